@@ -340,8 +340,12 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
     c.g_last_factorizations++;
     if (e < 0) return e;
     if (e == ECG_ESINGULAR) return ECG_ENOCONV;
-    // the converged eigenvalue is the bracket's; otherwise the bisection's own estimate
-    *energy = (lam >= lo && lam <= hi) ? lam : sigma;
+    // the converged eigenvalue is the bracket's; otherwise the bisection's own
+    // estimate.  A bisection point that met the eigenvalue to rounding (the
+    // first one does when the same basis is solved again) became an end of the
+    // bracket on either side of it, so the ends count with a margin.
+    const double margin = 1e-3 * (hi - lo) + 64.0 * DBL_EPSILON * fabs(sigma);
+    *energy = (lam >= lo - margin && lam <= hi + margin) ? lam : sigma;
     c.last_numiter = it;
     if (want_vector) CK(cudaMemcpyAsync(c.c, c.x, (size_t)n * sizeof(cd), cudaMemcpyDeviceToDevice, c.stream));
     CK(cudaStreamSynchronize(c.stream));
