@@ -728,6 +728,7 @@ int ensure_work(Ctx& c, int count)
     r |= dalloc_n(&cw.par, (size_t)c.npt * bcap);
     r |= dalloc_n(&cw.bra, (size_t)bcap * c.np);
     r |= dalloc_n(&cw.ket, (size_t)bcap * c.T * c.np);
+    r |= dalloc_n(&cw.ketn, (size_t)bcap * c.T * c.np);
     r |= dalloc_n(&cw.det, (size_t)bcap);
     r |= dalloc_n(&cw.dS, (size_t)bcap);
     r |= dalloc_n(&cw.mu, (size_t)bcap);
@@ -963,7 +964,7 @@ int tune_rows(Ctx& c, int nbase, int count, double approx_e)
 void cand_free(CandWork& cw)
 {
     drop_graphs(cw);
-    void* ptrs[] = {cw.par, cw.bra, cw.ket, cw.det, cw.dS, cw.mu, cw.Mcol, cw.Scol, cw.Acol, cw.Lcol, cw.V, cw.W,
+    void* ptrs[] = {cw.par, cw.bra, cw.ket, cw.ketn, cw.det, cw.dS, cw.mu, cw.Mcol, cw.Scol, cw.Acol, cw.Lcol, cw.V, cw.W,
                     cw.Y, cw.Z, cw.X, cw.X2, cw.brd, cw.nd, cw.st, cw.cmap, cw.Gm, cw.Pk, cw.flags, cw.bstart,
                     cw.abort_word, cw.gpart, cw.grad};
     for (void* p : ptrs)

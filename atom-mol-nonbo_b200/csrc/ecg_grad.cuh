@@ -1,11 +1,7 @@
 // ecg_grad.cuh -- derivatives of one ECG pair term.
 //
-// term_grad_plain: the derivative vectors Dk, Dl of src/matelem.f90:306-748
-//   (dH/dvechL, dH/dvechB, dS/dvechL, dS/dvechB of the bra and/or ket), in the
-//   reference's order, for the plain drop-in that materialises Glob_D.
-//
-// term_adjoint: the same derivatives already contracted into the form the
-//   energy gradient needs.  For one term with energy E fixed,
+// With the eigenvalue E fixed, the derivatives of one term
+// (src/matelem.f90:306-748) are
 //       dH/dvechL - E dS/dvechL  (entry (j,i), j >= i)
 //            = a * delta_ij / L_ii - 2 (Z L)_ji
 //       dH/dvechB - E dS/dvechB  (entry (i,j), weight 1 on the diagonal,
@@ -19,424 +15,252 @@
 //   from the reference's formulas: every Coulomb matrix tQ of
 //   src/matelem.f90:609-631 is the rank-one C^-1 (e_i-e_j)(e_i-e_j)' C^-1,
 //   so their weighted sum is C^-1 Q C^-1; and dS, dT, dV share the factors
-//   C^-1, F = C^-1 tCl M tCl C^-1 and G = P C^-1 Ck M Ck C^-1 P'.
+//   C^-1, F = C^-1 tCl M tCl C^-1 and G = P C^-1 Ck M Ck C^-1 P'.  E = 0
+//   gives dH alone, and dS has a = (3/2) S, Z = (3/2) S C^-1.
+//
+// Everything is S times a matrix that does not contain S, and with the unit
+// lower factor of pair_term (C^-1 = X^T D^-1 X)
+//       Z / S = X^T ( a' D^-1 - D^-1 (X R X^T) D^-1 ) X,
+//       a' = (3/2)(h - E),  R = N6 + Qs,
+// so one side costs two congruences with a unit triangular matrix (12
+// complex multiply-adds each at n = 3, against 45 for inv R inv).
 #pragma once
 #include "ecg_math.cuh"
 
 namespace ecg {
 
-// ---------------------------------------------------------------------------
-// Plain transcription (src/matelem.f90:306-748).  Lk, Ll are lower
-// triangular (upper entries zero), P the permutation matrix of this term.
-// Dk, Dl receive 4*NP complex values each (H-L, H-B, S-L, S-B blocks).
-// ---------------------------------------------------------------------------
-template <int N, bool GK, bool GL>
-__device__ __forceinline__ void term_grad_plain(const double (&Lk)[N][N], const double (&Ll)[N][N],
-                                                const double (&P)[N][N], const cd (&Ck)[N][N],
-                                                const cd (&tCl)[N][N], const TermEnergy<N>& te,
-                                                const SysParams& sp, cd* Dk, cd* Dl)
+// r_i r_j, packed, shared by the two sides of a term.
+template <int N>
+__device__ __forceinline__ void pivot_products(const cd (&r)[N], cd (&rr)[Sym<N>::NP])
 {
-    constexpr int NP = Sym<N>::NP;
-    const cd S = te.S;
-    const cd tos = cdiv(te.T, S);
-    const cd vos = cdiv(te.V, S);
-    cd Wc1[N][N];
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int j = i; j < N; j++) rr[vech_index(N, i, j)] = cmul(r[i], r[j]);
+}
 
-    // ---- dS (matelem.f90:306-423) ----
-    if (GK) {
+// Z (packed, vech order) = X^T (a D^-1 - D^-1 X R X^T D^-1) X for packed
+// symmetric R, unit lower X (strict part read) and ar_i = a r_i.
+template <int N>
+__device__ __forceinline__ void adj_congruence(const cd (&X)[N][N], const cd (&rr)[Sym<N>::NP], const cd (&ar)[N],
+                                               const cd (&R)[Sym<N>::NP], cd (&Z)[Sym<N>::NP])
+{
+    auto ix = [](int i, int j) { return i <= j ? vech_index(N, i, j) : vech_index(N, j, i); };
+    // A = X R, entries (i, b <= i); then B = A X^T, lower, scaled in place
+    cd A[N][N];
 #pragma unroll
-        for (int i = 0; i < N; i++)
+    for (int i = 0; i < N; i++)
 #pragma unroll
-            for (int j = 0; j < N; j++) {
-                cd s = mk(0.0, 0.0);
+        for (int b = 0; b <= i; b++) {
+            cd s = R[ix(i, b)];
 #pragma unroll
-                for (int k = j; k < N; k++) s = rfma(Lk[k][j], te.inv[i][k], s);
-                Wc1[i][j] = s;
-            }
-        double iL[N][N];
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) iL[j][i] = Lk[j][i];
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            iL[i][i] = 1.0 / iL[i][i];
-#pragma unroll
-            for (int j = i + 1; j < N; j++) {
-                double r = 0.0;
-#pragma unroll
-                for (int k = i; k <= j - 1; k++) r = fma(-iL[j][k], iL[k][i], r);
-                iL[j][i] = r / iL[j][j];
-            }
+            for (int k = 0; k < i; k++) s = cfma(X[i][k], R[ix(k, b)], s);
+            A[i][b] = s;
         }
-        const cd ct = 1.5 * S;
-        const cd cb = cmul(S, mk(0.0, 1.5));
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) {
-                const int x = vech_index(N, i, j);
-                const double d = (i == j) ? iL[i][i] : 0.0;
-                Dk[2 * NP + x] = cmul(mk(d - 2.0 * Wc1[j][i].x, -2.0 * Wc1[j][i].y), ct);
-                Dk[3 * NP + x] = (i == j) ? cmul(te.inv[i][i], cb) : cmul(te.inv[j][i], 2.0 * cb);
-            }
-    }
-    cd itt[N][N];  // inv_ttCkl = P C^-1 P'
-    if (GL) {
-        cd W[N][N];
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = 0; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = rfma(P[i][k], te.inv[k][j], s);
-                W[i][j] = s;
-            }
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = rfma(P[j][k], W[i][k], s);
-                itt[i][j] = s;
-                itt[j][i] = s;
-            }
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = 0; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = rfma(Ll[k][j], itt[i][k], s);
-                Wc1[i][j] = s;
-            }
-        double iL[N][N];
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) iL[j][i] = Ll[j][i];
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            iL[i][i] = 1.0 / iL[i][i];
-#pragma unroll
-            for (int j = i + 1; j < N; j++) {
-                double r = 0.0;
-#pragma unroll
-                for (int k = i; k <= j - 1; k++) r = fma(-iL[j][k], iL[k][i], r);
-                iL[j][i] = r / iL[j][j];
-            }
-        }
-        const cd ct = 1.5 * S;
-        const cd cb = cmul(S, mk(0.0, -1.5));
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) {
-                const int x = vech_index(N, i, j);
-                const double d = (i == j) ? iL[i][i] : 0.0;
-                Dl[2 * NP + x] = cmul(mk(d - 2.0 * Wc1[j][i].x, -2.0 * Wc1[j][i].y), ct);
-                Dl[3 * NP + x] = (i == j) ? cmul(itt[i][i], cb) : cmul(itt[j][i], 2.0 * cb);
-            }
-    }
-    // ---- dT (matelem.f90:427-598) ----
-    // X = C^-1 (Y M Y) C^-1 with Y = Ck (ket side, then G = P X P') or
-    // Y = tCl (bra side, F = X).
-    auto sandwich = [&](const cd (&Y)[N][N], cd (&X)[N][N]) {
-        cd A[N][N], B[N][N];
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = 0; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = rfma(sp.M[k * NMAX + j], Y[i][k], s);
-                A[i][j] = s;
-            }
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = 0; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = cfma(A[i][k], Y[k][j], s);
-                B[i][j] = s;
-            }
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = 0; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = cfma(te.inv[i][k], B[k][j], s);
-                A[i][j] = s;
-            }
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = cfma(A[i][k], te.inv[k][j], s);
-                X[i][j] = s;
-                X[j][i] = s;
-            }
-    };
-    if (GL) {
-        cd X[N][N], G[N][N], W[N][N];
-        sandwich(Ck, X);
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = 0; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = rfma(P[i][k], X[k][j], s);
-                W[i][j] = s;
-            }
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = rfma(P[j][k], W[i][k], s);
-                G[i][j] = s;
-                G[j][i] = s;
-            }
-        const cd c12 = 12.0 * S;
-        const cd c6 = cmul(S, mk(0.0, 6.0));
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) {
-                const int x = vech_index(N, i, j);
-                cd gl = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = i; k < N; k++) gl = rfma(Ll[k][i], G[j][k], gl);
-                Dl[x] = cfma(tos, Dl[2 * NP + x], cmul(c12, gl));
-                Dl[NP + x] = cfma(tos, Dl[3 * NP + x], (i == j) ? cmul(c6, G[i][i]) : cmul(2.0 * c6, G[j][i]));
-            }
-    }
-    if (GK) {
-        cd F[N][N];
-        sandwich(tCl, F);
-        const cd c12 = 12.0 * S;
-        const cd c6 = cmul(S, mk(0.0, -6.0));
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) {
-                const int x = vech_index(N, i, j);
-                cd fl = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = i; k < N; k++) fl = rfma(Lk[k][i], F[j][k], fl);
-                Dk[x] = cfma(tos, Dk[2 * NP + x], cmul(c12, fl));
-                Dk[NP + x] = cfma(tos, Dk[3 * NP + x], (i == j) ? cmul(c6, F[i][i]) : cmul(2.0 * c6, F[j][i]));
-            }
-    }
-    // ---- dV (matelem.f90:603-734) ----
-    cd Qw[N][N];
-    coulomb_weights<N>(te, sp, Qw);
-    cd WLk[NP], WBk[NP], WLl[NP], WBl[NP];
-#pragma unroll
-    for (int x = 0; x < NP; x++) {
-        WLk[x] = mk(0.0, 0.0); WBk[x] = mk(0.0, 0.0);
-        WLl[x] = mk(0.0, 0.0); WBl[x] = mk(0.0, 0.0);
-    }
+    cd Ee[Sym<N>::NP];
 #pragma unroll
     for (int i = 0; i < N; i++)
 #pragma unroll
         for (int j = 0; j <= i; j++) {
-            // tQ = C^-1 J_ij C^-1 = u u' with u = C^-1 (e_i - e_j) (u = C^-1 e_i if i == j)
-            cd u[N];
+            cd s = A[i][j];
 #pragma unroll
-            for (int k = 0; k < N; k++) u[k] = (i == j) ? te.inv[k][i] : te.inv[k][i] - te.inv[k][j];
-            const cd cn = Qw[i][j];
-            if (GK) {
-#pragma unroll
-                for (int k = 0; k < N; k++)
-#pragma unroll
-                    for (int kk = 0; kk <= k; kk++) {
-                        // (tQ Lk)(k,kk) = u_k * sum_{m>=kk} u_m Lk(m,kk)
-                        cd s = mk(0.0, 0.0);
-#pragma unroll
-                        for (int m = kk; m < N; m++) s = rfma(Lk[m][kk], u[m], s);
-                        const cd tl = cmul(u[k], s);
-                        const int x = vech_index(N, kk, k);
-                        WLk[x] = cfma(cn, tl, WLk[x]);
-                        const cd tq = cmul(u[k], u[kk]);
-                        WBk[x] = cfma((k == kk) ? cn : 2.0 * cn, tq, WBk[x]);
-                    }
-            }
-            if (GL) {
-                cd pu[N];  // P u, so that ttQ = (P u)(P u)'
-#pragma unroll
-                for (int k = 0; k < N; k++) {
-                    cd s = mk(0.0, 0.0);
-#pragma unroll
-                    for (int m = 0; m < N; m++) s = rfma(P[k][m], u[m], s);
-                    pu[k] = s;
-                }
-#pragma unroll
-                for (int k = 0; k < N; k++)
-#pragma unroll
-                    for (int kk = 0; kk <= k; kk++) {
-                        cd s = mk(0.0, 0.0);
-#pragma unroll
-                        for (int m = kk; m < N; m++) s = rfma(Ll[m][kk], pu[m], s);
-                        const cd tl = cmul(pu[k], s);
-                        const int x = vech_index(N, kk, k);
-                        WLl[x] = cfma(cn, tl, WLl[x]);
-                        const cd tq = cmul(pu[k], pu[kk]);
-                        WBl[x] = cfma((k == kk) ? cn : 2.0 * cn, tq, WBl[x]);
-                    }
-            }
+            for (int b = 0; b < j; b++) s = cfma(A[i][b], X[j][b], s);
+            Ee[ix(i, j)] = (i == j) ? cfms(rr[ix(i, i)], s, ar[i]) : cfms(rr[ix(i, j)], s, mk(0.0, 0.0));
         }
-    const cd c2 = TWO_OVER_SQRTPI * S;
-    const cd ci = cmul(mk(0.0, ONE_OVER_SQRTPI), S);
-    if (GK)
+    // G = E X, entries (a >= j, j); then Z = X^T G, lower
 #pragma unroll
-        for (int x = 0; x < NP; x++) {
-            Dk[x] = cfma(c2, WLk[x], cfma(vos, Dk[2 * NP + x], Dk[x]));
-            Dk[NP + x] = cfms(ci, WBk[x], cfma(vos, Dk[3 * NP + x], Dk[NP + x]));
+    for (int a = 0; a < N; a++)
+#pragma unroll
+        for (int j = 0; j <= a; j++) {
+            cd s = Ee[ix(a, j)];
+#pragma unroll
+            for (int b = j + 1; b < N; b++) s = cfma(Ee[ix(a, b)], X[b][j], s);
+            A[a][j] = s;
         }
-    if (GL)
 #pragma unroll
-        for (int x = 0; x < NP; x++) {
-            Dl[x] = cfma(c2, WLl[x], cfma(vos, Dl[2 * NP + x], Dl[x]));
-            Dl[NP + x] = cfma(ci, WBl[x], cfma(vos, Dl[3 * NP + x], Dl[NP + x]));
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int j = 0; j <= i; j++) {
+            cd s = A[i][j];
+#pragma unroll
+            for (int a = i + 1; a < N; a++) s = cfma(X[a][i], A[a][j], s);
+            Z[ix(i, j)] = s;
         }
 }
 
 // ---------------------------------------------------------------------------
-// Adjoint form: accumulate coef * Z_k, coef * Z_l (unpermuted) and coef * a.
-// Zk, Zl are stored as packed lower triangles (vech order, NP entries).
+// Z <- P Z P' for the ket side.  A product of particle transpositions acts
+// on the relative coordinates as rows e_x - e_b (x != b) and -e_b (the
+// image of the reference particle), b one coordinate or none, in some order
+// (src/workproc.f90:673-698).  perm_code packs that: b + 1 in bits 0..3
+// (0: none), and for every row i the slot it is swapped with, in bits
+// 4 + 3i.., so that P Z P' is a few additions and register swaps instead of
+// two products with P (45 real x complex multiply-adds at n = 3).  Any other
+// matrix has the code -1 and takes the general product.
 // ---------------------------------------------------------------------------
-template <int N>
-__device__ __forceinline__ void sym_sandwich(const cd (&inv)[N][N], const cd (&R)[N][N], cd (&X)[N][N])
+__host__ __device__ inline int perm_code(const double* P, int pitch, int n)
 {
-    cd A[N][N];
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = 0; j < N; j++) {
-            cd s = mk(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < N; k++) s = cfma(inv[i][k], R[k][j], s);
-            A[i][j] = s;
-        }
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = i; j < N; j++) {
-            cd s = mk(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < N; k++) s = cfma(A[i][k], inv[k][j], s);
-            X[i][j] = s;
-            X[j][i] = s;
-        }
-}
-
-// R = 6 S (Y M Y) + S/sqrt(pi) Q for symmetric complex Y.
-template <int N>
-__device__ __forceinline__ void adj_middle(const cd (&Y)[N][N], const cd (&Qs)[N][N], cd s6,
-                                           const SysParams& sp, cd (&R)[N][N])
-{
-    cd A[N][N];
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = 0; j < N; j++) {
-            cd s = mk(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < N; k++) s = rfma(sp.M[k * NMAX + j], Y[i][k], s);
-            A[i][j] = s;
-        }
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = i; j < N; j++) {
-            cd s = mk(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < N; k++) s = cfma(A[i][k], Y[k][j], s);
-            s = cfma(s6, s, Qs[i][j]);
-            R[i][j] = s;
-            R[j][i] = s;
-        }
-}
-
-template <int N, bool KET>
-__device__ __forceinline__ void term_adjoint(const double (&P)[N][N], const cd (&Ck)[N][N], const cd (&tCl)[N][N],
-                                             const TermEnergy<N>& te, const SysParams& sp, double E, double coef,
-                                             cd (&Zk)[Sym<N>::NP], cd (&Zl)[Sym<N>::NP], cd& a_acc)
-{
-    const cd S = te.S;
-    const cd H = te.T + te.V;
-    const cd a = 1.5 * (H - E * S);
-    a_acc = rfma(coef, a, a_acc);
-    // Qs = S/sqrt(pi) * Q
-    cd Qw[N][N], Qs[N][N];
-    coulomb_weights<N>(te, sp, Qw);
-    const cd sq = ONE_OVER_SQRTPI * S;
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        cd d = Qw[i][i];
-#pragma unroll
-        for (int j = 0; j < N; j++)
-            if (j != i) d = d + Qw[i][j];
-        Qs[i][i] = cmul(sq, d);
-#pragma unroll
-        for (int j = i + 1; j < N; j++) {
-            Qs[i][j] = -cmul(sq, Qw[i][j]);
-            Qs[j][i] = Qs[i][j];
-        }
+    int row_slot[NMAX], b = -1;
+    // b: the coordinate whose -1 stands in every row
+    for (int j = 0; j < n && b < 0; j++) {
+        bool all = true;
+        for (int i = 0; i < n; i++) all = all && P[i * pitch + j] == -1.0;
+        if (all) b = j;
     }
-    const cd s6 = 6.0 * S;
-    cd R[N][N], X[N][N];
-    adj_middle<N>(tCl, Qs, s6, sp, R);
-    sym_sandwich<N>(te.inv, R, X);
+    bool used[NMAX] = {false, false, false, false, false};
+    for (int i = 0; i < n; i++) {
+        int slot = -1;
+        for (int j = 0; j < n; j++) {
+            const double v = P[i * pitch + j];
+            if (j == b || v == 0.0) continue;
+            if (v != 1.0 || slot >= 0) return -1;
+            slot = j;
+        }
+        if (slot < 0) slot = b;  // the row -e_b
+        if (slot < 0 || used[slot]) return -1;
+        used[slot] = true;
+        row_slot[i] = slot;
+    }
+    int code = b + 1, cur[NMAX];
+    for (int i = 0; i < n; i++) cur[i] = i;
+    for (int i = 0; i + 1 < n; i++) {
+        int m = i;
+        while (cur[m] != row_slot[i]) m++;
+        const int c = cur[i];
+        cur[i] = cur[m];
+        cur[m] = c;
+        code |= m << (4 + 3 * i);
+    }
+    return code;
+}
+
+template <int N>
+__device__ __forceinline__ void perm_congruence(int code, const double* __restrict__ P, cd (&Z)[Sym<N>::NP])
+{
+    auto ix = [](int i, int j) { return i <= j ? vech_index(N, i, j) : vech_index(N, j, i); };
+    if (code >= 0) {
+        const int b = (code & 15) - 1;
+        if (b >= 0) {
+#pragma unroll
+            for (int x = 0; x < N; x++)
+                if (b == x) {
+                    cd e[N];
+#pragma unroll
+                    for (int a = 0; a < N; a++)
+                        if (a != x) e[a] = Z[ix(x, x)] - Z[ix(a, x)];
+#pragma unroll
+                    for (int a = 0; a < N; a++)
+#pragma unroll
+                        for (int c = a; c < N; c++)
+                            if (a != x && c != x) Z[ix(a, c)] = (Z[ix(a, c)] - Z[ix(c, x)]) + e[a];
+#pragma unroll
+                    for (int a = 0; a < N; a++)
+                        if (a != x) Z[ix(a, x)] = e[a];
+                }
+        }
+#pragma unroll
+        for (int i = 0; i + 1 < N; i++) {
+            const int m = (code >> (4 + 3 * i)) & 7;
+#pragma unroll
+            for (int x = i + 1; x < N; x++)
+                if (m == x) {
+#pragma unroll
+                    for (int a = 0; a < N; a++) {
+                        if (a == i || a == x) continue;
+                        const cd s = Z[ix(a, i)];
+                        Z[ix(a, i)] = Z[ix(a, x)];
+                        Z[ix(a, x)] = s;
+                    }
+                    const cd s = Z[ix(i, i)];
+                    Z[ix(i, i)] = Z[ix(x, x)];
+                    Z[ix(x, x)] = s;
+                }
+        }
+        return;
+    }
+    cd W[N][N];
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+            cd s = mk(0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < N; k++) s = rfma(__ldg(P + i * NMAX + k), Z[ix(k, j)], s);
+            W[i][j] = s;
+        }
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int j = i; j < N; j++) {
+            cd s = mk(0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < N; k++) s = rfma(__ldg(P + j * NMAX + k), W[i][k], s);
+            Z[ix(i, j)] = s;
+        }
+}
+
+// Bra and ket sides of one term over S (see the header): Zk, Zl (Zl only
+// with KET, already P Zl P') and a = (3/2)(h - E).  n6l(i, j) = 6 (tCl M
+// tCl)_ij.
+template <int N, bool KET, typename BRA, typename KETN>
+__device__ __forceinline__ cd term_adjoint(const BRA& bra, const KETN& n6l, const PairTerm<N>& te, double E,
+                                           int code, const double* __restrict__ P, cd (&Zk)[Sym<N>::NP],
+                                           cd (&Zl)[Sym<N>::NP])
+{
+    constexpr int NP = Sym<N>::NP;
+    const cd a = cd{1.5 * (te.h.x - E), 1.5 * te.h.y};
+    cd ar[N], rr[NP], R[NP];
+#pragma unroll
+    for (int i = 0; i < N; i++) ar[i] = cmul(a, te.r[i]);
+    pivot_products<N>(te.r, rr);
 #pragma unroll
     for (int i = 0; i < N; i++)
 #pragma unroll
         for (int j = i; j < N; j++) {
             const int x = vech_index(N, i, j);
-            Zk[x] = rfma(coef, cfms(mk(1.0, 0.0), X[j][i], cmul(a, te.inv[j][i])), Zk[x]);
+            R[x] = te.Qs[x] + n6l(i, j);
         }
+    adj_congruence<N>(te.X, rr, ar, R, Zk);
     if (KET) {
-        adj_middle<N>(Ck, Qs, s6, sp, R);
-        sym_sandwich<N>(te.inv, R, X);
-        // Zt = a C^-1 - X, then Zl += coef * P Zt P'
 #pragma unroll
         for (int i = 0; i < N; i++)
 #pragma unroll
             for (int j = i; j < N; j++) {
-                const cd z = cfms(mk(1.0, 0.0), X[j][i], cmul(a, te.inv[j][i]));
-                X[i][j] = z;
-                X[j][i] = z;
-            }
-        cd W[N][N];
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = 0; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = rfma(P[i][k], X[k][j], s);
-                W[i][j] = s;
-            }
-#pragma unroll
-        for (int i = 0; i < N; i++)
-#pragma unroll
-            for (int j = i; j < N; j++) {
-                cd s = mk(0.0, 0.0);
-#pragma unroll
-                for (int k = 0; k < N; k++) s = rfma(P[j][k], W[i][k], s);
                 const int x = vech_index(N, i, j);
-                Zl[x] = rfma(coef, s, Zl[x]);
+                R[x] = te.Qs[x] + bra.N6(i, j);
             }
+        adj_congruence<N>(te.X, rr, ar, R, Zl);
+        perm_congruence<N>(code, P, Zl);
     }
+    return a;
+}
+
+// The derivative vector of one function (the reference's order: H-L, H-B,
+// S-L, S-B blocks of NP entries) from its term sums: ZH, aH of H (E = 0),
+// ZS, aS of S; isign +1 for a bra, -1 for a ket.  L lower triangular.
+template <int N, typename GetH, typename GetS, typename Put>
+__device__ __forceinline__ void deriv_entries(const double (&L)[N][N], const GetH& ZH, cd aH, const GetS& ZS, cd aS,
+                                              double isign, const Put& put)
+{
+    constexpr int NP = Sym<N>::NP;
+    auto half = [&](const auto& Z, cd a, int off) {
+#pragma unroll
+        for (int i = 0; i < N; i++)
+#pragma unroll
+            for (int j = i; j < N; j++) {
+                cd s = mk(0.0, 0.0);
+#pragma unroll
+                for (int m = i; m < N; m++)
+                    s = rfma(L[m][i], Z(j >= m ? vech_index(N, m, j) : vech_index(N, j, m)), s);
+                cd g = -2.0 * s;
+                if (i == j) g = g + (1.0 / L[i][i]) * a;
+                put(off + vech_index(N, i, j), g);
+                const cd z = (i == j ? isign : 2.0 * isign) * Z(vech_index(N, i, j));
+                put(off + NP + vech_index(N, i, j), mk(-z.y, z.x));
+            }
+    };
+    half(ZH, aH, 0);
+    half(ZS, aS, 2 * NP);
 }
 
 }  // namespace ecg

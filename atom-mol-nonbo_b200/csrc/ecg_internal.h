@@ -34,7 +34,7 @@ inline long long tile_count(int Rlo, int Rhi)
 // Number of k_cand_row tile shapes the autotuner chooses from.
 constexpr int CAND_ROW_SHAPES = 5;
 // k_pair_energy shapes (warps per 32 x 32 tile x minimum CTAs per SM) and
-// k_adjoint shapes (minimum CTAs per SM) the autotuner chooses from.
+// k_adjoint shapes (likewise) the autotuner chooses from.
 constexpr int PAIR_SHAPES = 4;
 constexpr int ADJ_SHAPES = 2;
 // Columns (candidates) per work item of the batched triangular solves and
@@ -59,6 +59,7 @@ struct CandWork {
     double* par = nullptr;   // npt x bcap candidate parameters
     cd* bra = nullptr;       // bcap x NP
     cd* ket = nullptr;       // bcap x T x NP
+    cd* ketn = nullptr;      // bcap x T x NP: 6 tCl M tCl
     double* det = nullptr;   // bcap
     double* dS = nullptr;    // diagS of the candidate (its Re S_KK)
     double* mu = nullptr;    // M(K, K) = Re H_KK / diagS - lambda~
@@ -131,7 +132,9 @@ struct Ctx {
     std::vector<int> yhy_h;     // host copy of Glob_YHYMatr (n x n x T column-major)
     std::vector<int> yhy_coef_h;  // host copy of Glob_YHYCoeff
     cd* bra = nullptr;          // ld x NP: Ck = A - iB packed (vech order)
-    cd* ket = nullptr;          // ld x T x NP: P'AP + iP'BP packed
+    cd* ket = nullptr;          // ld x T x NP: P'AP + iP'BP packed (tCl)
+    cd* ketn = nullptr;         // ld x T x NP: 6 tCl M tCl packed
+    int* pcode = nullptr;       // T: the term matrices as row swaps (perm_code)
     double* detL = nullptr;     // ld
 
     // adjoint partial sums

@@ -112,142 +112,243 @@ __host__ __device__ constexpr int vech_index(int N, int i, int j)
     return i * N - i * (i - 1) / 2 + (j - i);
 }
 
-// Per-term energy quantities shared by the energy, plain-gradient and
-// adjoint kernels.  Inputs: Ck = A_k - iB_k (bra, conjugated), tCl =
-// P'A_lP + iP'B_lP (permuted ket), absdet = |det L_k det L_l|.
-// Outputs: inv = C^-1 (symmetric), S, T, V as in src/matelem.f90:182-299,
-// and with CUBE the Coulomb cubes tr32[i][j] = tr[C^-1 J_ij]^(-3/2) of
-// src/matelem.f90:284-296 (diagonal: (C^-1_ii)^(-3/2)).
-// Divisions are folded into reciprocals: each pseudo-Cholesky pivot is
-// inverted once and reused by the factor and by its inverse, and
-// 1/sqrt(a) = conj(sqrt a)/|a|.
+// 1/sqrt(x) for positive normal x without a branch: the hardware's seed y
+// (rsqrt.approx.ftz.f64, about 20 bits), then one step of Householder's
+// method of third order, the Taylor series of (1 - e)^(-1/2) to e^2 with
+// e = 1 - x y^2, whose remainder (5/16) e^3 is below 2^-60.  Zero,
+// subnormal, infinite or NaN x gives NaN.  rsqrt() and the divide are
+// accurate for every x and so end in a branch; the pair term takes up to
+// sixteen of them (n = 3), and without the branches their chains overlap.
+__device__ __forceinline__ double rsqrt_series(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+// x clamped to the normal range through its exponent word, x >= 0: what the
+// squared modulus of a pivot or a determinant needs where it over- or
+// underflows.  (A NaN stays visible in the factor the result multiplies.)
+__device__ __forceinline__ double normal_range(double x)
+{
+    const int hi = min(max(__double2hiint(x), 0x00100000), 0x7fe00000);
+    return __hiloint2double(hi, __double2loint(x));
+}
+// 1/b through the inverse modulus
+__device__ __forceinline__ cd crcp_series(cd b)
+{
+    const double q = rsqrt_series(normal_range(cnorm2(b)));
+    const double d = q * q;
+    return cd{b.x * d, -b.y * d};
+}
+
+// 1/sqrt(a) on the principal branch, and 1/a in ra.  With q = 1/|a| the
+// inverse is conj(a) q^2 and its modulus q itself, so Kahan's formulation
+// (csqrt_r above) of sqrt(1/a) needs two reciprocal square roots and no
+// division.
+__device__ __forceinline__ cd crsqrt(cd a, cd& ra)
+{
+    const double q = rsqrt_series(cnorm2(a));
+    const double q2 = q * q;
+    ra = cd{a.x * q2, -a.y * q2};
+    const double u = 0.5 * (fabs(ra.x) + q);
+    const double ri = rsqrt_series(u);
+    const double t = u * ri;
+    const double h = 0.5 * ra.y * ri;
+    const bool pos = ra.x >= 0.0;
+    return cd{pos ? t : fabs(h), pos ? h : copysign(t, ra.y)};
+}
+
+// The bra data a pair term reads, for one function k: C(i, j) = Ck,
+// KM(i, j) = (Ck M)_ij and N6(i, j) = 6 (Ck M Ck)_ij with M the mass matrix.
+// BraRegs keeps them in registers (or local memory), BraShared in shared
+// memory, entry e of the lane's function at p[e * stride].
 template <int N>
-struct TermEnergy {
-    cd inv[N][N];
-    cd S, T, V;
-    cd tr32[N][N];
+struct BraRegs {
+    cd c[N][N], km[N][N], n6[N][N];
+    __device__ __forceinline__ cd C(int i, int j) const { return c[i][j]; }
+    __device__ __forceinline__ cd KM(int i, int j) const { return km[i][j]; }
+    __device__ __forceinline__ cd N6(int i, int j) const { return n6[i][j]; }
+};
+template <int N>
+struct BraShared {
+    static constexpr int NP = Sym<N>::NP;
+    static constexpr int ENTRIES_E = NP + N * N;             // C, KM (energies)
+    static constexpr int ENTRIES = 2 * NP + N * N;           // and N6 (gradients)
+    const double2* p;
+    int stride;
+    __device__ __forceinline__ cd at(int e) const
+    {
+        const double2 v = p[e * stride];
+        return cd{v.x, v.y};
+    }
+    __device__ __forceinline__ cd C(int i, int j) const
+    {
+        return at(i <= j ? vech_index(N, i, j) : vech_index(N, j, i));
+    }
+    __device__ __forceinline__ cd KM(int i, int j) const { return at(NP + i * N + j); }
+    __device__ __forceinline__ cd N6(int i, int j) const
+    {
+        return at(NP + N * N + (i <= j ? vech_index(N, i, j) : vech_index(N, j, i)));
+    }
 };
 
-template <int N, bool CUBE>
-__device__ __forceinline__ void term_energy(const cd (&Ck)[N][N], const cd (&tCl)[N][N], double absdet,
-                                            const SysParams& sp, TermEnergy<N>& o)
+// X M for symmetric complex X.
+template <int N>
+__device__ __forceinline__ void mass_right(const cd (&X)[N][N], const SysParams& sp, cd (&XM)[N][N])
 {
-    cd G[N][N], rg[N];
-    // pseudo-Cholesky C = G G^T of C = Ck + tCl (matelem.f90:203-217)
-    cd det = mk(1.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        {
-            cd s = Ck[i][i] + tCl[i][i];
-#pragma unroll
-            for (int k = i - 1; k >= 0; k--) s = cfms(G[i][k], G[i][k], s);
-            G[i][i] = csqrt(s);
-            det = det * s;
-            rg[i] = crcp(G[i][i]);
-        }
-#pragma unroll
-        for (int j = i + 1; j < N; j++) {
-            cd s = Ck[i][j] + tCl[i][j];
-#pragma unroll
-            for (int k = i - 1; k >= 0; k--) s = cfms(G[i][k], G[j][k], s);
-            G[j][i] = cmul(s, rg[i]);
-        }
-    }
-    // X = G^-1 (lower) in place, then inv = X^T X (matelem.f90:221-241)
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        G[i][i] = rg[i];
-#pragma unroll
-        for (int j = i + 1; j < N; j++) {
-            cd s = mk(0.0, 0.0);
-#pragma unroll
-            for (int k = i; k <= j - 1; k++) s = cfms(G[j][k], G[k][i], s);
-            G[j][i] = cmul(s, rg[j]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-#pragma unroll
-        for (int j = i; j < N; j++) {
-            cd s = mk(0.0, 0.0);
-#pragma unroll
-            for (int k = j; k < N; k++) s = cfma(G[k][i], G[k][j], s);
-            o.inv[i][j] = s;
-            o.inv[j][i] = s;
-        }
-    }
-    // overlap (matelem.f90:244-245)
-    const cd c = rdiv(absdet, det);
-    o.S = sp.two_r3n2 * (c * csqrt(c));
-    // kinetic: T = 6 S tr[M tCl C^-1 Ck] (matelem.f90:248-274)
-    cd W1[N][N];
 #pragma unroll
     for (int i = 0; i < N; i++)
 #pragma unroll
         for (int j = 0; j < N; j++) {
             cd s = mk(0.0, 0.0);
 #pragma unroll
-            for (int k = 0; k < N; k++) s = cfma(o.inv[i][k], Ck[k][j], s);
-            W1[i][j] = s;
+            for (int k = 0; k < N; k++) s = rfma(sp.M[k * NMAX + j], X[i][k], s);
+            XM[i][j] = s;
         }
-    cd tr = mk(0.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int k = 0; k < N; k++) {
-            cd w2 = mk(0.0, 0.0);
-#pragma unroll
-            for (int m = 0; m < N; m++) w2 = cfma(tCl[k][m], W1[m][i], w2);
-            tr = rfma(sp.M[i * NMAX + k], w2, tr);
-        }
-    o.T = 6.0 * (o.S * tr);
-    // Coulomb (matelem.f90:280-299): cn / sqrt(a) = cn conj(sqrt a) / |a|
-    const cd cn = TWO_OVER_SQRTPI * o.S;
-    cd v = mk(0.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        const cd a = o.inv[i][i];
-        double r;
-        const cd sq = csqrt_r(a, r);
-        const double ir = 1.0 / r;
-        const cd is = mk(sq.x * ir, -sq.y * ir);  // 1/sqrt(a)
-        v = rfma(sp.q[i], cmul(cn, is), v);
-        if (CUBE) o.tr32[i][i] = cmul(is, mk(a.x * ir * ir, -a.y * ir * ir));  // a^(-1/2) a^(-1)
-    }
-    v = sp.q0 * v;
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = i + 1; j < N; j++) {
-            const cd a = o.inv[i][i] + o.inv[j][j] - o.inv[j][i] - o.inv[j][i];
-            double r;
-            const cd sq = csqrt_r(a, r);
-            const double ir = 1.0 / r;
-            const cd is = mk(sq.x * ir, -sq.y * ir);
-            v = rfma(sp.q[i] * sp.q[j], cmul(cn, is), v);
-            if (CUBE) {
-                o.tr32[j][i] = cmul(is, mk(a.x * ir * ir, -a.y * ir * ir));
-                o.tr32[i][j] = o.tr32[j][i];
-            }
-        }
-    o.V = v;
 }
 
-// Coulomb weights for the gradient: cnumb_ij = q_i q_j tr[C^-1 J_ij]^(-3/2)
-// (i != j) and q0 q_i (C^-1_ii)^(-3/2) on the diagonal, as cnumb of
-// src/matelem.f90:677-681, from the cubes kept by term_energy<N, true>.
+// 6 X M X from X and XM = X M.
 template <int N>
-__device__ __forceinline__ void coulomb_weights(const TermEnergy<N>& te, const SysParams& sp, cd (&Qw)[N][N])
+__device__ __forceinline__ void mass_sandwich(const cd (&X)[N][N], const cd (&XM)[N][N], cd (&N6)[N][N])
 {
-#pragma unroll
-    for (int i = 0; i < N; i++) Qw[i][i] = (sp.q0 * sp.q[i]) * te.tr32[i][i];
 #pragma unroll
     for (int i = 0; i < N; i++)
 #pragma unroll
-        for (int j = i + 1; j < N; j++) {
-            Qw[j][i] = (sp.q[i] * sp.q[j]) * te.tr32[j][i];
-            Qw[i][j] = Qw[j][i];
+        for (int j = i; j < N; j++) {
+            cd s = mk(0.0, 0.0);
+#pragma unroll
+            for (int k = 0; k < N; k++) s = cfma(XM[i][k], X[k][j], s);
+            N6[i][j] = 6.0 * s;
+            N6[j][i] = N6[i][j];
         }
+}
+
+// One pair term: what the energy, the derivative and the adjoint kernels
+// share.  Inputs: the bra data, tCl = P'A_lP + iP'B_lP (permuted ket),
+// absdet = |det L_k det L_l| and scale, a factor on S (2^(3n/2), times the
+// term's coefficient and whatever else a caller wants folded in).
+//   C = Ck + tCl = L D L^T (unit lower L, no square roots; its pivots are
+//   the squares of those of the pseudo-Cholesky factor of
+//   src/matelem.f90:203-217, so det C is the same product);
+//   X = L^-1 (strict lower part kept), r = 1/D, inv = C^-1 = X^T D^-1 X;
+//   S as src/matelem.f90:244-245, times scale;
+//   h = H/S: 6 tr[M tCl C^-1 Ck] (src/matelem.f90:248-274), taken as
+//   6 sum_k r_k (X Ck M)_k . (X tCl)_k, plus the Coulomb sum
+//   (src/matelem.f90:280-299) over S;
+//   with GRAD, Qs = Q/sqrt(pi) of ecg_grad.cuh: Q(i,i) = w_ii + sum_{j!=i}
+//   w_ij, Q(i,j) = -w_ij, w_ij the Coulomb weights cnumb of
+//   src/matelem.f90:677-681 over S.
+template <int N>
+struct PairTerm {
+    cd X[N][N];
+    cd r[N];
+    cd inv[N][N];
+    cd S, h;
+    cd Qs[Sym<N>::NP];
+};
+
+template <int N, bool GRAD, typename BRA>
+__device__ __forceinline__ void pair_term(const BRA& bra, const cd (&tCl)[N][N], double absdet, double scale,
+                                          const SysParams& sp, PairTerm<N>& o)
+{
+    // C = L D L^T by columns: G(j, i) the unscaled column, L(j, i) = G r_i
+    cd L[N][N], G[N][N];
+    cd det = mk(1.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        cd d = bra.C(i, i) + tCl[i][i];
+#pragma unroll
+        for (int k = 0; k < i; k++) d = cfms(L[i][k], G[i][k], d);
+        det = (i == 0) ? d : det * d;
+        o.r[i] = crcp_series(d);
+#pragma unroll
+        for (int j = i + 1; j < N; j++) {
+            cd g = bra.C(i, j) + tCl[i][j];
+#pragma unroll
+            for (int k = 0; k < i; k++) g = cfms(L[j][k], G[i][k], g);
+            G[j][i] = g;
+            L[j][i] = cmul(g, o.r[i]);
+        }
+    }
+    // X = L^-1, strict lower
+#pragma unroll
+    for (int j = 1; j < N; j++)
+#pragma unroll
+        for (int i = j - 1; i >= 0; i--) {
+            cd s = -L[j][i];
+#pragma unroll
+            for (int k = i + 1; k < j; k++) s = cfms(L[j][k], o.X[k][i], s);
+            o.X[j][i] = s;
+        }
+    // inv = X^T D^-1 X
+#pragma unroll
+    for (int j = 0; j < N; j++)
+#pragma unroll
+        for (int i = 0; i <= j; i++) {
+            cd s = (i == j) ? o.r[j] : cmul(o.r[j], o.X[j][i]);
+#pragma unroll
+            for (int k = j + 1; k < N; k++) s = cfma(cmul(o.r[k], o.X[k][j]), o.X[k][i], s);
+            o.inv[i][j] = s;
+            o.inv[j][i] = s;
+        }
+    // overlap: c = absdet / det, S = scale c sqrt(c)
+    {
+        const double q = rsqrt_series(normal_range(cnorm2(det)));
+        const double m = absdet * q;  // |c|
+        const cd c = cd{m * q * det.x, -m * q * det.y};
+        const double u = 0.5 * (fabs(c.x) + m);
+        const double ri = rsqrt_series(u);
+        const bool pos = c.x >= 0.0, tiny = !(u > 1e-300);  // a vanishing overlap
+        const double t = u * ri, hh = 0.5 * c.y * ri;
+        const cd sc = tiny ? cd{0.0 * u, 0.0} : cd{pos ? t : fabs(hh), pos ? hh : copysign(t, c.y)};
+        o.S = scale * cmul(c, sc);
+    }
+    // kinetic trace
+    cd tr = mk(0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        cd s = mk(0.0, 0.0);
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+            cd y = bra.KM(k, j), z = tCl[k][j];
+#pragma unroll
+            for (int a = 0; a < k; a++) {
+                y = cfma(o.X[k][a], bra.KM(a, j), y);
+                z = cfma(o.X[k][a], tCl[a][j], z);
+            }
+            s = cfma(y, z, s);
+        }
+        tr = cfma(o.r[k], s, tr);
+    }
+    // Coulomb sum over S / (2/sqrt(pi))
+    cd v = mk(0.0, 0.0);
+    if (GRAD)
+#pragma unroll
+        for (int i = 0; i < N; i++) o.Qs[vech_index(N, i, i)] = mk(0.0, 0.0);
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int j = i; j < N; j++) {
+            const cd a = (i == j) ? o.inv[i][i]
+                                  : cd{fma(-2.0, o.inv[i][j].x, o.inv[i][i].x + o.inv[j][j].x),
+                                       fma(-2.0, o.inv[i][j].y, o.inv[i][i].y + o.inv[j][j].y)};
+            cd ra;
+            const cd is = crsqrt(a, ra);
+            const double qq = (i == j) ? sp.q0 * sp.q[i] : sp.q[i] * sp.q[j];
+            v = rfma(qq, is, v);
+            if (GRAD) {
+                const cd w = (ONE_OVER_SQRTPI * qq) * cmul(is, ra);
+                cd& qi = o.Qs[vech_index(N, i, i)];
+                qi = qi + w;
+                if (i != j) {
+                    cd& qj = o.Qs[vech_index(N, j, j)];
+                    qj = qj + w;
+                    o.Qs[vech_index(N, i, j)] = -w;
+                }
+            }
+        }
+    o.h = cd{fma(6.0, tr.x, TWO_OVER_SQRTPI * v.x), fma(6.0, tr.y, TWO_OVER_SQRTPI * v.y)};
 }
 
 }  // namespace ecg

@@ -168,15 +168,21 @@ __device__ __forceinline__ void store_sym(cd* p, const cd (&M)[N][N])
 }
 
 // ---------------------------------------------------------------------------
+// Everything of one function: bra, permuted kets, det L; with ketn also
+// 6 tCl M tCl per term, which the adjoint pass reads.  The first T threads
+// describe the term matrices for it (perm_code).
 template <int N>
-__global__ void __launch_bounds__(128) k_prep(const double* __restrict__ params, const double* __restrict__ Pd,
-                                              int T, int nfun, cd* __restrict__ bra, cd* __restrict__ ket,
+__global__ void __launch_bounds__(128) k_prep(SysParams sp, const double* __restrict__ params,
+                                              const double* __restrict__ Pd, int T, int nfun, cd* __restrict__ bra,
+                                              cd* __restrict__ ket, cd* __restrict__ ketn, int* __restrict__ pcode,
                                               double* __restrict__ detL)
 {
     constexpr int NP = Sym<N>::NP;
     constexpr int NPT = 2 * NP;
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nfun) return;
+    if (pcode)
+        for (int t = f; t < T; t += nfun) pcode[t] = perm_code(Pd + t * NMAX * NMAX, NMAX, N);
     const double* p = params + (size_t)f * NPT;
     cd Ck[N][N];
     double det;
@@ -190,8 +196,69 @@ __global__ void __launch_bounds__(128) k_prep(const double* __restrict__ params,
         double d2;
         make_ket<N>(p, P, tCl, d2);
         store_sym<N>(ket + ((size_t)f * T + t) * NP, tCl);
+        if (ketn) {
+            cd KM[N][N], K6[N][N];
+            mass_right<N>(tCl, sp, KM);
+            mass_sandwich<N>(tCl, KM, K6);
+            store_sym<N>(ketn + ((size_t)f * T + t) * NP, K6);
+        }
     }
 }
+
+// The bra data of one function in registers.
+template <int N>
+__device__ __forceinline__ void load_bra(const cd* __restrict__ p, const SysParams& sp, BraRegs<N>& b)
+{
+    load_sym<N>(p, b.c);
+    mass_right<N>(b.c, sp, b.km);
+    mass_sandwich<N>(b.c, b.km, b.n6);
+}
+
+// The bra data of the lane's function into shared memory, entry e at
+// sm[e * stride]; GRAD: with 6 Ck M Ck.
+template <int N, bool GRAD>
+__device__ __forceinline__ void stage_bra(const cd* __restrict__ p, const SysParams& sp, double2* sm, int stride)
+{
+    constexpr int NP = Sym<N>::NP;
+    cd C[N][N], KM[N][N];
+    load_sym<N>(p, C);
+    mass_right<N>(C, sp, KM);
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int j = 0; j < N; j++) {
+            if (i <= j) sm[vech_index(N, i, j) * stride] = make_double2(C[i][j].x, C[i][j].y);
+            sm[(NP + i * N + j) * stride] = make_double2(KM[i][j].x, KM[i][j].y);
+        }
+    if (GRAD) {
+        cd K6[N][N];
+        mass_sandwich<N>(C, KM, K6);
+#pragma unroll
+        for (int i = 0; i < N; i++)
+#pragma unroll
+            for (int j = i; j < N; j++)
+                sm[(NP + N * N + vech_index(N, i, j)) * stride] = make_double2(K6[i][j].x, K6[i][j].y);
+    }
+}
+
+// 6 tCl M tCl of one ket and term: read (k_prep left it) or, where a caller
+// keeps only the kets, formed from tCl.
+template <int N>
+struct KetRead {
+    const cd* p;
+    __device__ __forceinline__ cd operator()(int i, int j) const { return ldcd(p + vech_index(N, i, j)); }
+};
+template <int N>
+struct KetFormed {
+    cd n6[N][N];
+    __device__ __forceinline__ KetFormed(const cd (&tCl)[N][N], const SysParams& sp)
+    {
+        cd KM[N][N];
+        mass_right<N>(tCl, sp, KM);
+        mass_sandwich<N>(tCl, KM, n6);
+    }
+    __device__ __forceinline__ cd operator()(int i, int j) const { return n6[i][j]; }
+};
 
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void tile_rc(long long b, int Rlo, int& R, int& C)
@@ -203,6 +270,29 @@ __device__ __forceinline__ void tile_rc(long long b, int Rlo, int& R, int& C)
     R = (int)r;
     C = (int)(bb - r * (r + 1) / 2);
 }
+
+// Term sums of one side's derivatives: dH (E = 0) and dS, see ecg_grad.cuh.
+template <int N>
+struct DerivSum {
+    static constexpr int NP = Sym<N>::NP;
+    cd zh[NP], zs[NP], ah, as;
+    __device__ __forceinline__ void zero()
+    {
+#pragma unroll
+        for (int x = 0; x < NP; x++) zh[x] = zs[x] = mk(0.0, 0.0);
+        ah = as = mk(0.0, 0.0);
+    }
+    // dS of a bra: a = (3/2) S, Z = (3/2) S C^-1
+    __device__ __forceinline__ void add_overlap(const PairTerm<N>& te, cd S)
+    {
+        const cd s = 1.5 * S;
+        as = as + s;
+#pragma unroll
+        for (int i = 0; i < N; i++)
+#pragma unroll
+            for (int j = i; j < N; j++) zs[vech_index(N, i, j)] = cfma(s, te.inv[i][j], zs[vech_index(N, i, j)]);
+    }
+};
 
 // Diagonal pairs k = l for k in [r0, r1).  deriv: also Glob_D(:,k-nfru,k).
 template <int N, bool DERIV>
@@ -217,33 +307,27 @@ __global__ void __launch_bounds__(128) k_pair_diag(SysParams sp, const double* _
     constexpr int NP = Sym<N>::NP;
     const int k = r0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= r1) return;
-    cd Ck[N][N];
-    load_sym<N>(bra + (size_t)k * NP, Ck);
+    BraRegs<N> b;
+    load_bra<N>(bra + (size_t)k * NP, sp, b);
     const double dk = detL[k];
     const double absdet = fabs(dk * dk);
     cd Hs = mk(0.0, 0.0), Ss = mk(0.0, 0.0);
-    cd Dks[4 * NP];
-    double Lk[N][N];
-    if (DERIV) {
-        load_L<N>(params + (size_t)k * 2 * NP, Lk);
-#pragma unroll
-        for (int m = 0; m < 4 * NP; m++) Dks[m] = mk(0.0, 0.0);
-    }
+    DerivSum<N> sum;
+    if (DERIV) sum.zero();
     for (int t = 0; t < sp.T; t++) {
         cd tCl[N][N];
         load_sym<N>(ket + ((size_t)k * sp.T + t) * NP, tCl);
-        TermEnergy<N> te;
-        term_energy<N, DERIV>(Ck, tCl, absdet, sp, te);
-        const double cf = coef[t];
-        Hs = rfma(cf, te.T + te.V, Hs);
-        Ss = rfma(cf, te.S, Ss);
+        PairTerm<N> te;
+        pair_term<N, DERIV>(b, tCl, absdet, sp.two_r3n2 * coef[t], sp, te);
+        Hs = cfma(te.S, te.h, Hs);
+        Ss = Ss + te.S;
         if (DERIV) {
-            double P[N][N];
-            load_P<N>(Pd, t, P);
-            cd Dk[4 * NP], Dl[1];
-            term_grad_plain<N, true, false>(Lk, Lk, P, Ck, tCl, te, sp, Dk, Dl);
+            cd Zk[NP], Zl[NP];
+            const cd a = term_adjoint<N, false>(b, KetFormed<N>(tCl, sp), te, 0.0, 0, Pd, Zk, Zl);
 #pragma unroll
-            for (int m = 0; m < 4 * NP; m++) Dks[m] = rfma(cf, Dk[m], Dks[m]);
+            for (int x = 0; x < NP; x++) sum.zh[x] = cfma(te.S, Zk[x], sum.zh[x]);
+            sum.ah = cfma(te.S, a, sum.ah);
+            sum.add_overlap(te, te.S);
         }
     }
     const double dS = Ss.x;
@@ -257,8 +341,11 @@ __global__ void __launch_bounds__(128) k_pair_diag(SysParams sp, const double* _
     }
     if (DERIV) {
         cd* d = D + ((size_t)(k - nfru) + (size_t)k * ldo) * (4 * NP);
-#pragma unroll
-        for (int m = 0; m < 4 * NP; m++) d[m] = mk(2.0 * Dks[m].x / dS, 0.0);
+        double Lk[N][N];
+        load_L<N>(params + (size_t)k * 2 * NP, Lk);
+        deriv_entries<N>(
+            Lk, [&](int x) { return sum.zh[x]; }, sum.ah, [&](int x) { return sum.zs[x]; }, sum.as, 1.0,
+            [&](int m, cd v) { d[m] = mk(2.0 * v.x / dS, 0.0); });
     }
 }
 
@@ -266,6 +353,12 @@ __global__ void __launch_bounds__(128) k_pair_diag(SysParams sp, const double* _
 // tile, NW warps (lanes along k, warps along l, 32 / NW columns each); the
 // shape (NW, MINB) is chosen by timing (PAIR_SHAPES); every shape computes
 // each element with the same instructions, so results do not depend on it.
+// FP64 issue bounds it: 437 FP64 instructions a term at n = 3 (ncu), 0.77 ms
+// of the pipe at K = 4000, T = 4, where it takes 1.07 ms; the form with a
+// square root per pivot, divisions and both matrix products of the kinetic
+// trace took 1.89 ms (n = 4, K = 1013, T = 14: 0.97 -> 0.55 ms).  The bra
+// matrices of the 32 rows sit in shared memory because C M is needed beside
+// C and both would not fit the register budget of 16 warps an SM.
 template <int N, int NW, int MINB>
 __global__ void __launch_bounds__(NW * 32, MINB) k_pair_energy(SysParams sp, const double* __restrict__ coef,
                                                      const cd* __restrict__ bra, const cd* __restrict__ ket,
@@ -275,13 +368,16 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_pair_energy(SysParams sp, con
                                                      char method, double approx_e, long long t0)
 {
     constexpr int NP = Sym<N>::NP;
+    extern __shared__ double2 bsm[];  // the 32 rows' bra data, [entry][lane]
     int R, C;
     tile_rc(t0 + blockIdx.x, Rlo, R, C);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = R * TILE + lane;
-    if (k < r0 || k >= r1) return;
-    cd Ck[N][N];
-    load_sym<N>(bra + (size_t)k * NP, Ck);
+    const bool row = k >= r0 && k < r1;
+    if (w == 0 && row) stage_bra<N, false>(bra + (size_t)k * NP, sp, bsm + lane, TILE);
+    __syncthreads();
+    if (!row) return;
+    const BraShared<N> b{bsm + lane, TILE};
     const double dk = detL[k];
     const double dSk = diagS[k];
 #pragma unroll 1
@@ -294,13 +390,12 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_pair_energy(SysParams sp, con
         for (int t = 0; t < sp.T; t++) {
             cd tCl[N][N];
             load_sym<N>(ket + ((size_t)l * sp.T + t) * NP, tCl);
-            TermEnergy<N> te;
-            term_energy<N, false>(Ck, tCl, absdet, sp, te);
-            const double cf = __ldg(coef + t);
-            Hs = rfma(cf, te.T + te.V, Hs);
-            Ss = rfma(cf, te.S, Ss);
+            PairTerm<N> te;
+            pair_term<N, false>(b, tCl, absdet, sp.two_r3n2 * __ldg(coef + t), sp, te);
+            Hs = cfma(te.S, te.h, Hs);
+            Ss = Ss + te.S;
         }
-        const double f = 1.0 / sqrt(dSk * diagS[l]);
+        const double f = (1.0 / sqrt(dSk * diagS[l]));
         const size_t kl = (size_t)k + (size_t)l * ld;
         const cd s = f * Ss;
         S[kl] = s;
@@ -313,73 +408,97 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_pair_energy(SysParams sp, con
     }
 }
 
-// Off-diagonal pairs with derivatives, one pair per thread at a time; the
-// per-term derivative sums live in shared memory ([value][thread]).
+// Off-diagonal pairs with derivatives, one pair per thread at a time.  Both
+// sides' term sums (Z and a of H and of S, as DerivSum) live in shared memory,
+// [value][thread]; L_k and L_l are applied once per pair, after the terms.
+// Summing the 8 NP derivative entries of every term instead, with their
+// matrices formed per entry, spilled 2 KB a thread at n = 3: 1.5 ms at K =
+// 1000, T = 4, against 0.3 ms (no spills), FP64 issue in both.
 template <int N, int NT>
 __global__ void __launch_bounds__(NT) k_pair_grad(SysParams sp, const double* __restrict__ coef,
-                                                  const double* __restrict__ Pd,
+                                                  const double* __restrict__ Pd, const int* __restrict__ pcode,
                                                   const double* __restrict__ params, const cd* __restrict__ bra,
-                                                  const cd* __restrict__ ket, const double* __restrict__ detL,
+                                                  const cd* __restrict__ ket, const cd* __restrict__ ketn,
+                                                  const double* __restrict__ detL,
                                                   const double* __restrict__ diagS, cd* __restrict__ H,
                                                   cd* __restrict__ S, int ld, int r0, int r1, int Rlo, char method,
                                                   double approx_e, cd* __restrict__ D, int ldo, int nfru)
 {
     constexpr int NP = Sym<N>::NP;
-    constexpr int NV = 8 * NP;  // complex values: Dk (4NP) + Dl (4NP)
-    extern __shared__ double acc[];
+    constexpr int NS = 4 * NP;  // Z sums: bra H, bra S, ket H, ket S
+    extern __shared__ double2 gsm[];
+    double2* bsm = gsm;                               // [entry][lane]
+    double2* acc = gsm + BraShared<N>::ENTRIES * TILE;  // [value][thread]
     int R, C;
     tile_rc(blockIdx.x, Rlo, R, C);
     const int tid = threadIdx.x;
     const int lane = tid & 31, w = tid >> 5;
     constexpr int NW = NT / 32;
     const int k = R * TILE + lane;
-    if (k < r0 || k >= r1) return;
-    cd Ck[N][N];
-    load_sym<N>(bra + (size_t)k * NP, Ck);
-    double Lk[N][N];
-    load_L<N>(params + (size_t)k * 2 * NP, Lk);
+    const bool row = k >= r0 && k < r1;
+    if (w == 0 && row) stage_bra<N, true>(bra + (size_t)k * NP, sp, bsm + lane, TILE);
+    __syncthreads();
+    if (!row) return;
+    const BraShared<N> b{bsm + lane, TILE};
     const double dk = detL[k];
     const double dSk = diagS[k];
-    auto A = [&](int v) -> double& { return acc[v * NT + tid]; };
+    auto A = [&](int v) -> double2& { return acc[v * NT + tid]; };
+    auto add = [&](int v, cd z) {
+        double2 o = A(v);
+        o.x += z.x;
+        o.y += z.y;
+        A(v) = o;
+    };
+    auto get = [&](int v) {
+        const double2 o = A(v);
+        return cd{o.x, o.y};
+    };
 #pragma unroll 1
     for (int j = 0; j < TILE / NW; j++) {
         const int l = C * TILE + w + NW * j;
         if (l >= k) break;
         const bool gl = (l >= nfru);
-        double Ll[N][N];
-        load_L<N>(params + (size_t)l * 2 * NP, Ll);
         const double absdet = fabs(detL[l] * dk);
-        for (int v = 0; v < 2 * NV; v++) A(v) = 0.0;
+#pragma unroll
+        for (int v = 0; v < NS; v++) A(v) = make_double2(0.0, 0.0);
         cd Hs = mk(0.0, 0.0), Ss = mk(0.0, 0.0);
 #pragma unroll 1
         for (int t = 0; t < sp.T; t++) {
             cd tCl[N][N];
             load_sym<N>(ket + ((size_t)l * sp.T + t) * NP, tCl);
-            TermEnergy<N> te;
-            term_energy<N, true>(Ck, tCl, absdet, sp, te);
-            const double cf = __ldg(coef + t);
-            Hs = rfma(cf, te.T + te.V, Hs);
-            Ss = rfma(cf, te.S, Ss);
-            double P[N][N];
-            load_P<N>(Pd, t, P);
-            cd Dk[4 * NP], Dl[4 * NP];
-            if (gl) {
-                term_grad_plain<N, true, true>(Lk, Ll, P, Ck, tCl, te, sp, Dk, Dl);
+            PairTerm<N> te;
+            pair_term<N, true>(b, tCl, absdet, sp.two_r3n2 * __ldg(coef + t), sp, te);
+            Hs = cfma(te.S, te.h, Hs);
+            Ss = Ss + te.S;
+            const KetRead<N> n6l{ketn + ((size_t)l * sp.T + t) * NP};
+            const double* Pt = Pd + t * NMAX * NMAX;
+            const int code = __ldg(pcode + t);
+            cd Zk[NP], Zl[NP];
+            if (gl)
+                term_adjoint<N, true>(b, n6l, te, 0.0, code, Pt, Zk, Zl);
+            else
+                term_adjoint<N, false>(b, n6l, te, 0.0, code, Pt, Zk, Zl);
+            const cd s15 = 1.5 * te.S;
+            cd I[NP];
 #pragma unroll
-                for (int m = 0; m < 4 * NP; m++) {
-                    A(2 * (4 * NP + m)) = fma(cf, Dl[m].x, A(2 * (4 * NP + m)));
-                    A(2 * (4 * NP + m) + 1) = fma(cf, Dl[m].y, A(2 * (4 * NP + m) + 1));
-                }
-            } else {
-                term_grad_plain<N, true, false>(Lk, Ll, P, Ck, tCl, te, sp, Dk, Dl);
+            for (int i = 0; i < N; i++)
+#pragma unroll
+                for (int jj = i; jj < N; jj++) I[vech_index(N, i, jj)] = te.inv[i][jj];
+#pragma unroll
+            for (int x = 0; x < NP; x++) {
+                add(x, cmul(te.S, Zk[x]));
+                add(NP + x, cmul(s15, I[x]));
             }
+            if (gl) {
+                perm_congruence<N>(code, Pt, I);
 #pragma unroll
-            for (int m = 0; m < 4 * NP; m++) {
-                A(2 * m) = fma(cf, Dk[m].x, A(2 * m));
-                A(2 * m + 1) = fma(cf, Dk[m].y, A(2 * m + 1));
+                for (int x = 0; x < NP; x++) {
+                    add(2 * NP + x, cmul(te.S, Zl[x]));
+                    add(3 * NP + x, cmul(s15, I[x]));
+                }
             }
         }
-        const double f = 1.0 / sqrt(dSk * diagS[l]);
+        const double f = (1.0 / sqrt(dSk * diagS[l]));
         const size_t kl = (size_t)k + (size_t)l * ld;
         const cd s = f * Ss;
         S[kl] = s;
@@ -389,12 +508,18 @@ __global__ void __launch_bounds__(NT) k_pair_grad(SysParams sp, const double* __
         } else {
             H[kl] = f * Hs;
         }
+        double L[N][N];
+        load_L<N>(params + (size_t)k * 2 * NP, L);
         cd* dkl = D + ((size_t)(k - nfru) + (size_t)l * ldo) * (4 * NP);
-        for (int m = 0; m < 4 * NP; m++) stcd(dkl + m, mk(f * A(2 * m), f * A(2 * m + 1)));
+        deriv_entries<N>(
+            L, [&](int x) { return get(x); }, 1.5 * Hs, [&](int x) { return get(NP + x); }, 1.5 * Ss, 1.0,
+            [&](int m, cd v) { stcd(dkl + m, f * v); });
         if (gl) {
+            load_L<N>(params + (size_t)l * 2 * NP, L);
             cd* dlk = D + ((size_t)(l - nfru) + (size_t)k * ldo) * (4 * NP);
-            for (int m = 0; m < 4 * NP; m++)
-                stcd(dlk + m, mk(f * A(2 * (4 * NP + m)), -f * A(2 * (4 * NP + m) + 1)));
+            deriv_entries<N>(
+                L, [&](int x) { return get(2 * NP + x); }, 1.5 * Hs, [&](int x) { return get(3 * NP + x); }, 1.5 * Ss,
+                -1.0, [&](int m, cd v) { stcd(dlk + m, mk(f * v.x, -f * v.y)); });
         }
     }
 }
@@ -412,99 +537,141 @@ struct AdjNV {
     static constexpr int value = 2 * Sym<N>::NP + 1;
 };
 
-template <int N, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_adjoint(SysParams sp, const double* __restrict__ coef,
-                                                 const double* __restrict__ Pd, const cd* __restrict__ bra,
-                                                 const cd* __restrict__ ket, const double* __restrict__ detL,
+// Sum v[0..M) (M a power of two, at most 32) over the warp's lanes: every
+// step exchanges half of the values a lane still holds, so 2 M - 1 values
+// travel instead of the 5 M of a butterfly per value.  Lane i returns the
+// sum of value i / (32 / M).
+template <int M>
+__device__ __forceinline__ double warp_transpose_sum(double (&v)[M])
+{
+    const int lane = threadIdx.x & 31;
+    int s = 16;
+#pragma unroll
+    for (int h = M / 2; h >= 1; h /= 2) {
+        const bool up = (lane & s) != 0;
+#pragma unroll
+        for (int i = 0; i < h; i++) {
+            const double send = up ? v[i] : v[i + h];
+            const double keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
+        }
+        s /= 2;
+    }
+#pragma unroll
+    for (int q = 16 / M; q >= 1; q /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], q);
+    return v[0];
+}
+
+// FP64 issue bounds it: 860 FP64 instructions a term at n = 3 (ncu), 1.52 ms
+// of the pipe at K = 4000, T = 4, where it takes 2.24 ms (4.35 ms with full
+// products C^-1 R C^-1, a product with P per term and a butterfly per
+// summed value); n = 4, K = 1013, T = 14: 2.43 -> 1.19 ms.
+// One CTA of NW warps per tile.  Column l = C*32 + v + 8 j belongs to
+// virtual warp v < 8; a CTA of fewer than eight warps takes several of them
+// in turn, so the sums do not depend on NW.
+template <int N, int NW, int MINB, bool KETN>
+__global__ void __launch_bounds__(NW * 32, MINB) k_adjoint(SysParams sp, const double* __restrict__ coef,
+                                                 const double* __restrict__ Pd, const int* __restrict__ pcode,
+                                                 const cd* __restrict__ bra, const cd* __restrict__ ket,
+                                                 const cd* __restrict__ ketn, const double* __restrict__ detL,
                                                  const double* __restrict__ diagS, const cd* __restrict__ cvec,
                                                  double E, int nfru, int nfa, int Rlo, double* __restrict__ part,
                                                  long long t0)
 {
     constexpr int NP = Sym<N>::NP;
     constexpr int NV = AdjNV<N>::value;
-    extern __shared__ double red[];  // [8][32][NV]
+    constexpr int M = NV <= 8 ? 8 : (NV <= 16 ? 16 : 32);  // NV rounded up for the lane sums
+    extern __shared__ double2 asm_[];
+    double2* bsm = asm_;  // the 32 rows' bra data, [entry][lane]
+    double* red = reinterpret_cast<double*>(asm_ + BraShared<N>::ENTRIES * TILE);  // [8][32][NV]
     int R, C;
     tile_rc(t0 + blockIdx.x, Rlo, R, C);
     const long long tile = blockIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = R * TILE + lane;
     const bool krow = (k >= nfru && k < nfa);
-    cd Ck[N][N];
     double dk = 1.0, dSk = 1.0;
     cd ck = mk(0.0, 0.0);
     if (krow) {
-        load_sym<N>(bra + (size_t)k * NP, Ck);
+        if (w == 0) stage_bra<N, true>(bra + (size_t)k * NP, sp, bsm + lane, TILE);
         dk = detL[k];
         dSk = diagS[k];
-        ck = ldcd(cvec + k);
+        ck = conj(ldcd(cvec + k));
     }
-    cd Ak[NP];
-    double dl_k = 0.0;
-#pragma unroll
-    for (int x = 0; x < NP; x++) Ak[x] = mk(0.0, 0.0);
+    __syncthreads();
+    const BraShared<N> b{bsm + lane, TILE};
 #pragma unroll 1
-    for (int j = 0; j < TILE / 8; j++) {
-        const int l = C * TILE + w + 8 * j;
-        const bool valid = krow && (l <= k);
-        const bool ketw = (l >= nfru);  // warp-uniform
-        cd Zk[NP], Zl[NP], a = mk(0.0, 0.0);
+    for (int vw = w; vw < 8; vw += NW) {
+        cd Ak[NP];
+        double dl_k = 0.0;
+#pragma unroll
+        for (int x = 0; x < NP; x++) Ak[x] = mk(0.0, 0.0);
+#pragma unroll 1
+        for (int j = 0; j < TILE / 8; j++) {
+            const int l = C * TILE + vw + 8 * j;
+            const bool valid = krow && (l <= k);
+            const bool ketw = (l >= nfru);  // warp-uniform
+            cd Al[NP];
+            double ra = 0.0;
+#pragma unroll
+            for (int x = 0; x < NP; x++) Al[x] = mk(0.0, 0.0);
+            if (valid) {
+                const double absdet = fabs(detL[l] * dk);
+                // the pair's weight conj(c_k) c_l f_kl goes into S of every term
+                const cd wkl = (1.0 / sqrt(dSk * diagS[l])) * cmul(ck, ldcd(cvec + l));
+#pragma unroll 1
+                for (int t = 0; t < sp.T; t++) {
+                    cd tCl[N][N];
+                    load_sym<N>(ket + ((size_t)l * sp.T + t) * NP, tCl);
+                    PairTerm<N> te;
+                    pair_term<N, true>(b, tCl, absdet, sp.two_r3n2 * __ldg(coef + t), sp, te);
+                    const cd Sw = cmul(wkl, te.S);
+                    const double* Pt = Pd + t * NMAX * NMAX;
+                    cd Zk[NP], Zl[NP], a;
+                    auto sides = [&](const auto& n6l) {
+                        const int code = __ldg(pcode + t);
+                        a = ketw ? term_adjoint<N, true>(b, n6l, te, E, code, Pt, Zk, Zl)
+                                 : term_adjoint<N, false>(b, n6l, te, E, code, Pt, Zk, Zl);
+                    };
+                    if (KETN)
+                        sides(KetRead<N>{ketn + ((size_t)l * sp.T + t) * NP});
+                    else
+                        sides(KetFormed<N>(tCl, sp));
+                    ra += cmul(Sw, a).x;
+#pragma unroll
+                    for (int x = 0; x < NP; x++) Ak[x] = cfma(Sw, Zk[x], Ak[x]);
+                    if (ketw)
+#pragma unroll
+                        for (int x = 0; x < NP; x++) Al[x] = cfma(Sw, Zl[x], Al[x]);
+                }
+            }
+            dl_k += ra;
+            if (ketw) {
+                const bool kc = valid && (l != k);
+                double v[M];
+#pragma unroll
+                for (int x = 0; x < M; x++) v[x] = 0.0;
+                if (kc) {
+#pragma unroll
+                    for (int x = 0; x < NP; x++) {
+                        v[2 * x] = Al[x].x;
+                        v[2 * x + 1] = -Al[x].y;
+                    }
+                    v[NV - 1] = ra;
+                }
+                const double sum = warp_transpose_sum<M>(v);
+                const int x = lane / (32 / M);
+                if (lane % (32 / M) == 0 && x < NV) part[((tile * 2 + 1) * TILE + (vw + 8 * j)) * NV + x] = sum;
+            }
+        }
+        double* r = red + ((size_t)vw * TILE + lane) * NV;
 #pragma unroll
         for (int x = 0; x < NP; x++) {
-            Zk[x] = mk(0.0, 0.0);
-            Zl[x] = mk(0.0, 0.0);
+            r[2 * x] = Ak[x].x;
+            r[2 * x + 1] = Ak[x].y;
         }
-        cd wkl = mk(0.0, 0.0);
-        if (valid) {
-            const double absdet = fabs(detL[l] * dk);
-#pragma unroll 1
-            for (int t = 0; t < sp.T; t++) {
-                cd tCl[N][N];
-                load_sym<N>(ket + ((size_t)l * sp.T + t) * NP, tCl);
-                TermEnergy<N> te;
-                term_energy<N, true>(Ck, tCl, absdet, sp, te);
-                double P[N][N];
-                load_P<N>(Pd, t, P);
-                const double cf = __ldg(coef + t);
-                if (ketw)
-                    term_adjoint<N, true>(P, Ck, tCl, te, sp, E, cf, Zk, Zl, a);
-                else
-                    term_adjoint<N, false>(P, Ck, tCl, te, sp, E, cf, Zk, Zl, a);
-            }
-            const double f = 1.0 / sqrt(dSk * diagS[l]);
-            wkl = f * cmul(conj(ck), ldcd(cvec + l));
-        }
-        const double ra = cmul(wkl, a).x;
-#pragma unroll
-        for (int x = 0; x < NP; x++) Ak[x] = cfma(wkl, Zk[x], Ak[x]);
-        dl_k += ra;
-        if (ketw) {
-            const bool kc = valid && (l != k);
-            double v[NV];
-#pragma unroll
-            for (int x = 0; x < NP; x++) {
-                const cd z = kc ? conj(cmul(wkl, Zl[x])) : mk(0.0, 0.0);
-                v[2 * x] = z.x;
-                v[2 * x + 1] = z.y;
-            }
-            v[NV - 1] = kc ? ra : 0.0;
-#pragma unroll
-            for (int s = 16; s >= 1; s >>= 1)
-#pragma unroll
-                for (int x = 0; x < NV; x++) v[x] += __shfl_xor_sync(0xffffffffu, v[x], s);
-            if (lane == 0) {
-                double* dst = part + ((tile * 2 + 1) * TILE + (w + 8 * j)) * NV;
-#pragma unroll
-                for (int x = 0; x < NV; x++) dst[x] = v[x];
-            }
-        }
+        r[NV - 1] = dl_k;
     }
-    double* r = red + ((size_t)w * TILE + lane) * NV;
-#pragma unroll
-    for (int x = 0; x < NP; x++) {
-        r[2 * x] = Ak[x].x;
-        r[2 * x + 1] = Ak[x].y;
-    }
-    r[NV - 1] = dl_k;
     __syncthreads();
     if (w == 0) {
         double* dst = part + ((tile * 2 + 0) * TILE + lane) * NV;
@@ -515,6 +682,11 @@ __global__ void __launch_bounds__(256, MINB) k_adjoint(SysParams sp, const doubl
             dst[x] = s;
         }
     }
+}
+template <int N>
+constexpr size_t adjoint_smem()
+{
+    return sizeof(double2) * BraShared<N>::ENTRIES * TILE + sizeof(double) * 8 * TILE * AdjNV<N>::value;
 }
 
 // dE/d(vech L, vech B) of one function from its summed adjoint values v
@@ -633,29 +805,41 @@ __global__ void __launch_bounds__(128) k_term_batch(SysParams sp, const double* 
     const double* b = pl + (size_t)i * 2 * NP;
     double P[N][N];
     load_P<N>(Pd, term[i], P);
-    cd Ck[N][N], tCl[N][N];
+    BraRegs<N> bk;
+    cd tCl[N][N];
     double dk, dl;
-    make_bra<N>(a, Ck, dk);
+    make_bra<N>(a, bk.c, dk);
+    mass_right<N>(bk.c, sp, bk.km);
+    mass_sandwich<N>(bk.c, bk.km, bk.n6);
     make_ket<N>(b, P, tCl, dl);
-    TermEnergy<N> te;
-    term_energy<N, true>(Ck, tCl, fabs(dl * dk), sp, te);
-    hs[2 * (size_t)i] = te.T + te.V;
+    PairTerm<N> te;
+    pair_term<N, true>(bk, tCl, fabs(dl * dk), sp.two_r3n2, sp, te);
+    hs[2 * (size_t)i] = cmul(te.S, te.h);
     hs[2 * (size_t)i + 1] = te.S;
     if (gradflag < 1 || gradflag > 3) return;
-    double Lk[N][N], Ll[N][N];
-    load_L<N>(a, Lk);
-    load_L<N>(b, Ll);
-    cd Dk[4 * NP], Dl[4 * NP];
-    if (gradflag == 1)
-        term_grad_plain<N, true, false>(Lk, Ll, P, Ck, tCl, te, sp, Dk, Dl);
-    else if (gradflag == 2)
-        term_grad_plain<N, false, true>(Lk, Ll, P, Ck, tCl, te, sp, Dk, Dl);
-    else
-        term_grad_plain<N, true, true>(Lk, Ll, P, Ck, tCl, te, sp, Dk, Dl);
-    if (gradflag & 1)
-        for (int m = 0; m < 4 * NP; m++) dko[(size_t)i * 4 * NP + m] = Dk[m];
-    if (gradflag & 2)
-        for (int m = 0; m < 4 * NP; m++) dlo[(size_t)i * 4 * NP + m] = Dl[m];
+    const double* Pt = Pd + term[i] * NMAX * NMAX;
+    const int code = perm_code(Pt, NMAX, N);
+    cd Zk[NP], Zl[NP], I[NP];
+    const cd a0 = cmul(te.S, term_adjoint<N, true>(bk, KetFormed<N>(tCl, sp), te, 0.0, code, Pt, Zk, Zl));
+    const cd s15 = 1.5 * te.S;
+#pragma unroll
+    for (int r = 0; r < N; r++)
+#pragma unroll
+        for (int q = r; q < N; q++) I[vech_index(N, r, q)] = te.inv[r][q];
+    double L[N][N];
+    if (gradflag & 1) {
+        load_L<N>(a, L);
+        deriv_entries<N>(
+            L, [&](int x) { return cmul(te.S, Zk[x]); }, a0, [&](int x) { return cmul(s15, I[x]); }, s15, 1.0,
+            [&](int m, cd v) { dko[(size_t)i * 4 * NP + m] = v; });
+    }
+    if (gradflag & 2) {
+        perm_congruence<N>(code, Pt, I);
+        load_L<N>(b, L);
+        deriv_entries<N>(
+            L, [&](int x) { return cmul(te.S, Zl[x]); }, a0, [&](int x) { return cmul(s15, I[x]); }, s15, -1.0,
+            [&](int m, cd v) { dlo[(size_t)i * 4 * NP + m] = v; });
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -677,19 +861,18 @@ __global__ void __launch_bounds__(128) k_cand_diag(SysParams sp, const double* _
     constexpr int NP = Sym<N>::NP;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= count) return;
-    cd Ck[N][N];
-    load_sym<N>(cbra + (size_t)j * NP, Ck);
+    BraRegs<N> b;
+    load_bra<N>(cbra + (size_t)j * NP, sp, b);
     const double dj = cdet[j];
     const double absdet = fabs(dj * dj);
     cd Hs = mk(0.0, 0.0), Ss = mk(0.0, 0.0);
     for (int t = 0; t < sp.T; t++) {
         cd tCl[N][N];
         load_sym<N>(cket + ((size_t)j * sp.T + t) * NP, tCl);
-        TermEnergy<N> te;
-        term_energy<N, false>(Ck, tCl, absdet, sp, te);
-        const double cf = coef[t];
-        Hs = rfma(cf, te.T + te.V, Hs);
-        Ss = rfma(cf, te.S, Ss);
+        PairTerm<N> te;
+        pair_term<N, false>(b, tCl, absdet, sp.two_r3n2 * coef[t], sp, te);
+        Hs = cfma(te.S, te.h, Hs);
+        Ss = Ss + te.S;
     }
     cdS[j] = Ss.x;
     cmu[j] = Hs.x / Ss.x - approx_e;
@@ -708,8 +891,14 @@ __global__ void __launch_bounds__(W * 32) k_cand_row(SysParams sp, const double*
                                                      int ldv)
 {
     constexpr int NP = Sym<N>::NP;
+    __shared__ double2 bsm[W * CPW][BraShared<N>::ENTRIES_E];  // the CTA's candidates as bras
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int q = blockIdx.x * 32 + lane;
+    if (threadIdx.x < W * CPW) {
+        const int j = blockIdx.y * W * CPW + threadIdx.x;
+        if (j < count) stage_bra<N, false>(cbra + (size_t)j * NP, sp, bsm[threadIdx.x], 1);
+    }
+    __syncthreads();
     if (q >= nbase) return;
     const double dq = detL[q];
     const double dSq = diagS[q];
@@ -717,21 +906,19 @@ __global__ void __launch_bounds__(W * 32) k_cand_row(SysParams sp, const double*
     for (int u = 0; u < CPW; u++) {
         const int j = (blockIdx.y * W + w) * CPW + u;
         if (j >= count) break;
-        cd Ck[N][N];
-        load_sym<N>(cbra + (size_t)j * NP, Ck);
+        const BraShared<N> b{bsm[w * CPW + u], 1};
         const double absdet = fabs(dq * cdet[j]);
         cd Hs = mk(0.0, 0.0), Ss = mk(0.0, 0.0);
 #pragma unroll 1
         for (int t = 0; t < sp.T; t++) {
             cd tCl[N][N];
             load_sym<N>(ket + ((size_t)q * sp.T + t) * NP, tCl);
-            TermEnergy<N> te;
-            term_energy<N, false>(Ck, tCl, absdet, sp, te);
-            const double cf = __ldg(coef + t);
-            Hs = rfma(cf, te.T + te.V, Hs);
-            Ss = rfma(cf, te.S, Ss);
+            PairTerm<N> te;
+            pair_term<N, false>(b, tCl, absdet, sp.two_r3n2 * __ldg(coef + t), sp, te);
+            Hs = cfma(te.S, te.h, Hs);
+            Ss = Ss + te.S;
         }
-        const double f = 1.0 / sqrt(cdS[j] * dSq);
+        const double f = (1.0 / sqrt(cdS[j] * dSq));
         const size_t o = (size_t)q + (size_t)j * ldv;
         const cd s = f * Ss;
         const cd m = f * (Hs - approx_e * Ss);
@@ -754,61 +941,63 @@ constexpr int CAND_ADJ_NT = 128;
 template <int N>
 __global__ void __launch_bounds__(CAND_ADJ_NT) k_cand_adjoint(
     SysParams sp, const double* __restrict__ coef, const double* __restrict__ Pd, const cd* __restrict__ cbra,
-    const cd* __restrict__ cket, const double* __restrict__ cdet, const double* __restrict__ cdS,
-    const cd* __restrict__ ket, const double* __restrict__ detL, const double* __restrict__ diagS, int nbase,
-    const cd* __restrict__ V, int ldv, const cd* __restrict__ vK, const double* __restrict__ t1,
+    const cd* __restrict__ cket, const cd* __restrict__ cketn, const double* __restrict__ cdet,
+    const double* __restrict__ cdS, const cd* __restrict__ ket, const cd* __restrict__ ketn,
+    const double* __restrict__ detL, const double* __restrict__ diagS, int nbase, const cd* __restrict__ V, int ldv, const cd* __restrict__ vK, const double* __restrict__ t1,
     const double* __restrict__ energy, const int* __restrict__ err, double* __restrict__ part)
 {
     constexpr int NP = Sym<N>::NP;
     constexpr int NV = AdjNV<N>::value;
-    __shared__ double red[CAND_ADJ_NT / 32][NV];
+    constexpr int M = NV <= 8 ? 8 : (NV <= 16 ? 16 : 32);
+    __shared__ double red[CAND_ADJ_NT / 32][M];
+    __shared__ double2 bsm[BraShared<N>::ENTRIES_E];
     const int j = blockIdx.y;
     const int q = blockIdx.x * CAND_ADJ_NT + threadIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    double v[NV];
+    if (threadIdx.x == 0) stage_bra<N, false>(cbra + (size_t)j * NP, sp, bsm, 1);
+    __syncthreads();
+    double v[M];
 #pragma unroll
-    for (int x = 0; x < NV; x++) v[x] = 0.0;
+    for (int x = 0; x < M; x++) v[x] = 0.0;
     if (q <= nbase && err[j] != 1) {
         const double rs = 1.0 / sqrt(t1[j]);
         const double E = energy[j];
         const cd cK = rs * vK[j];
         const bool dg = (q == nbase);
-        cd Ck[N][N];
-        load_sym<N>(cbra + (size_t)j * NP, Ck);
+        const BraShared<N> b{bsm, 1};
         const cd* kq = dg ? cket + (size_t)j * sp.T * NP : ket + (size_t)q * sp.T * NP;
+        const cd* kn = dg ? cketn + (size_t)j * sp.T * NP : ketn + (size_t)q * sp.T * NP;
         const double dq = dg ? cdet[j] : detL[q];
         const double dSq = dg ? cdS[j] : diagS[q];
         const cd cq = dg ? cK : rs * ldcd(V + (size_t)j * ldv + q);
         const double absdet = fabs(dq * cdet[j]);
-        cd Zk[NP], Zl[NP], a = mk(0.0, 0.0);
+        const cd wq = (1.0 / sqrt(cdS[j] * dSq)) * cmul(conj(cK), cq);
+        cd Ak[NP];
+        double ra = 0.0;
 #pragma unroll
-        for (int x = 0; x < NP; x++) Zk[x] = mk(0.0, 0.0);
+        for (int x = 0; x < NP; x++) Ak[x] = mk(0.0, 0.0);
 #pragma unroll 1
         for (int t = 0; t < sp.T; t++) {
             cd tCl[N][N];
             load_sym<N>(kq + (size_t)t * NP, tCl);
-            TermEnergy<N> te;
-            term_energy<N, true>(Ck, tCl, absdet, sp, te);
-            double P[N][N];
-            load_P<N>(Pd, t, P);
-            term_adjoint<N, false>(P, Ck, tCl, te, sp, E, __ldg(coef + t), Zk, Zl, a);
+            PairTerm<N> te;
+            pair_term<N, true>(b, tCl, absdet, sp.two_r3n2 * __ldg(coef + t), sp, te);
+            const cd Sw = cmul(wq, te.S);
+            cd Zk[NP], Zl[NP];
+            const cd a = term_adjoint<N, false>(b, KetRead<N>{kn + (size_t)t * NP}, te, E, 0, Pd, Zk, Zl);
+            ra += cmul(Sw, a).x;
+#pragma unroll
+            for (int x = 0; x < NP; x++) Ak[x] = cfma(Sw, Zk[x], Ak[x]);
         }
-        const cd wq = (1.0 / sqrt(cdS[j] * dSq)) * cmul(conj(cK), cq);
 #pragma unroll
         for (int x = 0; x < NP; x++) {
-            const cd z = cmul(wq, Zk[x]);
-            v[2 * x] = z.x;
-            v[2 * x + 1] = z.y;
+            v[2 * x] = Ak[x].x;
+            v[2 * x + 1] = Ak[x].y;
         }
-        v[NV - 1] = cmul(wq, a).x;
+        v[NV - 1] = ra;
     }
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1)
-#pragma unroll
-        for (int x = 0; x < NV; x++) v[x] += __shfl_xor_sync(0xffffffffu, v[x], s);
-    if (lane == 0)
-#pragma unroll
-        for (int x = 0; x < NV; x++) red[w][x] = v[x];
+    const double sum = warp_transpose_sum<M>(v);
+    if (lane % (32 / M) == 0) red[w][lane / (32 / M)] = sum;
     __syncthreads();
     if (threadIdx.x < NV) {
         double s = 0.0;
@@ -874,39 +1063,46 @@ constexpr int PEN_NT = 128;
 
 template <int N>
 __device__ void pen_pair_deriv(const SysParams& sp, const double* __restrict__ coef,
-                               const double* __restrict__ Pd, const double* __restrict__ params,
-                               const cd* __restrict__ bra, const cd* __restrict__ ket,
-                               const double* __restrict__ detL, int k, int l, bool want_row, cd* out)
+                               const double* __restrict__ Pd, const int* __restrict__ pcode,
+                               const double* __restrict__ params, const cd* __restrict__ bra,
+                               const cd* __restrict__ ket, const double* __restrict__ detL, int k, int l,
+                               bool want_row, cd* out)
 {
     // sum over terms of dS(k,l) w.r.t. the row function k (want_row) or the
     // column function l; out receives 2 NP complex values (vech L, vech B)
     constexpr int NP = Sym<N>::NP;
-    cd Ck[N][N];
-    load_sym<N>(bra + (size_t)k * NP, Ck);
-    double Lk[N][N], Ll[N][N];
-    load_L<N>(params + (size_t)k * 2 * NP, Lk);
-    load_L<N>(params + (size_t)l * 2 * NP, Ll);
+    BraRegs<N> b;
+    load_bra<N>(bra + (size_t)k * NP, sp, b);
     const double absdet = fabs(detL[l] * detL[k]);
-    for (int m = 0; m < 2 * NP; m++) out[m] = mk(0.0, 0.0);
+    DerivSum<N> sum;
+    sum.zero();
     for (int t = 0; t < sp.T; t++) {
         cd tCl[N][N];
         load_sym<N>(ket + ((size_t)l * sp.T + t) * NP, tCl);
-        TermEnergy<N> te;
-        term_energy<N, true>(Ck, tCl, absdet, sp, te);
-        double P[N][N];
-        load_P<N>(Pd, t, P);
-        cd Dk[4 * NP], Dl[4 * NP];
-        term_grad_plain<N, true, true>(Lk, Ll, P, Ck, tCl, te, sp, Dk, Dl);
-        const double cf = coef[t];
-        const cd* d = want_row ? Dk : Dl;
+        PairTerm<N> te;
+        pair_term<N, false>(b, tCl, absdet, sp.two_r3n2 * coef[t], sp, te);
+        const cd s15 = 1.5 * te.S;
+        cd I[NP];
 #pragma unroll
-        for (int m = 0; m < 2 * NP; m++) out[m] = rfma(cf, d[2 * NP + m], out[m]);
+        for (int i = 0; i < N; i++)
+#pragma unroll
+            for (int j = i; j < N; j++) I[vech_index(N, i, j)] = te.inv[i][j];
+        if (!want_row) perm_congruence<N>(pcode[t], Pd + t * NMAX * NMAX, I);
+#pragma unroll
+        for (int x = 0; x < NP; x++) sum.zs[x] = cfma(s15, I[x], sum.zs[x]);
+        sum.as = sum.as + s15;
     }
+    double L[N][N];
+    load_L<N>(params + (size_t)(want_row ? k : l) * 2 * NP, L);
+    auto zs = [&](int x) { return sum.zs[x]; };
+    deriv_entries<N>(L, zs, sum.as, zs, sum.as, want_row ? 1.0 : -1.0, [&](int m, cd v) {
+        if (m >= 2 * NP) out[m - 2 * NP] = v;
+    });
 }
 
 template <int N>
 __global__ void __launch_bounds__(PEN_NT) k_penalty(SysParams sp, const double* __restrict__ coef,
-                                                    const double* __restrict__ Pd,
+                                                    const double* __restrict__ Pd, const int* __restrict__ pcode,
                                                     const double* __restrict__ params, const cd* __restrict__ bra,
                                                     const cd* __restrict__ ket, const double* __restrict__ detL,
                                                     const double* __restrict__ diagS, const cd* __restrict__ S,
@@ -943,7 +1139,7 @@ __global__ void __launch_bounds__(PEN_NT) k_penalty(SysParams sp, const double* 
     if (tid == 0) {
         // Glob_D(npt+m, r-nfru, r) = 2 Re(sum_t coef_t dS_rr/dp_m) / diagS_r
         cd d[NPT];
-        pen_pair_deriv<N>(sp, coef, Pd, params, bra, ket, detL, r, r, true, d);
+        pen_pair_deriv<N>(sp, coef, Pd, pcode, params, bra, ket, detL, r, r, true, d);
         for (int m = 0; m < NPT; m++) sdd[m] = 2.0 * d[m].x / dr;
     }
     for (int m = 0; m < NPT; m++) sg[m][tid] = 0.0;
@@ -957,7 +1153,7 @@ __global__ void __launch_bounds__(PEN_NT) k_penalty(SysParams sp, const double* 
         if (!(aux > t2)) continue;
         cd d[NPT];
         const bool row = (r == j);
-        pen_pair_deriv<N>(sp, coef, Pd, params, bra, ket, detL, j, i, row, d);
+        pen_pair_deriv<N>(sp, coef, Pd, pcode, params, bra, ket, detL, j, i, row, d);
         const double f = 1.0 / sqrt(diagS[j] * diagS[i]);
         const double temp2 = (mode == 2) ? 1.0 : sqrt(diagS[i] / diagS[j]);
         for (int m = 0; m < NPT; m++) {
@@ -1000,7 +1196,8 @@ template <int N>
 static int prep_n(Ctx& c, int nfun)
 {
     if (nfun <= 0) return 0;
-    k_prep<N><<<(nfun + 127) / 128, 128, 0, c.stream>>>(c.params, c.Pd, c.T, nfun, c.bra, c.ket, c.detL);
+    k_prep<N><<<(nfun + 127) / 128, 128, 0, c.stream>>>(c.sp, c.params, c.Pd, c.T, nfun, c.bra, c.ket, c.ketn, c.pcode,
+                                                       c.detL);
     c.launches++;
     return last_err();
 }
@@ -1025,8 +1222,8 @@ static int diag_n(Ctx& c, int r0, int r1, double approx_e, int deriv, int nfru)
 template <int N>
 static int penalty_n(Ctx& c, int nfru, int nfa, double t2, double pc, int mode, double* part)
 {
-    k_penalty<N><<<nfa - nfru, PEN_NT, 0, c.stream>>>(c.sp, c.coef, c.Pd, c.params, c.bra, c.ket, c.detL, c.diagS,
-                                                      c.S, c.ld, nfru, nfa, t2, pc, mode, c.grad, part);
+    k_penalty<N><<<nfa - nfru, PEN_NT, 0, c.stream>>>(c.sp, c.coef, c.Pd, c.pcode, c.params, c.bra, c.ket, c.detL,
+                                                      c.diagS, c.S, c.ld, nfru, nfa, t2, pc, mode, c.grad, part);
     c.launches++;
     return last_err();
 }
@@ -1041,25 +1238,27 @@ int launch_pair_diag(Ctx& c, int r0, int r1, double approx_e, int deriv, int nfr
 }
 
 // The pair-kernel shapes the autotuner chooses from: k_pair_energy (warps
-// per tile, minimum CTAs per SM), k_adjoint (minimum CTAs per SM).
+// per tile, minimum CTAs per SM), k_adjoint (the same: 8 warps at 1 CTA, or 4
+// at 3, whose 168 registers spill a little at n = 3 and too much at n = 4).
 template <int N>
 static void pair_energy_launch(Ctx& c, int v, unsigned grid, int r0, int r1, int Rlo, double approx_e, long long t0)
 {
+    constexpr size_t smem = sizeof(double2) * BraShared<N>::ENTRIES_E * TILE;
     switch (v) {
         case 0:
-            k_pair_energy<N, 8, 2><<<grid, 256, 0, c.stream>>>(c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S,
+            k_pair_energy<N, 8, 2><<<grid, 256, smem, c.stream>>>(c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S,
                                                                c.ld, r0, r1, Rlo, c.method, approx_e, t0);
             break;
         case 1:
-            k_pair_energy<N, 8, 3><<<grid, 256, 0, c.stream>>>(c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S,
+            k_pair_energy<N, 4, 3><<<grid, 128, smem, c.stream>>>(c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S,
                                                                c.ld, r0, r1, Rlo, c.method, approx_e, t0);
             break;
         case 2:
-            k_pair_energy<N, 4, 2><<<grid, 128, 0, c.stream>>>(c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S,
+            k_pair_energy<N, 4, 2><<<grid, 128, smem, c.stream>>>(c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S,
                                                                c.ld, r0, r1, Rlo, c.method, approx_e, t0);
             break;
         default:
-            k_pair_energy<N, 4, 4><<<grid, 128, 0, c.stream>>>(c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S,
+            k_pair_energy<N, 4, 4><<<grid, 128, smem, c.stream>>>(c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S,
                                                                c.ld, r0, r1, Rlo, c.method, approx_e, t0);
             break;
     }
@@ -1171,7 +1370,7 @@ static int grad_n(Ctx& c, int r0, int r1, int nfru, double approx_e)
     if (r1 <= r0) return 0;
     constexpr int NT = (N <= 4) ? 128 : 64;
     constexpr int NP = Sym<N>::NP;
-    const size_t smem = (size_t)16 * NP * NT * sizeof(double);
+    const size_t smem = sizeof(double2) * ((size_t)4 * NP * NT + BraShared<N>::ENTRIES * TILE);
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(k_pair_grad<N, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1179,8 +1378,8 @@ static int grad_n(Ctx& c, int r0, int r1, int nfru, double approx_e)
     }
     const int Rlo = r0 / TILE, Rhi = (r1 + TILE - 1) / TILE;
     const long long nt = tile_count(Rlo, Rhi);
-    k_pair_grad<N, NT><<<(unsigned)nt, NT, smem, c.stream>>>(c.sp, c.coef, c.Pd, c.params, c.bra, c.ket, c.detL,
-                                                             c.diagS, c.H, c.S, c.ld, r0, r1, Rlo, c.method,
+    k_pair_grad<N, NT><<<(unsigned)nt, NT, smem, c.stream>>>(c.sp, c.coef, c.Pd, c.pcode, c.params, c.bra, c.ket,
+                                                             c.ketn, c.detL, c.diagS, c.H, c.S, c.ld, r0, r1, Rlo, c.method,
                                                              approx_e, c.D, c.max_nfo, nfru);
     c.launches++;
     return last_err();
@@ -1205,20 +1404,22 @@ static int adjoint_n(Ctx& c, int nfru, int nfa, double E)
         if (cudaMalloc(&c.part, need) != cudaSuccess) return -3;
         c.part_bytes = need;
     }
-    const size_t smem = (size_t)8 * TILE * NV * sizeof(double);
+    constexpr size_t smem = adjoint_smem<N>();
     static bool attr = false;
     if (!attr) {
-        cudaFuncSetAttribute(k_adjoint<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        cudaFuncSetAttribute(k_adjoint<N, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_adjoint<N, 8, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_adjoint<N, 4, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         attr = true;
     }
     auto run = [&](int v) {
         if (v == 0)
-            k_adjoint<N, 1><<<(unsigned)nt, 256, smem, c.stream>>>(c.sp, c.coef, c.Pd, c.bra, c.ket, c.detL, c.diagS,
-                                                                   c.c, E, nfru, nfa, Rlo, c.part, 0LL);
+            k_adjoint<N, 8, 1, true><<<(unsigned)nt, 256, smem, c.stream>>>(c.sp, c.coef, c.Pd, c.pcode, c.bra, c.ket,
+                                                                            c.ketn, c.detL, c.diagS, c.c, E, nfru,
+                                                                            nfa, Rlo, c.part, 0LL);
         else
-            k_adjoint<N, 2><<<(unsigned)nt, 256, smem, c.stream>>>(c.sp, c.coef, c.Pd, c.bra, c.ket, c.detL, c.diagS,
-                                                                   c.c, E, nfru, nfa, Rlo, c.part, 0LL);
+            k_adjoint<N, 4, 3, true><<<(unsigned)nt, 128, smem, c.stream>>>(c.sp, c.coef, c.Pd, c.pcode, c.bra, c.ket,
+                                                                            c.ketn, c.detL, c.diagS, c.c, E, nfru,
+                                                                            nfa, Rlo, c.part, 0LL);
     };
     c.launches++;
     if (c.tune_adj < 0 && nt >= 256) {
@@ -1242,12 +1443,13 @@ static int adjoint_tiles_n(Ctx& c, int nfru, int nfa, double E, const cd* cvec, 
                            double* part)
 {
     if (nfa <= nfru || count <= 0) return 0;
-    constexpr int NV = AdjNV<N>::value;
-    const size_t smem = (size_t)8 * TILE * NV * sizeof(double);
-    if (cudaFuncSetAttribute(k_adjoint<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    constexpr size_t smem = adjoint_smem<N>();
+    if (cudaFuncSetAttribute(k_adjoint<N, 8, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
         return -2;
-    k_adjoint<N, 1><<<(unsigned)count, 256, smem, c.stream>>>(c.sp, c.coef, c.Pd, c.bra, c.ket, c.detL, c.diagS,
-                                                              cvec, E, nfru, nfa, nfru / TILE, part, t0);
+    k_adjoint<N, 8, 1, true><<<(unsigned)count, 256, smem, c.stream>>>(c.sp, c.coef, c.Pd, c.pcode, c.bra, c.ket,
+                                                                       c.ketn, c.detL, c.diagS, cvec, E, nfru, nfa,
+                                                                       nfru / TILE, part, t0);
     c.launches++;
     return last_err();
 }
@@ -1312,7 +1514,8 @@ template <int N>
 static int cand_rows_n(Ctx& c, CandWork& cw, int nbase, int count, double approx_e, int variant)
 {
     if (count <= 0) return 0;
-    k_prep<N><<<(count + 127) / 128, 128, 0, c.stream>>>(cw.par, c.Pd, c.T, count, cw.bra, cw.ket, cw.det);
+    k_prep<N><<<(count + 127) / 128, 128, 0, c.stream>>>(c.sp, cw.par, c.Pd, c.T, count, cw.bra, cw.ket, cw.ketn, nullptr,
+                                                        cw.det);
     k_cand_diag<N><<<(count + 127) / 128, 128, 0, c.stream>>>(c.sp, c.coef, cw.bra, cw.ket, cw.det, count, approx_e,
                                                               cw.dS, cw.mu);
     c.launches += 2;
@@ -1340,8 +1543,8 @@ static int cand_adjoint_n(Ctx& c, CandWork& cw, int nbase, int count, const cd* 
     constexpr int NV = AdjNV<N>::value;
     const int nchunk = nbase / CAND_ADJ_NT + 1;  // q = 0..nbase
     if ((size_t)nchunk * count * NV > cw.gpart_n) return -1;
-    k_cand_adjoint<N><<<dim3(nchunk, count), CAND_ADJ_NT, 0, c.stream>>>(c.sp, c.coef, c.Pd, cw.bra, cw.ket, cw.det,
-                                                                         cw.dS, c.ket, c.detL, c.diagS, nbase, cw.V,
+    k_cand_adjoint<N><<<dim3(nchunk, count), CAND_ADJ_NT, 0, c.stream>>>(c.sp, c.coef, c.Pd, cw.bra, cw.ket,
+                                                                         cw.ketn, cw.det, cw.dS, c.ket, c.ketn, c.detL, c.diagS, nbase, cw.V,
                                                                          cw.ldv, vK, t1, energy, err, cw.gpart);
     k_cand_adjoint_final<N><<<(count * 32 + 255) / 256, 256, 0, c.stream>>>(cw.gpart, nchunk, cw.par, err, count,
                                                                            grad);
@@ -1394,7 +1597,8 @@ constexpr size_t OFF_COEF = OFF_P + align256(sizeof(double) * TMAXN * NMAX * NMA
 constexpr size_t OFF_BRA = OFF_COEF + align256(sizeof(double) * TMAXN);
 constexpr size_t OFF_KET = OFF_BRA + align256(sizeof(cd) * KMAX * NPMAX);
 constexpr size_t OFF_DET = OFF_KET + align256(sizeof(cd) * KMAX * TMAXN * NPMAX);
-constexpr size_t OFF_PART = OFF_DET + align256(sizeof(double) * KMAX);
+constexpr size_t OFF_CODE = OFF_DET + align256(sizeof(double) * KMAX);
+constexpr size_t OFF_PART = OFF_CODE + align256(sizeof(int) * TMAXN);
 constexpr size_t BYTES = OFF_PART + align256(sizeof(double) * TILES * 2 * TILE * NVMAX);
 
 // The one scratch array.  Host code must not take its address directly (on
@@ -1446,7 +1650,6 @@ template <int N>
 static int run(const SysParams& sp, const Terms& terms, unsigned char* base, const double* params, const cd* cvec, const double* diagS,
                double E, int nfru, int nfa, double* grad, cudaStream_t st)
 {
-    constexpr int NV = AdjNV<N>::value;
     double* Pd = reinterpret_cast<double*>(base + OFF_P);
     double* coef = reinterpret_cast<double*>(base + OFF_COEF);
     k_store_terms<<<1, 128, 0, st>>>(terms, sp.T, Pd, coef);
@@ -1454,16 +1657,19 @@ static int run(const SysParams& sp, const Terms& terms, unsigned char* base, con
     cd* ket = reinterpret_cast<cd*>(base + OFF_KET);
     double* detL = reinterpret_cast<double*>(base + OFF_DET);
     double* part = reinterpret_cast<double*>(base + OFF_PART);
-    k_prep<N><<<(nfa + 127) / 128, 128, 0, st>>>(params, Pd, sp.T, nfa, bra, ket, detL);
+    int* pcode = reinterpret_cast<int*>(base + OFF_CODE);
+    k_prep<N><<<(nfa + 127) / 128, 128, 0, st>>>(sp, params, Pd, sp.T, nfa, bra, ket, nullptr, pcode, detL);
     const int Rlo = nfru / TILE, Rhi = (nfa + TILE - 1) / TILE;
     const long long nt = tile_count(Rlo, Rhi);
-    const size_t smem = (size_t)8 * TILE * NV * sizeof(double);
-    if (cudaFuncSetAttribute(k_adjoint<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    constexpr size_t smem = adjoint_smem<N>();
+    // the fixed array has no room for 6 tCl M tCl: the kernel forms it
+    if (cudaFuncSetAttribute(k_adjoint<N, 8, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess) {
         cudaGetLastError();
         return ECG_ECUDA;
     }
-    k_adjoint<N, 1><<<(unsigned)nt, 256, smem, st>>>(sp, coef, Pd, bra, ket, detL, diagS, cvec, E, nfru, nfa, Rlo, part,
-                                                     0LL);
+    k_adjoint<N, 8, 1, false><<<(unsigned)nt, 256, smem, st>>>(sp, coef, Pd, pcode, bra, ket, nullptr, detL, diagS, cvec,
+                                                               E, nfru, nfa, Rlo, part, 0LL);
     const int nf = nfa - nfru;
     k_adjoint_final<N><<<(nf * 32 + 255) / 256, 256, 0, st>>>(part, params, nfru, nfa, Rlo, Rhi, grad);
     return cudaGetLastError() == cudaSuccess ? ECG_OK : ECG_ECUDA;
