@@ -701,8 +701,8 @@ static void enqueue_factor(Ctx& c, int m0, int n, const std::vector<int>& starts
 }
 
 // A whole factorisation (m0 = 0) as one persistent kernel (ldlp.cu): the
-// working upper triangle and diagonal, the tile tasks, then the inverse
-// diagonal blocks of the solves.
+// working upper triangle and diagonal, the tile tasks (which leave the
+// inverse diagonal blocks), then the neighbour products of the solves.
 static void enqueue_persist(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long long* trace = nullptr)
 {
     const int ct1 = (n + 31) / 32;
@@ -710,10 +710,9 @@ static void enqueue_persist(Ctx& c, int n, const unsigned* tasks, int ntasks, un
     c.launches++;
     ldlp_enqueue(c, n, tasks, ntasks, trace);
     const int nblk = (n + LDL_NB - 1) / LDL_NB;
-    k_ldl_linv<<<nblk, 256, 2 * LDL_NB * DG_LD * sizeof(double2), c.stream>>>(c.F, c.ld, c.dblk, 0, c.linv);
     k_ldl_mn<<<dim3(nblk, 2), 256, 2 * LDL_NB * DG_LD * sizeof(double2), c.stream>>>(c.F, c.ld, c.dblk, nblk, 0,
                                                                                     c.linv, c.lmf, c.lnb);
-    c.launches += 2;
+    c.launches++;
 }
 
 static void ldl_attrs()

@@ -7,8 +7,9 @@
 // working Schur complement W(r, c), r < c, lives in the upper triangle and
 // its diagonal in dw.  The factorisation is split into tasks on 64 x 64 tiles
 // (R, C), R <= C, of panel index s:
-//   D(s)        eliminate the diagonal tile (s, s): U_ss, invD, pivots d_s
-//               (written to dw over the consumed working diagonal);
+//   D(s)        eliminate the diagonal tile (s, s): U_ss, L_ss^-1 (also what
+//               the triangular solves need), invD, pivots d_s (written to dw
+//               over the consumed working diagonal);
 //   T(s, C)     panel rows of tile (s, C): U(s, C) = invD L_ss^-1 W(s, C);
 //   B(s, R, C)  W(R, C) -= conj(U(s, R))^T diag(d_s) U(s, C), s < R <= C
 //               (the unscaled rows of the reference's recurrence, d U, are
@@ -19,7 +20,7 @@
 //   D(s): cnt(s,s) >= s;  T(s,C): cnt(s,s) >= s+1, cnt(s,C) >= s;
 //   B(s,R,C): cnt(s,R) >= s+1, cnt(s,C) >= s+1, cnt(R,C) >= s.
 // CTA 0, alone on its SM, runs the chain D(s) -> T(s, s+1) -> B(s, s+1,
-// s+1) -> D(s+1) with the diagonal tile kept in shared memory.  The other
+// s+1) -> D(s+1) with the diagonal tile kept in registers.  The other
 // CTAs (all co-resident: cooperative launch) take every other task from a
 // list in a fixed order through one atomic counter; an update whose next
 // panels are already final applies them too (rank up to 256).  The list is
@@ -31,10 +32,17 @@
 // always proceed: the kernel cannot deadlock.  Waits are still bounded (the
 // poll limit of ecg_set_wait_limit); a CTA that gives up records
 // ST_SOLVE_TIMEOUT and sets the abort word, after which every CTA stops
-// taking tasks.  The kernel's code is kept compact (loops that are not
-// unrolled where unrolling gained nothing): the chain's per-panel loop has
-// to stay in the instruction cache, and a larger form measured D(s) at 42
-// instead of 21 us.
+// taking tasks.
+//
+// What bounds it: the FP64 tensor cores for the list (37 TFLOP/s; DFMA and
+// DMMA share that unit), the chain's latency where few panels are left.  On a
+// B200 the chain takes 32 us a panel (D 18, T 9, B 4 and a part overlapped
+// with D; 47 us with an elimination through shared memory and substitution
+// in T), so whole factorisations take 0.32 ms at K = 500 (0.46 before),
+// 0.88 at 1500 (1.24), 4.45 at 4000 (4.94).  Two CTAs an SM take 217 KB of
+// shared memory and leave about 28 KB of L1, so a spilled register comes back
+// from L2: the chain with 200 bytes of stack ran D(s) in 32 us, with 32 bytes
+// in 18.  Every array of the chain is sized to stay within 128 registers.
 #include <algorithm>
 #include <queue>
 #include <utility>
@@ -49,8 +57,6 @@ constexpr unsigned LP_NONE = 0xffffffffu;
 constexpr int LP_KC = 16;          // k rows per cp.async stage of an update
 constexpr int LP_P = 66;           // pitch (double2) of the staged operands: 2 mod 8, conflict-free fragments
 constexpr int LP_ST = 3;           // stages
-constexpr int LP_LD = LDL_NB + 1;  // pitch of the 64 x 64 shared tiles of D and T
-constexpr int LP_SUB = 8;          // sub-panel rows of the diagonal elimination
 constexpr int LP_MERGE = 4;        // most panels one trailing update applies at once
 constexpr size_t LP_SMEM_B = (size_t)(LP_ST * LP_KC * 2 * LP_P + LP_MERGE * LDL_NB) * sizeof(double2);
 
@@ -263,121 +269,86 @@ __device__ __forceinline__ bool lp_wait(const unsigned* p, unsigned v, unsigned*
     return true;
 }
 
-// T(s, C): U(s, C) = invD L_ss^-1 W(s, C) for the 64 columns of tile
-// (s, C), L_ss = U_ss^H unit lower, on the FP64 tensor cores by 8-row
-// blocks: with X_b = L_bb^-1 (the inverse of the b-th 8 x 8 diagonal block
-// of L) and the blocks L_ab below it,
-//     Wun_b = X_b W_b,   W_a -= L_ab Wun_b  (a > b),   b = 0..7,
-// which is the substitution of src/linalg.f90:384-389 for eight rows at a
-// time.  Each warp owns eight columns and runs the whole recurrence on them
-// (no barrier between the blocks); the eight X_b are formed first, one per
-// warp, by substitution on the identity.
-constexpr int LT_WP = 66;  // pitch (double2) of the working tile: fragment loads conflict-free
-constexpr size_t LP_SMEM_T = (size_t)(LDL_NB * LT_WP + 2016 + 8 * 64 + LDL_NB) * sizeof(double2);
+// T(s, C): U(s, C) = invD Linv_ss W(s, C) for the 64 columns of tile (s, C),
+// Linv_ss = L_ss^-1 (unit lower) as the diagonal task left it: one product
+// with a triangular matrix on the FP64 tensor cores, 288 independent-ordered
+// mma a warp and no step that waits for another.  (Substitution by 8-row
+// blocks, the form before, is a chain of eight dependent steps through
+// shared memory: 23.4 us a task with two CTAs an SM at K = 4000, 12.4 us on
+// the chain's own SM.)
+// Linv_ss sits in shared memory as its 36 lower 8 x 8 blocks, block (m, k)
+// at li_blk(m, k), element (r, q) of it at li_el(r, q): the exclusive or
+// spreads the fragment loads of two rows over all bank groups.
+constexpr int LT_WP = 66;  // pitch (double2) of a working tile: fragment loads conflict-free
+constexpr int LI_N = 36 * 64;
+__device__ __forceinline__ int li_blk(int m, int k) { return (m * (m + 1) / 2 + k) * 64; }
+__device__ __forceinline__ int li_el(int r, int q) { return r * 8 + (q ^ ((r & 1) << 2)); }
+constexpr size_t LP_SMEM_T = (size_t)(LI_N + LDL_NB * LT_WP + LDL_NB) * sizeof(double2);
 
-__device__ __forceinline__ int lt_li(int r, int q) { return r * (r - 1) / 2 + q; }  // packed strict lower, q < r
-
-__device__ void lp_trsm(cd* __restrict__ A, int ld, int n, int s, int C, const cd* __restrict__ invD, double2* sm)
+// Rows of Linv W for this warp's eight columns c0..: accr/acci[m][e] is
+// entry (8 m + g, c0 + 2 t4 + e).
+__device__ __forceinline__ void lp_linv_product(const double2* __restrict__ Li, const double2* __restrict__ Wt, int c0,
+                                                int g, int t4, double (&accr)[8][2], double (&acci)[8][2])
 {
-    double2* Wt = sm;                      // Wt[q * LT_WP + c]: the tile, then Wun
-    double2* Lp = Wt + LDL_NB * LT_WP;     // L(r, q) = conj(U(q, r)), q < r, packed
-    double2* Xb = Lp + 2016;               // X_b(i, j) at Xb[b * 64 + i * 8 + j]
-    double2* ids = Xb + 8 * 64;            // invD of the panel
-    const int p0 = s * LDL_NB, b = min(LDL_NB, n - p0);
+#pragma unroll
+    for (int m = 0; m < 8; m++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) accr[m][e] = acci[m][e] = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const double2 w = Wt[(8 * k + 4 * h + t4) * LT_WP + c0 + g];
+            const double wn = -w.y;
+#pragma unroll
+            for (int m = k; m < 8; m++) {
+                const double2 x = Li[li_blk(m, k) + li_el(g, 4 * h + t4)];
+                lp_mma(accr[m][0], accr[m][1], x.x, w.x);
+                lp_mma(acci[m][0], acci[m][1], x.x, w.y);
+                lp_mma(accr[m][0], accr[m][1], x.y, wn);
+                lp_mma(acci[m][0], acci[m][1], x.y, w.x);
+            }
+        }
+}
+
+__device__ void lp_panel(cd* __restrict__ A, int ld, int n, int s, int C, const cd* __restrict__ invD,
+                         const cd* __restrict__ linv, double2* sm)
+{
+    double2* Li = sm;
+    double2* Wt = Li + LI_N;                // Wt[q * LT_WP + c]
+    double2* ids = Wt + LDL_NB * LT_WP;     // invD of the panel
+    const int p0 = s * LDL_NB;              // a panel with columns beyond it is 64 rows high
     const int cb = C * LDL_NB, wd = min(LDL_NB, n - cb);
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll 3
+    for (int e = tid; e < LI_N; e += 256) {
+        const int blk = e >> 6, r = (e >> 3) & 7, q = e & 7;
+        const int m = (int)((sqrtf(8.0f * blk + 1.0f) - 1.0f) * 0.5f), k = blk - m * (m + 1) / 2;
+        cp_async16(Li + blk * 64 + li_el(r, q), linv + (size_t)(p0 + 8 * m + r) * LDL_NB + 8 * k + q, 16);
+    }
+#pragma unroll 4
     for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
         const int q = e & 63, c = e >> 6;
-        const bool in = q < b && c < wd;
+        const bool in = c < wd;
         cp_async16(Wt + q * LT_WP + c, in ? (const void*)(A + (size_t)(p0 + q) + (size_t)(cb + c) * ld) : (const void*)A,
                    in ? 16 : 0);
     }
     cp_async_commit();
-    for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
-        const int q = e & 63, r = e >> 6;
-        if (q < r) {
-            double2 v = make_double2(0.0, 0.0);
-            if (r < b) {
-                v = lp_ldcg(A + (size_t)(p0 + q) + (size_t)(p0 + r) * ld);
-                v.y = -v.y;
-            }
-            Lp[lt_li(r, q)] = v;
-        }
-    }
-    if (tid < LDL_NB) ids[tid] = tid < b ? lp_ldcg(invD + p0 + tid) : make_double2(0.0, 0.0);
-    __syncthreads();
-    // X_wp = L_bb^-1 for block bb = wp: lane j < 8 holds column j
-    {
-        const int bb = wp, j = lane;
-        cd x[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) x[i] = cd{(i == j) ? 1.0 : 0.0, 0.0};
-#pragma unroll
-        for (int q = 0; q < 8; q++)
-#pragma unroll
-            for (int r = q + 1; r < 8; r++) {
-                const double2 l = Lp[lt_li(8 * bb + r, 8 * bb + q)];
-                x[r] = cfms(cd{l.x, l.y}, x[q], x[r]);
-            }
-        if (j < 8)
-#pragma unroll
-            for (int i = 0; i < 8; i++) Xb[bb * 64 + i * 8 + j] = make_double2(x[i].x, x[i].y);
-    }
+    if (tid < LDL_NB) ids[tid] = lp_ldcg(invD + p0 + tid);
     cp_async_wait<0>();
     __syncthreads();
-    // the recurrence on this warp's eight columns
+    double accr[8][2], acci[8][2];
     const int c0 = 8 * wp;
-#pragma unroll 1
-    for (int bk = 0; bk < 8; bk++) {
-        // Wun_b = X_b W_b
-        double wr[2] = {0.0, 0.0}, wi[2] = {0.0, 0.0};
+    lp_linv_product(Li, Wt, c0, g, t4, accr, acci);
 #pragma unroll
-        for (int k0 = 0; k0 < 8; k0 += 4) {
-            const double2 xa = Xb[bk * 64 + g * 8 + k0 + t4];         // X_b(g, k)
-            const double2 wv = Wt[(8 * bk + k0 + t4) * LT_WP + c0 + g];  // W(k, c)
-            lp_mma(wr[0], wr[1], xa.x, wv.x);
-            lp_mma(wr[0], wr[1], -xa.y, wv.y);
-            lp_mma(wi[0], wi[1], xa.x, wv.y);
-            lp_mma(wi[0], wi[1], xa.y, wv.x);
-        }
-        __syncwarp();
+    for (int m = 0; m < 8; m++) {
+        const double2 d = ids[8 * m + g];
 #pragma unroll
-        for (int e = 0; e < 2; e++) Wt[(8 * bk + g) * LT_WP + c0 + 2 * t4 + e] = make_double2(wr[e], wi[e]);
-        __syncwarp();
-        // W_a -= L_ab Wun_b for the blocks a below
-        double2 un[2];
-#pragma unroll
-        for (int k0 = 0; k0 < 8; k0 += 4) un[k0 / 4] = Wt[(8 * bk + k0 + t4) * LT_WP + c0 + g];  // Wun(k, c)
-#pragma unroll 1
-        for (int a = bk + 1; a < 8; a++) {
-            double ar[2], ai[2];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const double2 o = Wt[(8 * a + g) * LT_WP + c0 + 2 * t4 + e];
-                ar[e] = o.x;
-                ai[e] = o.y;
-            }
-#pragma unroll
-            for (int k0 = 0; k0 < 8; k0 += 4) {
-                const double2 l = Lp[lt_li(8 * a + g, 8 * bk + k0 + t4)];  // L(r, k)
-                const double2 u = un[k0 / 4];
-                lp_mma(ar[0], ar[1], -l.x, u.x);
-                lp_mma(ar[0], ar[1], l.y, u.y);
-                lp_mma(ai[0], ai[1], -l.x, u.y);
-                lp_mma(ai[0], ai[1], -l.y, u.x);
-            }
-#pragma unroll
-            for (int e = 0; e < 2; e++) Wt[(8 * a + g) * LT_WP + c0 + 2 * t4 + e] = make_double2(ar[e], ai[e]);
-        }
-        __syncwarp();
-    }
-    // U = invD Wun
-    for (int e = lane; e < LDL_NB * 8; e += 32) {
-        const int q = e & 63, c = c0 + (e >> 6);
-        if (q < b && c < wd) {
-            const double2 v = Wt[q * LT_WP + c], d = ids[q];
-            A[(size_t)(p0 + q) + (size_t)(cb + c) * ld] = cmul(cd{v.x, v.y}, cd{d.x, d.y});
+        for (int e = 0; e < 2; e++) {
+            const int c = c0 + 2 * t4 + e;
+            if (c < wd)
+                A[(size_t)(p0 + 8 * m + g) + (size_t)(cb + c) * ld] = cmul(cd{accr[m][e], acci[m][e]}, cd{d.x, d.y});
         }
     }
 }
@@ -519,9 +490,11 @@ struct LpArgs {
     int ntasks;
     unsigned* cnt;          // tile counters
     unsigned* hc;           // per tile: column halves of band updates finished
+    unsigned* cl;           // per tile: panels claimed by a merged update under way
     unsigned* ctl;          // [0] next list index, [1] abort word, [2] trace records, [3] chain CTA's SM + 1
     cd* dw;
     cd* invD;
+    cd* linv;               // inverse unit-lower diagonal blocks, row r of panel p at [(64 p + r) * 64]
     int* status;
     const int* limitp;      // poll limit of the bounded waits
     unsigned long long* trace;  // optional: per task (code | cta << 32 | panels << 48, start, ready, done)
@@ -554,23 +527,27 @@ __device__ __forceinline__ int lp_deps(unsigned task, long long (&ix)[3], unsign
 }
 
 // Thread 0: wait until cnt[ix[i]] >= need[i] for the k (<= 3) conditions,
-// polling them together.  False when this CTA must stop.
-__device__ __forceinline__ bool lp_wait_all(const LpArgs& a, const long long (&ix)[3], const unsigned (&need)[3],
-                                            int k, int limit)
+// polling them together: 1 when they hold, 0 when this CTA must stop.  For
+// an update by panel need[0] also 2, as soon as a merged update that covers
+// this panel is under way in another CTA: waiting for it to finish, only to
+// find the panel applied, held CTAs for 13 % of the run at K = 4000.
+__device__ __forceinline__ int lp_wait_all(const LpArgs& a, const long long (&ix)[3], const unsigned (&need)[3],
+                                           int k, int limit, bool update = false)
 {
     int spins = 0;
     for (;;) {
+        if (update && *((volatile unsigned*)(a.cl + ix[0])) > need[0]) return 2;
         unsigned v[3];
 #pragma unroll
         for (int i = 0; i < 3; i++) v[i] = (i < k) ? lp_ld_acquire(a.cnt + ix[i]) : 0u;
         bool ok = true;
 #pragma unroll
         for (int i = 0; i < 3; i++) ok = ok && (i >= k || v[i] >= need[i]);
-        if (ok) return true;
+        if (ok) return 1;
         if (++spins > limit || *((volatile unsigned*)(a.ctl + 1)) != 0u) {
             atomicExch(a.status + ST_SOLVE_TIMEOUT, 1);
             atomicExch(a.ctl + 1, 1u);
-            return false;
+            return 0;
         }
         __nanosleep(32);
     }
@@ -595,7 +572,7 @@ __device__ __forceinline__ void lp_exec(const LpArgs& a, unsigned type, int s, i
                                         double2* sm)
 {
     if (type == LP_T)
-        lp_trsm(a.A, a.ld, a.n, s, C, a.invD, sm);
+        lp_panel(a.A, a.ld, a.n, s, C, a.invD, a.linv, sm);
     else if (lp_split(s, R, C))
         lp_update<2, 2, 4, 2>(a.A, a.ld, a.n, s, 1, R, C, half, a.dw, sm);
     else
@@ -610,370 +587,386 @@ __device__ __forceinline__ void lp_publish(const LpArgs& a, long long ix, unsign
 }
 
 // ---------------------------------------------------------------------------
-// The chain CTA.  It keeps the working diagonal tile (s, s) in shared
-// memory (its diagonal as dw holds it) and per panel s runs the three tasks
-// the next diagonal tile waits for:
-//   D(s)          elimination of the tile by 8-row sub-panels (8 x 8 blocks
-//                 by the lanes of warp 0, the rows beyond them by
-//                 substitution, rank-8 updates on the FP64 tensor cores,
-//                 the next block's elimination beside the update);
-//                 published at once, so the other panel rows start;
-//   T(s, s+1)     the tile to its right, by the blocked recurrence of
-//                 lp_trsm with L read from the tile in shared memory;
-//   B(s, s+1, s+1) tile (s+1, s+1) loaded once the other CTAs have applied
-//                 panels 0..s-1, then panel s applied from the panel rows
-//                 still in shared memory; it stays there for step s+1.
+// The chain CTA: per panel s the three tasks the next diagonal tile waits
+// for.
+//   D(s)          elimination of [tile | identity], so that L_ss^-1 comes
+//                 with U_ss.  Each warp keeps one column of 8 x 8 tiles in
+//                 registers: the rows up to its own diagonal tile are W, the
+//                 ones below it the identity's column (zero at first), so
+//                 every warp always holds eight.  They are held transposed
+//                 (lane (g, t4): column g, rows 2 t4 and 2 t4 + 1 of a tile)
+//                 because a product's result is then the next product's
+//                 first operand without a move.  Per row tile b: the warp of
+//                 column b eliminates the 8 x 8 block with the identity
+//                 beside it (X_b = L_bb^-1); the others take Y_b = X_b W_b,
+//                 write U = invD Y_b or the row of L_ss^-1 out, and share U
+//                 through shared memory; then every warp updates its tiles
+//                 below with conj(U(b, a))^T Y_b, the warp of column b + 1
+//                 only its diagonal tile, which it eliminates beside the
+//                 others' products.  Two barriers a row tile.  Published at
+//                 once, so the other panel rows start;
+//   T(s, s+1)     the tile to its right, as lp_panel does it, kept in shared
+//                 memory;
+//   B(s, s+1, s+1) the old values of tile (s+1, s+1) once the other CTAs
+//                 have applied panels 0..s-1, then panel s, straight into
+//                 the registers step s+1 starts from.
 // The tile (s+1, s+2) that T(s+1, s+2) needs comes from the other CTAs
 // (T(s, s+2), then B(s, s+1, s+2)) while this CTA runs D(s+1).
-constexpr int LC_NP = 2080;  // packed upper triangle of a 64 x 64 tile
-__device__ __forceinline__ int lc_pu(int r, int c) { return r * 64 - r * (r - 1) / 2 + (c - r); }  // r <= c
-constexpr size_t LP_SMEM_C = (size_t)(LC_NP + LDL_NB * LT_WP + 2 * LDL_NB + 8 * 64) * sizeof(double2);
+constexpr int LC_UP = 57;  // pitch of the shared rows of U (columns 8..63): 1 mod 4, conflict-free
+constexpr int LC_XP = 9;   // pitch of X_b
+constexpr size_t LP_SMEM_C = (size_t)(LI_N + LDL_NB * LT_WP + 2 * LDL_NB + 8 * LC_UP + 8 * LC_XP) * sizeof(double2);
 constexpr size_t lp_max(size_t a, size_t b) { return a > b ? a : b; }
 constexpr size_t LP_SMEM = lp_max(LP_SMEM_B, lp_max(LP_SMEM_C, LP_SMEM_T));
+
+// 1/d of a normal d, without a branch: the hardware's seed y (about 20 bits)
+// and the geometric series of 1 / (1 - e), e = 1 - d y, to e^2 (remainder
+// below 2^-60), which rounds once.  It stands in a chain of 64 a tile: the
+// 8 x 8 elimination measures 862 cycles with it and 1428 with a reciprocal
+// that also covers what lies outside the normal range.
+__device__ __forceinline__ double lp_rcp(double d)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
 
 template <bool CPLX>
 __device__ void lp_chain(const LpArgs& a, double2* sm, int limit)
 {
-    double2* P = sm;                      // packed tile: U_ss during T, tile (s+1, s+1) during B
-    double2* Rt = sm + LC_NP;             // right tile, Rt[q * LT_WP + c] (during T and B)
-    double2* Ws = Rt;                     // working diagonal tile, Ws[r * LP_LD + c] (during D)
-    double2* dpv = Rt + LDL_NB * LT_WP;   // pivots d of the panel
+    double2* Li = sm;                     // L_ss^-1 by 8 x 8 blocks, for T
+    double2* Rt = sm + LI_N;              // right tile, Rt[q * LT_WP + c]
+    // pivots d of the panel: real ones in two buffers, so that the next
+    // panel's first block can be eliminated while B still reads them
+    double2* dpv = Rt + LDL_NB * LT_WP;
+    double* dpr = reinterpret_cast<double*>(dpv);
     double2* sinv = dpv + LDL_NB;         // their inverses (invD)
-    double2* Xb = sinv + LDL_NB;          // X_b = L_bb^-1, Xb[b * 64 + i * 8 + j]
-    __shared__ double2 sid[LP_SUB];
-    __shared__ int s_go, s_v;
+    double2* Us = sinv + LDL_NB;          // -conj(U(b, c)), c >= 8: Us[(row of tile b) * LC_UP + c - 8]
+    double2* Xs = Us + 8 * LC_UP;         // X_b(i, j) at Xs[i * LC_XP + j]
+    __shared__ int s_go, s_v, s_pre;
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const int g = lane >> 2, t4 = lane & 3;
+    // the column of tiles this warp holds: 9 tiles of B for each pair of
+    // warps that shares a scheduler
+    const int cw = wp < 4 ? wp : 11 - wp;
     const int n = a.n, ld = a.ld;
     cd* A = a.A;
-    // tile (0, 0) from global memory (upper triangle and dw)
-    for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
-        const int r = e & 63, c = e >> 6;
-        double2 v = make_double2(0.0, 0.0);
-        if (r <= c && c < min(LDL_NB, n)) v = (r < c) ? lp_ldcg(A + (size_t)r + (size_t)c * ld) : lp_ldcg(a.dw + r);
-        Ws[r * LP_LD + c] = v;
-    }
-    __syncthreads();
+    auto times = [](cd v, cd r) { return CPLX ? cmul(v, r) : cd{v.x * r.x, v.y * r.x}; };
+    double wr[8][2], wi[8][2];  // row tile b + i of the column: rows 2 t4 + e, column g
+    double yr[2], yi[2];        // Y_b of the column, the same way
+    bool apply = false;         // panel s - 1 is still to be applied to tile (s, s)
     for (int s = 0; s < a.np; s++) {
         const int p0 = s * LDL_NB, b = min(LDL_NB, n - p0);
         const bool right = s + 1 < a.np;
         const int cb = p0 + LDL_NB, wd = right ? min(LDL_NB, n - cb) : 0;
         unsigned long long t0 = 0;
         if (tid == 0 && a.trace) t0 = lp_clock();
+        // ================= the rest of B(s-1, s, s)
+        // the tile's values from global memory, the whole of the diagonal
+        // 8 x 8 tile, the identity beyond the last row, zeros below
+        {
+            const int c = 8 * cw + g;
+            const bool cin = c < b;
+            const cd* col = A + (size_t)(p0 + 2 * t4) + (size_t)(p0 + c) * ld;
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    double2 w = make_double2(0.0, 0.0);
+                    if (i < cw && cin) w = lp_ldcg(col + 8 * i + e);
+                    wr[i][e] = w.x;
+                    wi[i][e] = w.y;
+                }
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int r = 8 * cw + 2 * t4 + e;
+                double2 w = make_double2((r == c) ? 1.0 : 0.0, 0.0);
+                if (max(r, c) < b) {
+                    w = lp_ldcg(r == c ? a.dw + p0 + r : A + (size_t)(p0 + min(r, c)) + (size_t)(p0 + max(r, c)) * ld);
+                    if (r >= c) w.y = -w.y;  // dw keeps the conjugate of the upper-triangle value
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (i == cw) {
+                        wr[i][e] = w.x;
+                        wi[i][e] = w.y;
+                    }
+            }
+        }
+        if (apply) {
+            // W(a, cw)^T -= (d U(:, cw))^T conj(U(:, a)); columns beyond the
+            // last row are zero in the right tile
+#pragma unroll 1
+            for (int k0 = 0; k0 < LDL_NB; k0 += 8) {
+                const double2* row = Rt + (k0 + t4) * LT_WP + g;
+                double vr[2], vi[2];
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const double2 uc = row[4 * k * LT_WP + 8 * cw];
+                    const int q = k0 + 4 * k + t4;
+                    const double2 d = CPLX ? dpv[q] : make_double2(dpr[((s - 1) & 1) * LDL_NB + q], 0.0);
+                    vr[k] = CPLX ? -fma(uc.x, d.x, -uc.y * d.y) : -uc.x * d.x;
+                    vi[k] = CPLX ? -fma(uc.x, d.y, uc.y * d.x) : -uc.y * d.x;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (i <= cw) {
+#pragma unroll
+                        for (int k = 0; k < 2; k++) {
+                            const double2 u = row[4 * k * LT_WP + 8 * i];
+                            lp_mma(wr[i][0], wr[i][1], vr[k], u.x);
+                            lp_mma(wi[i][0], wi[i][1], vi[k], u.x);
+                            lp_mma(wr[i][0], wr[i][1], vi[k], u.y);
+                            lp_mma(wi[i][0], wi[i][1], vr[k], -u.y);
+                        }
+                    }
+            }
+        }
+        if (CPLX) __syncthreads();  // one buffer of pivots
+        if (tid == 0 && s > 0) {
+            lp_trace(a, lp_code(LP_B, s - 1, s, s), apply ? 1 : 0, t0, t0);
+            if (a.trace) t0 = lp_clock();
+        }
         // ================= D(s)
-        auto eliminate = [&](int s0) {  // warp 0: the 8 x 8 sub-block at s0
-            const int nq = min(LP_SUB, b - s0);
-            const int j = lane;
-            const bool col = j < nq;
-            cd x[LP_SUB];
-#pragma unroll
-            for (int i = 0; i < LP_SUB; i++) {
-                double2 v = make_double2(0.0, 0.0);
-                if (col && i <= j) v = Ws[(s0 + i) * LP_LD + s0 + j];
-                x[i] = cd{v.x, v.y};
+        // bk = -1: the first diagonal tile alone; then per row tile (one
+        // call site of the elimination keeps the code small)
+        // this warp's eight columns of the right tile
+        auto load_right = [&]() {
+#pragma unroll 4
+            for (int e = lane; e < 8 * LDL_NB; e += 32) {
+                const int q = e & 63, c = 8 * wp + (e >> 6);
+                const bool in = c < wd;
+                cp_async16(Rt + q * LT_WP + c,
+                           in ? (const void*)(A + (size_t)(p0 + q) + (size_t)(cb + c) * ld) : (const void*)A, in ? 16 : 0);
             }
-#pragma unroll
-            for (int q = 0; q < LP_SUB; q++) {
-                if (q < nq) {
-                    const cd dq = lp_shfl(x[q], q);
-                    const double dr = dq.x, di = CPLX ? dq.y : 0.0;
-                    const bool zero = (dr == 0.0 && di == 0.0);
-                    double id, idi = 0.0;
-                    if (CPLX) {
-                        const double m = zero ? 0.0 : __drcp_rn(fma(dr, dr, di * di));
-                        id = dr * m;
-                        idi = -di * m;
-                    } else {
-                        id = zero ? 0.0 : __drcp_rn(dr);
-                    }
-                    if (lane == 0) {
-                        sid[q] = make_double2(id, idi);
-                        dpv[s0 + q] = make_double2(dr, di);
-                        sinv[s0 + q] = make_double2(id, idi);
-                        a.invD[p0 + s0 + q] = cd{id, idi};
-                        a.dw[p0 + s0 + q] = cd{dr, di};
-                        if (zero) atomicCAS(a.status + ST_ZERO_PIVOT, 0, p0 + s0 + q + 1);
-                    }
-                    cd u = cd{0.0, 0.0};
-                    if (col && j > q) u = CPLX ? cmul(x[q], cd{id, idi}) : cd{x[q].x * id, x[q].y * id};
-#pragma unroll
-                    for (int i = q + 1; i < LP_SUB; i++) {
-                        const cd ui = lp_shfl(u, i);
-                        if (col && j >= i) x[i] = cfms(conj(ui), x[q], x[i]);
-                    }
-                    if (col && j > q) x[q] = u;
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < LP_SUB; i++)
-                if (col && i < j) Ws[(s0 + i) * LP_LD + s0 + j] = make_double2(x[i].x, x[i].y);
+            cp_async_commit();
         };
-        // s0 = -8: the first sub-block's elimination alone; then per
-        // sub-panel (b), (c) and the next elimination (one call site keeps
-        // the code small)
-        for (int s0 = -LP_SUB; s0 < b; s0 += LP_SUB) {
-            if (s0 < 0) {
-                if (wp == 0) eliminate(0);
+        // is tile (s, s+1) ready already?  Then its columns are fetched during D
+        if (tid == 128) s_pre = right && lp_ld_acquire(a.cnt + lp_tix(s, s + (right ? 1 : 0))) >= (unsigned)s;
+#pragma unroll 1
+        for (int bk = -1; bk < 8; bk++) {
+            if (bk < 0) {
+                // L_ss^-1 is zero above its diagonal blocks
+                cd* z = a.linv + (size_t)(p0 + (lane >> 3)) * LDL_NB + 8 * cw + (lane & 7);
+                for (int r = lane >> 3; r < min(8 * cw, b); r += 4, z += 4 * LDL_NB) *z = cd{0.0, 0.0};
+            }
+            // each warp at a step at which no other waits for it
+            if (bk == ((cw + 4) & 7) && s_pre) load_right();
+            if (bk >= 0) {
+                if (cw != bk) {
+                    double zr[2][2], zi[2][2];  // the two halves of the sum, chains of two products each
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const double2 x = Xs[g * LC_XP + 2 * t4 + e];
+                        zr[e][0] = zr[e][1] = zi[e][0] = zi[e][1] = 0.0;
+                        lp_mma(zr[e][0], zr[e][1], wr[0][e], x.x);
+                        lp_mma(zi[e][0], zi[e][1], wr[0][e], x.y);
+                        lp_mma(zr[e][0], zr[e][1], -wi[0][e], x.y);
+                        lp_mma(zi[e][0], zi[e][1], wi[0][e], x.x);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        yr[e] = zr[0][e] + zr[1][e];
+                        yi[e] = zi[0][e] + zi[1][e];
+                    }
+                    if (cw > bk) {
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const double2 id = sinv[8 * bk + 2 * t4 + e];
+                            const cd u = times(cd{yr[e], yi[e]}, cd{id.x, id.y});
+                            Us[(2 * t4 + e) * LC_UP + 8 * cw + g - 8] = make_double2(-u.x, u.y);
+                            if (8 * cw + g < b)
+                                A[(size_t)(p0 + 8 * bk + 2 * t4 + e) + (size_t)(p0 + 8 * cw + g) * ld] = u;
+                        }
+                    }
+                } else {
+                    // what the elimination of this block left, written out
+                    // while the other warps multiply
+                    const double2* ub = Li + li_blk(7, 7);
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int i = (lane >> 3) + 4 * h, j = lane & 7, r = 8 * bk + i;
+                        const double2 v = Xs[i * LC_XP + j], u = ub[8 * i + j];
+                        if (bk < 7) Li[li_blk(bk, bk) + li_el(i, j)] = v;
+                        if (r < b) {
+                            cd* row = a.linv + (size_t)(p0 + r) * LDL_NB + 8 * bk + j;
+                            *row = cd{v.x, v.y};
+                            if (i < j && 8 * bk + j < b) A[(size_t)(p0 + r) + (size_t)(p0 + 8 * bk + j) * ld] = cd{u.x, u.y};
+                        }
+                    }
+                    if (lane < 8 && 8 * bk + lane < b) {
+                        const int r = 8 * bk + lane;
+                        const double2 id = sinv[r], d = CPLX ? dpv[r] : make_double2(dpr[(s & 1) * LDL_NB + r], 0.0);
+                        a.invD[p0 + r] = cd{id.x, id.y};
+                        a.dw[p0 + r] = cd{d.x, d.y};
+                        if (d.x == 0.0 && d.y == 0.0) atomicCAS(a.status + ST_ZERO_PIVOT, 0, p0 + r + 1);
+                    }
+                }
                 __syncthreads();
-                continue;
-            }
-            const int nq = min(LP_SUB, b - s0);
-            const int t0c = s0 + LP_SUB;
-            if (t0c >= b) break;
-            // (b) sub-panel rows beyond the sub-block, one thread per column
-            if (tid < b - t0c) {
-                const int c = t0c + tid;
-                cd wun[LP_SUB];
+                if (bk == 7 && cw == 7) {  // its own block last: it kept U(7, 7)'s place
 #pragma unroll
-                for (int q = 0; q < LP_SUB; q++) {
-                    if (q < nq) {
-                        double2* wq = Ws + (s0 + q) * LP_LD + c;
-                        const double2 w = *wq;
-                        cd v = cd{w.x, w.y};
+                    for (int h = 0; h < 2; h++) {
+                        const int i = (lane >> 3) + 4 * h, j = lane & 7;
+                        Li[li_blk(7, 7) + li_el(i, j)] = Xs[i * LC_XP + j];
+                    }
+                }
+                if (cw < bk) {
 #pragma unroll
-                        for (int q2 = 0; q2 < q; q2++) {
-                            const double2 u = Ws[(s0 + q2) * LP_LD + s0 + q];  // U(q2, q)
-                            v = cfms(cd{u.x, -u.y}, wun[q2], v);
+                    for (int e = 0; e < 2; e++) {
+                        const int rr = 2 * t4 + e;
+                        Li[li_blk(bk, cw) + li_el(rr, g)] = make_double2(yr[e], yi[e]);
+                        if (8 * bk + rr < b)
+                            a.linv[(size_t)(p0 + 8 * bk + rr) * LDL_NB + 8 * cw + g] = cd{yr[e], yi[e]};
+                    }
+                }
+                if (bk < 7) {
+                    // W(a, cw) -= conj(U(b, a))^T Y_b, the tiles moving up one place
+                    const int lim = cw > bk ? cw - bk : 7 - bk;
+                    const double2* u0 = Us + 2 * t4 * LC_UP + 8 * bk - 8 + g;
+#pragma unroll
+                    for (int i = 1; i < 8; i++) {
+                        if (i <= lim) {
+#pragma unroll
+                            for (int e = 0; e < 2; e++) {
+                                const double2 v = u0[e * LC_UP + 8 * i];
+                                lp_mma(wr[i][0], wr[i][1], yr[e], v.x);
+                                lp_mma(wi[i][0], wi[i][1], yi[e], v.x);
+                                lp_mma(wr[i][0], wr[i][1], yi[e], -v.y);
+                                lp_mma(wi[i][0], wi[i][1], yr[e], v.y);
+                            }
                         }
-                        wun[q] = v;
-                        const double2 id = sid[q];
-                        const cd uq = CPLX ? cmul(v, cd{id.x, id.y}) : cd{v.x * id.x, v.y * id.x};
-                        *wq = make_double2(uq.x, uq.y);
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            wr[i - 1][e] = wr[i][e];
+                            wi[i - 1][e] = wi[i][e];
+                        }
+                    }
+                }
+            }
+            if (cw == bk + 1) {
+                // eliminate the 8 x 8 block with the identity beside it: lane
+                // (hf, c) holds the rows 2 k + hf of column c (0..7 the
+                // block's, 8..15 the identity's), the pivot row goes round
+                // through Xs; row i takes conj(W(q, i)) W(q, :) / d, whose
+                // product does not wait for the reciprocal
+                const int c = lane & 15, hf = lane >> 4;
+                const bool col = c < 8;
+#pragma unroll
+                for (int e = 0; e < 2; e++) Xs[(2 * t4 + e) * LC_XP + g] = make_double2(wr[0][e], wi[0][e]);
+                __syncwarp();
+                cd x[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    double2 v = make_double2((2 * k + hf + 8 == c) ? 1.0 : 0.0, 0.0);
+                    if (col) v = Xs[(2 * k + hf) * LC_XP + c];
+                    x[k] = cd{v.x, v.y};
+                }
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const int kq = q >> 1, hq = q & 1;
+                    const cd d = lp_shfl(x[kq], q + 16 * hq), xq = lp_shfl(x[kq], c + 16 * hq);
+                    if (q > 0) {
+                        __syncwarp();
+                        if (col && hf == hq) Xs[q * LC_XP + c] = make_double2(x[kq].x, x[kq].y);
+                        __syncwarp();
+                    }
+                    cd id;
+                    if (CPLX) {
+                        const double r = __drcp_rn(fma(d.x, d.x, d.y * d.y));
+                        id = cd{d.x * r, -d.y * r};
                     } else {
-                        wun[q] = cd{0.0, 0.0};
-                    }
-                }
-            }
-            __syncthreads();
-            // (c) rank-8 update of rows and columns [t0c, b), B operand
-            // d_q U(q, c); warp 0 takes the next diagonal sub-block and
-            // eliminates it at once
-            {
-                const int T = (b - t0c + 7) >> 3;
-                const int ntiles = T * (T + 1) / 2;
-                for (int tile = (wp == 0) ? 0 : wp; tile < ntiles; tile += (wp == 0) ? ntiles : 7) {
-                    int Rr = 0, rem = tile;
-                    while (rem >= T - Rr) {
-                        rem -= T - Rr;
-                        Rr++;
-                    }
-                    const int Cc = Rr + rem;
-                    const int r = t0c + 8 * Rr + g, cgc = t0c + 8 * Cc + g, ca = t0c + 8 * Cc + 2 * t4;
-                    double accr[2], acci[2];
-#pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const int c = ca + e;
-                        double2 w = make_double2(0.0, 0.0);
-                        if (r < b && c < b && r <= c) w = Ws[(r) * LP_LD + c];
-                        accr[e] = w.x;
-                        acci[e] = w.y;
+                        id = cd{lp_rcp(d.x), 0.0};
                     }
 #pragma unroll
-                    for (int k0 = 0; k0 < LP_SUB; k0 += 4) {
-                        const int q = k0 + t4;
-                        double2 u = make_double2(0.0, 0.0), v = make_double2(0.0, 0.0);
-                        if (q < nq && r < b) u = Ws[(s0 + q) * LP_LD + r];  // U(q, r)
-                        if (q < nq && cgc < b) {
-                            const double2 uc = Ws[(s0 + q) * LP_LD + cgc];  // U(q, c)
-                            const double2 d = dpv[s0 + q];
-                            v = make_double2(fma(uc.x, d.x, -uc.y * d.y), fma(uc.x, d.y, uc.y * d.x));
-                        }
-                        lp_mma(accr[0], accr[1], -u.x, v.x);
-                        lp_mma(accr[0], accr[1], -u.y, v.y);
-                        lp_mma(acci[0], acci[1], -u.x, v.y);
-                        lp_mma(acci[0], acci[1], u.y, v.x);
+                    for (int k = kq; k < 4; k++) {
+                        const double2 w = Xs[q * LC_XP + 2 * k + hf];
+                        const cd t = cmul(cd{w.x, -w.y}, xq);
+                        const cd v = CPLX ? cfms(conj(id), t, x[k]) : cd{fma(-id.x, t.x, x[k].x), fma(-id.x, t.y, x[k].y)};
+                        if (k > kq || hf > hq) x[k] = v;
                     }
+                    if (col && hf == hq) x[kq] = times(x[kq], id);  // U(q, c)
+                    if (lane == q + 16 * hq) {
+                        // an exactly zero pivot is reported; its 1/d stays 0
+                        const bool zero = d.x == 0.0 && (!CPLX || d.y == 0.0);
+                        if (CPLX)
+                            dpv[8 * cw + q] = make_double2(d.x, d.y);
+                        else
+                            dpr[(s & 1) * LDL_NB + 8 * cw + q] = d.x;
+                        sinv[8 * cw + q] = make_double2(zero ? 0.0 : id.x, zero ? 0.0 : id.y);
+                    }
+                }
+                __syncwarp();
+                {
+                    // X_b to its place; U(b, b) waits where the last block of
+                    // L_ss^-1 goes
+                    double2* out = col ? Li + li_blk(7, 7) + 8 * hf + c : Xs + hf * LC_XP + c - 8;
+                    const int step = col ? 16 : 2 * LC_XP;
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const int c = ca + e;
-                        if (r < b && c < b && r <= c) Ws[(r) * LP_LD + c] = make_double2(accr[e], acci[e]);
-                    }
+                    for (int k = 0; k < 4; k++) out[k * step] = make_double2(x[k].x, x[k].y);
                 }
-                if (wp == 0) {
-                    __syncwarp();
-                    eliminate(t0c);
+                __syncwarp();
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const double2 v = Xs[(2 * t4 + e) * LC_XP + g];
+                    yr[e] = v.x;
+                    yi[e] = v.y;
                 }
+                // the column turns into the identity's: nothing below it yet
+#pragma unroll
+                for (int i = 0; i < 8; i++) wr[i][0] = wr[i][1] = wi[i][0] = wi[i][1] = 0.0;
             }
             __syncthreads();
         }
-        // U_ss out, and packed for T (the right tile overwrites Ws)
-        for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
-            const int r = e & 63, c = e >> 6;
-            if (r < c) {
-                const double2 v = Ws[r * LP_LD + c];
-                P[lc_pu(r, c)] = v;
-                if (c < b) A[(size_t)(p0 + r) + (size_t)(p0 + c) * ld] = cd{v.x, v.y};
-            }
-        }
-        __syncthreads();
         lp_publish(a, lp_tix(s, s), (unsigned)s + 1);
         if (tid == 0) lp_trace(a, lp_code(LP_D, s, s, s), 1, t0, t0);
         if (!right) break;
         // ================= T(s, s+1)
         if (tid == 0) {
             if (a.trace) t0 = lp_clock();
+            s_go = 1;
             long long ix[3] = {lp_tix(s, s + 1), 0, 0};
             unsigned need[3] = {(unsigned)s, 0u, 0u};
-            s_go = lp_wait_all(a, ix, need, 1, limit) ? 1 : 0;
+            if (!s_pre) s_go = lp_wait_all(a, ix, need, 1, limit);
         }
         __syncthreads();
         if (!s_go) return;
         unsigned long long t1 = 0;
         if (tid == 0 && a.trace) t1 = lp_clock();
-        for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
-            const int q = e & 63, c = e >> 6;
-            const bool in = c < wd;
-            cp_async16(Rt + q * LT_WP + c, in ? (const void*)(A + (size_t)(p0 + q) + (size_t)(cb + c) * ld) : (const void*)A,
-                       in ? 16 : 0);
-        }
-        cp_async_commit();
-        {
-            // X_wp = L_bb^-1 of block bb = wp, L(r, q) = conj(U(q, r)); lane j < 8 holds column j
-            const int bb = wp, j = lane;
-            cd x[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) x[i] = cd{(i == j) ? 1.0 : 0.0, 0.0};
-#pragma unroll
-            for (int q = 0; q < 8; q++)
-#pragma unroll
-                for (int r = q + 1; r < 8; r++) {
-                    const double2 u = P[lc_pu(8 * bb + q, 8 * bb + r)];
-                    x[r] = cfms(cd{u.x, -u.y}, x[q], x[r]);
-                }
-            if (j < 8)
-#pragma unroll
-                for (int i = 0; i < 8; i++) Xb[bb * 64 + i * 8 + j] = make_double2(x[i].x, x[i].y);
-        }
+        if (!s_pre) load_right();
         cp_async_wait<0>();
-        __syncthreads();
+        __syncwarp();  // a warp multiplies the columns it has loaded
         {
+            // each warp reads and rewrites its own eight columns of the right tile
             const int c0 = 8 * wp;
-#pragma unroll 1
-            for (int bk = 0; bk < 8; bk++) {
-                double wr[2] = {0.0, 0.0}, wi[2] = {0.0, 0.0};
+            lp_linv_product(Li, Rt, c0, g, t4, wr, wi);
+            __syncwarp();
 #pragma unroll
-                for (int k0 = 0; k0 < 8; k0 += 4) {
-                    const double2 xa = Xb[bk * 64 + g * 8 + k0 + t4];
-                    const double2 wv = Rt[(8 * bk + k0 + t4) * LT_WP + c0 + g];
-                    lp_mma(wr[0], wr[1], xa.x, wv.x);
-                    lp_mma(wr[0], wr[1], -xa.y, wv.y);
-                    lp_mma(wi[0], wi[1], xa.x, wv.y);
-                    lp_mma(wi[0], wi[1], xa.y, wv.x);
+            for (int m = 0; m < 8; m++) {
+                const double2 d = sinv[8 * m + g];
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int c = c0 + 2 * t4 + e;
+                    const cd u = times(cd{wr[m][e], wi[m][e]}, cd{d.x, d.y});
+                    Rt[(8 * m + g) * LT_WP + c] = make_double2(u.x, u.y);
+                    if (c < wd) A[(size_t)(p0 + 8 * m + g) + (size_t)(cb + c) * ld] = u;
                 }
-                __syncwarp();
-#pragma unroll
-                for (int e = 0; e < 2; e++) Rt[(8 * bk + g) * LT_WP + c0 + 2 * t4 + e] = make_double2(wr[e], wi[e]);
-                __syncwarp();
-                double2 un[2];
-#pragma unroll
-                for (int k0 = 0; k0 < 8; k0 += 4) un[k0 / 4] = Rt[(8 * bk + k0 + t4) * LT_WP + c0 + g];
-#pragma unroll 1
-                for (int a2 = bk + 1; a2 < 8; a2++) {
-                    double ar[2], ai[2];
-#pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const double2 o = Rt[(8 * a2 + g) * LT_WP + c0 + 2 * t4 + e];
-                        ar[e] = o.x;
-                        ai[e] = o.y;
-                    }
-#pragma unroll
-                    for (int k0 = 0; k0 < 8; k0 += 4) {
-                        const double2 uu = P[lc_pu(8 * bk + k0 + t4, 8 * a2 + g)];  // U(k, r): L(r, k) = conj
-                        const double2 u = un[k0 / 4];
-                        lp_mma(ar[0], ar[1], -uu.x, u.x);
-                        lp_mma(ar[0], ar[1], -uu.y, u.y);
-                        lp_mma(ai[0], ai[1], -uu.x, u.y);
-                        lp_mma(ai[0], ai[1], uu.y, u.x);
-                    }
-#pragma unroll
-                    for (int e = 0; e < 2; e++) Rt[(8 * a2 + g) * LT_WP + c0 + 2 * t4 + e] = make_double2(ar[e], ai[e]);
-                }
-                __syncwarp();
             }
-        }
-        __syncthreads();
-        // U(s, s+1) = invD Wun: kept in shared memory and written out
-        for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
-            const int q = e & 63, c = e >> 6;
-            const double2 v = Rt[q * LT_WP + c], d = sinv[q];
-            const cd u = cmul(cd{v.x, v.y}, cd{d.x, d.y});
-            Rt[q * LT_WP + c] = make_double2(u.x, u.y);
-            if (c < wd) A[(size_t)(p0 + q) + (size_t)(cb + c) * ld] = u;
         }
         __syncthreads();
         lp_publish(a, lp_tix(s, s + 1), (unsigned)s + 1);
         if (tid == 0) lp_trace(a, lp_code(LP_T, s, s, s + 1), 1, t0, t1);
-        // ================= B(s, s+1, s+1)
+        // ================= B(s, s+1, s+1): the wait; the products follow at
+        // the top of the next step
         if (tid == 0) {
-            if (a.trace) t0 = lp_clock();
             long long ix[3] = {lp_tix(s + 1, s + 1), 0, 0};
             unsigned need[3] = {(unsigned)s, 0u, 0u};
-            const int go = lp_wait_all(a, ix, need, 1, limit) ? 1 : 0;
+            const int go = lp_wait_all(a, ix, need, 1, limit);
             s_go = go;
             s_v = go ? (int)lp_ld_acquire(a.cnt + ix[0]) : 0;
-            if (a.trace) t1 = lp_clock();
         }
         __syncthreads();
         if (!s_go) return;
-        const int applied = s_v;  // panels already applied to tile (s+1, s+1)
-        const int q0 = p0 + LDL_NB, bn = min(LDL_NB, n - q0);
-        for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
-            const int r = e & 63, c = e >> 6;
-            if (r > c) continue;
-            double2 v = make_double2(0.0, 0.0);
-            if (c < bn) v = (r < c) ? lp_ldcg(A + (size_t)(q0 + r) + (size_t)(q0 + c) * ld) : lp_ldcg(a.dw + q0 + r);
-            P[lc_pu(r, c)] = v;
-        }
-        __syncthreads();
-        if (applied == s) {
-            // 8 x 8 tiles of the upper triangle; A = conj(U(q, r)), B = -(d_q U(q, c))
-            for (int tile = wp; tile < 36; tile += 8) {
-                int Rr = 0, rem = tile;
-                while (rem >= 8 - Rr) {
-                    rem -= 8 - Rr;
-                    Rr++;
-                }
-                const int Cc = Rr + rem;
-                const int r = 8 * Rr + g, cgc = 8 * Cc + g, ca = 8 * Cc + 2 * t4;
-                double accr[2], acci[2];
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int c = ca + e;
-                    double2 w = make_double2(0.0, 0.0);
-                    if (r <= c && c < bn) {
-                        w = P[lc_pu(r, c)];
-                        if (r == c) w.y = -w.y;  // dw keeps the conjugate of the upper-triangle value
-                    }
-                    accr[e] = w.x;
-                    acci[e] = w.y;
-                }
-#pragma unroll 2
-                for (int k0 = 0; k0 < LDL_NB; k0 += 4) {
-                    const int q = k0 + t4;
-                    const double2 u = Rt[q * LT_WP + r];
-                    const double2 uc = Rt[q * LT_WP + cgc];
-                    const double2 d = dpv[q];
-                    const double vr = -fma(uc.x, d.x, -uc.y * d.y), vi = -fma(uc.x, d.y, uc.y * d.x);
-                    lp_mma(accr[0], accr[1], u.x, vr);
-                    lp_mma(accr[0], accr[1], u.y, vi);
-                    lp_mma(acci[0], acci[1], u.x, vi);
-                    lp_mma(acci[0], acci[1], -u.y, vr);
-                }
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int c = ca + e;
-                    if (r <= c && c < bn) P[lc_pu(r, c)] = (r == c) ? make_double2(accr[e], -acci[e]) : make_double2(accr[e], acci[e]);
-                }
-            }
-        }
-        __syncthreads();
-        // the next diagonal tile into Ws (the right tile is no longer needed)
-        for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
-            const int r = e & 63, c = e >> 6;
-            Ws[r * LP_LD + c] = (r <= c) ? P[lc_pu(r, c)] : make_double2(0.0, 0.0);
-        }
-        __syncthreads();
-        if (tid == 0) lp_trace(a, lp_code(LP_B, s, s + 1, s + 1), applied == s ? 1 : 0, t0, t1);
+        apply = s_v == s;  // panels already applied to tile (s+1, s+1)
     }
 }
 
@@ -1040,11 +1033,12 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(LpArgs a)
                 long long ix[3] = {0, 0, 0};
                 unsigned need[3] = {0u, 0u, 0u};
                 const int k = lp_deps(task, ix, need);
-                go = lp_wait_all(a, ix, need, k, limit) ? 1 : 0;
-                if (go && type == LP_B) {
+                const bool whole = type == LP_B && !lp_split(s, R, C);
+                go = lp_wait_all(a, ix, need, k, limit, whole);
+                if (go == 1 && type == LP_B) {
                     if (lp_ld_acquire(a.cnt + ix[0]) > (unsigned)s) {
                         go = 2;  // applied already by a merged update
-                    } else if (!lp_split(s, R, C)) {
+                    } else if (whole) {
                         // following panels whose rows of R and C are final
                         unsigned fr[LP_MERGE - 1], fc[LP_MERGE - 1];
 #pragma unroll
@@ -1064,6 +1058,7 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(LpArgs a)
                             if (m == j && !own && s + j < R && fr[j - 1] >= want && (R == C || fc[j - 1] >= want))
                                 m = j + 1;
                         }
+                        if (m > 1) *((volatile unsigned*)(a.cl + ix[0])) = (unsigned)(s + m);
                     }
                 }
                 if (!go) task = LP_NONE;
@@ -1170,7 +1165,7 @@ long long ldlp_task_total(int n)
 // records, the chain CTA's SM) for np panels.
 int ldlp_reserve(Ctx& c, int np)
 {
-    const size_t need = (size_t)np * (np + 1) + 4;
+    const size_t need = (size_t)np * (np + 1) / 2 * 3 + 4;
     if (c.lp_cap >= need) return 0;
     if (c.lp_cnt) cudaFree(c.lp_cnt);
     c.lp_cnt = nullptr;
@@ -1190,7 +1185,7 @@ void ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned lon
 {
     const int np = (n + LDL_NB - 1) / LDL_NB;
     const size_t ntile = (size_t)np * (np + 1) / 2;
-    cudaMemsetAsync(c.lp_cnt, 0, (2 * ntile + 4) * sizeof(unsigned), c.stream);
+    cudaMemsetAsync(c.lp_cnt, 0, (3 * ntile + 4) * sizeof(unsigned), c.stream);
     LpArgs a;
     a.A = c.F;
     a.ld = c.ld;
@@ -1201,8 +1196,10 @@ void ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned lon
     a.cnt = c.lp_cnt;
     a.hc = c.lp_cnt + ntile;
     a.ctl = c.lp_cnt + 2 * ntile;
+    a.cl = c.lp_cnt + 2 * ntile + 4;
     a.dw = c.dw;
     a.invD = c.invD;
+    a.linv = c.linv;
     a.status = c.status;
     a.limitp = c.counters + 3;
     a.trace = trace;
