@@ -65,7 +65,7 @@ void free_ctx(Ctx& c)
     if (c.gcnt_h) cudaFreeHost(c.gcnt_h);
     void* ptrs[] = {c.gcnt, c.params, c.H, c.S, c.diagS, c.diagH, c.invD, c.c, c.x, c.w, c.D, c.grad, c.Pd, c.coef,
                     c.bra, c.ket, c.ketn, c.pcode, c.detL, c.part, c.dw, c.linv, c.lmf, c.lnb, c.vbuf, c.status, c.red, c.counters, c.yv,
-                    c.zv, c.spart, c.colval, c.dblk, c.flags};
+                    c.zv, c.xw, c.spart, c.colval, c.dblk};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (auto& g : c.ldl_graphs) {
@@ -532,7 +532,7 @@ int ecg_ctx_create(int n, const double* mass_matrix_host, const double* charges_
     r |= dalloc(&c.spart, (size_t)SOLVE_G_MAX * LDL_NB);
     r |= dalloc(&c.colval, 2 * L);
     r |= dalloc(&c.dblk, L + 2);
-    r |= dalloc(&c.flags, L + 2);
+    r |= dalloc(&c.xw, L);
     if (!r) {
         if (cudaMallocHost((void**)&c.status_h, ST_COUNT * sizeof(int)) != cudaSuccess ||
             cudaMallocHost((void**)&c.bounds_h, (L + 2) * sizeof(int)) != cudaSuccess ||
@@ -553,7 +553,6 @@ int ecg_ctx_create(int n, const double* mass_matrix_host, const double* charges_
               cudaMemset(c.S, 0, L * L * sizeof(cd)) == cudaSuccess &&
               cudaMemset(c.counters, 0, 4 * sizeof(int)) == cudaSuccess &&
               cudaMemcpy(c.counters + 3, &c.wait_limit, sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-              cudaMemset(c.flags, 0, (L + 2) * sizeof(unsigned)) == cudaSuccess &&
               cudaMemset(c.status, 0, ST_COUNT * sizeof(int)) == cudaSuccess &&
               cudaMemset(c.c, 0, L * sizeof(cd)) == cudaSuccess && cudaMemset(c.x, 0, L * sizeof(cd)) == cudaSuccess;
     if (!ok) {

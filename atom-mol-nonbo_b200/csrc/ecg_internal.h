@@ -161,8 +161,7 @@ struct Ctx {
     cd* spart = nullptr;        // per-CTA partial sums of the blocked solves
     double* colval = nullptr;   // per-column values of the quadratic forms (2 ld)
     int* dblk = nullptr;        // device copy of blk_start + end (ld + 2 ints)
-    unsigned* flags = nullptr;  // per-panel ready flags of the cooperative solves (ld + 2)
-    unsigned epoch = 0;         // value a panel flag takes when its panel is solved
+    cd* xw = nullptr;           // backward-solve result before its normalisation into x (ld)
     int coop_max_blocks = 0;    // co-resident CTAs of the cooperative solve kernels
     int coop_max_neigh = 0;     // the same with the neighbour products in shared memory
     std::vector<int> blk_start; // block starts of the current LDL^H factor

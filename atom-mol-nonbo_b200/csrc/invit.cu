@@ -13,6 +13,7 @@
 // block, so results are deterministic run to run.
 #include <algorithm>
 #include "ecg_internal.h"
+#include "warp_sums.cuh"
 
 namespace ecg {
 
@@ -38,9 +39,16 @@ __device__ __forceinline__ cd warp_sum(cd s)
     return s;
 }
 
+// The value that stands for "not computed yet" in the vectors the cooperative
+// solves pass between CTAs: a quiet NaN with a payload no arithmetic makes
+// (hardware NaNs are 0x7fff...).
+constexpr unsigned long long UNSET = 0xfff8c0de5eedfaceULL;
+__device__ __forceinline__ cd unset() { return cd{__longlong_as_double(UNSET), __longlong_as_double(UNSET)}; }
+
 // w(i) = sum_j conj(B(j,i)) v(j); one warp per column, four accumulators.
+// The solves' vectors y and x are marked as not computed on the way.
 __global__ void __launch_bounds__(256) k_hemv(const cd* __restrict__ B, int ld, int n, const cd* __restrict__ v,
-                                              cd* __restrict__ w)
+                                              cd* __restrict__ w, cd* __restrict__ y, cd* __restrict__ x)
 {
     const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -57,7 +65,11 @@ __global__ void __launch_bounds__(256) k_hemv(const cd* __restrict__ B, int ld, 
     }
     for (; j < n; j += 32) s0 = cfma(conj(ld2(b + j)), ld2(v + j), s0);
     const cd s = warp_sum((s0 + s1) + (s2 + s3));
-    if (lane == 0) w[col] = s;
+    if (lane == 0) {
+        w[col] = s;
+        y[col] = unset();
+        x[col] = unset();
+    }
 }
 
 // Forward solve of panel [j0, j1): y = Linv (w - U(0:j0, p)^H y(0:j0)),
@@ -150,61 +162,56 @@ __global__ void __launch_bounds__(256) k_bwd(const cd* __restrict__ A, int ld, i
 // ---------------------------------------------------------------------------
 // Cooperative triangular solves: one CTA per LDL^H panel, all CTAs
 // co-resident (cooperative launch).  CTA j accumulates the contributions of
-// the panels it depends on in panel order, each as soon as that panel's
-// flag carries the current epoch (acquire / release), then applies its
-// inverse diagonal block and publishes its own panel.  The neighbouring
-// panel (j-1 forward, j+1 backward) is left out of that sum: its term is
-// applied after the inverse block as one 64 x 64 product with the
-// precomputed M_j = Linv_j U(j-1, j)^H or N_j = Linv_j^H U(j, j+1)
-// (k_ldl_mn), so the step from one panel's flag to the next is that
-// product alone.  Every wait is
-// bounded: after SOLVE_SPIN_LIMIT polls, or as soon as any CTA has given
-// up (the abort word), the CTA records ST_SOLVE_TIMEOUT and finishes
-// without waiting; the host then reports the step as failed.
+// the panels it depends on in panel order, then applies its inverse diagonal
+// block and publishes its own panel.  The neighbouring panel (j-1 forward,
+// j+1 backward) is left out of that sum: its term is applied after the
+// inverse block as one 64 x 64 product with the precomputed M_j = Linv_j
+// U(j-1, j)^H or N_j = Linv_j^H U(j, j+1) (k_ldl_mn), so the step from one
+// panel to the next is that product alone.
+// The values are their own signal: the vector holds UNSET until a panel's
+// CTA stores its 64 values, and a reader polls the values themselves (each
+// 64-bit word is stored whole, and nothing else is read through them), so a
+// step is a store and a load that sees it.  A flag beside the data costs a
+// barrier, a release, the poll of the flag and then the load of the data:
+// 2.3 us a step at K = 2000..4000 against 1.2 us.  Every wait is bounded:
+// after SOLVE_SPIN_LIMIT polls, or as soon as any CTA has given up (the
+// abort word), the CTA records ST_SOLVE_TIMEOUT and finishes without
+// waiting; the host then reports the step as failed.
 static_assert(SOLVE_SPIN_LIMIT == (1 << 22), "the default poll limit of the solves' waits");
-constexpr int LS_LD = LDL_NB + 1;
+// pitch of the 64 x 64 blocks in shared memory: 4 mod 8 double2, so that two
+// rows' four columns fall on different banks
+constexpr int LS_LD = LDL_NB + 4;
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
+// The computed value at *p; ok turns false when this thread gives up: after
+// `limit` polls (abort_word[1]: SOLVE_SPIN_LIMIT unless a caller set another
+// through ecg_set_wait_limit), or when the abort word is set, which is looked
+// at every 64th poll (its load would otherwise stand between the polls).
+__device__ __forceinline__ double2 wait_value(const cd* p, int* status, int* abort_word, int limit, bool& ok)
 {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Wait (thread 0) for flags[a] == epoch; returns false if this CTA must stop.
-// abort_word[1] holds the poll limit (SOLVE_SPIN_LIMIT unless a caller set
-// another through ecg_set_wait_limit).
-__device__ __forceinline__ bool wait_panel(const unsigned* flags, int a, unsigned epoch, int* status, int* abort_word,
-                                           bool& ok)
-{
-    __shared__ int go;
-    if (threadIdx.x == 0) {
-        int g = 1;
-        if (ok) {
-            int spins = 0;
-            const int limit = ((volatile int*)abort_word)[1];
-            while (ld_acquire(flags + a) != epoch) {
-                if (++spins > limit || *((volatile int*)abort_word) != 0) {
-                    g = 0;
-                    break;
-                }
-            }
-            if (!g) {
-                atomicExch(status + ST_SOLVE_TIMEOUT, 1);
-                atomicExch(abort_word, 1);
-            }
-        } else {
-            g = 0;
+    unsigned long long a, b;
+    int spins = 0;
+    for (;;) {
+        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+        if ((a != UNSET && b != UNSET) || !ok) break;
+        ++spins;
+        if (spins > limit || ((spins & 63) == 0 && *((volatile int*)abort_word) != 0)) {
+            atomicExch(status + ST_SOLVE_TIMEOUT, 1);
+            atomicExch(abort_word, 1);
+            ok = false;
         }
-        go = g;
     }
-    __syncthreads();
-    ok = ok && go;
-    return ok;
+    return make_double2(__longlong_as_double((long long)a), __longlong_as_double((long long)b));
+}
+
+// Threads 0..63: the n <= 64 values at p into sv (zeros beyond), as they are
+// computed; every thread returns whether they all were.
+__device__ __forceinline__ bool wait_panel(const cd* p, int n, double2* sv, int* status, int* abort_word, int limit)
+{
+    bool ok = true;
+    if (threadIdx.x < LDL_NB)
+        sv[threadIdx.x] = (int)threadIdx.x < n ? wait_value(p + threadIdx.x, status, abort_word, limit, ok)
+                                               : make_double2(0.0, 0.0);
+    return __syncthreads_and(ok ? 1 : 0) != 0;
 }
 
 // Rows [j0, j0 + b) of a per-panel 64-column block (linv, lmf, lnb) into
@@ -223,42 +230,82 @@ __device__ __forceinline__ void load_linv(const cd* __restrict__ linv, int j0, i
     }
 }
 
+// Row r = tid / 4 of the product of a 64 x 64 block in shared memory with
+// the vector v: columns tid % 4, + 4, ..., summed over the four lanes, which
+// all return it.
+__device__ __forceinline__ cd row_product(const double2* __restrict__ B, const double2* __restrict__ v)
+{
+    const int r = threadIdx.x >> 2, q0 = threadIdx.x & 3;
+    cd s0 = mk(0.0, 0.0), s1 = s0;
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+        const double2 a = B[r * LS_LD + q0 + 4 * i], x = v[q0 + 4 * i];
+        const double2 b = B[r * LS_LD + q0 + 4 * i + 4], y = v[q0 + 4 * i + 4];
+        s0 = cfma(mk(a.x, a.y), mk(x.x, x.y), s0);
+        s1 = cfma(mk(b.x, b.y), mk(y.x, y.y), s1);
+    }
+    cd s = s0 + s1;
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    return s;
+}
+// The same for the conjugate transpose of the block.
+__device__ __forceinline__ cd row_product_h(const double2* __restrict__ B, const double2* __restrict__ v)
+{
+    const int r = threadIdx.x >> 2, q0 = threadIdx.x & 3;
+    cd s = mk(0.0, 0.0);
+#pragma unroll 4
+    for (int i = 0; i < 16; i++) {
+        const double2 a = B[(q0 + 4 * i) * LS_LD + r], x = v[q0 + 4 * i];
+        s = cfma(mk(a.x, -a.y), mk(x.x, x.y), s);
+    }
+#pragma unroll
+    for (int o = 1; o <= 2; o <<= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+    }
+    return s;
+}
+
 // Forward: y_j = Linv_j (w_j - sum_{a<j} U(a, j)^H y_a), z_j = invD_j y_j.
 template <bool NEIGH>
-__global__ void __launch_bounds__(256) k_fwd_coop(const cd* __restrict__ A, int ld, const int* __restrict__ bstart,
+__global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_fwd_coop(const cd* __restrict__ A, int ld, const int* __restrict__ bstart,
                                                   int nb, const cd* __restrict__ w, cd* __restrict__ y,
                                                   cd* __restrict__ z, const cd* __restrict__ invD,
                                                   const cd* __restrict__ linv, const cd* __restrict__ lmf,
-                                                  unsigned* __restrict__ flags, unsigned epoch,
                                                   int* __restrict__ status, int* abort_word)
 {
     extern __shared__ double2 sm[];
     double2* Ls = sm;                          // Linv_j, [r][q]
-    double2* red = sm + LDL_NB * LS_LD;        // [8][64] warp partials, then [4][64]
-    double2* Ms = red + 8 * LDL_NB;            // NEIGH: M_j, [r][q]
-    __shared__ double2 t[LDL_NB];
+    double2* Ms = sm + LDL_NB * LS_LD;         // NEIGH: M_j, [r][q]
+    __shared__ double2 t[LDL_NB], ys[2][LDL_NB];
     const int j = blockIdx.x;
     const int j0 = bstart[j], j1 = bstart[j + 1], b = j1 - j0;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     load_linv(linv, j0, b, Ls);
     if (NEIGH && j > 0) load_linv(lmf, j0, b, Ms, j0 - bstart[j - 1]);
     // this panel's right-hand side and pivots, read before the waits
+    const int r = threadIdx.x >> 2;
     const cd wj = (threadIdx.x < b) ? ld2(w + j0 + threadIdx.x) : mk(0.0, 0.0);
-    const cd dj = (threadIdx.x < b) ? ld2(invD + j0 + threadIdx.x) : mk(0.0, 0.0);
+    const cd dj = (r < b) ? ld2(invD + j0 + r) : mk(0.0, 0.0);
     // lane-partials for the 8 columns this warp owns
     cd acc[8];
 #pragma unroll
     for (int m = 0; m < 8; m++) acc[m] = mk(0.0, 0.0);
     bool ok = true;
+    const int limit = ((volatile int*)abort_word)[1];
     // every panel but the previous one; that one comes in below through
     // M_j = Linv_j U(j-1, j)^H
     const int alast = NEIGH ? j - 1 : j;
-    for (int a = 0; a < alast; a++) {
+    // the factor block U(panel a, panel j) does not depend on panel a's
+    // solution: it is loaded before the wait for that, with NEIGH (registers
+    // of one CTA an SM) while the panel before it is still waited for
+    auto load_u = [&](int a, cd (&u0)[8], cd (&u1)[8]) {
         const int a0 = bstart[a], a1 = bstart[a + 1];
         const int r0 = a0 + lane, r1 = a0 + lane + 32;
-        // the factor block U(panel a, panel j) does not depend on panel a's
-        // solution: load it before waiting for that panel's flag
-        cd u0[8], u1[8];
 #pragma unroll
         for (int m = 0; m < 8; m++) {
             const int c = wp * 8 + m;
@@ -266,110 +313,87 @@ __global__ void __launch_bounds__(256) k_fwd_coop(const cd* __restrict__ A, int 
             u0[m] = (c < b && r0 < a1) ? ld2(col + r0) : mk(0.0, 0.0);
             u1[m] = (c < b && r1 < a1) ? ld2(col + r1) : mk(0.0, 0.0);
         }
-        if (!wait_panel(flags, a, epoch, status, abort_word, ok)) break;
-        const cd y0 = (r0 < a1) ? ldcg2(y + r0) : mk(0.0, 0.0);
-        const cd y1 = (r1 < a1) ? ldcg2(y + r1) : mk(0.0, 0.0);
+    };
+    auto apply = [&](int a, const cd (&u0)[8], const cd (&u1)[8]) {
+        double2* sv = ys[a & 1];  // the other buffer may still be read
+        ok = wait_panel(y + bstart[a], bstart[a + 1] - bstart[a], sv, status, abort_word, limit);
+        const cd y0 = mk(sv[lane].x, sv[lane].y), y1 = mk(sv[lane + 32].x, sv[lane + 32].y);
 #pragma unroll
         for (int m = 0; m < 8; m++) {
             acc[m] = cfma(conj(u0[m]), y0, acc[m]);
             acc[m] = cfma(conj(u1[m]), y1, acc[m]);
         }
+    };
+    cd ua[8], va[8];
+    if (NEIGH) {
+        cd ub[8], vb[8];
+        if (alast > 0) load_u(0, ua, va);
+        for (int a = 0; a < alast && ok; a += 2) {
+            if (a + 1 < alast) load_u(a + 1, ub, vb);
+            apply(a, ua, va);
+            if (a + 1 < alast && ok) {
+                if (a + 2 < alast) load_u(a + 2, ua, va);
+                apply(a + 1, ub, vb);
+            }
+        }
+    } else {
+        for (int a = 0; a < alast && ok; a++) {
+            load_u(a, ua, va);
+            apply(a, ua, va);
+        }
     }
-#pragma unroll
-    for (int m = 0; m < 8; m++) acc[m] = warp_sum(acc[m]);
-    if (lane == 0)
+    {
+        double v[16];
 #pragma unroll
         for (int m = 0; m < 8; m++) {
-            const int c = wp * 8 + m;
-            if (c < b) t[c] = make_double2(0.0, 0.0), red[c] = make_double2(acc[m].x, acc[m].y);
+            v[2 * m] = acc[m].x;
+            v[2 * m + 1] = acc[m].y;
         }
-    __syncthreads();
-    if (threadIdx.x < b) {
-        const cd s = mk(red[threadIdx.x].x, red[threadIdx.x].y);
-        const cd v = wj - s;
-        t[threadIdx.x] = make_double2(v.x, v.y);
+        const double sum = warp_transpose_sum<16>(v);
+        if ((lane & 1) == 0) reinterpret_cast<double*>(t)[16 * wp + (lane >> 1)] = sum;
     }
     __syncthreads();
-    // y = Ls t: row r = tid & 63, four interleaved partial sums over q
-    {
-        const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
-        cd s = mk(0.0, 0.0);
-        if (r < b)
-            for (int q = g; q <= r; q += 4) {
-                const double2 l = Ls[r * LS_LD + q], tq = t[q];
-                s = cfma(mk(l.x, l.y), mk(tq.x, tq.y), s);
-            }
-        red[g * LDL_NB + r] = make_double2(s.x, s.y);
-    }
+    if (threadIdx.x < LDL_NB) t[threadIdx.x] = make_double2(wj.x - t[threadIdx.x].x, wj.y - t[threadIdx.x].y);
     __syncthreads();
-    cd ys = mk(0.0, 0.0);
-    if (threadIdx.x < b) {
-        const int r = threadIdx.x;
-#pragma unroll
-        for (int g = 0; g < 4; g++) ys = ys + mk(red[g * LDL_NB + r].x, red[g * LDL_NB + r].y);
-    }
+    cd yr = row_product(Ls, t);
     if (NEIGH && j > 0) {
-        // y_j -= M_j y_{j-1}: row r = tid & 63, columns g, g + 4, ...
-        const int a0 = bstart[j - 1], bp = j0 - a0;
-        const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
-        // (the barrier inside also orders the reads of red above before the writes below)
-        if (wait_panel(flags, j - 1, epoch, status, abort_word, ok)) {
-            cd s = mk(0.0, 0.0);
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const int q = g + 4 * i;
-                if (q < bp) {
-                    const double2 m = Ms[r * LS_LD + q];
-                    s = cfma(mk(m.x, m.y), ldcg2(y + a0 + q), s);
-                }
-            }
-            red[g * LDL_NB + r] = make_double2(s.x, s.y);
-        }
-        __syncthreads();
-        if (ok && threadIdx.x < b) {
-            const int rr = threadIdx.x;
-#pragma unroll
-            for (int g2 = 0; g2 < 4; g2++) ys = ys - mk(red[g2 * LDL_NB + rr].x, red[g2 * LDL_NB + rr].y);
-        }
+        // y_j -= M_j y_{j-1}
+        double2* sv = ys[(j - 1) & 1];
+        if (ok && wait_panel(y + bstart[j - 1], j0 - bstart[j - 1], sv, status, abort_word, limit)) yr = yr - row_product(Ms, sv);
     }
-    if (threadIdx.x < b) {
-        y[j0 + threadIdx.x] = ys;
-        z[j0 + threadIdx.x] = cmul(ys, dj);
+    if ((threadIdx.x & 3) == 0 && r < b) {
+        y[j0 + r] = yr;
+        z[j0 + r] = cmul(yr, dj);
     }
-    // the release by thread 0 after the barrier publishes every thread's
-    // stores above (cumulativity of the gpu-scope release)
-    __syncthreads();
-    if (threadIdx.x == 0) st_release(flags + j, epoch);
 }
 
 // Backward: x_j = Linv_j^H (z_j - sum_{c>j} U(j, c) x_c).
 template <bool NEIGH>
-__global__ void __launch_bounds__(256) k_bwd_coop(const cd* __restrict__ A, int ld, const int* __restrict__ bstart,
+__global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_bwd_coop(const cd* __restrict__ A, int ld, const int* __restrict__ bstart,
                                                   int nb, const cd* __restrict__ z, cd* __restrict__ x,
                                                   const cd* __restrict__ linv, const cd* __restrict__ lnb,
-                                                  unsigned* __restrict__ flags, unsigned epoch,
                                                   int* __restrict__ status, int* abort_word)
 {
     extern __shared__ double2 sm[];
     double2* Ls = sm;
-    double2* red = sm + LDL_NB * LS_LD;  // [8][64]
+    double2* red = sm + LDL_NB * LS_LD;  // [8][64] warp partials
     double2* Ns = red + 8 * LDL_NB;      // NEIGH: N_j, [r][q]
-    __shared__ double2 t[LDL_NB];
+    __shared__ double2 t[LDL_NB], xs[2][LDL_NB];
     const int j = blockIdx.x;
     const int j0 = bstart[j], j1 = bstart[j + 1], b = j1 - j0;
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     load_linv(linv, j0, b, Ls);
     if (NEIGH && j + 1 < nb) load_linv(lnb, j0, b, Ns, bstart[j + 2] - j1);
+    const int r = threadIdx.x >> 2;
     const cd zj = (threadIdx.x < b) ? ld2(z + j0 + threadIdx.x) : mk(0.0, 0.0);  // read before the waits
     cd a0 = mk(0.0, 0.0), a1 = mk(0.0, 0.0);  // rows lane, lane + 32
     bool ok = true;
+    const int limit = ((volatile int*)abort_word)[1];
     // every later panel but the next one; that one comes in below through
     // N_j = Linv_j^H U(j, j+1)
     const int clast = NEIGH ? j + 1 : j;
-    for (int c = nb - 1; c > clast; c--) {
+    auto load_u = [&](int c, cd (&u0)[8], cd (&u1)[8]) {
         const int c0 = bstart[c], c1 = bstart[c + 1];
-        // U(panel j, panel c) before the wait for panel c's solution
-        cd u0[8], u1[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
             const int col = c0 + wp + 8 * i;
@@ -377,70 +401,53 @@ __global__ void __launch_bounds__(256) k_bwd_coop(const cd* __restrict__ A, int 
             u0[i] = (col < c1 && lane < b) ? ld2(u + lane) : mk(0.0, 0.0);
             u1[i] = (col < c1 && lane + 32 < b) ? ld2(u + lane + 32) : mk(0.0, 0.0);
         }
-        if (!wait_panel(flags, c, epoch, status, abort_word, ok)) break;
+    };
+    auto apply = [&](int c, const cd (&u0)[8], const cd (&u1)[8]) {
+        double2* sv = xs[c & 1];
+        ok = wait_panel(x + bstart[c], bstart[c + 1] - bstart[c], sv, status, abort_word, limit);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            const int col = c0 + wp + 8 * i;
-            const cd xc = (col < c1) ? ldcg2(x + col) : mk(0.0, 0.0);
-            a0 = cfma(u0[i], xc, a0);
-            a1 = cfma(u1[i], xc, a1);
+            const double2 v = sv[wp + 8 * i];
+            a0 = cfma(u0[i], mk(v.x, v.y), a0);
+            a1 = cfma(u1[i], mk(v.x, v.y), a1);
+        }
+    };
+    cd ua[8], va[8];
+    if (NEIGH) {
+        cd ub[8], vb[8];
+        if (nb - 1 > clast) load_u(nb - 1, ua, va);
+        for (int c = nb - 1; c > clast && ok; c -= 2) {
+            if (c - 1 > clast) load_u(c - 1, ub, vb);
+            apply(c, ua, va);
+            if (c - 1 > clast && ok) {
+                if (c - 2 > clast) load_u(c - 2, ua, va);
+                apply(c - 1, ub, vb);
+            }
+        }
+    } else {
+        for (int c = nb - 1; c > clast && ok; c--) {
+            load_u(c, ua, va);
+            apply(c, ua, va);
         }
     }
     red[wp * LDL_NB + lane] = make_double2(a0.x, a0.y);
     red[wp * LDL_NB + lane + 32] = make_double2(a1.x, a1.y);
     __syncthreads();
-    if (threadIdx.x < b) {
-        const int r = threadIdx.x;
+    if (threadIdx.x < LDL_NB) {
         cd s = mk(0.0, 0.0);
 #pragma unroll
-        for (int q = 0; q < 8; q++) s = s + mk(red[q * LDL_NB + r].x, red[q * LDL_NB + r].y);
-        const cd v = zj - s;
-        t[r] = make_double2(v.x, v.y);
+        for (int q = 0; q < 8; q++) s = s + mk(red[q * LDL_NB + threadIdx.x].x, red[q * LDL_NB + threadIdx.x].y);
+        t[threadIdx.x] = make_double2(zj.x - s.x, zj.y - s.y);
     }
     __syncthreads();
-    {
-        const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
-        cd s = mk(0.0, 0.0);
-        if (r < b)
-            for (int q = r + g; q < b; q += 4) {
-                const double2 l = Ls[q * LS_LD + r], tq = t[q];
-                s = cfma(conj(mk(l.x, l.y)), mk(tq.x, tq.y), s);
-            }
-        red[g * LDL_NB + r] = make_double2(s.x, s.y);
-    }
-    __syncthreads();
-    cd xs = mk(0.0, 0.0);
-    if (threadIdx.x < b) {
-        const int r = threadIdx.x;
-#pragma unroll
-        for (int g = 0; g < 4; g++) xs = xs + mk(red[g * LDL_NB + r].x, red[g * LDL_NB + r].y);
-    }
+    cd xr = row_product_h(Ls, t);
     if (NEIGH && j + 1 < nb) {
-        // x_j -= N_j x_{j+1}: row r = tid & 63, columns g, g + 4, ...
-        const int c0 = bstart[j + 1], bn = bstart[j + 2] - c0;
-        const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
-        if (wait_panel(flags, j + 1, epoch, status, abort_word, ok)) {
-            cd s = mk(0.0, 0.0);
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const int q = g + 4 * i;
-                if (q < bn) {
-                    const double2 m = Ns[r * LS_LD + q];
-                    s = cfma(mk(m.x, m.y), ldcg2(x + c0 + q), s);
-                }
-            }
-            red[g * LDL_NB + r] = make_double2(s.x, s.y);
-        }
-        __syncthreads();
-        if (ok && threadIdx.x < b) {
-            const int rr = threadIdx.x;
-#pragma unroll
-            for (int g2 = 0; g2 < 4; g2++) xs = xs - mk(red[g2 * LDL_NB + rr].x, red[g2 * LDL_NB + rr].y);
-        }
+        // x_j -= N_j x_{j+1}
+        double2* sv = xs[(j + 1) & 1];
+        if (ok && wait_panel(x + bstart[j + 1], bstart[j + 2] - bstart[j + 1], sv, status, abort_word, limit))
+            xr = xr - row_product(Ns, sv);
     }
-    if (threadIdx.x < b) x[j0 + threadIdx.x] = xs;
-    __syncthreads();
-    if (threadIdx.x == 0) st_release(flags + j, epoch);
+    if ((threadIdx.x & 3) == 0 && r < b) x[j0 + r] = xr;
 }
 
 // Block-wide deterministic sums (1024 threads).
@@ -465,8 +472,10 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh)
     }
 }
 
-// Normalisation and convergence measure of one step; ends with v <- x.
-__global__ void __launch_bounds__(1024) k_iter_norm(int n, cd* __restrict__ x, cd* __restrict__ v, double sqrtn,
+// Normalisation and convergence measure of one step from the solution xw;
+// ends with v <- x.
+__global__ void __launch_bounds__(1024) k_iter_norm(int n, const cd* __restrict__ xw, cd* __restrict__ x,
+                                                    cd* __restrict__ v, double sqrtn,
                                                     double* __restrict__ red)
 {
     __shared__ double sh[32 * 3];
@@ -474,7 +483,7 @@ __global__ void __launch_bounds__(1024) k_iter_norm(int n, cd* __restrict__ x, c
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     double m = 0.0;
     for (int j = tid; j < n; j += 1024) {
-        const cd a = x[j];
+        const cd a = xw[j];
         m = fmax(m, fmax(fabs(a.x), fabs(a.y)));
     }
 #pragma unroll
@@ -486,7 +495,7 @@ __global__ void __launch_bounds__(1024) k_iter_norm(int n, cd* __restrict__ x, c
     const double ra = 1.0 / t1;
     double acc[3] = {0.0, 0.0, 0.0};
     for (int j = tid; j < n; j += 1024) {
-        cd a = x[j];
+        cd a = xw[j];
         a = cd{ra * a.x, ra * a.y};
         x[j] = a;
         const cd b = v[j];
@@ -617,7 +626,7 @@ static int solve_multi_launch(Ctx& c, int n)
         int G = (rest + 127) / 128;
         G = G < 1 ? 1 : (G > SOLVE_G_MAX ? SOLVE_G_MAX : G);
         const int chunk = (rest + G - 1) / G;
-        k_bwd<<<G, 256, 0, c.stream>>>(c.F, c.ld, j0, j1, n, chunk > 0 ? chunk : 1, c.zv, c.x, c.linv, c.spart,
+        k_bwd<<<G, 256, 0, c.stream>>>(c.F, c.ld, j0, j1, n, chunk > 0 ? chunk : 1, c.zv, c.xw, c.linv, c.spart,
                                       c.counters + 1);
         c.launches++;
     }
@@ -640,13 +649,11 @@ static int solve_cooperative(Ctx& c, int n, bool neigh)
     int ld = c.ld;
     const void* kf = neigh ? (const void*)k_fwd_coop<true> : (const void*)k_fwd_coop<false>;
     const void* kb = neigh ? (const void*)k_bwd_coop<true> : (const void*)k_bwd_coop<false>;
-    unsigned e1 = ++c.epoch;
     void* a1[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&w, &c.yv, &c.zv, (void*)&invD, (void*)&linv, (void*)&lmf,
-                  &c.flags, &e1, &c.status, &abort_word};
+                  &c.status, &abort_word};
     if (cudaLaunchCooperativeKernel(kf, nb, 256, a1, sm, c.stream) != cudaSuccess) return -2;
-    unsigned e2 = ++c.epoch;
     const cd* zv = c.zv;
-    void* a2[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&zv, &c.x, (void*)&linv, (void*)&lnb, &c.flags, &e2,
+    void* a2[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&zv, &c.xw, (void*)&linv, (void*)&lnb,
                   &c.status, &abort_word};
     if (cudaLaunchCooperativeKernel(kb, nb, 256, a2, sm, c.stream) != cudaSuccess) return -2;
     c.launches += 2;
@@ -655,7 +662,7 @@ static int solve_cooperative(Ctx& c, int n, bool neigh)
 
 int invit_step(Ctx& c, int n, bool /*first*/)
 {
-    k_hemv<<<(n * 32 + 255) / 256, 256, 0, c.stream>>>(c.S, c.ld, n, c.c, c.w);
+    k_hemv<<<(n * 32 + 255) / 256, 256, 0, c.stream>>>(c.S, c.ld, n, c.c, c.w, c.yv, c.xw);
     c.launches++;
     const int nb = (int)c.blk_start.size();
     // the neighbour products take a second 64 x 64 block of shared memory
@@ -668,7 +675,7 @@ int invit_step(Ctx& c, int n, bool /*first*/)
     else
         r = solve_multi_launch(c, n);
     if (r) return r;
-    k_iter_norm<<<1, 1024, 0, c.stream>>>(n, c.x, c.c, sqrt(2.0 * n), c.red);
+    k_iter_norm<<<1, 1024, 0, c.stream>>>(n, c.xw, c.x, c.c, sqrt(2.0 * n), c.red);
     c.launches++;
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -19,6 +19,7 @@
 #include <string.h>
 #include "ecg_internal.h"
 #include "ecg_grad.cuh"
+#include "warp_sums.cuh"
 
 namespace ecg {
 
@@ -536,31 +537,6 @@ template <int N>
 struct AdjNV {
     static constexpr int value = 2 * Sym<N>::NP + 1;
 };
-
-// Sum v[0..M) (M a power of two, at most 32) over the warp's lanes: every
-// step exchanges half of the values a lane still holds, so 2 M - 1 values
-// travel instead of the 5 M of a butterfly per value.  Lane i returns the
-// sum of value i / (32 / M).
-template <int M>
-__device__ __forceinline__ double warp_transpose_sum(double (&v)[M])
-{
-    const int lane = threadIdx.x & 31;
-    int s = 16;
-#pragma unroll
-    for (int h = M / 2; h >= 1; h /= 2) {
-        const bool up = (lane & s) != 0;
-#pragma unroll
-        for (int i = 0; i < h; i++) {
-            const double send = up ? v[i] : v[i + h];
-            const double keep = up ? v[i + h] : v[i];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
-        }
-        s /= 2;
-    }
-#pragma unroll
-    for (int q = 16 / M; q >= 1; q /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], q);
-    return v[0];
-}
 
 // FP64 issue bounds it: 860 FP64 instructions a term at n = 3 (ncu), 1.52 ms
 // of the pipe at K = 4000, T = 4, where it takes 2.24 ms (4.35 ms with full
