@@ -152,9 +152,14 @@ int ghepiis_core(Ctx& c, int k, int n, double apprlambda, double tol, int max_it
     CK(cudaStreamSynchronize(c.stream));
     mark(c, 2);
     if (c.status_h[ST_SOLVE_TIMEOUT]) {
-        // a bounded wait of the factorisation ran out: no factor
-        c.fact_n = 0;
-        c.blk_start.clear();
+        // a bounded wait of the factorisation ran out: no factor, or none of
+        // the one new row
+        const bool row = k > 1 && n == k;
+        c.fact_n = row ? k - 1 : 0;
+        if (!row)
+            c.blk_start.clear();
+        else if (!c.blk_start.empty() && c.blk_start.back() == k - 1)
+            c.blk_start.pop_back();
         return ECG_ECUDA;
     }
     if (c.status_h[ST_ZERO_PIVOT] != 0) {
@@ -224,7 +229,7 @@ int g_count(Ctx& c, int n, double sigma, int* nu, int* zero)
 {
     CKR(g_shift(c, c.H, c.S, c.diagH, nullptr, n, sigma));
     CK(cudaMemsetAsync(c.status, 0, ST_COUNT * sizeof(int), c.stream));
-    CKR(ldlh_factor(c, 0, n));
+    CKR(ldlh_factor(c, 0, n, false));
     CKR(g_inertia(c, n));
     CK(cudaMemcpyAsync(c.gcnt_h, c.gcnt, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     CK(cudaMemcpyAsync(c.status_h, c.status, ST_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
@@ -256,7 +261,7 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
     // S positive definite?  (ZPOTRF inside ZHEGVX: INFO = n + i)
     CKR(g_shift(c, c.S, nullptr, nullptr, nullptr, n, 0.0));
     CK(cudaMemsetAsync(c.status, 0, ST_COUNT * sizeof(int), c.stream));
-    CKR(ldlh_factor(c, 0, n));
+    CKR(ldlh_factor(c, 0, n, false));
     CKR(g_inertia(c, n));
     CK(cudaMemcpyAsync(c.gcnt_h, c.gcnt, 2 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     CK(cudaMemcpyAsync(c.status_h, c.status, ST_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c.stream));

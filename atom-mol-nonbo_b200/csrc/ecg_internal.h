@@ -269,7 +269,7 @@ int g_mirror_s(Ctx& c, int n);
 int g_inertia(Ctx& c, int n);
 
 // ---- launchers (ldlh.cu) ----
-int ldlh_factor(Ctx& c, int m0, int n);
+int ldlh_factor(Ctx& c, int m0, int n, bool solves = true);
 
 // ---- persistent factorisation (ldlp.cu) ----
 int ldlp_grid(Ctx& c);
@@ -284,6 +284,7 @@ int ldlh_factor_traced(Ctx& c, int n, unsigned long long* out, long long cap, lo
 // ---- launchers (invit.cu) ----
 int invit_step(Ctx& c, int n, bool first);
 int invit_rayleigh(Ctx& c, int n);
+int border_row(Ctx& c, int m0, int nexist);
 int vec_scale(Ctx& c, cd* v, int n, double s);
 
 inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? 0 : -2; }

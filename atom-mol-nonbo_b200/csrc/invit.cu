@@ -633,31 +633,126 @@ static int solve_multi_launch(Ctx& c, int n)
     return 0;
 }
 
-static int solve_cooperative(Ctx& c, int n, bool neigh)
+// ---------------------------------------------------------------------------
+// The bordered step of LDLHF for one new row (src/linalg.f90:356-391 with
+// m = n): column m0 of L^H is U(:, m0) = invD o a with a = L0^-1 M(:, m0),
+// one forward solve with the existing factor, and the pivot d = M(m0, m0) -
+// sum_q conj(a_q) U(q, m0).  At K = 2001: 70 us in three launches; a panel
+// solve and a rank-64 update of the one column per existing panel took 567
+// us in 64.
+// ---------------------------------------------------------------------------
+
+// w = M(0..m0-1, m0) from the row that holds its conjugate; y as the solve
+// wants it.
+__global__ void __launch_bounds__(256) k_border_rhs(const cd* __restrict__ A, int ld, int m0, cd* __restrict__ w,
+                                                    cd* __restrict__ y)
 {
-    int nb = (int)c.blk_start.size();
+    const int r = blockIdx.x * 256 + threadIdx.x;
+    if (r >= m0) return;
+    w[r] = conj(A[(size_t)m0 + (size_t)r * ld]);
+    y[r] = unset();
+}
+
+// The column, the pivot (its imaginary part kept with cplx, as the reference
+// keeps it) and the one-row panel's blocks for the solves: Linv = 1, M of the
+// new panel and N of the last existing one (rows [p0, m0)).
+__global__ void __launch_bounds__(1024) k_border_finish(cd* __restrict__ A, int ld, int m0, int p0,
+                                                        const cd* __restrict__ y, const cd* __restrict__ z,
+                                                        cd* __restrict__ invD, cd* __restrict__ linv,
+                                                        cd* __restrict__ lmf, cd* __restrict__ lnb,
+                                                        int* __restrict__ status, int cplx)
+{
+    __shared__ double sh[32 * 2];
+    const int tid = threadIdx.x;
+    double acc[2] = {0.0, 0.0};
+    for (int q = tid; q < m0; q += 1024) {
+        const cd u = z[q], s = cmul(conj(y[q]), u);
+        acc[0] += s.x;
+        acc[1] += s.y;
+        A[(size_t)q + (size_t)m0 * ld] = u;
+    }
+    block_sum<2>(acc, sh);
+    const int bp = m0 - p0;
+    if (tid == 0) {
+        const double xr = A[(size_t)m0 + (size_t)m0 * ld].x - acc[0], xi = cplx ? acc[1] : 0.0;
+        cd id = mk(0.0, 0.0);
+        if (xr == 0.0 && xi == 0.0)
+            atomicCAS(status + ST_ZERO_PIVOT, 0, m0 + 1);
+        else
+            id = cplx ? crcp(mk(xr, xi)) : mk(1.0 / xr, 0.0);
+        invD[m0] = id;
+    }
+    if (tid < LDL_NB) {
+        linv[(size_t)m0 * LDL_NB + tid] = mk(tid == 0 ? 1.0 : 0.0, 0.0);
+        lmf[(size_t)m0 * LDL_NB + tid] = tid < bp ? conj(z[p0 + tid]) : mk(0.0, 0.0);
+    }
+    // N(r, 0) = sum_q conj(Linv(q, r)) U(p0 + q, m0), four lanes a row
+    const int r = (tid >> 2) & 63;
+    if (tid < 4 * LDL_NB) {
+        cd s = mk(0.0, 0.0);
+        if (r < bp)
+            for (int q = r + (tid & 3); q < bp; q += 4)
+                s = cfma(conj(ld2(linv + (size_t)(p0 + q) * LDL_NB + r)), z[p0 + q], s);
+#pragma unroll
+        for (int o = 1; o <= 2; o <<= 1) {
+            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        }
+        if (r < bp)
+            for (int q = tid & 3; q < LDL_NB; q += 4)
+                lnb[(size_t)(p0 + r) * LDL_NB + q] = q == 0 ? s : mk(0.0, 0.0);
+    }
+}
+
+static int launch_fwd(Ctx& c, int nb, bool neigh)
+{
     const size_t sm = coop_smem(neigh);
     int* abort_word = c.counters + 2;
     if (cudaMemsetAsync(abort_word, 0, sizeof(int), c.stream) != cudaSuccess) return -2;
     const int* bs = c.dblk;
-    const cd* H = c.F;
-    const cd* w = c.w;
-    const cd* invD = c.invD;
-    const cd* linv = c.linv;
-    const cd* lmf = c.lmf;
-    const cd* lnb = c.lnb;
+    const cd *H = c.F, *w = c.w, *invD = c.invD, *linv = c.linv, *lmf = c.lmf;
     int ld = c.ld;
-    const void* kf = neigh ? (const void*)k_fwd_coop<true> : (const void*)k_fwd_coop<false>;
-    const void* kb = neigh ? (const void*)k_bwd_coop<true> : (const void*)k_bwd_coop<false>;
-    void* a1[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&w, &c.yv, &c.zv, (void*)&invD, (void*)&linv, (void*)&lmf,
-                  &c.status, &abort_word};
-    if (cudaLaunchCooperativeKernel(kf, nb, 256, a1, sm, c.stream) != cudaSuccess) return -2;
-    const cd* zv = c.zv;
-    void* a2[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&zv, &c.xw, (void*)&linv, (void*)&lnb,
-                  &c.status, &abort_word};
-    if (cudaLaunchCooperativeKernel(kb, nb, 256, a2, sm, c.stream) != cudaSuccess) return -2;
-    c.launches += 2;
+    void* args[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&w, &c.yv, &c.zv, (void*)&invD, (void*)&linv, (void*)&lmf,
+                    &c.status, &abort_word};
+    const void* k = neigh ? (const void*)k_fwd_coop<true> : (const void*)k_fwd_coop<false>;
+    if (cudaLaunchCooperativeKernel(k, nb, 256, args, sm, c.stream) != cudaSuccess) return -2;
+    c.launches++;
     return 0;
+}
+
+static int solve_cooperative(Ctx& c, bool neigh)
+{
+    int nb = (int)c.blk_start.size();
+    const int r = launch_fwd(c, nb, neigh);
+    if (r) return r;
+    int* abort_word = c.counters + 2;
+    const int* bs = c.dblk;
+    const cd *H = c.F, *linv = c.linv, *lnb = c.lnb, *zv = c.zv;
+    int ld = c.ld;
+    void* args[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&zv, &c.xw, (void*)&linv, (void*)&lnb,
+                    &c.status, &abort_word};
+    const void* k = neigh ? (const void*)k_bwd_coop<true> : (const void*)k_bwd_coop<false>;
+    if (cudaLaunchCooperativeKernel(k, nb, 256, args, coop_smem(neigh), c.stream) != cudaSuccess) return -2;
+    c.launches++;
+    return 0;
+}
+
+// Row m0 beside the factor of rows 0..m0-1, whose nexist panels (the last
+// one truncated at m0) are in c.dblk.  1: not available for so many panels.
+int border_row(Ctx& c, int m0, int nexist)
+{
+    const bool neigh = nexist <= coop_capacity(c, true);
+    if (nexist < 1 || (!neigh && nexist > coop_capacity(c, false))) return 1;
+    k_border_rhs<<<(m0 + 255) / 256, 256, 0, c.stream>>>(c.F, c.ld, m0, c.w, c.yv);
+    const int r = launch_fwd(c, nexist, neigh);
+    if (r) return r;
+    int p0 = 0;  // first row of the last existing panel
+    for (int s : c.blk_start)
+        if (s < m0) p0 = s;
+    k_border_finish<<<1, 1024, 0, c.stream>>>(c.F, c.ld, m0, p0, c.yv, c.zv, c.invD, c.linv, c.lmf, c.lnb, c.status,
+                                              c.pivot_mode);
+    c.launches += 2;
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 int invit_step(Ctx& c, int n, bool /*first*/)
@@ -669,9 +764,9 @@ int invit_step(Ctx& c, int n, bool /*first*/)
     // (one CTA per SM): used while every panel still has an SM of its own
     int r;
     if (nb <= coop_capacity(c, true))
-        r = solve_cooperative(c, n, true);
+        r = solve_cooperative(c, true);
     else if (nb <= coop_capacity(c, false))
-        r = solve_cooperative(c, n, false);
+        r = solve_cooperative(c, false);
     else
         r = solve_multi_launch(c, n);
     if (r) return r;

@@ -326,66 +326,70 @@ __global__ void __launch_bounds__(256) k_ldl_linv(const cd* __restrict__ A, int 
 // stored like linv, row r of panel j at [(p0 + r) * 64 + q].  With them a
 // solve's panel j applies the neighbouring panel's solution as one 64 x 64
 // product once that panel is published, everything else being done before.
+// One 64 x 64 x 64 complex product per CTA on the FP64 tensor cores, in two
+// chunks of the inner dimension: 8 us for all panels at K = 4000 (a product
+// of FMA loops over one chunk of 133 KB, one CTA an SM: 37 us).
+constexpr int MN_K = 32, MN_LDA = LDL_NB + 2, MN_LDB = MN_K + 4;  // pitches as zmma.cuh wants them
+constexpr size_t MN_SMEM = (size_t)(MN_K * MN_LDA + LDL_NB * MN_LDB) * sizeof(double2);
+
 __global__ void __launch_bounds__(256) k_ldl_mn(const cd* __restrict__ A, int ld, const int* __restrict__ bstart,
                                                  int nb, int first, const cd* __restrict__ linv, cd* __restrict__ lmf,
                                                  cd* __restrict__ lnb)
 {
     extern __shared__ double2 sm[];
-    double2* Ls = sm;                   // Ls[r * DG_LD + c] = Linv_j(r, c)
-    double2* Us = sm + LDL_NB * DG_LD;  // Us[c * DG_LD + q]: conj(U(o0 + q, p0 + c)) or U(p0 + c, o0 + q)
+    double2* As = sm;                    // [k][m]: Linv_j (forward) or its transpose (backward, conjugated in the product)
+    double2* Bs = sm + MN_K * MN_LDA;    // [n][k]: conj(U(o0 + n, p0 + k)) or U(p0 + k, o0 + n)
     const int j = first + blockIdx.x;
     const bool fwd = blockIdx.y == 0;
     if (fwd ? j < 1 : j + 1 >= nb) return;
     const int p0 = bstart[j], b = bstart[j + 1] - p0;
     const int o0 = fwd ? bstart[j - 1] : bstart[j + 1];
     const int bo = fwd ? p0 - o0 : bstart[j + 2] - o0;
-    const int tid = threadIdx.x;
-    for (int e = tid; e < LDL_NB * LDL_NB; e += 256) {
-        const int c = e & 63, r = e >> 6;
-        double2 v = make_double2(0.0, 0.0);
-        if (r < b && c < b) {
-            const cd x = linv[(size_t)(p0 + r) * LDL_NB + c];
-            v = make_double2(x.x, x.y);
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const int wm = (wp >> 2) * 32, wn = (wp & 3) * 16;
+    ZAcc<4, 2> acc;
+    acc.zero();
+    for (int k0 = 0; k0 < LDL_NB; k0 += MN_K) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int e = tid + 256 * u;
+            // linv's rows are contiguous, U's columns are
+            const int ma = fwd ? (e >> 5) : (e & 63), ka = k0 + (fwd ? (e & 31) : (e >> 6));
+            const int nn = fwd ? (e & 63) : (e >> 5), kb = k0 + (fwd ? (e >> 6) : (e & 31));
+            double2 x = make_double2(0.0, 0.0), y = x;
+            if (ma < b && ka < b) {
+                const cd v = ldg2(linv + (fwd ? (size_t)(p0 + ma) * LDL_NB + ka : (size_t)(p0 + ka) * LDL_NB + ma));
+                x = make_double2(v.x, v.y);
+            }
+            if (nn < bo && kb < b) {
+                const cd v = ldg2(A + (fwd ? (size_t)(o0 + nn) + (size_t)(p0 + kb) * ld
+                                           : (size_t)(p0 + kb) + (size_t)(o0 + nn) * ld));
+                y = make_double2(v.x, fwd ? -v.y : v.y);
+            }
+            As[(ka - k0) * MN_LDA + ma] = x;
+            Bs[nn * MN_LDB + kb - k0] = y;
         }
-        Ls[r * DG_LD + c] = v;
-        // the neighbour block, read along its columns
-        const int lo = e & 63, hi = e >> 6;
-        double2 u = make_double2(0.0, 0.0);
+        __syncthreads();
         if (fwd) {
-            if (hi < b && lo < bo) {
-                const cd x = A[(size_t)(o0 + lo) + (size_t)(p0 + hi) * ld];
-                u = make_double2(x.x, -x.y);
-            }
-            Us[hi * DG_LD + lo] = u;
+#pragma unroll
+            for (int kk = 0; kk < MN_K; kk += 4) zmma_k4<4, 2, MN_LDA, MN_LDB, false>(acc, As, Bs, wm, wn, kk, lane);
         } else {
-            if (lo < b && hi < bo) {
-                const cd x = A[(size_t)(p0 + lo) + (size_t)(o0 + hi) * ld];
-                u = make_double2(x.x, x.y);
+#pragma unroll
+            for (int kk = 0; kk < MN_K; kk += 4) zmma_k4<4, 2, MN_LDA, MN_LDB, true>(acc, As, Bs, wm, wn, kk, lane);
+        }
+        __syncthreads();
+    }
+    const int g = lane >> 2, t = lane & 3;
+    cd* out = fwd ? lmf : lnb;
+#pragma unroll
+    for (int mt = 0; mt < 4; mt++)
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int m = wm + mt * 8 + g, n = wn + nt * 8 + 2 * t + e;
+                if (m < b) out[(size_t)(p0 + m) * LDL_NB + n] = cd{acc.r[mt][nt][e], acc.i[mt][nt][e]};
             }
-            Us[lo * DG_LD + hi] = u;
-        }
-    }
-    __syncthreads();
-    const int r = tid >> 2, q0 = tid & 3;
-    double accr[16], acci[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) accr[i] = acci[i] = 0.0;
-    const int c0 = fwd ? 0 : r, c1 = fwd ? r + 1 : LDL_NB;
-    for (int c = c0; c < c1; c++) {
-        double2 l = fwd ? Ls[r * DG_LD + c] : Ls[c * DG_LD + r];
-        if (!fwd) l.y = -l.y;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const double2 u = Us[c * DG_LD + q0 + 4 * i];
-            accr[i] = fma(l.x, u.x, fma(-l.y, u.y, accr[i]));
-            acci[i] = fma(l.x, u.y, fma(l.y, u.x, acci[i]));
-        }
-    }
-    if (r < b) {
-        cd* out = (fwd ? lmf : lnb) + (size_t)(p0 + r) * LDL_NB;
-#pragma unroll
-        for (int i = 0; i < 16; i++) out[q0 + 4 * i] = cd{accr[i], acci[i]};
-    }
 }
 
 // Panel rows beyond the diagonal block, by substitution:
@@ -695,7 +699,7 @@ static void enqueue_factor(Ctx& c, int m0, int n, const std::vector<int>& starts
         k_ldl_linv<<<nblk - nexist, 256, 2 * sm1, c.stream>>>(c.F, c.ld, c.dblk, nexist, c.linv);
         // the last existing panel's N changes with the first new panel
         const int f = std::max(nexist - 1, 0);
-        k_ldl_mn<<<dim3(nblk - f, 2), 256, 2 * sm1, c.stream>>>(c.F, c.ld, c.dblk, nblk, f, c.linv, c.lmf, c.lnb);
+        k_ldl_mn<<<dim3(nblk - f, 2), 256, MN_SMEM, c.stream>>>(c.F, c.ld, c.dblk, nblk, f, c.linv, c.lmf, c.lnb);
         c.launches += 2;
     }
 }
@@ -703,15 +707,16 @@ static void enqueue_factor(Ctx& c, int m0, int n, const std::vector<int>& starts
 // A whole factorisation (m0 = 0) as one persistent kernel (ldlp.cu): the
 // working upper triangle and diagonal, the tile tasks (which leave the
 // inverse diagonal blocks), then the neighbour products of the solves.
-static void enqueue_persist(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long long* trace = nullptr)
+static void enqueue_persist(Ctx& c, int n, const unsigned* tasks, int ntasks, bool solves,
+                            unsigned long long* trace = nullptr)
 {
     const int ct1 = (n + 31) / 32;
     k_ldl_mirror<<<dim3(ct1, ct1), 256, 0, c.stream>>>(c.F, c.ld, 0, n, c.dw, 0);
     c.launches++;
     ldlp_enqueue(c, n, tasks, ntasks, trace);
+    if (!solves) return;
     const int nblk = (n + LDL_NB - 1) / LDL_NB;
-    k_ldl_mn<<<dim3(nblk, 2), 256, 2 * LDL_NB * DG_LD * sizeof(double2), c.stream>>>(c.F, c.ld, c.dblk, nblk, 0,
-                                                                                    c.linv, c.lmf, c.lnb);
+    k_ldl_mn<<<dim3(nblk, 2), 256, MN_SMEM, c.stream>>>(c.F, c.ld, c.dblk, nblk, 0, c.linv, c.lmf, c.lnb);
     c.launches++;
 }
 
@@ -723,7 +728,7 @@ static void ldl_attrs()
     cudaFuncSetAttribute(k_ldl_diag<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DG_SMEM);
     cudaFuncSetAttribute(k_ldl_diag<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DG_SMEM);
     cudaFuncSetAttribute(k_ldl_linv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * sm1));
-    cudaFuncSetAttribute(k_ldl_mn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * sm1));
+    cudaFuncSetAttribute(k_ldl_mn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MN_SMEM);
     cudaFuncSetAttribute(k_ldl_bulk<32, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)blk_smem<32>());
     cudaFuncSetAttribute(k_ldl_bulk<16, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)blk_smem<16>());
     g_ldl_attr = true;
@@ -734,8 +739,10 @@ static void ldl_attrs()
 // panel boundaries, so it is captured once into a CUDA graph (both streams)
 // and replayed.  A whole factorisation (m0 = 0) runs as the persistent
 // kernel of ldlp.cu unless ecg_set_factor_mode selected the launch-per-panel
-// form.
-int ldlh_factor(Ctx& c, int m0, int n)
+// form.  One new row beside an existing factor (the trial loops) is a single
+// forward solve and takes neither.  Without `solves` only the pivots are
+// wanted (the inertia counts): the factor is then not kept for use.
+int ldlh_factor(Ctx& c, int m0, int n, bool solves)
 {
     if (m0 < 0 || m0 > n || n > c.ld) return -1;
     if (m0 > c.fact_n) return -1;
@@ -757,7 +764,17 @@ int ldlh_factor(Ctx& c, int m0, int n)
     // rows (at 10000 rows the panel pairs' rank-128 launches measured 57.2
     // against its 59.4 ms)
     const bool persist = (m0 == 0 && n > 0 && n < LDL_PAIR_MIN && c.factor_mode == 0 && ldlp_grid(c) > 0);
-    std::vector<int> key = {m0, n, c.pivot_mode, persist ? 1 : 0};
+    if (m0 > 0 && n - m0 == 1) {
+        const int r = border_row(c, m0, nexist);
+        if (r <= 0) {
+            if (r == 0) {
+                c.blk_start = starts;
+                c.fact_n = n;
+            }
+            return r;
+        }
+    }
+    std::vector<int> key = {m0, n, c.pivot_mode, persist ? (solves ? 1 : 2) : 0};
     key.insert(key.end(), starts.begin(), starts.begin() + nexist);
     Ctx::LdlGraph* g = nullptr;
     for (auto& e : c.ldl_graphs)
@@ -773,7 +790,7 @@ int ldlh_factor(Ctx& c, int m0, int n)
         }
         auto enqueue = [&]() {
             if (persist)
-                enqueue_persist(c, n, tasks, ntasks);
+                enqueue_persist(c, n, tasks, ntasks, solves);
             else
                 enqueue_factor(c, m0, n, starts, nexist);
         };
@@ -805,8 +822,8 @@ int ldlh_factor(Ctx& c, int m0, int n)
             }
             enqueue();
             if (cudaGetLastError() != cudaSuccess) return -2;
-            c.blk_start = starts;
-            c.fact_n = n;
+            c.blk_start = solves ? starts : std::vector<int>();
+            c.fact_n = solves ? n : 0;
             return 0;
         }
         if (c.ldl_graphs.size() >= 8) {
@@ -823,8 +840,8 @@ int ldlh_factor(Ctx& c, int m0, int n)
     }
     if (cudaGraphLaunch(g->exec, c.stream) != cudaSuccess) return -2;
     c.launches += g->launches;
-    c.blk_start = starts;
-    c.fact_n = n;
+    c.blk_start = solves ? starts : std::vector<int>();
+    c.fact_n = solves ? n : 0;
     return 0;
 }
 
@@ -858,7 +875,7 @@ int ldlh_factor_traced(Ctx& c, int n, unsigned long long* out, long long cap, lo
         cudaFree(tasks);
         return -3;
     }
-    enqueue_persist(c, n, tasks, ntasks, d);
+    enqueue_persist(c, n, tasks, ntasks, true, d);
     unsigned recs = 0;
     const size_t ntile = (size_t)nb * (nb + 1) / 2;  // trace records at ctl[2], ctl = counters + 2 ntile
     int r = 0;

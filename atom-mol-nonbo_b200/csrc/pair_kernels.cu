@@ -409,6 +409,50 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_pair_energy(SysParams sp, con
     }
 }
 
+// The same pairs for a few rows (one in the trial loops, where a tile of 32
+// rows would leave 31 lanes of every warp idle): lanes run along the column
+// index l, blockIdx.y along the rows.  One row at K = 2001, n = 3, T = 4: 12
+// us against 89 (ncu), bound by the latency of one pair's terms.
+constexpr int PAIR_ROW_NT = 64;
+template <int N>
+__global__ void __launch_bounds__(PAIR_ROW_NT) k_pair_row(SysParams sp, const double* __restrict__ coef,
+                                                          const cd* __restrict__ bra, const cd* __restrict__ ket,
+                                                          const double* __restrict__ detL,
+                                                          const double* __restrict__ diagS, cd* __restrict__ H,
+                                                          cd* __restrict__ S, int ld, int r0, char method,
+                                                          double approx_e)
+{
+    constexpr int NP = Sym<N>::NP;
+    __shared__ double2 bsm[BraShared<N>::ENTRIES_E];
+    const int k = r0 + blockIdx.y;
+    const int l = blockIdx.x * PAIR_ROW_NT + threadIdx.x;
+    if (threadIdx.x == 0) stage_bra<N, false>(bra + (size_t)k * NP, sp, bsm, 1);
+    __syncthreads();
+    if (l >= k) return;
+    const BraShared<N> b{bsm, 1};
+    const double absdet = fabs(detL[l] * detL[k]);
+    cd Hs = mk(0.0, 0.0), Ss = mk(0.0, 0.0);
+#pragma unroll 1
+    for (int t = 0; t < sp.T; t++) {
+        cd tCl[N][N];
+        load_sym<N>(ket + ((size_t)l * sp.T + t) * NP, tCl);
+        PairTerm<N> te;
+        pair_term<N, false>(b, tCl, absdet, sp.two_r3n2 * __ldg(coef + t), sp, te);
+        Hs = cfma(te.S, te.h, Hs);
+        Ss = Ss + te.S;
+    }
+    const double f = (1.0 / sqrt(diagS[k] * diagS[l]));
+    const size_t kl = (size_t)k + (size_t)l * ld;
+    const cd s = f * Ss;
+    S[kl] = s;
+    if (method == 'I') {
+        S[(size_t)l + (size_t)k * ld] = conj(s);
+        H[kl] = f * (Hs - approx_e * Ss);
+    } else {
+        H[kl] = f * Hs;
+    }
+}
+
 // Off-diagonal pairs with derivatives, one pair per thread at a time.  Both
 // sides' term sums (Z and a of H and of S, as DerivSum) live in shared memory,
 // [value][thread]; L_k and L_l are applied once per pair, after the terms.
@@ -659,6 +703,72 @@ __global__ void __launch_bounds__(NW * 32, MINB) k_adjoint(SysParams sp, const d
         }
     }
 }
+// The same partials where only one function is optimised (EnergyIB(K-1, K)):
+// of a tile's rows only k = nfru counts, and no column, so the tile kernel
+// would keep one lane of every warp busy.  One warp per tile, lanes along
+// its 32 columns, the row's sums over the lanes.  Whole passes and ranges of
+// tiles both take it, so their sums are the same.  The gradient stage of one
+// function: 103 -> 81 us at K = 2000, n = 3, T = 4; 286 -> 97 us at K = 1000,
+// n = 4, T = 14.
+template <int N>
+__global__ void __launch_bounds__(TILE) k_adjoint_row(SysParams sp, const double* __restrict__ coef,
+                                                      const double* __restrict__ Pd, const cd* __restrict__ bra,
+                                                      const cd* __restrict__ ket, const cd* __restrict__ ketn,
+                                                      const double* __restrict__ detL,
+                                                      const double* __restrict__ diagS,
+                                                      const cd* __restrict__ cvec, double E, int k, int Rlo,
+                                                      double* __restrict__ part, long long t0)
+{
+    constexpr int NP = Sym<N>::NP;
+    constexpr int NV = AdjNV<N>::value;
+    constexpr int M = NV <= 8 ? 8 : (NV <= 16 ? 16 : 32);
+    __shared__ double2 bsm[BraShared<N>::ENTRIES_E];
+    int R, C;
+    tile_rc(t0 + blockIdx.x, Rlo, R, C);
+    const long long tile = blockIdx.x;
+    const int lane = threadIdx.x;
+    if (lane == 0) stage_bra<N, false>(bra + (size_t)k * NP, sp, bsm, 1);
+    __syncwarp();
+    const BraShared<N> b{bsm, 1};
+    const int l = C * TILE + lane;
+    cd Ak[NP];
+    double ra = 0.0;
+#pragma unroll
+    for (int x = 0; x < NP; x++) Ak[x] = mk(0.0, 0.0);
+    if (l <= k) {
+        const double absdet = fabs(detL[l] * detL[k]);
+        const cd wkl = (1.0 / sqrt(diagS[k] * diagS[l])) * cmul(conj(ldcd(cvec + k)), ldcd(cvec + l));
+#pragma unroll 1
+        for (int t = 0; t < sp.T; t++) {
+            cd tCl[N][N];
+            load_sym<N>(ket + ((size_t)l * sp.T + t) * NP, tCl);
+            PairTerm<N> te;
+            pair_term<N, true>(b, tCl, absdet, sp.two_r3n2 * __ldg(coef + t), sp, te);
+            const cd Sw = cmul(wkl, te.S);
+            cd Zk[NP], Zl[NP];
+            const cd a = term_adjoint<N, false>(b, KetRead<N>{ketn + ((size_t)l * sp.T + t) * NP}, te, E, 0, Pd, Zk, Zl);
+            ra += cmul(Sw, a).x;
+#pragma unroll
+            for (int x = 0; x < NP; x++) Ak[x] = cfma(Sw, Zk[x], Ak[x]);
+        }
+    }
+    double v[M];
+#pragma unroll
+    for (int x = 0; x < M; x++) v[x] = 0.0;
+#pragma unroll
+    for (int x = 0; x < NP; x++) {
+        v[2 * x] = Ak[x].x;
+        v[2 * x + 1] = Ak[x].y;
+    }
+    v[NV - 1] = ra;
+    const double sum = warp_transpose_sum<M>(v);
+    const int x = lane / (32 / M);
+    if (lane % (32 / M) == 0 && x < NV) {
+        part[((tile * 2 + 0) * TILE + k % TILE) * NV + x] = sum;
+        part[((tile * 2 + 1) * TILE + k % TILE) * NV + x] = 0.0;
+    }
+}
+
 template <int N>
 constexpr size_t adjoint_smem()
 {
@@ -1274,6 +1384,10 @@ static int tune(Ctx& c, int nshapes, int& choice, float* ms_out, F run)
     return last_err();
 }
 
+// Ranges of at most this many rows take k_pair_row: a tile of 32 rows takes
+// the same time however few of them are computed.
+constexpr int PAIR_ROWS_MAX = 8;
+
 template <int N>
 static int energy_n(Ctx& c, int r0, int r1, double approx_e)
 {
@@ -1281,6 +1395,11 @@ static int energy_n(Ctx& c, int r0, int r1, double approx_e)
     const int Rlo = r0 / TILE, Rhi = (r1 + TILE - 1) / TILE;
     const long long nt = tile_count(Rlo, Rhi);
     c.launches++;
+    if (r1 - r0 <= PAIR_ROWS_MAX && r0 > 0) {
+        k_pair_row<N><<<dim3((r1 - 1 + PAIR_ROW_NT - 1) / PAIR_ROW_NT, r1 - r0), PAIR_ROW_NT, 0, c.stream>>>(
+            c.sp, c.coef, c.bra, c.ket, c.detL, c.diagS, c.H, c.S, c.ld, r0, c.method, approx_e);
+        return last_err();
+    }
     // shapes are tuned on the first launch with at least 256 tiles
     if (c.tune_pair < 0 && nt >= 256)
         return tune(c, PAIR_SHAPES, c.tune_pair, c.tune_pair_ms, [&](int v) {
@@ -1398,7 +1517,10 @@ static int adjoint_n(Ctx& c, int nfru, int nfa, double E)
                                                                             nfa, Rlo, c.part, 0LL);
     };
     c.launches++;
-    if (c.tune_adj < 0 && nt >= 256) {
+    if (nfa - nfru == 1) {
+        k_adjoint_row<N><<<(unsigned)nt, TILE, 0, c.stream>>>(c.sp, c.coef, c.Pd, c.bra, c.ket, c.ketn, c.detL, c.diagS,
+                                                              c.c, E, nfru, Rlo, c.part, 0LL);
+    } else if (c.tune_adj < 0 && nt >= 256) {
         const int r = tune(c, ADJ_SHAPES, c.tune_adj, c.tune_adj_ms, run);
         if (r) return r;
     } else {
@@ -1419,6 +1541,12 @@ static int adjoint_tiles_n(Ctx& c, int nfru, int nfa, double E, const cd* cvec, 
                            double* part)
 {
     if (nfa <= nfru || count <= 0) return 0;
+    if (nfa - nfru == 1) {
+        k_adjoint_row<N><<<(unsigned)count, TILE, 0, c.stream>>>(c.sp, c.coef, c.Pd, c.bra, c.ket, c.ketn, c.detL,
+                                                                 c.diagS, cvec, E, nfru, nfru / TILE, part, t0);
+        c.launches++;
+        return last_err();
+    }
     constexpr size_t smem = adjoint_smem<N>();
     if (cudaFuncSetAttribute(k_adjoint<N, 8, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
