@@ -276,7 +276,7 @@ int ldlp_grid(Ctx& c);
 int ldlp_tasks(Ctx& c, int n, unsigned** tasks, int* count);
 long long ldlp_task_total(int n);
 int ldlp_reserve(Ctx& c, int np);
-void ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long long* trace = nullptr);
+int ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long long* trace = nullptr);
 // One persistent factorisation of rows 0..n-1 of the current matrix with a
 // per-task timing record (4 values per task, see ecg_factor_trace).
 int ldlh_factor_traced(Ctx& c, int n, unsigned long long* out, long long cap, long long* count);

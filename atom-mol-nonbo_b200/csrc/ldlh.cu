@@ -707,17 +707,18 @@ static void enqueue_factor(Ctx& c, int m0, int n, const std::vector<int>& starts
 // A whole factorisation (m0 = 0) as one persistent kernel (ldlp.cu): the
 // working upper triangle and diagonal, the tile tasks (which leave the
 // inverse diagonal blocks), then the neighbour products of the solves.
-static void enqueue_persist(Ctx& c, int n, const unsigned* tasks, int ntasks, bool solves,
+static int enqueue_persist(Ctx& c, int n, const unsigned* tasks, int ntasks, bool solves,
                             unsigned long long* trace = nullptr)
 {
     const int ct1 = (n + 31) / 32;
     k_ldl_mirror<<<dim3(ct1, ct1), 256, 0, c.stream>>>(c.F, c.ld, 0, n, c.dw, 0);
     c.launches++;
-    ldlp_enqueue(c, n, tasks, ntasks, trace);
-    if (!solves) return;
+    const int r = ldlp_enqueue(c, n, tasks, ntasks, trace);
+    if (r || !solves) return r;
     const int nblk = (n + LDL_NB - 1) / LDL_NB;
     k_ldl_mn<<<dim3(nblk, 2), 256, MN_SMEM, c.stream>>>(c.F, c.ld, c.dblk, nblk, 0, c.linv, c.lmf, c.lnb);
     c.launches++;
+    return 0;
 }
 
 static void ldl_attrs()
@@ -788,21 +789,20 @@ int ldlh_factor(Ctx& c, int m0, int n, bool solves)
             const int t = ldlp_tasks(c, n, &tasks, &ntasks);
             if (t) return t;
         }
-        auto enqueue = [&]() {
-            if (persist)
-                enqueue_persist(c, n, tasks, ntasks, solves);
-            else
-                enqueue_factor(c, m0, n, starts, nexist);
+        auto enqueue = [&]() -> int {
+            if (persist) return enqueue_persist(c, n, tasks, ntasks, solves);
+            enqueue_factor(c, m0, n, starts, nexist);
+            return 0;
         };
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         bool ok = cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
         if (ok) {
             const long long l0 = c.launches;
-            enqueue();
+            const int r = enqueue();
             c.graph_launches = c.launches - l0;
             c.launches = l0;
-            ok = cudaStreamEndCapture(c.stream, &graph) == cudaSuccess && graph &&
+            ok = cudaStreamEndCapture(c.stream, &graph) == cudaSuccess && graph && r == 0 &&
                  cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
         }
         if (graph) cudaGraphDestroy(graph);
@@ -820,8 +820,7 @@ int ldlh_factor(Ctx& c, int m0, int n, bool solves)
                 c.lp_direct_n = n;
                 c.lp_direct_count = ntasks;
             }
-            enqueue();
-            if (cudaGetLastError() != cudaSuccess) return -2;
+            if (enqueue() || cudaGetLastError() != cudaSuccess) return -2;
             c.blk_start = solves ? starts : std::vector<int>();
             c.fact_n = solves ? n : 0;
             return 0;
@@ -875,10 +874,9 @@ int ldlh_factor_traced(Ctx& c, int n, unsigned long long* out, long long cap, lo
         cudaFree(tasks);
         return -3;
     }
-    enqueue_persist(c, n, tasks, ntasks, true, d);
+    int r = enqueue_persist(c, n, tasks, ntasks, true, d);
     unsigned recs = 0;
     const size_t ntile = (size_t)nb * (nb + 1) / 2;  // trace records at ctl[2], ctl = counters + 2 ntile
-    int r = 0;
     if (cudaMemcpyAsync(&recs, c.lp_cnt + 2 * ntile + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, c.stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(c.stream) != cudaSuccess)

@@ -47,6 +47,7 @@
 #include <queue>
 #include <utility>
 #include <vector>
+#include <cuda.h>  // CUtensorMap
 #include "ecg_internal.h"
 #include "zmma.cuh"
 
@@ -54,11 +55,12 @@ namespace ecg {
 
 constexpr unsigned LP_D = 0, LP_T = 1, LP_B = 2;
 constexpr unsigned LP_NONE = 0xffffffffu;
-constexpr int LP_KC = 16;          // k rows per cp.async stage of an update
-constexpr int LP_P = 66;           // pitch (double2) of the staged operands: 2 mod 8, conflict-free fragments
-constexpr int LP_ST = 3;           // stages
+constexpr int LP_KC = 8;           // k rows per TMA stage of an update: 128 bytes, the width of the swizzle
+constexpr int LP_ST = 6;           // stages
+constexpr int LP_OP = LP_KC * LDL_NB;  // double2 of one staged operand (8 KB)
 constexpr int LP_MERGE = 4;        // most panels one trailing update applies at once
-constexpr size_t LP_SMEM_B = (size_t)(LP_ST * LP_KC * 2 * LP_P + LP_MERGE * LDL_NB) * sizeof(double2);
+// 1 KB to align the stages, which the swizzle wants
+constexpr size_t LP_SMEM_B = 1024 + (size_t)(LP_ST * 2 * LP_OP + LP_MERGE * LDL_NB) * sizeof(double2);
 
 __host__ __device__ __forceinline__ unsigned lp_code(unsigned type, int s, int R, int C, unsigned half = 0)
 {
@@ -269,6 +271,55 @@ __device__ __forceinline__ bool lp_wait(const unsigned* p, unsigned v, unsigned*
     return true;
 }
 
+// ---------------------------------------------------------------------------
+// TMA and mbarriers of the updates.
+// ---------------------------------------------------------------------------
+constexpr int LP_TMA_LIMIT = 1 << 21;  // bound on the polls for a copy or a stage (tens of ms)
+
+__device__ __forceinline__ unsigned lp_s32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void lp_bar_init(unsigned bar, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void lp_bar_arrive(unsigned bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void lp_bar_expect(unsigned bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Wait for the phase of the given parity to end; false when the limit runs out.
+__device__ __forceinline__ bool lp_bar_wait(unsigned bar, unsigned parity)
+{
+    for (int i = 0; i < LP_TMA_LIMIT; i++) {
+        unsigned done;
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+    }
+    return false;
+}
+// Box of 8 complex rows from row k0 (16 doubles, x = 2 k0: 16-byte aligned)
+// and the map's columns from column c.
+__device__ __forceinline__ void lp_tma(unsigned dst, const CUtensorMap* map, int k0, int c, unsigned bar)
+{
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            dst),
+        "l"(map), "r"(2 * k0), "r"(c), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void lp_fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
+__device__ __forceinline__ void lp_fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 // T(s, C): U(s, C) = invD Linv_ss W(s, C) for the 64 columns of tile (s, C),
 // Linv_ss = L_ss^-1 (unit lower) as the diagonal task left it: one product
 // with a triangular matrix on the FP64 tensor cores, 288 independent-ordered
@@ -351,139 +402,12 @@ __device__ void lp_panel(cd* __restrict__ A, int ld, int n, int s, int C, const 
                 A[(size_t)(p0 + 8 * m + g) + (size_t)(cb + c) * ld] = cmul(cd{accr[m][e], acci[m][e]}, cd{d.x, d.y});
         }
     }
+    lp_fence_async_global();  // read by TMA in the updates
+    lp_fence_async_shared();  // and this memory is written by TMA next
 }
 
-// B(s, R, C): W(r, c) -= sum_q conj(U(q, r)) d_q U(q, c) over the 64 x 64
-// tile, r <= c on a diagonal tile (its diagonal in dw).  Eight warps as
-// 2 x 4, each a 32 x 16 complex sub-tile of 8 x 8 mma tiles; the tile's
-// old values are the accumulators' initial values (the minus sign is folded
-// into the operand -d U(q, c)), so a product is accumulated straight onto
-// them; U(s, R) and U(s, C) stream through three cp.async stages of 16 k
-// rows.  m consecutive panels s..s+m-1 (whose rows are contiguous) are
-// applied in one pass when they are all ready: a rank-64m update, the
-// tile read and written once.
-// MT x NT mma tiles per warp, WR x WC warps: <4, 2, 2, 4> covers the whole
-// 64 x 64 tile, <2, 2, 4, 2> the 64 x 32 column half `half` of it.
-template <int MT, int NT, int WR, int WC>
-__device__ void lp_update(cd* __restrict__ A, int ld, int n, int s, int m, int R, int C, int half,
-                          cd* __restrict__ dw, double2* sm)
-{
-    static_assert(WR * WC == 8 && WR * MT * 8 == LDL_NB, "eight warps over the 64 tile rows");
-    constexpr int CW = WC * NT * 8;  // columns covered
-    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int wr = wp / WC, wc = wp % WC;
-    const int g = lane >> 2, t4 = lane & 3;
-    const int p0 = s * LDL_NB, b = min(m * LDL_NB, n - p0);
-    const int rb = R * LDL_NB, cb = C * LDL_NB + half * CW;
-    const bool dtile = (R == C);
-    double2* dp = sm + LP_ST * LP_KC * 2 * LP_P;  // pivots d_q of panels s..s+m-1
-    for (int q = tid; q < m * LDL_NB; q += 256) dp[q] = q < b ? lp_ldcg(dw + p0 + q) : make_double2(0.0, 0.0);
-    // a warp whose sub-tile lies wholly below the diagonal has nothing to do
-    const bool wact = !dtile || (wr * MT * 8 <= half * CW + (wc + 1) * NT * 8 - 1);
-    auto stage = [&](int ch, int buf) {
-        const int k0 = ch * LP_KC;
-        double2* Us = sm + buf * LP_KC * 2 * LP_P;
-        double2* Vs = Us + LP_KC * LP_P;
-#pragma unroll
-        for (int e = tid; e < LP_KC * LDL_NB; e += 256) {
-            const int q = e % LP_KC, mm = e / LP_KC;
-            const bool kq = k0 + q < b;
-            const int r = rb + mm;
-            const bool ku = kq && r < n;
-            cp_async16(Us + q * LP_P + mm, ku ? (const void*)(A + (size_t)(p0 + k0 + q) + (size_t)r * ld) : (const void*)A,
-                       ku ? 16 : 0);
-        }
-#pragma unroll
-        for (int e = tid; e < LP_KC * CW; e += 256) {
-            const int q = e % LP_KC, mm = e / LP_KC;
-            const int c = cb + mm;
-            const bool kv = (k0 + q < b) && c < n;
-            cp_async16(Vs + q * LP_P + mm, kv ? (const void*)(A + (size_t)(p0 + k0 + q) + (size_t)c * ld) : (const void*)A,
-                       kv ? 16 : 0);
-        }
-        cp_async_commit();
-    };
-    const int nch = (b + LP_KC - 1) / LP_KC;
-    stage(0, 0);
-    if (nch > 1) stage(1, 1);
-    double accr[MT][NT][2], acci[MT][NT][2];
-#pragma unroll
-    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int r = rb + (wr * MT + mt) * 8 + g;
-                const int c = cb + (wc * NT + nt) * 8 + 2 * t4 + e;
-                double2 o = make_double2(0.0, 0.0);
-                if (r < n && c < n && r <= c) {
-                    if (r == c) {
-                        o = lp_ldcg(dw + c);
-                        o.y = -o.y;  // dw keeps the conjugate of the upper-triangle value
-                    } else {
-                        o = lp_ldcg(A + (size_t)r + (size_t)c * ld);
-                    }
-                }
-                accr[mt][nt][e] = o.x;
-                acci[mt][nt][e] = o.y;
-            }
-    for (int ch = 0; ch < nch; ch++) {
-        if (ch + 2 < nch) {
-            __syncthreads();  // buffer (ch + 2) % 3 was read in step ch - 1
-            stage(ch + 2, (ch + 2) % LP_ST);
-            cp_async_wait<2>();
-        } else if (ch + 1 < nch) {
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        if (wact) {
-            const double2* Us = sm + (ch % LP_ST) * LP_KC * 2 * LP_P;
-            const double2* Vs = Us + LP_KC * LP_P;
-#pragma unroll
-            for (int kk = 0; kk < LP_KC; kk += 4) {
-                const double2 d = dp[ch * LP_KC + kk + t4];
-                double2 a[MT];
-                double vr[NT], vi[NT];
-#pragma unroll
-                for (int mt = 0; mt < MT; mt++) a[mt] = Us[(kk + t4) * LP_P + (wr * MT + mt) * 8 + g];
-#pragma unroll
-                for (int nt = 0; nt < NT; nt++) {
-                    const double2 v = Vs[(kk + t4) * LP_P + (wc * NT + nt) * 8 + g];
-                    // -(d v): the unscaled row, negated
-                    vr[nt] = -fma(v.x, d.x, -v.y * d.y);
-                    vi[nt] = -fma(v.x, d.y, v.y * d.x);
-                }
-#pragma unroll
-                for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-                    for (int nt = 0; nt < NT; nt++) {
-                        lp_mma(accr[mt][nt][0], accr[mt][nt][1], a[mt].x, vr[nt]);
-                        lp_mma(accr[mt][nt][0], accr[mt][nt][1], a[mt].y, vi[nt]);
-                        lp_mma(acci[mt][nt][0], acci[mt][nt][1], a[mt].x, vi[nt]);
-                        lp_mma(acci[mt][nt][0], acci[mt][nt][1], -a[mt].y, vr[nt]);
-                    }
-            }
-        }
-    }
-#pragma unroll
-    for (int mt = 0; mt < MT; mt++)
-#pragma unroll
-        for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int r = rb + (wr * MT + mt) * 8 + g;
-                const int c = cb + (wc * NT + nt) * 8 + 2 * t4 + e;
-                if (r >= n || c >= n || c < r) continue;
-                if (c == r)
-                    dw[c] = cd{accr[mt][nt][e], -acci[mt][nt][e]};
-                else
-                    A[(size_t)r + (size_t)c * ld] = cd{accr[mt][nt][e], acci[mt][nt][e]};
-            }
-}
-
-struct LpArgs {
+struct alignas(64) LpArgs {
+    CUtensorMap t64, t32;   // F's rows 0..n-1 as doubles by columns: boxes of 8 complex rows x 64 and x 32 columns
     cd* A;
     int ld, n, np;
     const unsigned* tasks;  // the list of the CTAs other than the chain CTA
@@ -499,6 +423,168 @@ struct LpArgs {
     const int* limitp;      // poll limit of the bounded waits
     unsigned long long* trace;  // optional: per task (code | cta << 32 | panels << 48, start, ready, done)
 };
+
+// The stages' ring as it goes on from one update to the next: the next
+// stage and the parity of its current use.
+struct LpRing {
+    unsigned full, empty;  // shared addresses of LP_ST mbarriers each
+    int st = 0;
+    unsigned ph = 0;
+    __device__ __forceinline__ void step(int& i, unsigned& p) const
+    {
+        if (++i == LP_ST) {
+            i = 0;
+            p ^= 1u;
+        }
+    }
+};
+
+// B(s, R, C): W(r, c) -= sum_q conj(U(q, r)) d_q U(q, c) over the 64 x 64
+// tile, r <= c on a diagonal tile (its diagonal in dw).  Eight warps as
+// 2 x 4, each a 32 x 16 complex sub-tile of 8 x 8 mma tiles; the tile's
+// old values are the accumulators' initial values (the minus sign is folded
+// into the operand -d U(q, c)), so a product is accumulated straight onto
+// them.  m consecutive panels s..s+m-1 (whose rows are contiguous) are
+// applied in one pass when they are all ready: a rank-64m update, the
+// tile read and written once.
+// U(s, R) and U(s, C) come by TMA, eight k rows a stage, through a ring of
+// LP_ST stages: thread 0 refills a stage once the eight warps have left it
+// (two chunks behind its own), each warp waits only for its data, and no
+// barrier stands between chunks.  The 128-byte swizzle puts row k of column
+// c at 16-byte slot c * 8 + (k ^ (c & 7)); with the columns of an 8 x 8 mma
+// tile taken in the order p(g) = 0 4 1 5 2 6 3 7 a quarter-warp's fragment
+// load meets eight different bank groups.  What bounds it: the FP64 tensor
+// cores (8.4 us of an SM per panel).  Two CTAs an SM, four panels a pass:
+// XX us per panel and SM against 12.3 with cp.async stages and two barriers
+// a chunk, whose address arithmetic and waits kept the pipe at 68 %.
+// MT x NT mma tiles per warp, WR x WC warps: <4, 2, 2, 4> covers the whole
+// 64 x 64 tile, <2, 2, 4, 2> the 64 x 32 column half `half` of it.
+template <bool CPLX, int MT, int NT, int WR, int WC>
+__device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half, double2* sm, LpRing& ring)
+{
+    static_assert(WR * WC == 8 && WR * MT * 8 == LDL_NB, "eight warps over the 64 tile rows");
+    constexpr int CW = WC * NT * 8;  // columns covered
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
+    const int wr = wp / WC, wc = wp % WC;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int pg = (g & 1) << 2 | g >> 1;
+    const int n = a.n, ld = a.ld;
+    cd* __restrict__ A = a.A;
+    const int p0 = s * LDL_NB;
+    const int rb = R * LDL_NB, cb = C * LDL_NB + half * CW;
+    const bool dtile = (R == C);
+    const unsigned base = (lp_s32(sm) + 1023u) & ~1023u;
+    double2* stages = sm + (base - lp_s32(sm)) / sizeof(double2);
+    double2* dp = stages + LP_ST * 2 * LP_OP;  // pivots d_q of panels s..s+m-1
+    const int nch = m * (LDL_NB / LP_KC);      // panels with rows below them are whole
+    auto issue = [&](int ch, int st) {
+        const unsigned bar = ring.full + 8u * st, dst = base + (unsigned)(st * 2 * LP_OP * sizeof(double2));
+        lp_bar_expect(bar, (unsigned)((LP_OP + LP_KC * CW) * sizeof(double2)));
+        lp_tma(dst, &a.t64, p0 + ch * LP_KC, rb, bar);
+        lp_tma(dst + (unsigned)(LP_OP * sizeof(double2)), CW == LDL_NB ? &a.t64 : &a.t32, p0 + ch * LP_KC, cb, bar);
+    };
+    // the stage refilled next (thread 0) and the parity its last use ends with
+    int rst = ring.st;
+    unsigned rph = ring.ph;
+    if (tid == 0) {
+        lp_fence_async_global();  // the panel rows were written by other CTAs' ordinary stores
+        int st = ring.st;
+        unsigned ph = ring.ph;
+        for (int ch = 0; ch < min(LP_ST, nch); ch++) {
+            issue(ch, st);
+            ring.step(st, ph);
+        }
+    }
+    for (int q = tid; q < m * LDL_NB; q += 256) dp[q] = lp_ldcg(a.dw + p0 + q);
+    // a warp whose sub-tile lies wholly below the diagonal has nothing to do
+    const bool wact = !dtile || (wr * MT * 8 <= half * CW + (wc + 1) * NT * 8 - 1);
+    double accr[MT][NT][2], acci[MT][NT][2];
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int r = rb + (wr * MT + mt) * 8 + pg;
+                const int c = cb + (wc * NT + nt) * 8 + 4 * e + t4;
+                double2 o = make_double2(0.0, 0.0);
+                if (r < n && c < n && r <= c) {
+                    if (r == c) {
+                        o = lp_ldcg(a.dw + c);
+                        o.y = -o.y;  // dw keeps the conjugate of the upper-triangle value
+                    } else {
+                        o = lp_ldcg(A + (size_t)r + (size_t)c * ld);
+                    }
+                }
+                accr[mt][nt][e] = o.x;
+                acci[mt][nt][e] = o.y;
+            }
+    __syncthreads();  // dp
+    bool ok = true;
+    const int f0 = pg * LP_KC + (t4 ^ pg);  // fragment slots of k = t4 and, with ^ 4, of k = 4 + t4
+    for (int ch = 0; ch < nch; ch++) {
+        ok = lp_bar_wait(ring.full + 8u * ring.st, ring.ph);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        if (wact) {
+            const double2* Us = stages + ring.st * 2 * LP_OP + (wr * MT) * 64;
+            const double2* Vs = stages + ring.st * 2 * LP_OP + LP_OP + (wc * NT) * 64;
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int f = f0 ^ (4 * j);
+                const double2 d = dp[ch * LP_KC + 4 * j + t4];
+                double2 u[MT];
+                double vr[NT], vi[NT];
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) u[mt] = Us[mt * 64 + f];
+#pragma unroll
+                for (int nt = 0; nt < NT; nt++) {
+                    const double2 v = Vs[nt * 64 + f];
+                    // -(d v): the unscaled row, negated
+                    vr[nt] = CPLX ? -fma(v.x, d.x, -v.y * d.y) : -v.x * d.x;
+                    vi[nt] = CPLX ? -fma(v.x, d.y, v.y * d.x) : -v.y * d.x;
+                }
+#pragma unroll
+                for (int nt = 0; nt < NT; nt++) {
+                    const double nr = -vr[nt];
+#pragma unroll
+                    for (int mt = 0; mt < MT; mt++) {
+                        lp_mma(accr[mt][nt][0], accr[mt][nt][1], u[mt].x, vr[nt]);
+                        lp_mma(acci[mt][nt][0], acci[mt][nt][1], u[mt].x, vi[nt]);
+                    }
+#pragma unroll
+                    for (int mt = 0; mt < MT; mt++) {
+                        lp_mma(accr[mt][nt][0], accr[mt][nt][1], u[mt].y, vi[nt]);
+                        lp_mma(acci[mt][nt][0], acci[mt][nt][1], u[mt].y, nr);
+                    }
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) lp_bar_arrive(ring.empty + 8u * ring.st);
+        ring.step(ring.st, ring.ph);
+        if (tid == 0 && ch >= 2 && ch - 2 + LP_ST < nch) {
+            // (without its stage a chunk is not asked for, and its wait runs out)
+            if (lp_bar_wait(ring.empty + 8u * rst, rph)) issue(ch - 2 + LP_ST, rst);
+            ring.step(rst, rph);
+        }
+    }
+    if (__syncthreads_or(ok ? 0 : 1)) return false;
+#pragma unroll
+    for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int r = rb + (wr * MT + mt) * 8 + pg;
+                const int c = cb + (wc * NT + nt) * 8 + 4 * e + t4;
+                if (r >= n || c >= n || c < r) continue;
+                if (c == r)
+                    a.dw[c] = cd{accr[mt][nt][e], -acci[mt][nt][e]};
+                else
+                    A[(size_t)r + (size_t)c * ld] = cd{accr[mt][nt][e], acci[mt][nt][e]};
+            }
+    return true;
+}
 
 __device__ __forceinline__ unsigned long long lp_clock()
 {
@@ -568,15 +654,17 @@ __device__ __forceinline__ void lp_trace(const LpArgs& a, unsigned code, int m, 
 
 // One task, all threads.  Thread 0 has checked the dependencies; on return
 // the task's stores are done (a barrier follows).  m: panels of an update.
-__device__ __forceinline__ void lp_exec(const LpArgs& a, unsigned type, int s, int m, int R, int C, int half,
-                                        double2* sm)
+// False when a copy did not arrive.
+template <bool CPLX>
+__device__ __forceinline__ bool lp_exec(const LpArgs& a, unsigned type, int s, int m, int R, int C, int half,
+                                        double2* sm, LpRing& ring)
 {
-    if (type == LP_T)
+    if (type == LP_T) {
         lp_panel(a.A, a.ld, a.n, s, C, a.invD, a.linv, sm);
-    else if (lp_split(s, R, C))
-        lp_update<2, 2, 4, 2>(a.A, a.ld, a.n, s, 1, R, C, half, a.dw, sm);
-    else
-        lp_update<4, 2, 2, 4>(a.A, a.ld, a.n, s, m, R, C, 0, a.dw, sm);
+        return true;
+    }
+    if (lp_split(s, R, C)) return lp_update<CPLX, 2, 2, 4, 2>(a, s, 1, R, C, half, sm, ring);
+    return lp_update<CPLX, 4, 2, 2, 4>(a, s, m, R, C, 0, sm, ring);
 }
 
 // After the task's barrier: thread 0 publishes the tile's new count.  The
@@ -616,7 +704,8 @@ constexpr int LC_UP = 57;  // pitch of the shared rows of U (columns 8..63): 1 m
 constexpr int LC_XP = 9;   // pitch of X_b
 constexpr size_t LP_SMEM_C = (size_t)(LI_N + LDL_NB * LT_WP + 2 * LDL_NB + 8 * LC_UP + 8 * LC_XP) * sizeof(double2);
 constexpr size_t lp_max(size_t a, size_t b) { return a > b ? a : b; }
-constexpr size_t LP_SMEM = lp_max(LP_SMEM_B, lp_max(LP_SMEM_C, LP_SMEM_T));
+constexpr size_t LP_SMEM_BAR = lp_max(LP_SMEM_B, lp_max(LP_SMEM_C, LP_SMEM_T));  // the ring's mbarriers
+constexpr size_t LP_SMEM = LP_SMEM_BAR + 2 * LP_ST * 8;
 
 // 1/d of a normal d, without a branch: the hardware's seed y (about 20 bits)
 // and the geometric series of 1 / (1 - e), e = 1 - d y, to e^2 (remainder
@@ -952,6 +1041,7 @@ __device__ void lp_chain(const LpArgs& a, double2* sm, int limit)
                 }
             }
         }
+        lp_fence_async_global();
         __syncthreads();
         lp_publish(a, lp_tix(s, s + 1), (unsigned)s + 1);
         if (tid == 0) lp_trace(a, lp_code(LP_T, s, s, s + 1), 1, t0, t1);
@@ -979,7 +1069,7 @@ __device__ void lp_chain(const LpArgs& a, double2* sm, int limit)
 // panels s+1.. (up to LP_MERGE in all, below R) whose panel rows of R and
 // C are already final.
 template <bool CPLX>
-__global__ void __launch_bounds__(256, 2) k_ldl_persist(LpArgs a)
+__global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ LpArgs a)
 {
     extern __shared__ double2 lsm[];
     __shared__ unsigned s_next;
@@ -1015,6 +1105,17 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(LpArgs a)
         lp_chain<CPLX>(a, lsm, limit);
         return;
     }
+    LpRing ring;
+    ring.full = lp_s32(lsm) + (unsigned)LP_SMEM_BAR;
+    ring.empty = ring.full + 8u * LP_ST;
+    if (tid == 0) {
+        for (int i = 0; i < LP_ST; i++) {
+            lp_bar_init(ring.full + 8u * i, 1);
+            lp_bar_init(ring.empty + 8u * i, 8);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
     for (;;) {
         unsigned long long t0 = 0, t1 = 0;
         if (tid == 0) {
@@ -1076,7 +1177,15 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(LpArgs a)
         const int s = (task >> 20) & 511, R = (task >> 10) & 1023, C = task & 1023;
         const int half = (task >> 29) & 1;
         if (go == 1) {
-            lp_exec(a, type, s, m, R, C, half, lsm);
+            if (!lp_exec<CPLX>(a, type, s, m, R, C, half, lsm, ring)) {
+                // a copy did not arrive: wait for the others in flight, report, stop
+                for (int i = 0; i < LP_ST; i++) lp_bar_wait(ring.full + 8u * i, ring.ph);
+                if (tid == 0) {
+                    atomicExch(a.status + ST_SOLVE_TIMEOUT, 1);
+                    atomicExch(a.ctl + 1, 1u);
+                }
+                return;
+            }
             __syncthreads();
             const long long tt = (type == LP_B) ? lp_tix(R, C) : lp_tix(s, (type == LP_D) ? s : C);
             if (type == LP_B && lp_split(s, R, C)) {
@@ -1096,6 +1205,27 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(LpArgs a)
 }
 
 static bool g_lp_attr = false;
+
+// Tensor map of the n x n matrix at A (column-major complex) as doubles by
+// columns, boxes of LP_KC complex rows x `cols` columns, 128-byte swizzle.
+static bool lp_map(CUtensorMap* map, void* A, int ld, int n, int cols)
+{
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess || !fn) {
+        cudaGetLastError();
+        return false;
+    }
+    const cuuint64_t dim[2] = {2 * (cuuint64_t)n, (cuuint64_t)n}, stride[1] = {(cuuint64_t)ld * sizeof(cd)};
+    const cuuint32_t box[2] = {2 * LP_KC, (cuuint32_t)cols}, one[2] = {1, 1};
+    return reinterpret_cast<Encode>(fn)(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, A, dim, stride, box, one,
+                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // Grid of the persistent kernel (co-resident CTAs), 0 if unavailable.
 int ldlp_grid(Ctx& c)
@@ -1181,12 +1311,13 @@ int ldlp_reserve(Ctx& c, int np)
 // Queue one persistent factorisation of rows 0..n-1 (the working upper
 // triangle and dw already initialised by k_ldl_mirror); trace (device,
 // 4 x ldlp_task_total(n) values) may be null.
-void ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long long* trace)
+int ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long long* trace)
 {
     const int np = (n + LDL_NB - 1) / LDL_NB;
     const size_t ntile = (size_t)np * (np + 1) / 2;
     cudaMemsetAsync(c.lp_cnt, 0, (3 * ntile + 4) * sizeof(unsigned), c.stream);
     LpArgs a;
+    if (!lp_map(&a.t64, c.F, c.ld, n, LDL_NB) || !lp_map(&a.t32, c.F, c.ld, n, LDL_NB / 2)) return -2;
     a.A = c.F;
     a.ld = c.ld;
     a.n = n;
@@ -1218,6 +1349,7 @@ void ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned lon
     else
         cudaLaunchKernelEx(&cfg, k_ldl_persist<false>, a);
     c.launches++;
+    return 0;
 }
 
 }  // namespace ecg
