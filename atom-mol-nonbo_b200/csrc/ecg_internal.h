@@ -17,9 +17,13 @@ constexpr int SOLVE_SPIN_LIMIT = 1 << 22;
 
 // LDL^H block size (rows of one panel).
 constexpr int LDL_NB = 64;
-// Factorisations of at least this many new rows take the panels in pairs
-// with rank-128 trailing updates (ldlh.cu); the buffers of unscaled panel
-// rows hold a pair's rows per column.
+// Whole factorisations of at most this many rows run as the persistent tile
+// kernel (its task codes hold 200 panels; at K = 10000 it measures 47.2 ms
+// against 57.2 with one launch per panel step).
+constexpr int LDL_PERSIST_MAX = 12800;
+// Among the launch-per-panel factorisations (ldlh.cu) those of at least this
+// many new rows take the panels in pairs with rank-128 trailing updates; the
+// buffers of unscaled panel rows hold a pair's rows per column.
 constexpr int LDL_PAIR_MIN = 6000;
 constexpr int LDL_VLD = 2 * LDL_NB;
 

@@ -21,7 +21,7 @@
 // src/linalg.f90:359-391 term for term; only the summation order differs,
 // and the pivots are kept real (the reference's complex arithmetic leaves a
 // rounding-level imaginary part in them).
-// A whole factorisation (m0 = 0) below LDL_PAIR_MIN rows runs instead as
+// A whole factorisation (m0 = 0) of up to LDL_PERSIST_MAX rows runs instead as
 // the persistent tile kernel of ldlp.cu; ldlh_factor captures either form
 // into a CUDA graph.
 #include "ecg_internal.h"
@@ -761,10 +761,7 @@ int ldlh_factor(Ctx& c, int m0, int n, bool solves)
     if (cudaMemcpyAsync(c.dblk, c.bounds_h, (nb + 1) * sizeof(int), cudaMemcpyHostToDevice, c.stream) !=
         cudaSuccess)
         return -2;
-    // whole factorisations take the persistent kernel below LDL_PAIR_MIN
-    // rows (at 10000 rows the panel pairs' rank-128 launches measured 57.2
-    // against its 59.4 ms)
-    const bool persist = (m0 == 0 && n > 0 && n < LDL_PAIR_MIN && c.factor_mode == 0 && ldlp_grid(c) > 0);
+    const bool persist = (m0 == 0 && n > 0 && n <= LDL_PERSIST_MAX && c.factor_mode == 0 && ldlp_grid(c) > 0);
     if (m0 > 0 && n - m0 == 1) {
         const int r = border_row(c, m0, nexist);
         if (r <= 0) {

@@ -38,8 +38,9 @@
 // DMMA share that unit), the chain's latency where few panels are left.  On a
 // B200 the chain takes 32 us a panel (D 18, T 9, B 4 and a part overlapped
 // with D; 47 us with an elimination through shared memory and substitution
-// in T), so whole factorisations take 0.32 ms at K = 500 (0.46 before),
-// 0.88 at 1500 (1.24), 4.45 at 4000 (4.94).  Two CTAs an SM take 217 KB of
+// in T), and the list's updates run at 95 % of the tensor cores, so whole
+// factorisations take 0.31 ms at K = 500 (0.46 before both), 0.88 at 1500
+// (1.24), 3.79 at 4000 (4.94), 47.2 at 10000 (57.2 per panel step).  Two CTAs an SM take 217 KB of
 // shared memory and leave about 28 KB of L1, so a spilled register comes back
 // from L2: the chain with 200 bytes of stack ran D(s) in 32 us, with 32 bytes
 // in 18.  Every array of the chain is sized to stay within 128 registers.
@@ -455,8 +456,9 @@ struct LpRing {
 // tile taken in the order p(g) = 0 4 1 5 2 6 3 7 a quarter-warp's fragment
 // load meets eight different bank groups.  What bounds it: the FP64 tensor
 // cores (8.4 us of an SM per panel).  Two CTAs an SM, four panels a pass:
-// XX us per panel and SM against 12.3 with cp.async stages and two barriers
-// a chunk, whose address arithmetic and waits kept the pipe at 68 %.
+// 17.6 us per panel and pair of CTAs (95 % of the pipe) against 22.0 with
+// cp.async stages and two barriers a chunk, whose address arithmetic and
+// waits kept the pipe at 68 % (ncu).
 // MT x NT mma tiles per warp, WR x WC warps: <4, 2, 2, 4> covers the whole
 // 64 x 64 tile, <2, 2, 4, 2> the 64 x 32 column half `half` of it.
 template <bool CPLX, int MT, int NT, int WR, int WC>
@@ -1263,7 +1265,7 @@ int ldlp_tasks(Ctx& c, int n, unsigned** tasks, int* count)
     const int grid = ldlp_grid(c);
     if (grid <= 0) return -1;
     const int np = (n + LDL_NB - 1) / LDL_NB;
-    if (np > 200) return -1;
+    if (n > LDL_PERSIST_MAX) return -1;
     const int per_sm = std::max(1, c.lp_grid / std::max(1, c.lp_sms));
     std::vector<unsigned> list;
     lp_schedule(np, std::max(1, grid - per_sm), LpCost(), list);
