@@ -60,6 +60,10 @@ constexpr int LP_KC = 8;           // k rows per TMA stage of an update: 128 byt
 constexpr int LP_ST = 6;           // stages
 constexpr int LP_OP = LP_KC * LDL_NB;  // double2 of one staged operand (8 KB)
 constexpr int LP_MERGE = 4;        // most panels one trailing update applies at once
+// Aligned groups of LP_MERGE panels whose update of a tile row at least this
+// far from the group's first panel is one task of the list: nearer rows are
+// wanted before the group's last panel is there.
+constexpr int LP_FAR = 8;
 // 1 KB to align the stages, which the swizzle wants
 constexpr size_t LP_SMEM_B = 1024 + (size_t)(LP_ST * 2 * LP_OP + LP_MERGE * LDL_NB) * sizeof(double2);
 
@@ -74,6 +78,12 @@ __host__ __device__ __forceinline__ bool lp_split(int s, int R, int C)
 {
     return R <= s + 2 && !(R == s + 1 && C == s + 1);
 }
+// One list task for panels s..s+LP_MERGE-1 on tile (R, C) (s a multiple of
+// LP_MERGE); its code has the half bit, which whole updates do not use.
+__host__ __device__ __forceinline__ bool lp_grouped(int s, int R)
+{
+    return R >= s - s % LP_MERGE + LP_FAR;
+}
 // counter of tile (R, C), R <= C: column-wise packed triangle
 __host__ __device__ __forceinline__ long long lp_tix(int R, int C) { return (long long)C * (C + 1) / 2 + R; }
 
@@ -83,50 +93,60 @@ __host__ __device__ __forceinline__ long long lp_tix(int R, int C) { return (lon
 // Task weights (us) for the list scheduler: the time a CTA is held by a
 // task on a B200 with two CTAs per SM, waits and merged updates included
 // (globaltimer records of ecg_factor_trace); a split update counts half.
-// Only the ratios matter: at K = 4000 this set measured 4.82 ms, the raw
-// run times (21, 24, 24, 15) 5.0 ms, and a T weighted above B 5.1-5.2 ms.
+// Only the ratios matter.  Measured for g (ms at K = 2500, 4000, 9000):
+// 75 1.62, 3.81, 33.5; 140 1.59, 3.61, 33.3; 180 1.55, 3.63, 33.2; 320
+// 1.55, 3.74, 33.3.  Per-panel tasks in place of groups: 1.52, 3.79, 34.9.
 struct LpCost {
-    double d = 21.0, t = 40.0, b = 60.0, bd = 40.0;
+    double d = 21.0, t = 40.0, b = 60.0, bd = 40.0, g = 180.0;  // g: one task for LP_MERGE panels
 };
 
 // Tasks of a factorisation with np panels: the list the P CTAs other than
 // the chain CTA take, and (if full is given) every task in the simulated
-// start order, the chain's included.
-static void lp_schedule(int np, int P, const LpCost& cost, std::vector<unsigned>& list,
+// start order, the chain's included.  With `group` the far updates are one
+// task for LP_MERGE panels: found merged one by one at run time they left
+// 440,000 empty tasks at K = 10000, and the list took the host 290 ms.
+static void lp_schedule(int np, int P, const LpCost& cost, bool group, std::vector<unsigned>& list,
                         std::vector<unsigned>* full = nullptr)
 {
     std::vector<unsigned> code;
-    std::vector<long long> idD(np);
-    std::vector<long long> idT((size_t)np * np, -1);
-    std::vector<long long> idB((size_t)np * np * np, -1);  // first node of B(s, R, C)
+    std::vector<int> idD(np);
+    std::vector<int> idT((size_t)np * np, -1);
+    std::vector<int> idB((size_t)np * np * np, -1);  // first node of B(s, R, C)
     auto bix = [&](int s, int R, int C) -> size_t { return ((size_t)s * np + R) * np + C; };
     for (int s = 0; s < np; s++) {
-        idD[s] = (long long)code.size();
+        idD[s] = (int)code.size();
         code.push_back(lp_code(LP_D, s, s, s));
         for (int C = s + 1; C < np; C++) {
-            idT[(size_t)s * np + C] = (long long)code.size();
+            idT[(size_t)s * np + C] = (int)code.size();
             code.push_back(lp_code(LP_T, s, s, C));
         }
         for (int R = s + 1; R < np; R++)
             for (int C = R; C < np; C++) {
-                idB[bix(s, R, C)] = (long long)code.size();
+                if (group && lp_grouped(s, R)) {  // created with the group's last panel
+                    if (s % LP_MERGE == LP_MERGE - 1) {
+                        idB[bix(s, R, C)] = (int)code.size();
+                        code.push_back(lp_code(LP_B, s - s % LP_MERGE, R, C, 1));
+                    }
+                    continue;
+                }
+                idB[bix(s, R, C)] = (int)code.size();
                 code.push_back(lp_code(LP_B, s, R, C));
                 if (lp_split(s, R, C)) code.push_back(lp_code(LP_B, s, R, C, 1));  // the second column half
             }
     }
-    const long long N = (long long)code.size();
+    const int N = (int)code.size();
     // predecessors in creation order, which is topological: an update that
     // is split in two column halves counts as both halves
     constexpr int NPRED = 6;
-    std::vector<long long> pred((size_t)N * NPRED, -1);
+    std::vector<int> pred((size_t)N * NPRED, -1);
     std::vector<double> w((size_t)N);
-    for (long long t = 0; t < N; t++) {
+    for (int t = 0; t < N; t++) {
         const unsigned c = code[t];
         const int type = c >> 30, s = (c >> 20) & 511, R = (c >> 10) & 1023, C = c & 1023;
-        long long* p = &pred[(size_t)t * NPRED];
+        int* p = &pred[(size_t)t * NPRED];
         int k = 0;
         auto addB = [&](int s2, int R2, int C2) {
-            const long long b = idB[bix(s2, R2, C2)];
+            const int b = idB[bix(s2, R2, C2)];
             p[k++] = b;
             if (lp_split(s2, R2, C2)) p[k++] = b + 1;
         };
@@ -138,32 +158,34 @@ static void lp_schedule(int np, int P, const LpCost& cost, std::vector<unsigned>
             if (s > 0) addB(s - 1, s, C);
             w[t] = cost.t;
         } else {
-            p[k++] = idT[(size_t)s * np + R];
-            if (C != R) p[k++] = idT[(size_t)s * np + C];
+            const bool g = group && lp_grouped(s, R);
+            const int last = g ? s + LP_MERGE - 1 : s;
+            p[k++] = idT[(size_t)last * np + R];
+            if (C != R) p[k++] = idT[(size_t)last * np + C];
             if (s > 0) addB(s - 1, R, C);
-            w[t] = ((R == C) ? cost.bd : cost.b) * (lp_split(s, R, C) ? 0.5 : 1.0);
+            w[t] = g ? cost.g : ((R == C) ? cost.bd : cost.b) * (lp_split(s, R, C) ? 0.5 : 1.0);
         }
     }
     // successors (CSR)
-    std::vector<long long> so((size_t)N + 1, 0), sl;
-    for (long long t = 0; t < N; t++)
+    std::vector<int> so((size_t)N + 1, 0), sl;
+    for (int t = 0; t < N; t++)
         for (int k = 0; k < NPRED; k++)
             if (pred[(size_t)t * NPRED + k] >= 0) so[(size_t)pred[(size_t)t * NPRED + k] + 1]++;
-    for (long long t = 0; t < N; t++) so[(size_t)t + 1] += so[(size_t)t];
+    for (int t = 0; t < N; t++) so[(size_t)t + 1] += so[(size_t)t];
     sl.resize((size_t)so[(size_t)N]);
     {
-        std::vector<long long> fill(so.begin(), so.end() - 1);
-        for (long long t = 0; t < N; t++)
+        std::vector<int> fill(so.begin(), so.end() - 1);
+        for (int t = 0; t < N; t++)
             for (int k = 0; k < NPRED; k++) {
-                const long long p = pred[(size_t)t * NPRED + k];
+                const int p = pred[(size_t)t * NPRED + k];
                 if (p >= 0) sl[(size_t)fill[(size_t)p]++] = t;
             }
     }
     // upward rank: own duration plus the longest path through the successors
     std::vector<double> rank((size_t)N);
-    for (long long t = N - 1; t >= 0; t--) {
+    for (int t = N - 1; t >= 0; t--) {
         double m = 0.0;
-        for (long long e = so[(size_t)t]; e < so[(size_t)t + 1]; e++) m = std::max(m, rank[(size_t)sl[(size_t)e]]);
+        for (int e = so[(size_t)t]; e < so[(size_t)t + 1]; e++) m = std::max(m, rank[(size_t)sl[(size_t)e]]);
         rank[(size_t)t] = w[(size_t)t] + m;
     }
     // list scheduling: the chain worker runs D(s), T(s, s+1), B(s, s+1,
@@ -172,24 +194,24 @@ static void lp_schedule(int np, int P, const LpCost& cost, std::vector<unsigned>
     // whenever one of them is free.  `full` receives every task in start
     // order.
     std::vector<char> pool((size_t)N, 1);  // 0 chain, 1 list
-    std::vector<long long> cseq;
+    std::vector<int> cseq;
     for (int s = 0; s < np; s++) {
         pool[(size_t)idD[s]] = 0;
         cseq.push_back(idD[s]);
         if (s + 1 < np) {
-            const long long t = idT[(size_t)s * np + s + 1], b = idB[bix(s, s + 1, s + 1)];
+            const int t = idT[(size_t)s * np + s + 1], b = idB[bix(s, s + 1, s + 1)];
             pool[(size_t)t] = pool[(size_t)b] = 0;
             cseq.push_back(t);
             cseq.push_back(b);
         }
     }
     std::vector<int> npred((size_t)N, 0);
-    for (long long t = 0; t < N; t++)
+    for (int t = 0; t < N; t++)
         for (int k = 0; k < NPRED; k++) npred[(size_t)t] += pred[(size_t)t * NPRED + k] >= 0;
-    typedef std::pair<double, long long> Item;
+    typedef std::pair<double, int> Item;
     std::priority_queue<Item> ready;                                        // (rank, -id)
     std::priority_queue<Item, std::vector<Item>, std::greater<Item>> busy;  // (finish, id)
-    for (long long t = 0; t < N; t++)
+    for (int t = 0; t < N; t++)
         if (npred[(size_t)t] == 0 && pool[(size_t)t]) ready.push({rank[(size_t)t], -t});
     list.clear();
     if (full) {
@@ -198,18 +220,18 @@ static void lp_schedule(int np, int P, const LpCost& cost, std::vector<unsigned>
     }
     int free_w[2] = {1, std::max(1, P)};
     size_t ci = 0;
-    long long started = 0;
+    int started = 0;
     double now = 0.0;
     while (started < N) {
         if (free_w[0] > 0 && ci < cseq.size() && npred[(size_t)cseq[ci]] == 0) {
-            const long long t = cseq[ci];
+            const int t = cseq[ci];
             if (full) full->push_back(code[(size_t)t]);
             busy.push({now + w[(size_t)t], t});
             free_w[0]--;
             started++;
         }
         while (free_w[1] > 0 && !ready.empty()) {
-            const long long t = -ready.top().second;
+            const int t = -ready.top().second;
             ready.pop();
             list.push_back(code[(size_t)t]);
             if (full) full->push_back(code[(size_t)t]);
@@ -224,8 +246,8 @@ static void lp_schedule(int np, int P, const LpCost& cost, std::vector<unsigned>
         const int fp = pool[(size_t)f.second];
         free_w[fp]++;
         if (fp == 0) ci++;
-        for (long long e = so[(size_t)f.second]; e < so[(size_t)f.second + 1]; e++) {
-            const long long q = sl[(size_t)e];
+        for (int e = so[(size_t)f.second]; e < so[(size_t)f.second + 1]; e++) {
+            const int q = sl[(size_t)e];
             if (--npred[(size_t)q] == 0 && pool[(size_t)q]) ready.push({rank[(size_t)q], -q});
         }
     }
@@ -254,22 +276,6 @@ __device__ __forceinline__ void lp_mma(double& c0, double& c1, double a, double 
 __device__ __forceinline__ cd lp_shfl(cd v, int src)
 {
     return cd{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
-}
-
-// Thread 0: wait until *p >= v.  False when this CTA must stop (the poll
-// limit ran out here or the abort word is set).
-__device__ __forceinline__ bool lp_wait(const unsigned* p, unsigned v, unsigned* ctl, int* status, int limit)
-{
-    int spins = 0;
-    while (lp_ld_acquire(p) < v) {
-        if (++spins > limit || *((volatile unsigned*)(ctl + 1)) != 0u) {
-            atomicExch(status + ST_SOLVE_TIMEOUT, 1);
-            atomicExch(ctl + 1, 1u);
-            return false;
-        }
-        __nanosleep(32);
-    }
-    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -608,9 +614,10 @@ __device__ __forceinline__ int lp_deps(unsigned task, long long (&ix)[3], unsign
         ix[1] = lp_tix(s, C), need[1] = (unsigned)s;
         return 2;
     }
+    const int last = lp_grouped(s, R) ? s + LP_MERGE - 1 : s;
     ix[0] = lp_tix(R, C), need[0] = (unsigned)s;
-    ix[1] = lp_tix(s, R), need[1] = (unsigned)s + 1;
-    ix[2] = lp_tix(s, C), need[2] = (unsigned)s + 1;
+    ix[1] = lp_tix(last, R), need[1] = (unsigned)last + 1;
+    ix[2] = lp_tix(last, C), need[2] = (unsigned)last + 1;
     return (R == C) ? 2 : 3;
 }
 
@@ -665,7 +672,7 @@ __device__ __forceinline__ bool lp_exec(const LpArgs& a, unsigned type, int s, i
         lp_panel(a.A, a.ld, a.n, s, C, a.invD, a.linv, sm);
         return true;
     }
-    if (lp_split(s, R, C)) return lp_update<CPLX, 2, 2, 4, 2>(a, s, 1, R, C, half, sm, ring);
+    if (!lp_grouped(s, R) && lp_split(s, R, C)) return lp_update<CPLX, 2, 2, 4, 2>(a, s, 1, R, C, half, sm, ring);
     return lp_update<CPLX, 4, 2, 2, 4>(a, s, m, R, C, 0, sm, ring);
 }
 
@@ -1136,9 +1143,11 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
                 long long ix[3] = {0, 0, 0};
                 unsigned need[3] = {0u, 0u, 0u};
                 const int k = lp_deps(task, ix, need);
-                const bool whole = type == LP_B && !lp_split(s, R, C);
+                const bool group = type == LP_B && lp_grouped(s, R);
+                const bool whole = type == LP_B && !group && !lp_split(s, R, C);
+                if (group) m = LP_MERGE;
                 go = lp_wait_all(a, ix, need, k, limit, whole);
-                if (go == 1 && type == LP_B) {
+                if (go == 1 && type == LP_B && !group) {
                     if (lp_ld_acquire(a.cnt + ix[0]) > (unsigned)s) {
                         go = 2;  // applied already by a merged update
                     } else if (whole) {
@@ -1146,7 +1155,7 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
                         unsigned fr[LP_MERGE - 1], fc[LP_MERGE - 1];
 #pragma unroll
                         for (int j = 1; j < LP_MERGE; j++) {
-                            const bool in = s + j < R;
+                            const bool in = s % LP_MERGE + j < LP_MERGE && s + j < R;
                             fr[j - 1] = in ? lp_ld_acquire(a.cnt + lp_tix(s + j, R)) : 0u;
                             fc[j - 1] = (in && R != C) ? lp_ld_acquire(a.cnt + lp_tix(s + j, C)) : 0u;
                         }
@@ -1158,7 +1167,7 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
                             // tasks: a long merged update would hold up the panel rows
                             // the chain waits for
                             const bool own = lp_split(s + j, R, C) || (s + j == R - 1);
-                            if (m == j && !own && s + j < R && fr[j - 1] >= want && (R == C || fc[j - 1] >= want))
+                            if (m == j && !own && s % LP_MERGE + j < LP_MERGE && s + j < R && fr[j - 1] >= want && (R == C || fc[j - 1] >= want))
                                 m = j + 1;
                         }
                         if (m > 1) *((volatile unsigned*)(a.cl + ix[0])) = (unsigned)(s + m);
@@ -1190,7 +1199,7 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
             }
             __syncthreads();
             const long long tt = (type == LP_B) ? lp_tix(R, C) : lp_tix(s, (type == LP_D) ? s : C);
-            if (type == LP_B && lp_split(s, R, C)) {
+            if (type == LP_B && !lp_grouped(s, R) && lp_split(s, R, C)) {
                 // a column half: the second of the two to finish publishes the tile
                 if (tid == 0) {
                     unsigned old;
@@ -1268,7 +1277,7 @@ int ldlp_tasks(Ctx& c, int n, unsigned** tasks, int* count)
     if (n > LDL_PERSIST_MAX) return -1;
     const int per_sm = std::max(1, c.lp_grid / std::max(1, c.lp_sms));
     std::vector<unsigned> list;
-    lp_schedule(np, std::max(1, grid - per_sm), LpCost(), list);
+    lp_schedule(np, std::max(1, grid - per_sm), LpCost(), true, list);
     unsigned* d = nullptr;
     if (cudaMalloc(&d, std::max<size_t>(1, list.size()) * sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
@@ -1367,7 +1376,7 @@ extern "C" int ecg_ldl_schedule(int n, int workers, unsigned* out, long long cap
     const int np = (n + LDL_NB - 1) / LDL_NB;
     if (np > 200) return -1;
     std::vector<unsigned> full, list;
-    lp_schedule(np, workers, LpCost(), list, &full);
+    lp_schedule(np, workers, LpCost(), false, list, &full);
     *count = (long long)full.size();
     if (out && cap >= (long long)full.size()) std::copy(full.begin(), full.end(), out);
     return 0;
