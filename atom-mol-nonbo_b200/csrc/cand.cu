@@ -41,6 +41,7 @@
 #include <algorithm>
 #include "../../include/ecg_abi.h"
 #include "ecg_internal.h"
+#include "wait_value.cuh"
 #include "zmma.cuh"
 
 namespace ecg {
@@ -51,17 +52,6 @@ __device__ __forceinline__ cd ldcd(const cd* p)
 {
     const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
     return cd{v.x, v.y};
-}
-
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -190,21 +180,53 @@ __global__ void __launch_bounds__(256) k_zgemm(const cd* __restrict__ A, int lda
 //   BWD (L^H x = z - U(:,K) x_K):
 //     X_p = Linv_p^H (Z_p - U(p,K) x_K) - sum_{q>p} G_pq X_q,  G_pq = Linv_p^H U_pq
 // (L_pq(m, k) = conj(U(q0+k, p0+m)), U_pq(m, k) = U(p0+m, q0+k)).  The
-// diagonal-block product needs no other panel, so it runs before the first
-// wait; each dependency's G tile (static) is loaded while the CTA waits for
-// that panel's flag, so a step of the panel chain is one flag hand-off, one
-// 64 x 16 tile load and one 64 x 64 x 16 product.
-// Work item (panel p, column block cb of CAND_NC columns); items are ordered
-// so that every item depends only on items with smaller indices, and each
-// CTA takes items blockIdx.x, blockIdx.x + gridDim.x, ... in order, so with
-// all CTAs co-resident every wait ends.  Each wait is bounded
-// (abort_word[1] polls, SOLVE_SPIN_LIMIT by default, or at once after any
-// CTA gave up); a CTA that gives
-// up records ST_SOLVE_TIMEOUT and publishes nothing.
+// diagonal-block product needs no other panel, so it comes first.
+//
+// Work item (panel p, column block cb of NC columns); items are ordered so
+// that every item depends only on items with smaller indices, and each CTA
+// takes items blockIdx.x, blockIdx.x + gridDim.x, ... in order, so with all
+// CTAs co-resident every wait ends.  An item is 2 (dependencies + 1) steps
+// of 32 inner rows: the operand from the factor through a ring of three
+// half tiles (two steps ahead), the values of the panel waited for straight
+// into registers while the step before is computed.  The values are their
+// own signal (wait_value.cuh): Y starts as UNSET and each solve marks the
+// other's output for the next one.  Bounded waits: a thread that gives up
+// records ST_SOLVE_TIMEOUT and goes on without waiting.
+// What bounds it: the chain over the panels, one 64 x 64 x NC product (2.1
+// us of an SM at NC = 16) and one hand-off a panel; at 256 columns the
+// FP64 tensor cores' 117 us too.  At K = 2000 a pair of solves takes 490 us
+// with 256 columns and 210 us with 64; with a flag per panel, whole tiles
+// and blocks of 16 columns throughout 566 and 363 us.
 // ---------------------------------------------------------------------------
-constexpr int TS_LDA = 64 + 2;
-constexpr int TS_LDB = 64 + 4;
-constexpr size_t TS_SMEM = (size_t)(64 * TS_LDA + CAND_NC * TS_LDB) * sizeof(double2);
+// As(k, m) of a half tile (32 x 64) and Bs(n, k) of a half right-hand side
+// (NC x 32): the exclusive or takes the fragment loads of a quarter-warp to
+// eight different bank groups.
+__device__ __forceinline__ int cs_a(int k, int m) { return k * 64 + (m ^ ((k & 3) << 1)); }
+__device__ __forceinline__ int cs_b(int n, int k) { return n * 32 + (k ^ ((n & 1) << 2)); }
+constexpr int CS_A = 32 * 64;
+template <int NC>
+constexpr size_t cs_smem() { return (size_t)(3 * CS_A + 2 * NC * 32) * sizeof(double2); }
+
+// acc += op(A) B over the 32 inner rows of a step: MT 8-row tiles from row
+// wm, the 8 columns from wn.
+template <int MT, bool CONJA>
+__device__ __forceinline__ void cs_mma(ZAcc<MT, 1>& acc, const double2* __restrict__ As,
+                                       const double2* __restrict__ Bs, int wm, int wn, int g, int t)
+{
+#pragma unroll
+    for (int kk = 0; kk < 32; kk += 4) {
+        const double2 b = Bs[cs_b(wn + g, kk + t)];
+#pragma unroll
+        for (int mt = 0; mt < MT; mt++) {
+            const double2 a = As[cs_a(kk + t, wm + mt * 8 + g)];
+            const double ai = CONJA ? -a.y : a.y;
+            dmma(acc.r[mt][0][0], acc.r[mt][0][1], a.x, b.x);
+            dmma(acc.r[mt][0][0], acc.r[mt][0][1], -ai, b.y);
+            dmma(acc.i[mt][0][0], acc.i[mt][0][1], a.x, b.y);
+            dmma(acc.i[mt][0][0], acc.i[mt][0][1], ai, b.x);
+        }
+    }
+}
 
 // G tiles: one CTA per ordered panel pair (p, q), p != q; FWD blocks (p > q)
 // and BWD blocks (p < q) share the array, G(p0+m, q0+n) at Gm[(p0+m) + (q0+n) ld].
@@ -270,130 +292,130 @@ __global__ void __launch_bounds__(256) k_cand_gmat(const cd* __restrict__ H, int
             }
 }
 
-template <bool FWD>
-__global__ void __launch_bounds__(256) k_cand_solve(const cd* __restrict__ Gm, int ld, const int* __restrict__ bstart,
-                                                    int nb, const cd* __restrict__ linv, const cd* __restrict__ invD,
-                                                    const cd* __restrict__ Win, cd* __restrict__ Yout,
-                                                    cd* __restrict__ Zout, const cd* __restrict__ lcol,
-                                                    const cd* __restrict__ xK, int ldv, int ncb,
-                                                    const int* __restrict__ cmap, unsigned* __restrict__ flags,
-                                                    int* __restrict__ status, int* __restrict__ abort_word)
+template <bool FWD, int NC>
+__global__ void __launch_bounds__(256, 2) k_cand_solve(const cd* __restrict__ Gm, int ld,
+                                                       const int* __restrict__ bstart, int nb,
+                                                       const cd* __restrict__ linv, const cd* __restrict__ invD,
+                                                       const cd* __restrict__ Win, cd* Yout, cd* __restrict__ Zout,
+                                                       cd* __restrict__ unset_next, const cd* __restrict__ lcol,
+                                                       const cd* __restrict__ xK, int ldv, int ncb,
+                                                       const int* __restrict__ cmap, int* __restrict__ status,
+                                                       int* __restrict__ abort_word)
 {
     extern __shared__ double2 tsm[];
-    double2* As = tsm;                // [k][m]
-    double2* Bs = tsm + 64 * TS_LDA;  // [n][k]
-    __shared__ int go;
+    double2* As = tsm;             // three half tiles
+    double2* Bs = tsm + 3 * CS_A;  // two half right-hand sides
+    constexpr int MT = NC / 8, U = NC * 32 / 256;
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int wm = (wp >> 1) * 16, wn = (wp & 1) * 8;  // 4 x 2 warps of 16 x 8
+    const int wm = (NC == 16) ? (wp >> 1) * 16 : wp * 8, wn = (NC == 16) ? (wp & 1) * 8 : 0;
     const int g = lane >> 2, t = lane & 3;
+    const int kb = tid & 31;  // this thread's inner row of a step's right-hand side, columns tid / 32 + 8 u
+    const int limit = ((volatile int*)abort_word)[1];
     const int nitems = nb * ncb;
     bool ok = true;
-    // G tile of dependency q into As (m contiguous in memory)
-    auto load_g = [&](int p0, int bp, int q) {
-        const int q0 = bstart[q], bq = bstart[q + 1] - q0;
-#pragma unroll 4
-        for (int u = 0; u < 16; u++) {
-            const int e = tid + 256 * u;
-            const int m = e & 63, k = e >> 6;
-            const bool in = (m < bp) && (k < bq);
-            cp_async16(As + k * TS_LDA + m, in ? Gm + (size_t)(p0 + m) + (size_t)(q0 + k) * ld : Gm, in ? 16 : 0);
-        }
-        cp_async_commit();
-    };
-    for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
         const int pi = item / ncb, cb = item % ncb;
         const int p = FWD ? pi : nb - 1 - pi;
         const int p0 = bstart[p], bp = bstart[p + 1] - p0;
-        const int col0 = cb * CAND_NC;
-        // (1) diagonal block: Linv_p rhs (FWD) / Linv_p^H (rhs - U(p,K) x_K) (BWD)
+        const int nstep = 2 * ((FWD ? p : nb - 1 - p) + 1);
+        size_t col[U];
+        int jc[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int slot = cb * NC + (tid >> 5) + 8 * u;
+            jc[u] = cmap ? cmap[slot] : slot;
+            col[u] = (size_t)jc[u] * ldv;
+        }
+        // first row and height of the panel step s multiplies: this one's
+        // own right-hand side, then the dependencies
+        auto panel = [&](int s, int& q0, int& bq) {
+            const int d = (s >> 1) - 1;
+            const int q = d < 0 ? p : (FWD ? d : nb - 1 - d);
+            q0 = bstart[q];
+            bq = bstart[q + 1] - q0;
+        };
+        // step s of the factor's operand into slot s % 3
+        auto load_a = [&](int s) {
+            int q0, bq;
+            panel(s, q0, bq);
+            const int k0 = (s & 1) * 32;
+            double2* a = As + (s % 3) * CS_A;
+            if (s < 2 && FWD) {  // Linv_p, k contiguous
 #pragma unroll 4
-        for (int u = 0; u < 16; u++) {
-            const int e = tid + 256 * u;
-            const int m = FWD ? (e >> 6) : (e & 63);
-            const int k = FWD ? (e & 63) : (e >> 6);
-            const bool in = (m < bp) && (k < bp);
-            const cd* src = FWD ? linv + (size_t)(p0 + m) * LDL_NB + k : linv + (size_t)(p0 + k) * LDL_NB + m;
-            cp_async16(As + k * TS_LDA + m, in ? src : linv, in ? 16 : 0);
-        }
+                for (int u = 0; u < 8; u++) {
+                    const int e = tid + 256 * u, k = e & 31, m = e >> 5;
+                    const bool in = m < bp && k0 + k < bq;
+                    cp_async16(a + cs_a(k, m), in ? linv + (size_t)(p0 + m) * LDL_NB + k0 + k : linv, in ? 16 : 0);
+                }
+            } else {  // Linv_p^H before its conjugation, or G(p, q): m contiguous
+                const cd* src = s < 2 ? linv + (size_t)(p0 + k0) * LDL_NB : Gm + p0 + (size_t)(q0 + k0) * ld;
+                const size_t pitch = s < 2 ? (size_t)LDL_NB : (size_t)ld;
+#pragma unroll 4
+                for (int u = 0; u < 8; u++) {
+                    const int e = tid + 256 * u, m = e & 63, k = e >> 6;
+                    const bool in = m < bp && k0 + k < bq;
+                    cp_async16(a + cs_a(k, m), in ? src + m + k * pitch : src, in ? 16 : 0);
+                }
+            }
+        };
+        load_a(0);
         cp_async_commit();
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const int e = tid + 256 * u;
-            const int m = e & 63, n = e >> 6;
-            cd v = mk(0.0, 0.0);
-            if (m < bp) {
-                const int jp = cmap ? cmap[col0 + n] : col0 + n;
-                const size_t o = (size_t)(p0 + m) + (size_t)jp * ldv;
-                v = ldcd(Win + o);
-                if (!FWD) v = cfms(ldcd(lcol + o), ldcd(xK + jp), v);
-            }
-            Bs[n * TS_LDB + m] = make_double2(v.x, v.y);
-        }
-        cp_async_wait<0>();
-        __syncthreads();
-        ZAcc<2, 1> acc;
+        load_a(1);
+        cp_async_commit();
+        ZAcc<MT, 1> acc, dep;
         acc.zero();
-#pragma unroll
-        for (int kk = 0; kk < 64; kk += 4) zmma_k4<2, 1, TS_LDA, TS_LDB, !FWD>(acc, As, Bs, wm, wn, kk, lane);
-        __syncthreads();
-        // (2) the panels this one depends on
-        ZAcc<2, 1> dep;
         dep.zero();
-        const int ndep = FWD ? p : nb - 1 - p;
-        if (ndep > 0) load_g(p0, bp, FWD ? 0 : nb - 1);
-        for (int d = 0; d < ndep; d++) {
-            const int q = FWD ? d : nb - 1 - d;
-            if (tid == 0) {
-                int gg = 1;
-                int spins = 0;
-                const int limit = ((volatile int*)abort_word)[1];
-                while (ld_acquire_u32(flags + q * ncb + cb) != 1u) {
-                    if (++spins > limit || *((volatile int*)abort_word) != 0) {
-                        gg = 0;
-                        break;
+        for (int s = -1; s < nstep; s++) {
+            if (s >= 0) {
+                cp_async_wait<1>();
+                __syncthreads();
+                if (s + 2 < nstep) load_a(s + 2);
+                cp_async_commit();
+            }
+            // the next step's right-hand side: the first look before this
+            // step's products, the waiting after them
+            const int sn = s + 1;
+            unsigned long long v0[U], v1[U];
+            int q0 = 0, bq = 0;
+            if (sn < nstep) panel(sn, q0, bq);
+            const int kq = (sn & 1) * 32 + kb;
+            const bool in = sn < nstep && kq < bq;
+            if (in && sn >= 2)
+#pragma unroll
+                for (int u = 0; u < U; u++) look_value(Yout + col[u] + q0 + kq, v0[u], v1[u]);
+            if (s >= 0) {
+                const double2* a = As + (s % 3) * CS_A;
+                const double2* b = Bs + (s & 1) * NC * 32;
+                if (s < 2)
+                    cs_mma<MT, !FWD>(acc, a, b, wm, wn, g, t);
+                else
+                    cs_mma<MT, false>(dep, a, b, wm, wn, g, t);
+            }
+            if (sn < nstep)
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    double2 v = make_double2(0.0, 0.0);
+                    if (in && sn >= 2) {
+                        v = (v0[u] != UNSET && v1[u] != UNSET)
+                                ? make_double2(__longlong_as_double((long long)v0[u]),
+                                               __longlong_as_double((long long)v1[u]))
+                                : wait_value(Yout + col[u] + q0 + kq, status, abort_word, limit, ok);
+                    } else if (in) {
+                        cd w = ldcd(Win + col[u] + p0 + kq);
+                        if (!FWD) w = cfms(ldcd(lcol + col[u] + p0 + kq), ldcd(xK + jc[u]), w);
+                        v = make_double2(w.x, w.y);
                     }
-                    __nanosleep(64);
+                    Bs[(sn & 1) * NC * 32 + cs_b((tid >> 5) + 8 * u, kb)] = v;
                 }
-                if (!gg) {
-                    atomicExch(status + ST_SOLVE_TIMEOUT, 1);
-                    atomicExch(abort_word, 1);
-                }
-                go = gg;
-            }
-            __syncthreads();
-            if (!go) {
-                ok = false;
-                break;
-            }
-            const int q0 = bstart[q], bq = bstart[q + 1] - q0;
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int e = tid + 256 * u;
-                const int k = e & 63, n = e >> 6;
-                const bool in = k < bq;
-                const int jp = cmap ? cmap[col0 + n] : col0 + n;
-                cp_async16(Bs + n * TS_LDB + k, in ? Yout + (size_t)(q0 + k) + (size_t)jp * ldv : Yout, in ? 16 : 0);
-            }
-            cp_async_commit();
-            cp_async_wait<0>();
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < 64; kk += 4) zmma_k4<2, 1, TS_LDA, TS_LDB, false>(dep, As, Bs, wm, wn, kk, lane);
-            __syncthreads();
-            if (d + 1 < ndep) load_g(p0, bp, FWD ? d + 1 : nb - 2 - d);  // overlaps the next wait
         }
-        if (!ok) {
-            cp_async_wait<0>();
-            break;
-        }
-        // (3) publish this panel
+        // publish this panel
 #pragma unroll
-        for (int mt = 0; mt < 2; mt++)
+        for (int mt = 0; mt < MT; mt++)
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                const int m = wm + mt * 8 + g, n = wn + 2 * t + e;
+                const int m = wm + mt * 8 + g, slot = cb * NC + wn + 2 * t + e;
                 if (m < bp) {
-                    const int jp = cmap ? cmap[col0 + n] : col0 + n;
+                    const int jp = cmap ? cmap[slot] : slot;
                     const size_t o = (size_t)(p0 + m) + (size_t)jp * ldv;
                     const cd y = mk(acc.r[mt][0][e] - dep.r[mt][0][e], acc.i[mt][0][e] - dep.i[mt][0][e]);
                     *reinterpret_cast<double2*>(Yout + o) = make_double2(y.x, y.y);
@@ -401,11 +423,10 @@ __global__ void __launch_bounds__(256) k_cand_solve(const cd* __restrict__ Gm, i
                         const cd z = cmul(y, ldcd(invD + p0 + m));
                         *reinterpret_cast<double2*>(Zout + o) = make_double2(z.x, z.y);
                     }
+                    unset_next[o] = unset();
                 }
             }
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) st_release_u32(flags + p * ncb + cb, 1u);
+        __syncthreads();  // the next item loads over the ring
     }
 }
 
@@ -469,10 +490,10 @@ __device__ __forceinline__ double block_max256(double v, double* sh)
 // Per-column state, stride `bcap` in the kernels (CandWork::ccap):
 // CandWork::st (ints): [0] active  [1] iterations  [2] ErrorCode, then the active count
 // CandWork::nd (doubles): [0] NormOfDiff  [1] NormOfDiffPrev  [2] t1  [3] t2  [4] E
-// border entries (CandWork::brd, complex): [0] v_K  [1] w_K  [2] invD_K  [3] x_K
+// border entries (CandWork::brd, complex): [0] v_K  [1] invD_K  [2] x_K
 enum { ST_ACTIVE = 0, ST_ITERS = 1, ST_ERR = 2 };
 enum { ND_ND = 0, ND_PREV = 1, ND_T1 = 2, ND_T2 = 3, ND_E = 4 };
-enum { BR_V = 0, BR_W = 1, BR_INVD = 2, BR_X = 3 };
+enum { BR_V = 0, BR_INVD = 1, BR_X = 2 };
 
 // Bordered LDLHF step for row K (src/linalg.f90:359-383):
 // x = M(K,K) - sum_q conj(a_q) U(q,K);  d_K = conj(x);  invD_K = 1/d_K,
@@ -528,45 +549,30 @@ __global__ void __launch_bounds__(256) k_cand_init(const cd* __restrict__ x0, in
     }
 }
 
-// w_K = sum_q conj(S(q,K)) v_q + v_K  (row K of MHMV's B^H v)
-__global__ void __launch_bounds__(256) k_cand_wk(const cd* __restrict__ Scol, const cd* __restrict__ V, int nbase,
-                                                 int ldv, int bcap, cd* __restrict__ brd, const int* __restrict__ cmap,
-                                                 int count)
-{
-    __shared__ double sh[8 * 2];
-    const int j = cmap[blockIdx.x];
-    if (j >= count) return;
-    const cd* s = Scol + (size_t)j * ldv;
-    const cd* v = V + (size_t)j * ldv;
-    double a[2] = {0.0, 0.0};
-    for (int q = threadIdx.x; q < nbase; q += 256) {
-        const cd p = cmul(conj(ldcd(s + q)), ldcd(v + q));
-        a[0] += p.x;
-        a[1] += p.y;
-    }
-    block_sum256<2>(a, sh);
-    if (threadIdx.x == 0) brd[BR_W * bcap + j] = mk(a[0], a[1]) + brd[BR_V * bcap + j];
-}
-
+// w_K = sum_q conj(S(q,K)) v_q + v_K  (row K of MHMV's B^H v);
 // y_K = w_K - sum_q conj(U(q,K)) y_q;  x_K = z_K = invD_K y_K
-__global__ void __launch_bounds__(256) k_cand_mid(const cd* __restrict__ Lcol, const cd* __restrict__ Y, int nbase,
-                                                  int ldv, int bcap, cd* __restrict__ brd, const int* __restrict__ cmap,
-                                                  int count)
+__global__ void __launch_bounds__(256) k_cand_mid(const cd* __restrict__ Scol, const cd* __restrict__ V,
+                                                  const cd* __restrict__ Lcol, const cd* __restrict__ Y, int nbase,
+                                                  int ldv, int bcap, cd* __restrict__ brd,
+                                                  const int* __restrict__ cmap, int count)
 {
-    __shared__ double sh[8 * 2];
+    __shared__ double sh[8 * 4];
     const int j = cmap[blockIdx.x];
     if (j >= count) return;
-    const cd* l = Lcol + (size_t)j * ldv;
-    const cd* y = Y + (size_t)j * ldv;
-    double a[2] = {0.0, 0.0};
+    const size_t o = (size_t)j * ldv;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
     for (int q = threadIdx.x; q < nbase; q += 256) {
-        const cd p = cmul(conj(ldcd(l + q)), ldcd(y + q));
-        a[0] += p.x;
-        a[1] += p.y;
+        const cd w = cmul(conj(ldcd(Scol + o + q)), ldcd(V + o + q));
+        const cd p = cmul(conj(ldcd(Lcol + o + q)), ldcd(Y + o + q));
+        a[0] += w.x;
+        a[1] += w.y;
+        a[2] += p.x;
+        a[3] += p.y;
     }
-    block_sum256<2>(a, sh);
+    block_sum256<4>(a, sh);
     if (threadIdx.x == 0) {
-        const cd yk = brd[BR_W * bcap + j] - mk(a[0], a[1]);
+        const cd wk = mk(a[0], a[1]) + brd[BR_V * bcap + j];
+        const cd yk = wk - mk(a[2], a[3]);
         brd[BR_X * bcap + j] = cmul(yk, brd[BR_INVD * bcap + j]);
     }
 }
@@ -641,19 +647,39 @@ __global__ void __launch_bounds__(256) k_cand_norm(const cd* __restrict__ X, cd*
 // multiple of CAND_PAD (bcap here is the column stride, CAND_PAD beyond
 // the candidate capacity); the active count goes to st[3 bcap].  init:
 // start from candidates 0..count-1.
-__global__ void k_cand_compact(int* __restrict__ cmap, int* __restrict__ st, int bcap, int count, int nslots,
-                               int init)
+__global__ void __launch_bounds__(256) k_cand_compact(int* __restrict__ cmap, int* __restrict__ st, int bcap,
+                                                      int count, int nslots, int init)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int na = 0;
+    __shared__ int wsum[8];
+    const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
     const int n = init ? count : nslots;
-    for (int s = 0; s < n; s++) {
-        const int j = init ? s : cmap[s];
-        if (j < count && st[ST_ACTIVE * bcap + j]) cmap[na++] = j;
+    int na = 0;
+    for (int s0 = 0; s0 < n; s0 += 256) {  // 256 slots at a time: written at or before where they were read
+        const int s = s0 + tid;
+        const int j = s < n ? (init ? s : cmap[s]) : count;
+        const bool on = j < count && st[ST_ACTIVE * bcap + j] != 0;
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) wsum[wp] = __popc(m);
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            before += w < wp ? wsum[w] : 0;
+            all += wsum[w];
+        }
+        if (on) cmap[na + before + __popc(m & ((1u << lane) - 1u))] = j;
+        na += all;
+        __syncthreads();
     }
     const int pad = ((na + CAND_PAD - 1) / CAND_PAD) * CAND_PAD;
-    for (int s = na; s < pad; s++) cmap[s] = bcap - CAND_PAD + (s - na);  // spare physical columns
-    st[3 * bcap] = na;
+    for (int s = na + tid; s < pad; s += 256) cmap[s] = bcap - CAND_PAD + (s - na);  // spare physical columns
+    if (tid == 0) st[3 * bcap] = na;
+}
+
+// Mark two solve outputs as not computed.
+__global__ void __launch_bounds__(256) k_cand_unset(cd* __restrict__ a, cd* __restrict__ b, size_t n)
+{
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) a[i] = b[i] = unset();
 }
 
 // Rayleigh quotient (src/linalg.f90:1913-1917) of the final iterate:
@@ -723,7 +749,6 @@ int ensure_work(Ctx& c, int count)
     const size_t col = (size_t)ldv * ccap;
     cw.ldv = ldv;
     const int maxpanels = c.ld + 2;  // panel count never exceeds the row count
-    cw.nflags = maxpanels * (ccap / CAND_NC);
     int r = 0;
     r |= dalloc_n(&cw.par, (size_t)c.npt * bcap);
     r |= dalloc_n(&cw.bra, (size_t)bcap * c.np);
@@ -742,13 +767,12 @@ int ensure_work(Ctx& c, int count)
     r |= dalloc_n(&cw.Z, col);
     r |= dalloc_n(&cw.X, col);
     r |= dalloc_n(&cw.X2, col);
-    r |= dalloc_n(&cw.brd, (size_t)4 * ccap);
+    r |= dalloc_n(&cw.brd, (size_t)3 * ccap);
     r |= dalloc_n(&cw.nd, (size_t)5 * ccap);
     r |= dalloc_n(&cw.st, (size_t)3 * ccap + 1);
     r |= dalloc_n(&cw.cmap, (size_t)ccap);
     r |= dalloc_n(&cw.Gm, (size_t)c.ld * c.ld);
     r |= dalloc_n(&cw.Pk, (size_t)CAND_KSPLIT * ldv * 2 * CAND_PAD);
-    r |= dalloc_n(&cw.flags, (size_t)cw.nflags);
     r |= dalloc_n(&cw.bstart, (size_t)maxpanels + 1);
     r |= dalloc_n(&cw.abort_word, 2);  // abort word, wait poll limit
     cw.gpart_n = (size_t)bcap * (c.ld / 128 + 2) * (2 * c.np + 1);
@@ -772,7 +796,7 @@ int ensure_work(Ctx& c, int count)
     void* zc[] = {cw.Mcol, cw.Scol, cw.Acol, cw.Lcol, cw.V, cw.W, cw.Y, cw.Z, cw.X, cw.X2};
     for (void* p : zc)
         if (cudaMemsetAsync(p, 0, col * sizeof(cd), c.stream) != cudaSuccess) return -2;
-    if (cudaMemsetAsync(cw.brd, 0, 4 * (size_t)ccap * sizeof(cd), c.stream) != cudaSuccess) return -2;
+    if (cudaMemsetAsync(cw.brd, 0, 3 * (size_t)ccap * sizeof(cd), c.stream) != cudaSuccess) return -2;
     if (cudaMemcpyAsync(cw.abort_word + 1, &c.wait_limit, sizeof(int), cudaMemcpyHostToDevice, c.stream) !=
             cudaSuccess ||
         cudaStreamSynchronize(c.stream) != cudaSuccess)
@@ -784,32 +808,42 @@ int solve_grid(Ctx& c)
 {
     CandWork& cw = c.cand;
     if (cw.solve_grid) return cw.solve_grid;
-    int coop = 0, nsm = 0, a = 0, b = 0;
+    int coop = 0, nsm = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c.dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.dev);
-    cudaFuncSetAttribute(k_cand_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM);
-    cudaFuncSetAttribute(k_cand_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM);
     cudaFuncSetAttribute(k_zgemm<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM);
     cudaFuncSetAttribute(k_zgemm<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM);
     cudaFuncSetAttribute(k_cand_gmat, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(G_STAGE * sizeof(double2)));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_cand_solve<true>, 256, TS_SMEM);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cand_solve<false>, 256, TS_SMEM);
+    int per = 1 << 30;
+    auto fit = [&](const void* f, size_t smem) {
+        int a = 0;
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, f, 256, smem);
+        per = std::min(per, a);
+    };
+    fit((const void*)k_cand_solve<true, 8>, cs_smem<8>());
+    fit((const void*)k_cand_solve<false, 8>, cs_smem<8>());
+    fit((const void*)k_cand_solve<true, 16>, cs_smem<16>());
+    fit((const void*)k_cand_solve<false, 16>, cs_smem<16>());
     cudaGetLastError();
-    cw.solve_grid = (coop && std::min(a, b) > 0) ? nsm * std::min(a, b) : -1;
+    cw.solve_grid = (coop && per > 0) ? nsm * per : -1;
     return cw.solve_grid;
 }
 
 // One cooperative triangular solve over ncols columns (through cmap when
-// it is not null).
-int launch_solve(Ctx& c, bool fwd, int nb, int ncols, const cd* Win, cd* Yout, cd* Zout, const int* cmap)
+// it is not null); `next` is marked as not computed for the next solve.
+// Up to CAND_NC8_MAX columns the chain over the panels decides, and blocks
+// of 8 columns halve its products; beyond, blocks of 16 halve the reads of
+// the factor.  Whole calls at K = 2000, blocks of 8 and 16, ms: 64 columns
+// 2.21, 2.77; 256 4.43, 4.68; 512 8.01, 7.63; K = 4000, 512 27.3, 25.9.
+template <bool FWD, int NC>
+int launch_solve_nc(Ctx& c, int nb, int ncols, const cd* Win, cd* Yout, cd* Zout, cd* next, const int* cmap)
 {
     CandWork& cw = c.cand;
-    const int ncb = ncols / CAND_NC;
+    const int ncb = ncols / NC;
     const int items = nb * ncb;
     if (items <= 0) return 0;
-    if (cudaMemsetAsync(cw.flags, 0, sizeof(unsigned) * (size_t)items, c.stream) != cudaSuccess) return -2;
-    if (cudaMemsetAsync(cw.abort_word, 0, sizeof(int), c.stream) != cudaSuccess) return -2;
     const int grid = std::min(items, solve_grid(c));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -817,22 +851,23 @@ int launch_solve(Ctx& c, bool fwd, int nb, int ncols, const cd* Win, cd* Yout, c
     attr[0].val.cooperative = 1;
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = TS_SMEM;
+    cfg.dynamicSmemBytes = cs_smem<NC>();
     cfg.stream = c.stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const cd* xk = cw.brd + BR_X * cw.ccap;
-    cudaError_t e;
-    if (fwd)
-        e = cudaLaunchKernelEx(&cfg, k_cand_solve<true>, (const cd*)cw.Gm, c.ld, (const int*)cw.bstart, nb,
-                               (const cd*)c.linv, (const cd*)c.invD, Win, Yout, Zout, (const cd*)cw.Lcol, xk, cw.ldv,
-                               ncb, cmap, cw.flags, c.status, cw.abort_word);
-    else
-        e = cudaLaunchKernelEx(&cfg, k_cand_solve<false>, (const cd*)cw.Gm, c.ld, (const int*)cw.bstart, nb,
-                               (const cd*)c.linv, (const cd*)c.invD, Win, Yout, Zout, (const cd*)cw.Lcol, xk, cw.ldv,
-                               ncb, cmap, cw.flags, c.status, cw.abort_word);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_cand_solve<FWD, NC>, (const cd*)cw.Gm, c.ld, (const int*)cw.bstart,
+                                             nb, (const cd*)c.linv, (const cd*)c.invD, Win, Yout, Zout, next,
+                                             (const cd*)cw.Lcol, xk, cw.ldv, ncb, cmap, c.status, cw.abort_word);
     c.launches++;
     return e == cudaSuccess ? 0 : -2;
+}
+
+template <bool FWD>
+int launch_solve(Ctx& c, int nb, int ncols, const cd* Win, cd* Yout, cd* Zout, cd* next, const int* cmap)
+{
+    return ncols <= CAND_NC8_MAX ? launch_solve_nc<FWD, 8>(c, nb, ncols, Win, Yout, Zout, next, cmap)
+                                 : launch_solve_nc<FWD, 16>(c, nb, ncols, Win, Yout, Zout, next, cmap);
 }
 
 int launch_gemm(Ctx& c, int amode, const cd* A, int M, int ncols, const cd* B, cd* C, const cd* E1, const cd* e2,
@@ -869,15 +904,13 @@ int enqueue_iteration(Ctx& c, int nbase, int count, int ncols, int nb, double to
     const int cc = cw.ccap;
     int r;
     if ((r = launch_gemm(c, 0, c.S, nbase, ncols, cw.V, cw.W, cw.Scol, cw.brd + BR_V * cc, cw.cmap))) return r;
-    k_cand_wk<<<ncols, 256, 0, c.stream>>>(cw.Scol, cw.V, nbase, cw.ldv, cc, cw.brd, cw.cmap, count);
+    if ((r = launch_solve<true>(c, nb, ncols, cw.W, cw.Y, cw.Z, cw.X, cw.cmap))) return r;
+    k_cand_mid<<<ncols, 256, 0, c.stream>>>(cw.Scol, cw.V, cw.Lcol, cw.Y, nbase, cw.ldv, cc, cw.brd, cw.cmap, count);
     c.launches++;
-    if ((r = launch_solve(c, true, nb, ncols, cw.W, cw.Y, cw.Z, cw.cmap))) return r;
-    k_cand_mid<<<ncols, 256, 0, c.stream>>>(cw.Lcol, cw.Y, nbase, cw.ldv, cc, cw.brd, cw.cmap, count);
-    c.launches++;
-    if ((r = launch_solve(c, false, nb, ncols, cw.Z, cw.X, nullptr, cw.cmap))) return r;
+    if ((r = launch_solve<false>(c, nb, ncols, cw.Z, cw.X, nullptr, cw.Y, cw.cmap))) return r;
     k_cand_norm<<<ncols, 256, 0, c.stream>>>(cw.X, cw.V, nbase, cw.ldv, cc, cw.brd, cw.nd, cw.st,
                                              sqrt(2.0 * (nbase + 1)), tol, cw.cmap, count);
-    k_cand_compact<<<1, 32, 0, c.stream>>>(cw.cmap, cw.st, cc, count, ncols, 0);
+    k_cand_compact<<<1, 256, 0, c.stream>>>(cw.cmap, cw.st, cc, count, ncols, 0);
     c.launches += 2;
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -965,7 +998,7 @@ void cand_free(CandWork& cw)
 {
     drop_graphs(cw);
     void* ptrs[] = {cw.par, cw.bra, cw.ket, cw.ketn, cw.det, cw.dS, cw.mu, cw.Mcol, cw.Scol, cw.Acol, cw.Lcol, cw.V, cw.W,
-                    cw.Y, cw.Z, cw.X, cw.X2, cw.brd, cw.nd, cw.st, cw.cmap, cw.Gm, cw.Pk, cw.flags, cw.bstart,
+                    cw.Y, cw.Z, cw.X, cw.X2, cw.brd, cw.nd, cw.st, cw.cmap, cw.Gm, cw.Pk, cw.bstart,
                     cw.abort_word, cw.gpart, cw.grad};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -1053,7 +1086,10 @@ int eval_candidates(Ctx& c, int nbase, int count, const double* cand_host, doubl
         c.launches++;
     }
     // bordered factor row: Acol = L0^-1 Mcol, Lcol = invD o Acol, then d_K
-    if (launch_solve(c, true, nb, ncols, cw.Mcol, cw.Acol, cw.Lcol, nullptr)) return ECG_ECUDA;
+    k_cand_unset<<<296, 256, 0, c.stream>>>(cw.Acol, cw.Y, (size_t)cw.ldv * cc);
+    c.launches++;
+    if ((r = CKc(cudaMemsetAsync(cw.abort_word, 0, sizeof(int), c.stream)))) return r;
+    if (launch_solve<true>(c, nb, ncols, cw.Mcol, cw.Acol, cw.Lcol, cw.X, nullptr)) return ECG_ECUDA;
     k_cand_border<<<count, 256, 0, c.stream>>>(cw.Acol, cw.Lcol, cw.mu, nbase, cw.ldv, cc, cw.brd, cw.st,
                                                c.pivot_mode);
     {
@@ -1061,7 +1097,7 @@ int eval_candidates(Ctx& c, int nbase, int count, const double* cand_host, doubl
         if (g.x > 16) g.x = 16;
         k_cand_init<<<g, 256, 0, c.stream>>>(c.x, nbase, count, cw.ldv, cc, cw.V, cw.brd, cw.nd, cw.st);
     }
-    k_cand_compact<<<1, 32, 0, c.stream>>>(cw.cmap, cw.st, cc, count, 0, 1);
+    k_cand_compact<<<1, 256, 0, c.stream>>>(cw.cmap, cw.st, cc, count, 0, 1);
     c.launches += 3;
     int nact = count;
     for (int it = 0; it < max_iter; it++) {

@@ -41,9 +41,9 @@ constexpr int CAND_ROW_SHAPES = 5;
 // k_adjoint shapes (likewise) the autotuner chooses from.
 constexpr int PAIR_SHAPES = 4;
 constexpr int ADJ_SHAPES = 2;
-// Columns (candidates) per work item of the batched triangular solves and
-// the padding unit of the candidate column blocks.
-constexpr int CAND_NC = 16;
+// Most columns (candidates) the batched triangular solves take in blocks of
+// 8, not 16, and the padding unit of the candidate column blocks.
+constexpr int CAND_NC8_MAX = 256;
 constexpr int CAND_PAD = 64;
 // Largest split of the inner dimension of the candidates' GEMM.
 constexpr int CAND_KSPLIT = 4;
@@ -77,13 +77,11 @@ struct CandWork {
     cd* Z = nullptr;         // invD o Y
     cd* X = nullptr;         // backward solve (new x); Rayleigh products
     cd* X2 = nullptr;        // second Rayleigh product
-    cd* brd = nullptr;       // border entries: [0] vK [1] wK [2] invDK [3] xK
+    cd* brd = nullptr;       // border entries: [0] vK [1] invDK [2] xK
     double* nd = nullptr;    // NormOfDiff, NormOfDiffPrev, t1, t2, E
     int* st = nullptr;       // active, iterations, ErrorCode, then the active count
     int* st_h = nullptr;     // pinned host mirror of st
     double* nd_h = nullptr;  // pinned host mirror of nd
-    unsigned* flags = nullptr;  // work-item flags of the cooperative solves
-    int nflags = 0;
     int* bstart = nullptr;   // device panel boundaries of the base factor
     int* bstart_h = nullptr; // pinned staging
     int* abort_word = nullptr;

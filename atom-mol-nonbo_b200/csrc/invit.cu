@@ -13,6 +13,7 @@
 // block, so results are deterministic run to run.
 #include <algorithm>
 #include "ecg_internal.h"
+#include "wait_value.cuh"
 #include "warp_sums.cuh"
 
 namespace ecg {
@@ -38,12 +39,6 @@ __device__ __forceinline__ cd warp_sum(cd s)
     }
     return s;
 }
-
-// The value that stands for "not computed yet" in the vectors the cooperative
-// solves pass between CTAs: a quiet NaN with a payload no arithmetic makes
-// (hardware NaNs are 0x7fff...).
-constexpr unsigned long long UNSET = 0xfff8c0de5eedfaceULL;
-__device__ __forceinline__ cd unset() { return cd{__longlong_as_double(UNSET), __longlong_as_double(UNSET)}; }
 
 // w(i) = sum_j conj(B(j,i)) v(j); one warp per column, four accumulators.
 // The solves' vectors y and x are marked as not computed on the way.
@@ -181,27 +176,6 @@ static_assert(SOLVE_SPIN_LIMIT == (1 << 22), "the default poll limit of the solv
 // pitch of the 64 x 64 blocks in shared memory: 4 mod 8 double2, so that two
 // rows' four columns fall on different banks
 constexpr int LS_LD = LDL_NB + 4;
-
-// The computed value at *p; ok turns false when this thread gives up: after
-// `limit` polls (abort_word[1]: SOLVE_SPIN_LIMIT unless a caller set another
-// through ecg_set_wait_limit), or when the abort word is set, which is looked
-// at every 64th poll (its load would otherwise stand between the polls).
-__device__ __forceinline__ double2 wait_value(const cd* p, int* status, int* abort_word, int limit, bool& ok)
-{
-    unsigned long long a, b;
-    int spins = 0;
-    for (;;) {
-        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-        if ((a != UNSET && b != UNSET) || !ok) break;
-        ++spins;
-        if (spins > limit || ((spins & 63) == 0 && *((volatile int*)abort_word) != 0)) {
-            atomicExch(status + ST_SOLVE_TIMEOUT, 1);
-            atomicExch(abort_word, 1);
-            ok = false;
-        }
-    }
-    return make_double2(__longlong_as_double((long long)a), __longlong_as_double((long long)b));
-}
 
 // Threads 0..63: the n <= 64 values at p into sv (zeros beyond), as they are
 // computed; every thread returns whether they all were.
