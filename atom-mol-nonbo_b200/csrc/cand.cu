@@ -27,7 +27,8 @@
 //               cooperative launch over (panel, column block) work items;
 //               the bordered row and column enter as rank-one terms.
 //   Rayleigh    VMMHMV on S and on M (src/linalg.f90:1913-1917) as two
-//               GEMMs (S0 V and the Hermitian M0 V) plus border terms.
+//               GEMMs with the lower triangles of S0 and M0, plus border
+//               terms.
 //
 // One iteration (GEMM, solves, norms) is captured once into a CUDA graph
 // and replayed until every candidate has converged or MaxIter is reached;
@@ -42,6 +43,7 @@
 #include "../../include/ecg_abi.h"
 #include "ecg_internal.h"
 #include "wait_value.cuh"
+#include "tma_ring.cuh"
 #include "zmma.cuh"
 
 namespace ecg {
@@ -55,119 +57,226 @@ __device__ __forceinline__ cd ldcd(const cd* p)
 }
 
 // ---------------------------------------------------------------------------
-// C = op(A) B (+ E1 o e2 per column): M x N complex, inner dimension Kd.
-// Column j of B, C, E1 and e2 is physical column cmap[j] (j itself when
-// cmap is null): the iterations run on the still-active candidates only.
-//   AMODE 0: A(i, k) = A[i + k lda]
-//   AMODE 1: A Hermitian, stored in its lower triangle (the lower triangle
-//            of Glob_H holds M = H - lambda~ S): A(i, k) = A[i + k lda] for
-//            i >= k, conj(A[k + i lda]) for i < k.
-// 64 x 64 output tile per CTA, 8 warps as 2 x 4 (32 x 16 each), inner
-// chunks of 32 staged by cp.async into two shared-memory stages.
+// C(i, j) = sum_k conj(A(k, i)) B(k, j) (+ E1 o e2 per column) over the
+// nbase rows of a Hermitian A and of B; TRI: only k >= i of the column, its
+// diagonal halved, i.e. P with v^H A v = 2 Re v^H P from A's lower triangle
+// (half the products of the whole one; the matrix F keeps M there and the
+// factor in its upper triangle).  Column j of B is slot j, of C, E1 and e2
+// physical column cmap[j] (j itself when cmap is null).
+//
+// 64 x 64 tiles, 8 warps as 2 x 4 (32 x 16 each), the operands by TMA eight
+// inner rows a chunk through the six-stage ring, as in the trailing updates
+// of the factorisation (same fragment slots).  The chunks of all tiles are
+// one sequence, cut into equal pieces for two CTAs an SM: a tile that falls
+// into several pieces is written as partial sums, which k_cgemm_sum adds in
+// their order.  No barrier stands in the loop, and the stages run on from
+// tile to tile.  Bound by the FP64 tensor cores (8.2 GFLOP at K = 2000 and
+// 256 columns: 234 us at the measured peak).  At K = 2000 and 256, 192 and 64
+// columns, sum included: 268, 206 and 74 us; with cp.async stages and one CTA
+// a tile or an even split 336, 336 and 92 us.  TRI: 163 us, the whole
+// products of S and of M before 330 and 387 us.
 // ---------------------------------------------------------------------------
-constexpr int GM = 64, GN = 64, GK = 32;
-constexpr int G_LDA = GM + 2;  // % 8 == 2
-constexpr int G_LDB = GK + 4;  // % 8 == 4
-constexpr int G_STAGE = GK * G_LDA + GN * G_LDB;
-constexpr size_t G_SMEM = 2 * (size_t)G_STAGE * sizeof(double2);
+constexpr int CG_OP = TMA_KC * LDL_NB;  // double2 of one staged operand
+constexpr int CG_TILE = 64 * 64;
+constexpr size_t CG_RING = (size_t)TMA_ST * 2 * CG_OP * sizeof(double2);
+constexpr size_t CG_SMEM = 1024 + CG_RING + 2 * TMA_ST * 8;  // 1 KB to align the stages
 
-template <int AMODE>
-__global__ void __launch_bounds__(256) k_zgemm(const cd* __restrict__ A, int lda, int M, int Kd,
-                                               const cd* __restrict__ B, int ldb, cd* __restrict__ C, int ldc,
-                                               const cd* __restrict__ E1, const cd* __restrict__ e2,
-                                               const int* __restrict__ cmap, cd* __restrict__ P, size_t pstride)
+struct CgArgs {
+    CUtensorMap a, b;  // boxes of 8 complex rows x 64 columns
+    int M, mt;         // rows and tile rows of C (and columns of A)
+    int nk, ntile;     // chunks of a whole tile, tiles
+    long long total;   // chunks of all tiles
+    const int* cmap;
+    cd* C;
+    int ldc;
+    const cd *E1, *e2;
+    cd* P;             // two partial tiles a CTA
+    int* status;
+};
+
+// first chunk of tile row it, and the chunks before tile t (column by column)
+template <bool TRI>
+__host__ __device__ __forceinline__ int cg_first(int it)
 {
-    extern __shared__ double2 gsm[];
-    const int i0 = blockIdx.x * GM, j0 = blockIdx.y * GN;
+    return TRI ? it * (64 / TMA_KC) : 0;
+}
+template <bool TRI>
+__host__ __device__ __forceinline__ long long cg_before(int t, int mt, int nk)
+{
+    if (!TRI) return (long long)t * nk;
+    const int jt = t / mt, it = t % mt;
+    const long long col = (long long)mt * nk - (long long)(64 / TMA_KC) * mt * (mt - 1) / 2;
+    return jt * col + (long long)it * nk - (long long)(64 / TMA_KC) * it * (it - 1) / 2;
+}
+
+__device__ __forceinline__ void cg_store(const CgArgs& a, int i, int j, double re, double im)
+{
+    if (i >= a.M) return;
+    const int jp = a.cmap ? a.cmap[j] : j;
+    cd v = mk(re, im);
+    const size_t o = (size_t)i + (size_t)jp * a.ldc;
+    if (a.E1) v = cfma(ldcd(a.E1 + o), ldcd(a.e2 + jp), v);
+    *reinterpret_cast<double2*>(a.C + o) = make_double2(v.x, v.y);
+}
+
+template <bool TRI>
+__global__ void __launch_bounds__(256, 2) k_cgemm(const __grid_constant__ CgArgs a)
+{
+    extern __shared__ __align__(16) unsigned char cgsm[];
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int wm = (wp >> 2) * 32, wn = (wp & 3) * 16;
-    ZAcc<4, 2> acc;
-    acc.zero();
-    // split K: slice blockIdx.z of gridDim.z takes chunks [kc0, kc1)
-    const int nkt = (Kd + GK - 1) / GK;
-    const int per = (nkt + gridDim.z - 1) / gridDim.z;
-    const int kc0 = blockIdx.z * per, kc1 = min(nkt, kc0 + per);
-    const int nk = kc1 > kc0 ? kc1 - kc0 : 0;
-    auto stage = [&](int s, int kcl) {
-        const int kc = kc0 + kcl;
-        double2* As = gsm + s * G_STAGE;
-        double2* Bs = As + GK * G_LDA;
-        const int k0 = kc * GK;
-        // a tile wholly above the diagonal reads A's transpose: walk k fastest
-        const bool up = (AMODE == 1) && (i0 + GM <= k0);
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int e = tid + 256 * u;
-            const int m = up ? (e >> 5) : (e & 63);
-            const int k = up ? (e & 31) : (e >> 6);
-            const int i = i0 + m, kk = k0 + k;
-            const cd* src = A;
-            int bytes = 0;
-            if (i < M && kk < Kd) {
-                bytes = 16;
-                src = (AMODE == 1 && i < kk) ? A + kk + (size_t)i * lda : A + i + (size_t)kk * lda;
-            }
-            cp_async16(As + k * G_LDA + m, src, bytes);
+    const int wr = wp >> 2, wc = wp & 3;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int pg = (g & 1) << 2 | g >> 1;
+    const unsigned base = (smem32(cgsm) + 1023u) & ~1023u;
+    const double2* stages = reinterpret_cast<const double2*>(cgsm + (base - smem32(cgsm)));
+    TmaRing ring;
+    ring.init(base + (unsigned)CG_RING, tid);
+    const long long u0 = a.total * blockIdx.x / gridDim.x, u1 = a.total * (blockIdx.x + 1) / gridDim.x;
+    // the tile and the chunk the piece begins with
+    int t = TRI ? 0 : (int)(u0 / a.nk);
+    if (TRI)
+        for (int lo = 0, hi = a.ntile; hi - lo > 1;) {
+            const int mid = (lo + hi) / 2;
+            if (cg_before<true>(mid, a.mt, a.nk) <= u0)
+                t = lo = mid;
+            else
+                hi = mid;
         }
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int e = tid + 256 * u;
-            const int k = e & 31, n = e >> 5;
-            const int kk = k0 + k;
-            const bool ok = kk < Kd;
-            const int jp = cmap ? cmap[j0 + n] : j0 + n;
-            cp_async16(Bs + n * G_LDB + k, ok ? B + kk + (size_t)jp * ldb : B, ok ? 16 : 0);
+    int k = cg_first<TRI>(t % a.mt) + (int)(u0 - cg_before<TRI>(t, a.mt, a.nk));
+    __syncthreads();
+    int qt = t, qk = k;  // thread 0: what the next stage is filled with
+    auto issue = [&](int st) {
+        const unsigned bar = ring.full + 8u * st, dst = base + (unsigned)(st * 2 * CG_OP * sizeof(double2));
+        bar_expect(bar, (unsigned)(2 * CG_OP * sizeof(double2)));
+        tma_box(dst, &a.a, qk * TMA_KC, (qt % a.mt) * 64, bar);
+        tma_box(dst + (unsigned)(CG_OP * sizeof(double2)), &a.b, qk * TMA_KC, (qt / a.mt) * 64, bar);
+        if (++qk == a.nk) {
+            qt++;
+            qk = cg_first<TRI>(qt % a.mt);
         }
-        cp_async_commit();
     };
-    if (nk > 0) stage(0, 0);
-    for (int kcl = 0; kcl < nk; kcl++) {
-        if (kcl + 1 < nk) {
-            stage((kcl + 1) & 1, kcl + 1);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        double2* As = gsm + (kcl & 1) * G_STAGE;
-        const double2* Bs = As + GK * G_LDA;
-        const int kc = kc0 + kcl;
-        if (AMODE == 1 && i0 < (kc + 1) * GK) {
-            // elements read from the upper triangle enter conjugated
-            const int k0 = kc * GK;
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int e = tid + 256 * u;
-                const int m = e & 63, k = e >> 6;
-                if (i0 + m < k0 + k) As[k * G_LDA + m].y = -As[k * G_LDA + m].y;
-            }
-            __syncthreads();
-        }
-#pragma unroll
-        for (int kk = 0; kk < GK; kk += 4) zmma_k4<4, 2, G_LDA, G_LDB, false>(acc, As, Bs, wm, wn, kk, lane);
-        __syncthreads();
+    int rst = 0;
+    unsigned rph = 0;
+    if (tid == 0) {
+        fence_async_global();
+        for (int i = 0; i < TMA_ST && u0 + i < u1; i++) issue(i);
     }
-    const int g = lane >> 2, t = lane & 3;
+    constexpr int MT = 4, NT = 2;
+    double accr[MT][NT][2], acci[MT][NT][2];
+    auto zero = [&] {
 #pragma unroll
-    for (int mt = 0; mt < 4; mt++)
+        for (int mt = 0; mt < MT; mt++)
 #pragma unroll
-        for (int nt = 0; nt < 2; nt++)
+            for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int i = i0 + wm + mt * 8 + g;
-                const int j = j0 + wn + nt * 8 + 2 * t + e;
-                if (i >= M) continue;
-                if (gridDim.z > 1) {  // partial sum of this K slice, by slot
-                    *reinterpret_cast<double2*>(P + blockIdx.z * pstride + (size_t)i + (size_t)j * ldc) =
-                        make_double2(acc.r[mt][nt][e], acc.i[mt][nt][e]);
-                    continue;
+                for (int e = 0; e < 2; e++) accr[mt][nt][e] = acci[mt][nt][e] = 0.0;
+    };
+    zero();
+    int k0 = k;  // where the tile's segment begins
+    bool first = true;
+    const int f0 = pg * TMA_KC + (t4 ^ pg);  // fragment slots of k = t4 and, with ^ 4, of k = 4 + t4
+    for (long long u = u0; u < u1; u++) {
+        const bool ok = bar_wait(ring.full + 8u * ring.st, ring.ph);
+        if (!__all_sync(0xffffffffu, ok)) {
+            if (lane == 0) atomicExch(a.status + ST_SOLVE_TIMEOUT, 1);
+            return;
+        }
+        const int it = t % a.mt;
+        const double2* Us = stages + ring.st * 2 * CG_OP + (wr * MT) * 64;
+        const double2* Vs = stages + ring.st * 2 * CG_OP + CG_OP + (wc * NT) * 64;
+        const bool diag = TRI && k < cg_first<TRI>(it) + 64 / TMA_KC;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int f = f0 ^ (4 * j);
+            double2 u2[MT], v[NT];
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++) u2[mt] = Us[mt * 64 + f];
+            if (diag) {
+                const int kq = k * TMA_KC + 4 * j + t4 - it * 64;
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    const int i = (wr * MT + mt) * 8 + pg;
+                    const double h = kq > i ? 1.0 : 0.5;
+                    u2[mt] = kq < i ? make_double2(0.0, 0.0) : make_double2(h * u2[mt].x, h * u2[mt].y);
                 }
-                const int jp = cmap ? cmap[j] : j;
-                cd v = mk(acc.r[mt][nt][e], acc.i[mt][nt][e]);
-                const size_t o = (size_t)i + (size_t)jp * ldc;
-                if (E1) v = cfma(ldcd(E1 + o), ldcd(e2 + jp), v);
-                *reinterpret_cast<double2*>(C + o) = make_double2(v.x, v.y);
             }
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) v[nt] = Vs[nt * 64 + f];
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                const double nr = -v[nt].x;
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    dmma(accr[mt][nt][0], accr[mt][nt][1], u2[mt].x, v[nt].x);
+                    dmma(acci[mt][nt][0], acci[mt][nt][1], u2[mt].x, v[nt].y);
+                }
+#pragma unroll
+                for (int mt = 0; mt < MT; mt++) {
+                    dmma(accr[mt][nt][0], accr[mt][nt][1], u2[mt].y, v[nt].y);
+                    dmma(acci[mt][nt][0], acci[mt][nt][1], u2[mt].y, nr);
+                }
+            }
+        }
+        __syncwarp();
+        if (lane == 0) bar_arrive(ring.empty + 8u * ring.st);
+        ring.step(ring.st, ring.ph);
+        if (tid == 0 && u - u0 >= 2 && u - 2 + TMA_ST < u1) {
+            // (without its stage a chunk is not asked for, and its wait runs out)
+            if (bar_wait(ring.empty + 8u * rst, rph)) issue(rst);
+            ring.step(rst, rph);
+        }
+        if (++k == a.nk || u + 1 == u1) {
+            const bool whole = k == a.nk && k0 == cg_first<TRI>(it);
+            cd* part = a.P + ((size_t)2 * blockIdx.x + (first ? 0 : 1)) * CG_TILE;
+#pragma unroll
+            for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+                for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        if (whole)
+                            cg_store(a, it * 64 + (wr * MT + mt) * 8 + pg,
+                                     (t / a.mt) * 64 + (wc * NT + nt) * 8 + 4 * e + t4, accr[mt][nt][e],
+                                     acci[mt][nt][e]);
+                        else
+                            *reinterpret_cast<double2*>(part + ((mt * NT + nt) * 2 + e) * 256 + tid) =
+                                make_double2(accr[mt][nt][e], acci[mt][nt][e]);
+                    }
+            zero();
+            t++;
+            k = k0 = cg_first<TRI>(t % a.mt);
+            first = false;
+        }
+    }
+}
+
+// Tiles that fell into several pieces: their partial sums, in order.  One
+// CTA for 256 values of a tile; `pieces` is k_cgemm's grid.
+template <bool TRI>
+__global__ void __launch_bounds__(256) k_cgemm_sum(const __grid_constant__ CgArgs a, int pieces)
+{
+    const int t = blockIdx.x, tid = threadIdx.x;
+    const long long ub = cg_before<TRI>(t, a.mt, a.nk), ue = cg_before<TRI>(t + 1, a.mt, a.nk);
+    // the piece a chunk falls into is the last that begins at or before it
+    const int b0 = (int)(((ub + 1) * pieces - 1) / a.total), b1 = (int)((ue * pieces - 1) / a.total);
+    if (b0 == b1) return;
+    const int lane = tid & 31, wp = tid >> 5, g = lane >> 2, t4 = lane & 3, pg = (g & 1) << 2 | g >> 1;
+    const int e = blockIdx.y;
+    const cd* part = a.P + e * 256 + tid;
+    // a piece that begins before the tile ends in it: its second partial tile
+    cd v = ldcd(part + ((size_t)2 * b0 + (a.total * b0 / pieces < ub ? 1 : 0)) * CG_TILE);
+#pragma unroll 8
+    for (int b = b0 + 1; b <= b1; b++) v = v + ldcd(part + (size_t)2 * b * CG_TILE);
+    cg_store(a, (t % a.mt) * 64 + ((wp >> 2) * 4 + (e >> 2)) * 8 + pg,
+             (t / a.mt) * 64 + ((wp & 3) * 2 + (e >> 1 & 1)) * 8 + 4 * (e & 1) + t4, v.x, v.y);
+}
+
+// The active columns in slot order, for the GEMM's boxes.
+__global__ void __launch_bounds__(256) k_cand_gather(const cd* __restrict__ V, cd* __restrict__ Vs, int nbase, int ldv,
+                                                     const int* __restrict__ cmap)
+{
+    const int q = blockIdx.x * 256 + threadIdx.x;
+    if (q < nbase) Vs[q + (size_t)blockIdx.y * ldv] = ldcd(V + q + (size_t)cmap[blockIdx.y] * ldv);
 }
 
 // ---------------------------------------------------------------------------
@@ -227,6 +336,11 @@ __device__ __forceinline__ void cs_mma(ZAcc<MT, 1>& acc, const double2* __restri
         }
     }
 }
+
+constexpr int GM = 64, GN = 64, GK = 32;
+constexpr int G_LDA = GM + 2;  // % 8 == 2
+constexpr int G_LDB = GK + 4;  // % 8 == 4
+constexpr int G_STAGE = GK * G_LDA + GN * G_LDB;
 
 // G tiles: one CTA per ordered panel pair (p, q), p != q; FWD blocks (p > q)
 // and BWD blocks (p < q) share the array, G(p0+m, q0+n) at Gm[(p0+m) + (q0+n) ld].
@@ -428,23 +542,6 @@ __global__ void __launch_bounds__(256, 2) k_cand_solve(const cd* __restrict__ Gm
             }
         __syncthreads();  // the next item loads over the ring
     }
-}
-
-// Split-K partial sums of k_zgemm are added in a fixed order:
-// C(:, slot j) = sum_z P[z](:, j) (+ E1 o e2), through the column map.
-__global__ void __launch_bounds__(256) k_zsum(const cd* __restrict__ P, int nz, size_t pstride, int M, int ncols,
-                                              int ldc, cd* __restrict__ C, const cd* __restrict__ E1,
-                                              const cd* __restrict__ e2, const int* __restrict__ cmap)
-{
-    const long long idx = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (idx >= (long long)M * ncols) return;
-    const int i = (int)(idx % M), j = (int)(idx / M);
-    cd v = mk(0.0, 0.0);
-    for (int z = 0; z < nz; z++) v = v + ldcd(P + z * pstride + (size_t)i + (size_t)j * ldc);
-    const int jp = cmap ? cmap[j] : j;
-    const size_t o = (size_t)i + (size_t)jp * ldc;
-    if (E1) v = cfma(ldcd(E1 + o), ldcd(e2 + jp), v);
-    *reinterpret_cast<double2*>(C + o) = make_double2(v.x, v.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -683,7 +780,8 @@ __global__ void __launch_bounds__(256) k_cand_unset(cd* __restrict__ a, cd* __re
 }
 
 // Rayleigh quotient (src/linalg.f90:1913-1917) of the final iterate:
-// t1 = v^H S v, t2 = v^H M v with P = S0 V, Q = M0 V; E = t2 / t1 + lambda~.
+// t1 = v^H S v, t2 = v^H M v, E = t2 / t1 + lambda~, with P and Q the lower
+// halves of S0 V and M0 V (k_cgemm<true>).
 __global__ void __launch_bounds__(256) k_cand_rayleigh(const cd* __restrict__ P, const cd* __restrict__ Q,
                                                        const cd* __restrict__ V, const cd* __restrict__ Scol,
                                                        const cd* __restrict__ Mcol, const double* __restrict__ mu,
@@ -710,8 +808,8 @@ __global__ void __launch_bounds__(256) k_cand_rayleigh(const cd* __restrict__ P,
     block_sum256<6>(a, sh);
     if (threadIdx.x == 0) {
         const cd vk = brd[BR_V * bcap + j];
-        const double t1 = a[0] + 2.0 * cmul(conj(vk), mk(a[2], a[3])).x + cnorm2(vk);
-        const double t2 = a[1] + 2.0 * cmul(conj(vk), mk(a[4], a[5])).x + mu[j] * cnorm2(vk);
+        const double t1 = 2.0 * a[0] + 2.0 * cmul(conj(vk), mk(a[2], a[3])).x + cnorm2(vk);
+        const double t2 = 2.0 * a[1] + 2.0 * cmul(conj(vk), mk(a[4], a[5])).x + mu[j] * cnorm2(vk);
         nd[ND_T1 * bcap + j] = t1;
         nd[ND_T2 * bcap + j] = t2;
         nd[ND_E * bcap + j] = (st[ST_ERR * bcap + j] == 1) ? __longlong_as_double(0x7ff8000000000000LL) : t2 / t1 + lam;
@@ -772,7 +870,14 @@ int ensure_work(Ctx& c, int count)
     r |= dalloc_n(&cw.st, (size_t)3 * ccap + 1);
     r |= dalloc_n(&cw.cmap, (size_t)ccap);
     r |= dalloc_n(&cw.Gm, (size_t)c.ld * c.ld);
-    r |= dalloc_n(&cw.Pk, (size_t)CAND_KSPLIT * ldv * 2 * CAND_PAD);
+    int nsm = 0, per = 0;
+    for (const void* f : {(const void*)k_cgemm<false>, (const void*)k_cgemm<true>})
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CG_SMEM);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cgemm<false>, 256, CG_SMEM);
+    cudaGetLastError();
+    cw.gemm_grid = std::max(1, nsm * per);
+    r |= dalloc_n(&cw.Pk, (size_t)cw.gemm_grid * 2 * CG_TILE);
     r |= dalloc_n(&cw.bstart, (size_t)maxpanels + 1);
     r |= dalloc_n(&cw.abort_word, 2);  // abort word, wait poll limit
     cw.gpart_n = (size_t)bcap * (c.ld / 128 + 2) * (2 * c.np + 1);
@@ -811,8 +916,6 @@ int solve_grid(Ctx& c)
     int coop = 0, nsm = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c.dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c.dev);
-    cudaFuncSetAttribute(k_zgemm<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM);
-    cudaFuncSetAttribute(k_zgemm<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G_SMEM);
     cudaFuncSetAttribute(k_cand_gmat, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(G_STAGE * sizeof(double2)));
     int per = 1 << 30;
@@ -870,29 +973,30 @@ int launch_solve(Ctx& c, int nb, int ncols, const cd* Win, cd* Yout, cd* Zout, c
                                  : launch_solve_nc<FWD, 16>(c, nb, ncols, Win, Yout, Zout, next, cmap);
 }
 
-int launch_gemm(Ctx& c, int amode, const cd* A, int M, int ncols, const cd* B, cd* C, const cd* E1, const cd* e2,
-                const int* cmap)
+// C = A^H B over nbase rows for ncols columns of B (see k_cgemm).
+template <bool TRI>
+int launch_gemm(Ctx& c, cd* A, int nbase, int ncols, cd* B, cd* C, const cd* E1, const cd* e2, const int* cmap)
 {
     CandWork& cw = c.cand;
-    if (M <= 0) return 0;
-    const int mt = (M + GM - 1) / GM, nt = ncols / GN;
-    // few output tiles (the late iterations run on one or two 64-column
-    // slots): split the inner dimension so that the GPU stays busy
-    int nz = 1;
-    if (ncols <= 2 * CAND_PAD) nz = std::max(1, std::min(CAND_KSPLIT, 148 / std::max(1, mt * nt)));
-    dim3 g(mt, nt, nz);
-    const size_t pstride = (size_t)cw.ldv * 2 * CAND_PAD;
-    if (amode == 0)
-        k_zgemm<0><<<g, 256, G_SMEM, c.stream>>>(A, c.ld, M, M, B, cw.ldv, C, cw.ldv, E1, e2, cmap, cw.Pk, pstride);
-    else
-        k_zgemm<1><<<g, 256, G_SMEM, c.stream>>>(A, c.ld, M, M, B, cw.ldv, C, cw.ldv, E1, e2, cmap, cw.Pk, pstride);
-    c.launches++;
-    if (nz > 1) {
-        const long long cnt = (long long)M * ncols;
-        k_zsum<<<(unsigned)((cnt + 255) / 256), 256, 0, c.stream>>>(cw.Pk, nz, pstride, M, ncols, cw.ldv, C, E1, e2,
-                                                                    cmap);
-        c.launches++;
-    }
+    if (nbase <= 0 || ncols <= 0) return 0;
+    CgArgs a{};
+    if (!tma_map(&a.a, A, c.ld, nbase, nbase, 64) || !tma_map(&a.b, B, cw.ldv, nbase, ncols, 64)) return -2;
+    a.M = nbase;
+    a.mt = (nbase + 63) / 64;
+    a.nk = (nbase + TMA_KC - 1) / TMA_KC;
+    a.ntile = a.mt * (ncols / 64);
+    a.total = cg_before<TRI>(a.ntile, a.mt, a.nk);
+    a.cmap = cmap;
+    a.C = C;
+    a.ldc = cw.ldv;
+    a.E1 = E1;
+    a.e2 = e2;
+    a.P = cw.Pk;
+    a.status = c.status;
+    const int pieces = (int)std::min<long long>(cw.gemm_grid, a.total);
+    k_cgemm<TRI><<<pieces, 256, CG_SMEM, c.stream>>>(a);
+    k_cgemm_sum<TRI><<<dim3(a.ntile, CG_TILE / 256), 256, 0, c.stream>>>(a, pieces);
+    c.launches += 2;
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -903,7 +1007,9 @@ int enqueue_iteration(Ctx& c, int nbase, int count, int ncols, int nb, double to
     CandWork& cw = c.cand;
     const int cc = cw.ccap;
     int r;
-    if ((r = launch_gemm(c, 0, c.S, nbase, ncols, cw.V, cw.W, cw.Scol, cw.brd + BR_V * cc, cw.cmap))) return r;
+    k_cand_gather<<<dim3((nbase + 255) / 256, ncols), 256, 0, c.stream>>>(cw.V, cw.X2, nbase, cw.ldv, cw.cmap);
+    c.launches++;
+    if ((r = launch_gemm<false>(c, c.S, nbase, ncols, cw.X2, cw.W, cw.Scol, cw.brd + BR_V * cc, cw.cmap))) return r;
     if ((r = launch_solve<true>(c, nb, ncols, cw.W, cw.Y, cw.Z, cw.X, cw.cmap))) return r;
     k_cand_mid<<<ncols, 256, 0, c.stream>>>(cw.Scol, cw.V, cw.Lcol, cw.Y, nbase, cw.ldv, cc, cw.brd, cw.cmap, count);
     c.launches++;
@@ -1115,8 +1221,8 @@ int eval_candidates(Ctx& c, int nbase, int count, const double* cand_host, doubl
         if (run_iteration(c, nbase, count, nslots, nb, tol)) return ECG_ECUDA;
     }
     // Rayleigh quotients of the final iterates (all candidates)
-    if (launch_gemm(c, 0, c.S, nbase, ncols, cw.V, cw.X, nullptr, nullptr, nullptr)) return ECG_ECUDA;
-    if (launch_gemm(c, 1, c.F, nbase, ncols, cw.V, cw.X2, nullptr, nullptr, nullptr)) return ECG_ECUDA;
+    if (launch_gemm<true>(c, c.S, nbase, ncols, cw.V, cw.X, nullptr, nullptr, nullptr)) return ECG_ECUDA;
+    if (launch_gemm<true>(c, c.F, nbase, ncols, cw.V, cw.X2, nullptr, nullptr, nullptr)) return ECG_ECUDA;
     k_cand_rayleigh<<<count, 256, 0, c.stream>>>(cw.X, cw.X2, cw.V, cw.Scol, cw.Mcol, cw.mu, nbase, cw.ldv, cc,
                                                  cw.brd, cw.nd, cw.st, approx_e);
     c.launches++;

@@ -45,8 +45,6 @@ constexpr int ADJ_SHAPES = 2;
 // 8, not 16, and the padding unit of the candidate column blocks.
 constexpr int CAND_NC8_MAX = 256;
 constexpr int CAND_PAD = 64;
-// Largest split of the inner dimension of the candidates' GEMM.
-constexpr int CAND_KSPLIT = 4;
 
 // Workspace of the batched candidate evaluation (allocated on first use).
 // Column blocks are ldv x ccap, column j = candidate j, rows = base
@@ -59,7 +57,8 @@ struct CandWork {
     int ldv = 0;             // rows of the column blocks (ld rounded up to 64)
     int* cmap = nullptr;     // slot -> physical column of the active candidates (ccap)
     cd* Gm = nullptr;        // ld x ld: off-diagonal factor blocks premultiplied by Linv (solves)
-    cd* Pk = nullptr;        // CAND_KSPLIT x ldv x 2 CAND_PAD: split-K partial sums of the GEMM
+    cd* Pk = nullptr;        // two 64 x 64 partial tiles for each CTA of the GEMM
+    int gemm_grid = 0;       // CTAs of the GEMM (two an SM)
     double* par = nullptr;   // npt x bcap candidate parameters
     cd* bra = nullptr;       // bcap x NP
     cd* ket = nullptr;       // bcap x T x NP
@@ -76,7 +75,7 @@ struct CandWork {
     cd* Y = nullptr;         // forward solve
     cd* Z = nullptr;         // invD o Y
     cd* X = nullptr;         // backward solve (new x); Rayleigh products
-    cd* X2 = nullptr;        // second Rayleigh product
+    cd* X2 = nullptr;        // active columns of V in slot order; second Rayleigh product
     cd* brd = nullptr;       // border entries: [0] vK [1] invDK [2] xK
     double* nd = nullptr;    // NormOfDiff, NormOfDiffPrev, t1, t2, E
     int* st = nullptr;       // active, iterations, ErrorCode, then the active count

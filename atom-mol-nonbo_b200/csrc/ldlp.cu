@@ -48,24 +48,22 @@
 #include <queue>
 #include <utility>
 #include <vector>
-#include <cuda.h>  // CUtensorMap
 #include "ecg_internal.h"
 #include "zmma.cuh"
+#include "tma_ring.cuh"
 
 namespace ecg {
 
 constexpr unsigned LP_D = 0, LP_T = 1, LP_B = 2;
 constexpr unsigned LP_NONE = 0xffffffffu;
-constexpr int LP_KC = 8;           // k rows per TMA stage of an update: 128 bytes, the width of the swizzle
-constexpr int LP_ST = 6;           // stages
-constexpr int LP_OP = LP_KC * LDL_NB;  // double2 of one staged operand (8 KB)
+constexpr int LP_OP = TMA_KC * LDL_NB;  // double2 of one staged operand (8 KB)
 constexpr int LP_MERGE = 4;        // most panels one trailing update applies at once
 // Aligned groups of LP_MERGE panels whose update of a tile row at least this
 // far from the group's first panel is one task of the list: nearer rows are
 // wanted before the group's last panel is there.
 constexpr int LP_FAR = 8;
 // 1 KB to align the stages, which the swizzle wants
-constexpr size_t LP_SMEM_B = 1024 + (size_t)(LP_ST * 2 * LP_OP + LP_MERGE * LDL_NB) * sizeof(double2);
+constexpr size_t LP_SMEM_B = 1024 + (size_t)(TMA_ST * 2 * LP_OP + LP_MERGE * LDL_NB) * sizeof(double2);
 
 __host__ __device__ __forceinline__ unsigned lp_code(unsigned type, int s, int R, int C, unsigned half = 0)
 {
@@ -278,55 +276,6 @@ __device__ __forceinline__ cd lp_shfl(cd v, int src)
     return cd{__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src)};
 }
 
-// ---------------------------------------------------------------------------
-// TMA and mbarriers of the updates.
-// ---------------------------------------------------------------------------
-constexpr int LP_TMA_LIMIT = 1 << 21;  // bound on the polls for a copy or a stage (tens of ms)
-
-__device__ __forceinline__ unsigned lp_s32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void lp_bar_init(unsigned bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void lp_bar_arrive(unsigned bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void lp_bar_expect(unsigned bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Wait for the phase of the given parity to end; false when the limit runs out.
-__device__ __forceinline__ bool lp_bar_wait(unsigned bar, unsigned parity)
-{
-    for (int i = 0; i < LP_TMA_LIMIT; i++) {
-        unsigned done;
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-// Box of 8 complex rows from row k0 (16 doubles, x = 2 k0: 16-byte aligned)
-// and the map's columns from column c.
-__device__ __forceinline__ void lp_tma(unsigned dst, const CUtensorMap* map, int k0, int c, unsigned bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            dst),
-        "l"(map), "r"(2 * k0), "r"(c), "r"(bar)
-        : "memory");
-}
-__device__ __forceinline__ void lp_fence_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
-__device__ __forceinline__ void lp_fence_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
 // T(s, C): U(s, C) = invD Linv_ss W(s, C) for the 64 columns of tile (s, C),
 // Linv_ss = L_ss^-1 (unit lower) as the diagonal task left it: one product
 // with a triangular matrix on the FP64 tensor cores, 288 independent-ordered
@@ -409,8 +358,8 @@ __device__ void lp_panel(cd* __restrict__ A, int ld, int n, int s, int C, const 
                 A[(size_t)(p0 + 8 * m + g) + (size_t)(cb + c) * ld] = cmul(cd{accr[m][e], acci[m][e]}, cd{d.x, d.y});
         }
     }
-    lp_fence_async_global();  // read by TMA in the updates
-    lp_fence_async_shared();  // and this memory is written by TMA next
+    fence_async_global();  // read by TMA in the updates
+    fence_async_shared();  // and this memory is written by TMA next
 }
 
 struct alignas(64) LpArgs {
@@ -431,21 +380,6 @@ struct alignas(64) LpArgs {
     unsigned long long* trace;  // optional: per task (code | cta << 32 | panels << 48, start, ready, done)
 };
 
-// The stages' ring as it goes on from one update to the next: the next
-// stage and the parity of its current use.
-struct LpRing {
-    unsigned full, empty;  // shared addresses of LP_ST mbarriers each
-    int st = 0;
-    unsigned ph = 0;
-    __device__ __forceinline__ void step(int& i, unsigned& p) const
-    {
-        if (++i == LP_ST) {
-            i = 0;
-            p ^= 1u;
-        }
-    }
-};
-
 // B(s, R, C): W(r, c) -= sum_q conj(U(q, r)) d_q U(q, c) over the 64 x 64
 // tile, r <= c on a diagonal tile (its diagonal in dw).  Eight warps as
 // 2 x 4, each a 32 x 16 complex sub-tile of 8 x 8 mma tiles; the tile's
@@ -455,7 +389,7 @@ struct LpRing {
 // applied in one pass when they are all ready: a rank-64m update, the
 // tile read and written once.
 // U(s, R) and U(s, C) come by TMA, eight k rows a stage, through a ring of
-// LP_ST stages: thread 0 refills a stage once the eight warps have left it
+// TMA_ST stages: thread 0 refills a stage once the eight warps have left it
 // (two chunks behind its own), each warp waits only for its data, and no
 // barrier stands between chunks.  The 128-byte swizzle puts row k of column
 // c at 16-byte slot c * 8 + (k ^ (c & 7)); with the columns of an 8 x 8 mma
@@ -468,7 +402,7 @@ struct LpRing {
 // MT x NT mma tiles per warp, WR x WC warps: <4, 2, 2, 4> covers the whole
 // 64 x 64 tile, <2, 2, 4, 2> the 64 x 32 column half `half` of it.
 template <bool CPLX, int MT, int NT, int WR, int WC>
-__device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half, double2* sm, LpRing& ring)
+__device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half, double2* sm, TmaRing& ring)
 {
     static_assert(WR * WC == 8 && WR * MT * 8 == LDL_NB, "eight warps over the 64 tile rows");
     constexpr int CW = WC * NT * 8;  // columns covered
@@ -481,24 +415,24 @@ __device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half,
     const int p0 = s * LDL_NB;
     const int rb = R * LDL_NB, cb = C * LDL_NB + half * CW;
     const bool dtile = (R == C);
-    const unsigned base = (lp_s32(sm) + 1023u) & ~1023u;
-    double2* stages = sm + (base - lp_s32(sm)) / sizeof(double2);
-    double2* dp = stages + LP_ST * 2 * LP_OP;  // pivots d_q of panels s..s+m-1
-    const int nch = m * (LDL_NB / LP_KC);      // panels with rows below them are whole
+    const unsigned base = (smem32(sm) + 1023u) & ~1023u;
+    double2* stages = sm + (base - smem32(sm)) / sizeof(double2);
+    double2* dp = stages + TMA_ST * 2 * LP_OP;  // pivots d_q of panels s..s+m-1
+    const int nch = m * (LDL_NB / TMA_KC);      // panels with rows below them are whole
     auto issue = [&](int ch, int st) {
         const unsigned bar = ring.full + 8u * st, dst = base + (unsigned)(st * 2 * LP_OP * sizeof(double2));
-        lp_bar_expect(bar, (unsigned)((LP_OP + LP_KC * CW) * sizeof(double2)));
-        lp_tma(dst, &a.t64, p0 + ch * LP_KC, rb, bar);
-        lp_tma(dst + (unsigned)(LP_OP * sizeof(double2)), CW == LDL_NB ? &a.t64 : &a.t32, p0 + ch * LP_KC, cb, bar);
+        bar_expect(bar, (unsigned)((LP_OP + TMA_KC * CW) * sizeof(double2)));
+        tma_box(dst, &a.t64, p0 + ch * TMA_KC, rb, bar);
+        tma_box(dst + (unsigned)(LP_OP * sizeof(double2)), CW == LDL_NB ? &a.t64 : &a.t32, p0 + ch * TMA_KC, cb, bar);
     };
     // the stage refilled next (thread 0) and the parity its last use ends with
     int rst = ring.st;
     unsigned rph = ring.ph;
     if (tid == 0) {
-        lp_fence_async_global();  // the panel rows were written by other CTAs' ordinary stores
+        fence_async_global();  // the panel rows were written by other CTAs' ordinary stores
         int st = ring.st;
         unsigned ph = ring.ph;
-        for (int ch = 0; ch < min(LP_ST, nch); ch++) {
+        for (int ch = 0; ch < min(TMA_ST, nch); ch++) {
             issue(ch, st);
             ring.step(st, ph);
         }
@@ -529,9 +463,9 @@ __device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half,
             }
     __syncthreads();  // dp
     bool ok = true;
-    const int f0 = pg * LP_KC + (t4 ^ pg);  // fragment slots of k = t4 and, with ^ 4, of k = 4 + t4
+    const int f0 = pg * TMA_KC + (t4 ^ pg);  // fragment slots of k = t4 and, with ^ 4, of k = 4 + t4
     for (int ch = 0; ch < nch; ch++) {
-        ok = lp_bar_wait(ring.full + 8u * ring.st, ring.ph);
+        ok = bar_wait(ring.full + 8u * ring.st, ring.ph);
         if (!__all_sync(0xffffffffu, ok)) break;
         if (wact) {
             const double2* Us = stages + ring.st * 2 * LP_OP + (wr * MT) * 64;
@@ -539,7 +473,7 @@ __device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half,
 #pragma unroll
             for (int j = 0; j < 2; j++) {
                 const int f = f0 ^ (4 * j);
-                const double2 d = dp[ch * LP_KC + 4 * j + t4];
+                const double2 d = dp[ch * TMA_KC + 4 * j + t4];
                 double2 u[MT];
                 double vr[NT], vi[NT];
 #pragma unroll
@@ -568,11 +502,11 @@ __device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half,
             }
         }
         __syncwarp();
-        if (lane == 0) lp_bar_arrive(ring.empty + 8u * ring.st);
+        if (lane == 0) bar_arrive(ring.empty + 8u * ring.st);
         ring.step(ring.st, ring.ph);
-        if (tid == 0 && ch >= 2 && ch - 2 + LP_ST < nch) {
+        if (tid == 0 && ch >= 2 && ch - 2 + TMA_ST < nch) {
             // (without its stage a chunk is not asked for, and its wait runs out)
-            if (lp_bar_wait(ring.empty + 8u * rst, rph)) issue(ch - 2 + LP_ST, rst);
+            if (bar_wait(ring.empty + 8u * rst, rph)) issue(ch - 2 + TMA_ST, rst);
             ring.step(rst, rph);
         }
     }
@@ -666,7 +600,7 @@ __device__ __forceinline__ void lp_trace(const LpArgs& a, unsigned code, int m, 
 // False when a copy did not arrive.
 template <bool CPLX>
 __device__ __forceinline__ bool lp_exec(const LpArgs& a, unsigned type, int s, int m, int R, int C, int half,
-                                        double2* sm, LpRing& ring)
+                                        double2* sm, TmaRing& ring)
 {
     if (type == LP_T) {
         lp_panel(a.A, a.ld, a.n, s, C, a.invD, a.linv, sm);
@@ -714,7 +648,7 @@ constexpr int LC_XP = 9;   // pitch of X_b
 constexpr size_t LP_SMEM_C = (size_t)(LI_N + LDL_NB * LT_WP + 2 * LDL_NB + 8 * LC_UP + 8 * LC_XP) * sizeof(double2);
 constexpr size_t lp_max(size_t a, size_t b) { return a > b ? a : b; }
 constexpr size_t LP_SMEM_BAR = lp_max(LP_SMEM_B, lp_max(LP_SMEM_C, LP_SMEM_T));  // the ring's mbarriers
-constexpr size_t LP_SMEM = LP_SMEM_BAR + 2 * LP_ST * 8;
+constexpr size_t LP_SMEM = LP_SMEM_BAR + 2 * TMA_ST * 8;
 
 // 1/d of a normal d, without a branch: the hardware's seed y (about 20 bits)
 // and the geometric series of 1 / (1 - e), e = 1 - d y, to e^2 (remainder
@@ -1050,7 +984,7 @@ __device__ void lp_chain(const LpArgs& a, double2* sm, int limit)
                 }
             }
         }
-        lp_fence_async_global();
+        fence_async_global();
         __syncthreads();
         lp_publish(a, lp_tix(s, s + 1), (unsigned)s + 1);
         if (tid == 0) lp_trace(a, lp_code(LP_T, s, s, s + 1), 1, t0, t1);
@@ -1114,16 +1048,8 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
         lp_chain<CPLX>(a, lsm, limit);
         return;
     }
-    LpRing ring;
-    ring.full = lp_s32(lsm) + (unsigned)LP_SMEM_BAR;
-    ring.empty = ring.full + 8u * LP_ST;
-    if (tid == 0) {
-        for (int i = 0; i < LP_ST; i++) {
-            lp_bar_init(ring.full + 8u * i, 1);
-            lp_bar_init(ring.empty + 8u * i, 8);
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+    TmaRing ring;
+    ring.init(smem32(lsm) + (unsigned)LP_SMEM_BAR, tid);
     __syncthreads();
     for (;;) {
         unsigned long long t0 = 0, t1 = 0;
@@ -1190,7 +1116,7 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
         if (go == 1) {
             if (!lp_exec<CPLX>(a, type, s, m, R, C, half, lsm, ring)) {
                 // a copy did not arrive: wait for the others in flight, report, stop
-                for (int i = 0; i < LP_ST; i++) lp_bar_wait(ring.full + 8u * i, ring.ph);
+                for (int i = 0; i < TMA_ST; i++) bar_wait(ring.full + 8u * i, ring.ph);
                 if (tid == 0) {
                     atomicExch(a.status + ST_SOLVE_TIMEOUT, 1);
                     atomicExch(a.ctl + 1, 1u);
@@ -1216,27 +1142,6 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
 }
 
 static bool g_lp_attr = false;
-
-// Tensor map of the n x n matrix at A (column-major complex) as doubles by
-// columns, boxes of LP_KC complex rows x `cols` columns, 128-byte swizzle.
-static bool lp_map(CUtensorMap* map, void* A, int ld, int n, int cols)
-{
-    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult found;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &found) != cudaSuccess || !fn) {
-        cudaGetLastError();
-        return false;
-    }
-    const cuuint64_t dim[2] = {2 * (cuuint64_t)n, (cuuint64_t)n}, stride[1] = {(cuuint64_t)ld * sizeof(cd)};
-    const cuuint32_t box[2] = {2 * LP_KC, (cuuint32_t)cols}, one[2] = {1, 1};
-    return reinterpret_cast<Encode>(fn)(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, A, dim, stride, box, one,
-                                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 
 // Grid of the persistent kernel (co-resident CTAs), 0 if unavailable.
 int ldlp_grid(Ctx& c)
@@ -1328,7 +1233,7 @@ int ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long
     const size_t ntile = (size_t)np * (np + 1) / 2;
     cudaMemsetAsync(c.lp_cnt, 0, (3 * ntile + 4) * sizeof(unsigned), c.stream);
     LpArgs a;
-    if (!lp_map(&a.t64, c.F, c.ld, n, LDL_NB) || !lp_map(&a.t32, c.F, c.ld, n, LDL_NB / 2)) return -2;
+    if (!tma_map(&a.t64, c.F, c.ld, n, n, LDL_NB) || !tma_map(&a.t32, c.F, c.ld, n, n, LDL_NB / 2)) return -2;
     a.A = c.F;
     a.ld = c.ld;
     a.n = n;

@@ -13,11 +13,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nbase,count,grown", [(1, 257, 0), (31, 257, 0), (33, 320, 0), (64, 258, 0), (65, 257, 0),
-                                               (127, 300, 0), (129, 257, 0), (70, 257, 5), (130, 300, 3)])
+                                               (127, 300, 0), (129, 257, 0), (70, 257, 5), (130, 300, 3), (100, 20100, 0), (700, 300, 0)])
 def test_batches_of_both_widths_agree(nbase, count, grown):
     """Below the spectrum, where the iteration is well conditioned, the two
     widths multiply and add the same numbers in the same order except in the
-    GEMM, whose inner sum is split for few columns: energies agree to 1e-11
+    GEMM, whose inner sum is cut into pieces by the number of tiles (from
+    pieces of one chunk to several tiles a piece): energies agree to 1e-11
     (a stationary value of vectors converged to 1e-9), ErrorCodes exactly."""
     sysm, params, lam0, _ = problem(1, nbase)
     cands = synth.candidates(params, count, 5)
