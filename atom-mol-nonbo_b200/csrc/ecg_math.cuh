@@ -50,40 +50,6 @@ __device__ __forceinline__ cd crcp(cd b)
     const double d = 1.0 / cnorm2(b);
     return cd{b.x * d, -b.y * d};
 }
-__device__ __forceinline__ cd cdiv(cd a, cd b)
-{
-    const double d = 1.0 / cnorm2(b);
-    return cd{fma(a.x, b.x, a.y * b.y) * d, fma(a.y, b.x, -a.x * b.y) * d};
-}
-// real / complex
-__device__ __forceinline__ cd rdiv(double r, cd b)
-{
-    const double d = r / cnorm2(b);
-    return cd{b.x * d, -b.y * d};
-}
-// Principal square root (branch cut on the negative real axis, as the
-// Fortran intrinsic): Kahan's formulation, "Branch cuts for complex
-// elementary functions" (1987): t = sqrt((|x| + |z|)/2), then the other
-// component y/(2t).  One sqrt for |z| and one reciprocal square root give
-// both t and 1/t.  Also returns |z| (= |sqrt z|^2).
-__device__ __forceinline__ cd csqrt_r(cd z, double& absz)
-{
-    const double r = sqrt(fma(z.x, z.x, z.y * z.y));
-    absz = r;
-    if (r == 0.0) return cd{0.0, z.y};
-    const double u = 0.5 * (fabs(z.x) + r);
-    const double ri = rsqrt(u);
-    const double t = u * ri;
-    const double h = 0.5 * z.y * ri;
-    if (z.x >= 0.0) return cd{t, h};
-    return cd{fabs(h), copysign(t, z.y)};
-}
-__device__ __forceinline__ cd csqrt(cd z)
-{
-    double r;
-    return csqrt_r(z, r);
-}
-
 // Physical constants of one system: the n x n mass matrix
 // Glob_MassMatrix (src/workproc.f90:606-610), pseudo-charges q0, q_i and
 // 2^(3n/2) (src/globvars.f90:69).
@@ -143,9 +109,11 @@ __device__ __forceinline__ cd crcp_series(cd b)
 }
 
 // 1/sqrt(a) on the principal branch, and 1/a in ra.  With q = 1/|a| the
-// inverse is conj(a) q^2 and its modulus q itself, so Kahan's formulation
-// (csqrt_r above) of sqrt(1/a) needs two reciprocal square roots and no
-// division.
+// inverse is conj(a) q^2 and its modulus q itself, so Kahan's formulation of
+// the square root ("Branch cuts for complex elementary functions", 1987: t =
+// sqrt((|x| + |z|)/2), the other component y/(2t)) needs two reciprocal
+// square roots and no division.  The branch cut is on the negative real axis,
+// as the Fortran intrinsic's.
 __device__ __forceinline__ cd crsqrt(cd a, cd& ra)
 {
     const double q = rsqrt_series(cnorm2(a));

@@ -4,24 +4,28 @@
 //
 // One thread evaluates one pair (row i >= column j) for every symmetry term
 // of the list, and adds each value's weight  factor * coef * Re(c_i^* c_j O)
-// and its rounding-error bound (the reference's MEkl_s / MEkl_e) into
-// per-thread shared-memory accumulators as the value is produced, so no
-// pair term is stored.  Blocks then sum their threads in a fixed order and
-// a second kernel sums the blocks in a fixed order: the result does not
+// and its rounding-error bound (the reference's MEkl_s / MEkl_e) to sums over
+// its warp as the value is produced, so no pair term is stored.  A second
+// kernel sums the blocks; every order is fixed, so the result does not
 // depend on scheduling.  Correlation functions and particle densities
 // (the grid parts) run as a second pair kernel whose blocks also split the
 // grid, with the same two-level reduction.
 //
-// The n x n algebra is restated with vectors: for a pair index P = (a, b),
-// u_P = e_a (a = b) or e_a - e_b, d_P = C^-1 u_P and TrCJ_P = u_P' C^-1 u_P;
-// then tr[C^-1 X C^-1 J_P] = d_P' X d_P, which is what the reference's
-// ME_rXr_over_rij / ME_rXr_rYr_over_rij (src/matelem.f90:753-945) sum
-// element by element.  Most matrices the reference builds for these traces
-// are rank one or sums of rank-one terms (J C, C J_ii C in the
-// mass-velocity terms, the Wc1..Wc3 of the orbit-orbit loops, E_ii / E_jj
-// and the all-ones matrix of the Drachmanised Darwin term), so their traces
-// are taken as dot products.  Results agree with the reference's to
-// rounding.
+// The n x n algebra is restated through three matrices.  With C = tCk + tCl,
+// a pair index P = (a, b), u_P = e_a (a = b) or e_a - e_b and TrCJ_P =
+// u_P' C^-1 u_P, the traces of ME_rXr_over_rij, ME_rXr_rYr_over_rij, ME_dXd
+// and ME_dXd_dYd (src/matelem.f90:753-945) are quadratic forms in C^-1 tCl,
+// C^-1 tCk and X = tCk C^-1 tCl, and tCk C^-1 tCk = tCk - X, tCl C^-1 tCl =
+// tCl - X (all symmetric).  Put in, the long sums the reference takes term
+// by term leave
+//   kinetic            6 S tr[M X]
+//   mass-velocity      -(36/8) (5/3) S (X_k l summed squared / m0^3 + sum_i X_ii^2 / m_i^3)
+//   ME_dXd_dYd         36 X_ii X_jj + 24 X_ij^2 (X = E_ii, Y = E_jj)
+//   orbit-orbit        -8 X_ij <1/r_P> of each (i, j)
+// so the Drachmanised mass-velocity and Darwin sums are one value (the
+// reference's own check of them), and the cancellation between the terms,
+// which cost the orbit-orbit term up to seven digits, does not happen.
+// Results agree with the reference's to its rounding.
 //
 // TrCJCJ(i,j,p,q) of src/matelem.f90:1270-1300 is never assigned for
 // i = j < p < q (n >= 3) but is read by the 1/(r_ij r_pq) loop; the
@@ -30,12 +34,15 @@
 #include <float.h>
 #include <algorithm>
 #include "ecg_internal.h"
+#include "warp_sums.cuh"
 
 namespace ecg {
 
 namespace {
 
-constexpr int EXPC_BLK = 64;
+constexpr int EXPC_BLK = 128;
+constexpr int EXPC_MINB = 2;  // CTAs an SM
+constexpr int GRID_BLK = 64;
 constexpr double PI_D = 3.14159265358979323846264338327950;
 
 __device__ __forceinline__ cd cexp_(cd z)
@@ -45,8 +52,6 @@ __device__ __forceinline__ cd cexp_(cd z)
     const double e = exp(z.x);
     return mk(e * c, e * s);
 }
-// principal branch, as Fortran's log of a complex argument
-__device__ __forceinline__ cd clog_(cd z) { return mk(log(hypot(z.x, z.y)), atan2(z.y, z.x)); }
 
 template <int N>
 __device__ __forceinline__ void mm(const cd (&A)[N][N], const cd (&B)[N][N], cd (&C)[N][N])
@@ -61,110 +66,16 @@ __device__ __forceinline__ void mm(const cd (&A)[N][N], const cd (&B)[N][N], cd 
             C[i][j] = s;
         }
 }
-// tr(A B)
-template <int N>
-__device__ __forceinline__ cd trmm(const cd (&A)[N][N], const cd (&B)[N][N])
-{
-    cd s = mk(0.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-        for (int j = 0; j < N; j++) s = cfma(A[i][j], B[j][i], s);
-    return s;
-}
-template <int N>
-__device__ __forceinline__ cd trace(const cd (&A)[N][N])
-{
-    cd s = mk(0.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < N; i++) s = s + A[i][i];
-    return s;
-}
-// u' A v
-template <int N>
-__device__ __forceinline__ cd quad(const cd (&u)[N], const cd (&A)[N][N], const cd (&v)[N])
-{
-    cd s = mk(0.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        cd t = mk(0.0, 0.0);
-#pragma unroll
-        for (int j = 0; j < N; j++) t = cfma(A[i][j], v[j], t);
-        s = cfma(u[i], t, s);
-    }
-    return s;
-}
-template <int N>
-__device__ __forceinline__ cd dot(const cd (&u)[N], const cd (&v)[N])
-{
-    cd s = mk(0.0, 0.0);
-#pragma unroll
-    for (int i = 0; i < N; i++) s = cfma(u[i], v[i], s);
-    return s;
-}
-
-// v[k] for a runtime k, by selects (keeps v in registers)
-template <int N>
-__device__ __forceinline__ cd pick(const cd (&v)[N], int k)
-{
-    cd r = v[0];
-#pragma unroll
-    for (int m = 1; m < N; m++)
-        if (k == m) r = v[m];
-    return r;
-}
-template <int N>
-__device__ __forceinline__ double pickd(const double (&v)[N], int k)
-{
-    double r = v[0];
-#pragma unroll
-    for (int m = 1; m < N; m++)
-        if (k == m) r = v[m];
-    return r;
-}
-
-// Per pair index P = (a, b) in vech order: d_P = C^-1 u_P and TrCJ_P.
-template <int N>
-struct PairVecs {
-    static constexpr int NP = N * (N + 1) / 2;
-    cd d[NP][N];
-    cd tr[NP];
-};
-
-template <int N>
-__device__ __forceinline__ void pair_vecs(const cd (&inv)[N][N], PairVecs<N>& pv)
-{
-    int P = 0;
-#pragma unroll
-    for (int a = 0; a < N; a++)
-#pragma unroll
-        for (int b = a; b < N; b++, P++) {
-            if (a == b) {
-#pragma unroll
-                for (int m = 0; m < N; m++) pv.d[P][m] = inv[m][a];
-                pv.tr[P] = inv[a][a];
-            } else {
-#pragma unroll
-                for (int m = 0; m < N; m++) pv.d[P][m] = inv[m][a] - inv[m][b];
-                // inv(i,i) + inv(j,j) - inv(j,i) - inv(j,i), src/matelem.f90:1252
-                pv.tr[P] = inv[a][a] + inv[b][b] - inv[b][a] - inv[b][a];
-            }
-        }
-}
-
-// tCl X tCl and tr(tCl X) (the products of ME_dXd / ME_dXd_over_rij)
-template <int N>
-__device__ __forceinline__ cd clxcl(const cd (&X)[N][N], const cd (&tCl)[N][N], cd (&M)[N][N])
-{
-    cd T1[N][N];
-    mm(X, tCl, T1);
-    mm(tCl, T1, M);
-    return trmm(tCl, X);
-}
-
 struct ExpcArgs {
     SysParams sp;
-    double mass[NMAX + 1];       // Glob_Mass: m0, m1..mn
+    // what the values take of the masses and charges, so that no thread
+    // divides by them
+    double im2[NMAX + 1], im3[NMAX + 1];  // 1 / m^2, 1 / m^3 of m0, m1..mn
+    double cw[NMAX][NMAX];       // (m_k + m_p) / (m_k m_p)^2, k < p; [p][p]: with m0 for m_k
+    double wq[NMAX][NMAX];       // q0 q_a, or q_a q_b for a < b
+    double wdw[NMAX][NMAX];      // wq (1 / m0^2 + 1 / m_a^2), or with m_a, m_b
+    double woo[NMAX][NMAX];      // wq / (m0 m_a), or -wq / (m_a m_b)
+    double icm[NMAX][NMAX];      // 1 / (2 pi (M_aa or M_aa + M_bb - 2 M_ab))
     double bvc[NMAX][NMAX + 1];  // Glob_bvc
     double energy;               // Glob_CurrEnergy
     double err_mult;             // 2 (SymmAdaptMethod 1) or 3 (2)
@@ -173,20 +84,38 @@ struct ExpcArgs {
     long long npairs;
 };
 
-// Weighted accumulation of one value (src/workproc.f90:8218-8225).
+// Weighted accumulation of the values in MEkl order (src/workproc.f90:
+// 8218-8225), four at a time: their weights and error bounds are summed over
+// the warp, and lane l keeps the running sum of entry l / 4 of each group
+// (entries 2k and 2k + 1: weight and bound of the group's value k).  A thread
+// of the warp without a pair has w = 0.
+template <int NV>
 struct Acc {
-    double* s;
-    double* e;
+    static constexpr int G = (NV + 3) / 4;
+    double sum[G];
+    double buf[8];
     double p1, p2;                 // Re(c_i^* c_j), -Im(c_i^* c_j)
     double rci, ici, rcj, icj;
     double w, em;
-    __device__ __forceinline__ void add(int a, cd O) const
+    __device__ __forceinline__ void zero()
+    {
+#pragma unroll
+        for (int g = 0; g < G; g++) sum[g] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) buf[k] = 0.0;
+    }
+    __device__ __forceinline__ void add(int a, cd O)
     {
         const double beta = p1 * O.x + p2 * O.y;
         const double mu = fabs(rci * (rcj * O.x - icj * O.y)) + fabs(rcj * (rci * O.x + ici * O.y)) +
                           fabs(ici * (icj * O.x + rcj * O.y)) + fabs(icj * (ici * O.x - rci * O.y));
-        s[a * EXPC_BLK] += w * beta;
-        e[a * EXPC_BLK] += fabs(w * (mu + em * fabs(beta)));
+        buf[2 * (a & 3)] = w * beta;
+        buf[2 * (a & 3) + 1] = fabs(w * (mu + em * fabs(beta)));
+        if ((a & 3) == 3 || a == NV - 1) {
+            sum[a >> 2] += warp_transpose_sum<8>(buf);
+#pragma unroll
+            for (int k = 0; k < 8; k++) buf[k] = 0.0;
+        }
     }
 };
 
@@ -257,55 +186,60 @@ __device__ __forceinline__ void congruence(const double (&X)[N][N], const double
         }
 }
 
-// Pseudo-Cholesky C = G G' of C = tCk + tCl, its inverse and the overlap
-// (src/matelem.f90:1152-1201).
+// C = tCk + tCl = L D L' (its pivots are the squares of those of the
+// pseudo-Cholesky factor of src/matelem.f90:1152-1201), its inverse and the
+// overlap.
 template <int N>
 __device__ __forceinline__ void inverse_overlap(const cd (&C)[N][N], double absdet, double two_r3n2,
                                                 cd (&inv)[N][N], cd& S)
 {
-    cd G[N][N], rg[N];
+    cd L[N][N], G[N][N], X[N][N], r[N];
     cd det = mk(1.0, 0.0);
 #pragma unroll
     for (int i = 0; i < N; i++) {
-        {
-            cd s = C[i][i];
+        cd d = C[i][i];
 #pragma unroll
-            for (int k = i - 1; k >= 0; k--) s = cfms(G[i][k], G[i][k], s);
-            G[i][i] = csqrt(s);
-            det = det * s;
-            rg[i] = crcp(G[i][i]);
-        }
+        for (int k = 0; k < i; k++) d = cfms(L[i][k], G[i][k], d);
+        det = (i == 0) ? d : det * d;
+        r[i] = crcp_series(d);
 #pragma unroll
         for (int j = i + 1; j < N; j++) {
-            cd s = C[i][j];
+            cd g = C[i][j];
 #pragma unroll
-            for (int k = i - 1; k >= 0; k--) s = cfms(G[i][k], G[j][k], s);
-            G[j][i] = cmul(s, rg[i]);
+            for (int k = 0; k < i; k++) g = cfms(L[j][k], G[i][k], g);
+            G[j][i] = g;
+            L[j][i] = cmul(g, r[i]);
         }
     }
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        G[i][i] = rg[i];
+    for (int j = 1; j < N; j++)
 #pragma unroll
-        for (int j = i + 1; j < N; j++) {
-            cd s = mk(0.0, 0.0);
+        for (int i = j - 1; i >= 0; i--) {
+            cd s = -L[j][i];
 #pragma unroll
-            for (int k = i; k <= j - 1; k++) s = cfms(G[j][k], G[k][i], s);
-            G[j][i] = cmul(s, rg[j]);
+            for (int k = i + 1; k < j; k++) s = cfms(L[j][k], X[k][i], s);
+            X[j][i] = s;
         }
-    }
 #pragma unroll
-    for (int i = 0; i < N; i++)
+    for (int j = 0; j < N; j++)
 #pragma unroll
-        for (int j = i; j < N; j++) {
-            cd s = mk(0.0, 0.0);
+        for (int i = 0; i <= j; i++) {
+            cd s = (i == j) ? r[j] : cmul(r[j], X[j][i]);
 #pragma unroll
-            for (int k = j; k < N; k++) s = cfma(G[k][i], G[k][j], s);
+            for (int k = j + 1; k < N; k++) s = cfma(cmul(r[k], X[k][j]), X[k][i], s);
             inv[i][j] = s;
             inv[j][i] = s;
         }
-    const cd c = rdiv(absdet, det);
-    S = two_r3n2 * (c * csqrt(c));
+    // c = absdet / det, S = 2^(3n/2) c sqrt(c)
+    const double q = rsqrt_series(normal_range(cnorm2(det)));
+    const double m = absdet * q;  // |c|
+    const cd c = mk(m * q * det.x, -m * q * det.y);
+    const double u = 0.5 * (fabs(c.x) + m);
+    const double ri = rsqrt_series(u);
+    const bool pos = c.x >= 0.0, tiny = !(u > 1e-300);  // a vanishing overlap
+    const double t = u * ri, h = 0.5 * c.y * ri;
+    const cd sc = tiny ? cd{0.0 * u, 0.0} : cd{pos ? t : fabs(h), pos ? h : copysign(t, c.y)};
+    S = two_r3n2 * cmul(c, sc);
 }
 
 // The permuted bra tCk = tAk - i tBk and ket tCl = tAl + i tBl of one term.
@@ -330,599 +264,284 @@ __device__ __forceinline__ void term_matrices(const double (&Ak)[N][N], const do
         for (int j = 0; j < N; j++) tCl[i][j] = mk(R1[i][j], R2[i][j]);
 }
 
-// 1/(r_P r_Q) for pair indices P = (a,b) before Q = (c,d) in vech order
-// (src/matelem.f90:1302-1339), from dP = C^-1 u_P and the two TrCJ:
-// TrCJCJ is the square of u_Q' C^-1 u_P, zero where the reference leaves it
-// unassigned (a = b < c < d).
+// arcsin(z) / z, what 1/(r_P r_Q) takes of z = u_Q' C^-1 u_P / sqrt(TrCJ_P
+// TrCJ_Q) (src/matelem.f90:1302-1339), as -i log(i z + sqrt(1 - z^2)) / z;
+// 1 at z = 0.  Even in z, so the sign of the reference's sqrt(TrCJCJ) does
+// not matter.
+__device__ __forceinline__ cd asin_ratio(cd z)
+{
+    const cd w = mk(fma(-z.x, z.x, fma(z.y, z.y, 1.0)), -2.0 * z.x * z.y);
+    // sqrt(w) on the principal branch, Re >= 0
+    const double m2 = cnorm2(w);
+    const double q = rsqrt_series(normal_range(m2));
+    const double m = m2 * q;
+    const double u = 0.5 * (fabs(w.x) + m);
+    const double ri = rsqrt_series(normal_range(u));
+    const double t = u * ri, h = 0.5 * w.y * ri;
+    const cd sw = w.x >= 0.0 ? mk(t, h) : mk(fabs(h), copysign(t, w.y));
+    const cd l = mk(sw.x - z.y, sw.y + z.x);
+    const cd a = mk(atan2(l.y, l.x), -0.5 * log(cnorm2(l)));
+    const cd o = cmul(a, crcp_series(z));
+    const bool zero = z.x == 0.0 && z.y == 0.0;
+    return mk(zero ? 1.0 : o.x, zero ? 0.0 : o.y);
+}
+
+// 1/(r_P r_Q), P before Q in vech order, are computed EXPC_PQ at a time: the
+// z go to the thread's column of shared memory, one loop takes them to
+// arcsin(z) / z, and the unrolled code reads these back.  (Unrolled, the
+// logarithms of all pairs are more code than the instruction cache holds;
+// a loop over the pairs themselves spends its time on selecting operands.)
+constexpr int EXPC_PQ = 15;
+// vech pair index of (P, Q), P < Q < np, and back
+__host__ __device__ constexpr int pq_count(int np) { return np * (np - 1) / 2; }
+
+// values per pair term, and their MEkl indices: all are produced by k_expc
 template <int N>
-__device__ __forceinline__ cd pair_pair(const cd (&dP)[N], cd trP, cd trQ, bool same, int a, int b, int c, int d,
-                                        cd S)
-{
-    const cd cnumb = (4.0 / PI_D) * S;
-    if (same) return cdiv(2.0 * S, trP);
-    cd x;
-    if (c == d)
-        x = pick(dP, c);
-    else if (a == b && a < c)
-        x = mk(0.0, 0.0);
-    else
-        x = pick(dP, c) - pick(dP, d);
-    const cd tt = x * x;
-    const cd caux = csqrt(tt);
-    const cd sq = csqrt(trP * trQ);
-    if (caux.x != 0.0 || caux.y != 0.0) {
-        const cd caux1 = cdiv(caux, sq);
-        const cd w = mk(1.0, 0.0) - caux1 * caux1;
-        const cd lg = clog_(mk(-caux1.y, caux1.x) + csqrt(w));  // log(i caux1 + sqrt(1 - caux1^2))
-        const cd csum = mk(lg.y, -lg.x);                          // -i log(...)
-        return cdiv(cnumb * csum, caux);
-    }
-    return cdiv(cnumb, sq);
-}
+__host__ __device__ constexpr int expc_nv() { return 6 * (N * (N + 1) / 2) + 9; }
 
-// (a, b) of vech index P, a <= b
+// All 6 np + 9 values of the pairs of one CTA, summed: partial[CTA][values,
+// then bounds].  Bound by FP64 arithmetic at two CTAs an SM (255 registers):
+// the arcsines of the pairs of pairs are most of it (15 for n = 3).  K =
+// 1000, n = 3, four terms: 1.07 ms a call, with the reference's sums term by
+// term in four kernels (accumulators in shared memory, divisions by masses
+// and branching roots in every thread) 4.9 ms; n = 2 0.24 and 0.98 ms, n =
+// 4, K = 150, 14 terms 1.0 and 2.4 ms.  Three CTAs an SM: 1.24 ms.
 template <int N>
-__device__ __forceinline__ void vech_pair(int P, int& a, int& b)
-{
-    a = 0;
-    while (P >= N - a) {
-        P -= N - a;
-        a++;
-    }
-    b = a + P;
-}
-
-// The pass is split into four kernels by the values they produce, each
-// recomputing the short common part (matrices, inverse, overlap): 0 = T, V,
-// H, S, the pair quantities and Darwin; 1 = orbit-orbit; 2 = mass-velocity
-// and its Drachmanised form; 3 = Drachmanised Darwin.  Smaller kernels keep
-// their code in the instruction cache and their matrices in registers.
-constexpr int EXPC_SECTIONS = 4;
-
-// values of section SEC (local index order), and local -> MEkl index
-template <int N, int SEC>
-__host__ __device__ constexpr int sec_nv()
-{
-    return SEC == 0 ? 6 * (N * (N + 1) / 2) + 5 : (SEC == 2 ? 2 : 1);
-}
-template <int N, int SEC>
-__device__ __forceinline__ int sec_global(int l)
-{
-    constexpr int B = 6 * (N * (N + 1) / 2);
-    if (SEC == 0) return l < B + 4 ? l : B + 6;  // ..., H, S, T, V, then Darwin
-    if (SEC == 1) return B + 8;                   // OO
-    if (SEC == 2) return B + 4 + l;               // MV, drach_MV
-    return B + 7;                                 // drach_Darwin
-}
-
-template <int N, int SEC>
-__global__ void __launch_bounds__(EXPC_BLK) k_expc(const double* __restrict__ params, int npt,
-                                                   const cd* __restrict__ cvec, const double* __restrict__ diagS,
-                                                   const double* __restrict__ terms, ExpcArgs ea,
-                                                   double* __restrict__ partial)
+__global__ void __launch_bounds__(EXPC_BLK, EXPC_MINB)
+    k_expc(const double* __restrict__ params, int npt, const cd* __restrict__ cvec, const double* __restrict__ diagS,
+           const double* __restrict__ terms, const __grid_constant__ ExpcArgs ea, double* __restrict__ partial)
 {
     constexpr int NP = N * (N + 1) / 2;
-    constexpr int nvs = sec_nv<N, SEC>();
-    extern __shared__ double sacc[];
-    const int tid = threadIdx.x;
-    const int nv = ea.nv;
-    for (int a = 0; a < 2 * nvs; a++) sacc[a * EXPC_BLK + tid] = 0.0;
+    constexpr int NV = expc_nv<N>();
+    constexpr int NPQ = pq_count(NP);
+    __shared__ double2 zsm[EXPC_PQ < NPQ ? EXPC_PQ : NPQ][EXPC_BLK];
+    __shared__ double red[EXPC_BLK / 32][Acc<NV>::G * 8];
+    const int tid = threadIdx.x, lane = tid & 31;
     const SysParams& sp = ea.sp;
-    const double(&mass)[NMAX + 1] = ea.mass;
-    for (long long pidx = (long long)blockIdx.x * EXPC_BLK + tid; pidx < ea.npairs;
-         pidx += (long long)gridDim.x * EXPC_BLK) {
+    Acc<NV> acc;
+    acc.zero();
+    acc.em = ea.err_mult;
+    for (long long base = (long long)blockIdx.x * EXPC_BLK; base < ea.npairs; base += (long long)gridDim.x * EXPC_BLK) {
+        const bool active = base + tid < ea.npairs;
         int pi, pj;
-        pair_of(pidx, pi, pj);
+        pair_of(active ? base + tid : 0, pi, pj);
         double Ak[N][N], Bk[N][N], Al[N][N], Bl[N][N], dk, dl;
         unpack<N>(params + (size_t)pi * npt, Ak, Bk, dk);
         unpack<N>(params + (size_t)pj * npt, Al, Bl, dl);
         const double absdet = fabs(dl * dk);
         const cd ci = cvec[pi], cj = cvec[pj];
-        const double factor = (pi == pj) ? 1.0 / sqrt(diagS[pi] * diagS[pi]) : 2.0 / sqrt(diagS[pi] * diagS[pj]);
-        Acc acc;
-        acc.s = sacc + tid;
-        acc.e = sacc + nvs * EXPC_BLK + tid;
+        double factor = (pi == pj) ? 1.0 / sqrt(diagS[pi] * diagS[pi]) : 2.0 / sqrt(diagS[pi] * diagS[pj]);
+        if (!active) factor = 0.0;
         acc.rci = ci.x; acc.ici = ci.y; acc.rcj = cj.x; acc.icj = cj.y;
         acc.p1 = ci.x * cj.x + ci.y * cj.y;
         acc.p2 = ci.y * cj.x - ci.x * cj.y;
-        acc.em = ea.err_mult;
         for (int t = 0; t < ea.nterms; t++) {
             const double* tp = terms + (size_t)t * (2 * NMAX * NMAX + 2);
             acc.w = factor * __ldg(tp + 2 * NMAX * NMAX) * __ldg(tp + 2 * NMAX * NMAX + 1);
-            cd tCk[N][N], tCl[N][N], tCkl[N][N], inv[N][N], S;
-            term_matrices<N>(Ak, Bk, Al, Bl, tp, tp + NMAX * NMAX, tCk, tCl);
-#pragma unroll
-            for (int i = 0; i < N; i++)
-#pragma unroll
-                for (int j = 0; j < N; j++) tCkl[i][j] = tCk[i][j] + tCl[i][j];
-            inverse_overlap<N>(tCkl, absdet, sp.two_r3n2, inv, S);
-            PairVecs<N> pv;
-            pair_vecs<N>(inv, pv);
-            cd rm[NP];  // <1/r_P>
-            if constexpr (SEC != 0) {
-                const cd cn = TWO_OVER_SQRTPI * S;
-#pragma unroll
-                for (int P = 0; P < NP; P++) rm[P] = cdiv(cn, csqrt(pv.tr[P]));
-            }
-
-            if constexpr (SEC == 0) {
-            // kinetic energy, src/matelem.f90:1203-1229
-            cd T;
+            cd inv[N][N], X[N][N], Vk[N][N], Vl[N][N], S;
             {
-                cd W1[N][N], W2[N][N];
-                mm(inv, tCk, W1);
-                mm(tCl, W1, W2);
-                cd tr = mk(0.0, 0.0);
+                cd tCk[N][N], tCl[N][N], C[N][N];
+                term_matrices<N>(Ak, Bk, Al, Bl, tp, tp + NMAX * NMAX, tCk, tCl);
 #pragma unroll
                 for (int i = 0; i < N; i++)
 #pragma unroll
-                    for (int k = 0; k < N; k++) tr = rfma(sp.M[i * NMAX + k], W2[k][i], tr);
-                T = 6.0 * (S * tr);
+                    for (int j = 0; j < N; j++) C[i][j] = tCk[i][j] + tCl[i][j];
+                inverse_overlap<N>(C, absdet, sp.two_r3n2, inv, S);
+                mm(inv, tCk, Vk);
+                mm(inv, tCl, Vl);
+#pragma unroll
+                for (int i = 0; i < N; i++)
+#pragma unroll
+                    for (int j = i; j < N; j++) {
+                        cd s = mk(0.0, 0.0);
+#pragma unroll
+                        for (int k = 0; k < N; k++) s = cfma(tCk[i][k], Vl[k][j], s);
+                        X[i][j] = s;
+                        X[j][i] = s;
+                    }
             }
-            // 1/r, r, r^2, delta(r), V, src/matelem.f90:1231-1268
-            cd V = mk(0.0, 0.0), V0 = mk(0.0, 0.0);
+            const cd cn = TWO_OVER_SQRTPI * S;
+            const cd cdl = (1.0 / (PI_D * SQRTPI)) * S;
+            // 1/sqrt(TrCJ_P) and 1/TrCJ_P
+            cd tr[NP], rs[NP], rt[NP], rm[NP];
+            double wq[NP];
             {
-                const cd cn = TWO_OVER_SQRTPI * S;
-                const cd c15 = 1.5 * S;
-                const cd cdl = (1.0 / (PI_D * SQRTPI)) * S;
                 int P = 0;
 #pragma unroll
                 for (int a = 0; a < N; a++)
 #pragma unroll
                     for (int b = a; b < N; b++, P++) {
-                        const cd tr = pv.tr[P];
-                        const cd sq = csqrt(tr);
-                        rm[P] = cdiv(cn, sq);
-                        acc.add(NP + P, rm[P]);
-                        acc.add(2 * NP + P, cn * sq);
-                        acc.add(3 * NP + P, c15 * tr);
-                        acc.add(4 * NP + P, cdiv(cdl, sq * tr));
-                        acc.add(P, cdiv(2.0 * S, tr));  // 1/r^2: the P == Q term of pair_pair
-                        if (a == b)
-                            V0 = rfma(sp.q[a], rm[P], V0);
-                        else
-                            V = rfma(sp.q[a] * sp.q[b], rm[P], V);
+                        // inv(i,i) + inv(j,j) - inv(j,i) - inv(j,i), src/matelem.f90:1252
+                        tr[P] = (a == b) ? inv[a][a] : inv[a][a] + inv[b][b] - inv[b][a] - inv[b][a];
+                        rs[P] = crsqrt(tr[P], rt[P]);
+                        rm[P] = cn * rs[P];  // <1/r_P>
+                        wq[P] = ea.wq[a][b];
                     }
-                V = sp.q0 * V0 + V;
             }
+            // 1/r^2, 1/r, r, r^2, delta(r), src/matelem.f90:1231-1268; Darwin
+            // from delta(r), src/matelem.f90:1850-1873
+#pragma unroll
+            for (int P = 0; P < NP; P++) acc.add(P, (2.0 * S) * rt[P]);
+#pragma unroll
+            for (int P = 0; P < NP; P++) acc.add(NP + P, rm[P]);
+#pragma unroll
+            for (int P = 0; P < NP; P++) acc.add(2 * NP + P, cn * (tr[P] * rs[P]));
+#pragma unroll
+            for (int P = 0; P < NP; P++) acc.add(3 * NP + P, (1.5 * S) * tr[P]);
+            cd dw = mk(0.0, 0.0);
+            {
+                int P = 0;
+#pragma unroll
+                for (int a = 0; a < N; a++)
+#pragma unroll
+                    for (int b = a; b < N; b++, P++) {
+                        const cd dr = cdl * (rs[P] * rt[P]);
+                        acc.add(4 * NP + P, dr);
+                        dw = rfma(ea.wdw[a][b], dr, dw);
+                    }
+            }
+            // tr[M X]; rows of X summed; 1'X1
+            cd trM = mk(0.0, 0.0), sX[N], s1 = mk(0.0, 0.0);
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                sX[i] = mk(0.0, 0.0);
+#pragma unroll
+                for (int k = 0; k < N; k++) {
+                    trM = rfma(sp.M[i * NMAX + k], X[k][i], trM);
+                    sX[i] = sX[i] + X[k][i];
+                }
+                s1 = s1 + sX[i];
+            }
+            // mass-velocity, src/matelem.f90:1487-1597
+            cd mv = ea.im3[0] * (s1 * s1);
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                mv = rfma(ea.im3[i + 1], X[i][i] * X[i][i], mv);
+            mv = -7.5 * (S * mv);
+            // Drachmanised mass-velocity (src/matelem.f90:1675-1848) and Darwin
+            // (src/matelem.f90:1875-1929): W1 = 1/m0^2 + diag(1/m_i^2)
+            cd trW = ea.im2[0] * s1;
+#pragma unroll
+            for (int i = 0; i < N; i++) trW = rfma(ea.im2[i + 1], X[i][i], trW);
+            cd dd = mk(0.0, 0.0);  // the ME_dXd_dYd terms, over S/8
+#pragma unroll
+            for (int p = 0; p < N; p++) {
+                dd = rfma(ea.cw[p][p], 36.0 * (s1 * X[p][p]) + 24.0 * (sX[p] * sX[p]), dd);
+#pragma unroll
+                for (int k = 0; k < p; k++)
+                    dd = rfma(ea.cw[k][p], 36.0 * (X[k][k] * X[p][p]) + 24.0 * (X[k][p] * X[k][p]), dd);
+            }
+            dd = 0.125 * (S * dd) - (1.5 * ea.energy) * (S * trW);
+            // orbit-orbit, src/matelem.f90:1394-1485
+            cd oo = mk(0.0, 0.0);
+            // the sums over pairs: Drachmanised delta (src/matelem.f90:1349-1392,
+            // num without its 1/(r_P r_Q)) and the second Drachmanised terms
+            cd num[NP], V = mk(0.0, 0.0);
+            {
+                int P = 0;
+#pragma unroll
+                for (int a = 0; a < N; a++)
+#pragma unroll
+                    for (int b = a; b < N; b++, P++) {
+                        V = rfma(wq[P], rm[P], V);
+                        oo = rfma(ea.woo[a][b], rm[P] * (a == b ? sX[a] : X[a][b]), oo);
+                        // tCk C^-1 u_P, tCl C^-1 u_P
+                        cd yk[N], yl[N];
+#pragma unroll
+                        for (int m = 0; m < N; m++) {
+                            yk[m] = a == b ? Vk[a][m] : Vk[a][m] - Vk[b][m];
+                            yl[m] = a == b ? Vl[a][m] : Vl[a][m] - Vl[b][m];
+                        }
+                        cd tM = mk(0.0, 0.0), tW = mk(0.0, 0.0), ys = mk(0.0, 0.0);
+#pragma unroll
+                        for (int m = 0; m < N; m++) {
+                            cd u = mk(0.0, 0.0);
+#pragma unroll
+                            for (int k = 0; k < N; k++) u = rfma(sp.M[m * NMAX + k], yl[k], u);
+                            tM = cfma(yk[m], u, tM);
+                            tW = rfma(ea.im2[m + 1], yl[m] * yl[m], tW);
+                            ys = ys + yl[m];
+                        }
+                        tW = rfma(ea.im2[0], ys * ys, tW);
+                        dd = rfma(wq[P], rm[P] * (1.5 * trW + 0.5 * (tW * rt[P])), dd);
+                        num[P] = rm[P] * (mk(ea.energy, 0.0) - 6.0 * trM + 2.0 * (tM * rt[P])) -
+                                 wq[P] * ((2.0 * S) * rt[P]);
+                    }
+            }
+            // 1/(r_P r_Q), P before Q
+            const cd cpq = (4.0 / PI_D) * S;
+#pragma unroll
+            for (int ch = 0; ch * EXPC_PQ < NPQ; ch++) {
+                int e = 0, P = 0;
+#pragma unroll
+                for (int a = 0; a < N; a++)
+#pragma unroll
+                    for (int b = a; b < N; b++, P++) {
+                        int Q = 0;
+#pragma unroll
+                        for (int c = 0; c < N; c++)
+#pragma unroll
+                            for (int d = c; d < N; d++, Q++) {
+                                if (Q <= P) continue;
+                                if (e / EXPC_PQ == ch) {
+                                    cd x = mk(0.0, 0.0);
+                                    if (!(a == b && a < c && c < d)) {  // (see the file header)
+                                        x = a == b ? inv[a][c] : inv[a][c] - inv[b][c];
+                                        if (c != d) x = x - (a == b ? inv[a][d] : inv[a][d] - inv[b][d]);
+                                    }
+                                    x = x * (rs[P] * rs[Q]);
+                                    zsm[e % EXPC_PQ][tid] = make_double2(x.x, x.y);
+                                }
+                                e++;
+                            }
+                    }
+#pragma unroll 1
+                for (int k = 0; k < (NPQ - ch * EXPC_PQ < EXPC_PQ ? NPQ - ch * EXPC_PQ : EXPC_PQ); k++) {
+                    const double2 z = zsm[k][tid];
+                    const cd r = asin_ratio(mk(z.x, z.y));
+                    zsm[k][tid] = make_double2(r.x, r.y);
+                }
+                e = 0;
+#pragma unroll
+                for (int P2 = 0; P2 < NP; P2++)
+#pragma unroll
+                    for (int Q = P2 + 1; Q < NP; Q++, e++)
+                        if (e / EXPC_PQ == ch) {
+                            const double2 z = zsm[e % EXPC_PQ][tid];
+                            const cd R = (cpq * (rs[P2] * rs[Q])) * mk(z.x, z.y);
+                            num[P2] = rfma(-wq[Q], R, num[P2]);
+                            num[Q] = rfma(-wq[P2], R, num[Q]);
+                        }
+            }
+            {
+                int P = 0;
+#pragma unroll
+                for (int a = 0; a < N; a++)
+#pragma unroll
+                    for (int b = a; b < N; b++, P++) {
+                        acc.add(5 * NP + P, ea.icm[a][b] * num[P]);
+                    }
+            }
+            const cd T = 6.0 * (S * trM);  // src/matelem.f90:1203-1229
             acc.add(6 * NP + 0, T + V);
             acc.add(6 * NP + 1, S);
             acc.add(6 * NP + 2, T);
             acc.add(6 * NP + 3, V);
-
-            // Darwin, src/matelem.f90:1850-1873, from delta(r_P)
-            {
-                const cd cdl = (1.0 / (PI_D * SQRTPI)) * S;
-                cd dw = mk(0.0, 0.0);
-                int P = 0;
-#pragma unroll
-                for (int a = 0; a < N; a++)
-#pragma unroll
-                    for (int b = a; b < N; b++, P++) {
-                        const cd dr = cdiv(cdl, csqrt(pv.tr[P]) * pv.tr[P]);
-                        if (a == b) {
-                            const double f = (1.0 / (mass[0] * mass[0]) + 1.0 / (mass[a + 1] * mass[a + 1])) *
-                                             sp.q0 * sp.q[a];
-                            dw = rfma(f, dr, dw);
-                        } else {
-                            // delta(r_ab) enters twice: weights 1/m_a^2 and 1/m_b^2
-                            const double f = (1.0 / (mass[a + 1] * mass[a + 1]) + 1.0 / (mass[b + 1] * mass[b + 1])) *
-                                             sp.q[a] * sp.q[b];
-                            dw = rfma(f, dr, dw);
-                        }
-                    }
-                acc.add(6 * NP + 4, (-0.5 * PI_D) * dw);
-            }
-
-            // Drachmanised delta(r_P), src/matelem.f90:1349-1392
-            {
-                cd sumq[NP];
-#pragma unroll
-                for (int P = 0; P < NP; P++) sumq[P] = mk(0.0, 0.0);
-                // charge weights per pair index, q0 q_a or q_a q_b
-                double wq[NP];
-                {
-                    int P = 0;
-#pragma unroll
-                    for (int a = 0; a < N; a++)
-#pragma unroll
-                        for (int b = a; b < N; b++, P++) wq[P] = (a == b) ? sp.q0 * sp.q[a] : sp.q[a] * sp.q[b];
-                }
-                // one loop over the pairs (P, Q >= P); each R adds to both
-                // sums, so every sum runs over Q in ascending order
-#pragma unroll 1
-                for (int P = 0; P < NP; P++) {
-                    int a, b;
-                    vech_pair<N>(P, a, b);
-                    cd dP[N];
-#pragma unroll
-                    for (int m = 0; m < N; m++) {
-                        cd r = pv.d[0][m];
-#pragma unroll
-                        for (int X = 1; X < NP; X++)
-                            if (X == P) r = pv.d[X][m];
-                        dP[m] = r;
-                    }
-                    const cd trP = pick(pv.tr, P);
-                    const double wP = pickd(wq, P);
-#pragma unroll 1
-                    for (int Q = P; Q < NP; Q++) {
-                        int c, d;
-                        vech_pair<N>(Q, c, d);
-                        const cd R = pair_pair<N>(dP, trP, pick(pv.tr, Q), Q == P, a, b, c, d, S);
-                        const double wQ = pickd(wq, Q);
-#pragma unroll
-                        for (int X = 0; X < NP; X++) {
-                            if (X == P) sumq[X] = rfma(wQ, R, sumq[X]);
-                            if (X == Q && Q != P) sumq[X] = rfma(wP, R, sumq[X]);
-                        }
-                    }
-                }
-                int P = 0;
-                cd W1[N][N], W2[N][N], Mc[N][N];
-#pragma unroll
-                for (int i = 0; i < N; i++)
-#pragma unroll
-                    for (int j = 0; j < N; j++) Mc[i][j] = mk(sp.M[i * NMAX + j], 0.0);
-                mm(Mc, tCl, W1);
-                mm(tCk, W1, W2);  // Wc2 = tCk M tCl, src/matelem.f90:1351-1366
-                const cd trcx = trmm(inv, W2);
-                P = 0;
-#pragma unroll
-                for (int a = 0; a < N; a++)
-#pragma unroll
-                    for (int b = a; b < N; b++, P++) {
-                        const double cm = (a == b) ? 2.0 * PI_D * sp.M[a * NMAX + a]
-                                                   : 2.0 * PI_D *
-                                                         (sp.M[a * NMAX + a] + sp.M[b * NMAX + b] -
-                                                          sp.M[a * NMAX + b] - sp.M[a * NMAX + b]);
-                        const cd t = quad(pv.d[P], W2, pv.d[P]);
-                        const cd rxr = rm[P] * (0.5 * (3.0 * trcx - cdiv(t, pv.tr[P])));
-                        const cd num = ea.energy * rm[P] - sumq[P] - 4.0 * rxr;
-                        acc.add(5 * NP + P, (1.0 / cm) * num);
-                    }
-            }
-
-            }
-
-            if constexpr (SEC == 1) {
-            // orbit-orbit, src/matelem.f90:1394-1485
-            // Each iteration's matrices are rank one or sums of rank-one
-            // terms: Wc2 = x y', Wc3 = u z' and Wc1 = z y' + y z' + t x u'
-            // + u v' with x = tCkl(:,j), y = tCl(:,j), z = tCl(:,i),
-            // t = tCl(j,i), v = tCl(i,j) y + 3 tCl(j,j) z, u = e_j (first
-            // loop) or e_j - e_i (second loop), so the traces of
-            // ME_rXr_over_rij / ME_rXr_rYr_over_rij reduce to dot products
-            // with C^-1 u, C^-1 x and C^-1 z.  The iterations run as one
-            // loop; columns are picked with selects, so the matrices stay in
-            // registers.
-            {
-                const cd cn = TWO_OVER_SQRTPI * S;
-                double qv[N], mv[N];
-#pragma unroll
-                for (int p = 0; p < N; p++) {
-                    qv[p] = sp.q[p];
-                    mv[p] = mass[p + 1];
-                }
-                cd oo1 = mk(0.0, 0.0), oo2 = mk(0.0, 0.0);
-#pragma unroll 1
-                for (int it = 0; it < N * N + N * (N - 1) / 2; it++) {
-                    int i, j;
-                    const bool second = it >= N * N;
-                    if (!second) {
-                        i = it / N;
-                        j = it - i * N;
-                    } else {
-                        int r = it - N * N;
-                        i = 0;
-                        while (r >= N - 1 - i) {
-                            r -= N - 1 - i;
-                            i++;
-                        }
-                        j = i + 1 + r;
-                    }
-                    cd x[N], y[N], z[N], iu[N];
-#pragma unroll
-                    for (int p = 0; p < N; p++) {
-                        x[p] = pick(tCkl[p], j);
-                        y[p] = pick(tCl[p], j);
-                        z[p] = pick(tCl[p], i);
-                        iu[p] = pick(inv[p], j);
-                        if (second) iu[p] = iu[p] - pick(inv[p], i);
-                    }
-                    auto udot = [&](const cd (&w)[N]) -> cd {
-                        cd r = pick(w, j);
-                        if (second) r = r - pick(w, i);
-                        return r;
-                    };
-                    const cd t = pick(z, j);           // tCl(j,i)
-                    const cd tr3 = 3.0 * pick(y, j);   // 3 tCl(j,j)
-                    cd v[N], ix[N], iz[N];
-#pragma unroll
-                    for (int p = 0; p < N; p++) v[p] = t * y[p] + tr3 * z[p];
-#pragma unroll
-                    for (int p = 0; p < N; p++) {
-                        cd a = mk(0.0, 0.0), b = mk(0.0, 0.0);
-#pragma unroll
-                        for (int q = 0; q < N; q++) {
-                            a = cfma(inv[p][q], x[q], a);
-                            b = cfma(inv[p][q], z[q], b);
-                        }
-                        ix[p] = a;
-                        iz[p] = b;
-                    }
-                    // d = C^-1 u_P (up to sign, which cancels) = iu; TrCJ = u' C^-1 u
-                    const cd trcj = udot(iu);
-                    const cd me1 = cdiv(cn, csqrt(trcj));
-                    const cd yiz = dot(y, iz), xiu = dot(x, iu), viu = dot(v, iu), yiu = dot(y, iu);
-                    const cd xiz = dot(x, iz), ziu = dot(z, iu), yix = dot(y, ix);
-                    const cd dx = xiu, dy = yiu, dz = ziu, dv = viu, du = trcj;
-                    // <r'Wc1 r / r_P>
-                    const cd trw = 2.0 * yiz + t * xiu + viu;
-                    const cd dwd = 2.0 * (dz * dy) + t * (dx * du) + du * dv;
-                    const cd cnumb = me1 * (0.5 * (3.0 * trw - cdiv(dwd, trcj)));
-                    // <(r'Wc2 r)(r'Wc3 r) / r_P>
-                    const cd trcx = yix, trcy = ziu;
-                    const cd trcxcy = 0.5 * (yiu * xiz + yiz * xiu);
-                    const cd txj = dx * dy, tyj = du * dz;
-                    const cd txyj = 0.25 * ((dy * dz) * xiu + (dy * du) * xiz + (dx * dz) * yiu + (dx * du) * yiz);
-                    const cd r = 9.0 * (trcy * trcx) + 6.0 * trcxcy -
-                                 cdiv(3.0 * (trcy * txj + trcx * tyj) + 4.0 * txyj, trcj) +
-                                 cdiv(3.0 * (txj * tyj), trcj * trcj);
-                    const cd ctemp = me1 * (0.25 * r);
-                    const cd caux = -6.0 * ((t + t) * me1) + 4.0 * cnumb - 8.0 * ctemp;
-                    const double qj = pickd(qv, j), mj = pickd(mv, j);
-                    if (!second)
-                        oo1 = oo1 - (qj / mj) * caux;
-                    else
-                        oo2 = oo2 + (pickd(qv, i) * qj / (pickd(mv, i) * mj)) * caux;
-                }
-                oo1 = (sp.q0 / mass[0]) * oo1;
-                acc.add(0, 0.5 * (oo1 + oo2));
-            }
-
-            }
-
-            if constexpr (SEC == 2) {
-            // mass-velocity, src/matelem.f90:1487-1597: tCk J tCk = s_k s_k',
-            // tCk J_ii tCk = tCk(:,i) tCk(i,:) (rank one), so every trace is a
-            // quadratic form in C^-1.
-            {
-                auto mv_term = [&](const cd (&a)[N], const cd (&b)[N], cd tr1, cd tr2) -> cd {
-                    const cd tr4 = quad(a, inv, a);  // tr[C^-1 a a']
-                    const cd tr5 = quad(b, inv, b);
-                    const cd x = quad(a, inv, b);
-                    const cd caux = tr1 * tr5 + tr2 * tr4;
-                    return tr4 * tr5 + (2.0 / 3.0) * (x * x) - caux + tr1 * tr2;
-                };
-                cd sk[N], sl[N];
-                cd t1 = mk(0.0, 0.0), t2 = mk(0.0, 0.0);
-#pragma unroll
-                for (int p = 0; p < N; p++) {
-                    cd u = mk(0.0, 0.0), v = mk(0.0, 0.0);
-#pragma unroll
-                    for (int q = 0; q < N; q++) {
-                        u = u + tCk[q][p];
-                        v = v + tCl[q][p];
-                    }
-                    sk[p] = u;
-                    sl[p] = v;
-                    t1 = t1 + u;
-                    t2 = t2 + v;
-                }
-                cd mv = (1.0 / (mass[0] * mass[0] * mass[0])) * mv_term(sk, sl, t1, t2);
-#pragma unroll
-                for (int i = 0; i < N; i++) {
-                    cd a[N], b[N];
-#pragma unroll
-                    for (int p = 0; p < N; p++) {
-                        a[p] = tCk[p][i];
-                        b[p] = tCl[p][i];
-                    }
-                    mv = mv + (1.0 / (mass[i + 1] * mass[i + 1] * mass[i + 1])) * mv_term(a, b, tCk[i][i], tCl[i][i]);
-                }
-                acc.add(0, (-36.0 / 8.0) * (S * mv));
-            }
-
-            // Drachmanised mass-velocity, src/matelem.f90:1675-1848
-            {
-                cd W1[N][N], W3[N][N];
-                const double im0 = 1.0 / (mass[0] * mass[0]);
-#pragma unroll
-                for (int p = 0; p < N; p++)
-#pragma unroll
-                    for (int q = 0; q < N; q++)
-                        W1[p][q] = mk(p == q ? im0 + 1.0 / (mass[p + 1] * mass[p + 1]) : im0, 0.0);
-                const cd tr1 = clxcl(W1, tCl, W3);  // W3 = tCl W1 tCl
-                const cd tr2 = trmm(inv, W3);
-                cd dmv = (6.0 / 4.0) * (ea.energy * (S * (tr2 - tr1)));
-                // second term: sum over pairs of 4 <r'W3r / r_P> - 6 tr1 <1/r_P>
-                {
-                    cd s = mk(0.0, 0.0);
-                    int P = 0;
-#pragma unroll
-                    for (int a = 0; a < N; a++)
-#pragma unroll
-                        for (int b = a; b < N; b++, P++) {
-                            const double wq = (a == b) ? sp.q0 * sp.q[a] : sp.q[a] * sp.q[b];
-                            const cd t = quad(pv.d[P], W3, pv.d[P]);
-                            const cd rxr = rm[P] * (0.5 * (3.0 * tr2 - cdiv(t, pv.tr[P])));
-                            s = rfma(wq, 4.0 * rxr - 6.0 * (tr1 * rm[P]), s);
-                        }
-                    dmv = dmv - 0.25 * s;
-                }
-                // third term: J tCk = 1 s_k', so C^-1 tCk J tCk... = (C^-1 s_k) s_k'
-                auto third = [&](const cd (&a)[N], cd t1, const double (&cw)[N]) -> cd {
-                    // Wc2 = tCl diag(cw), Wc4 = C^-1 Wc2 tCl
-                    cd W2[N][N], W4[N][N], Ti[N][N];
-                    cd t2 = mk(0.0, 0.0);
-#pragma unroll
-                    for (int q = 0; q < N; q++)
-#pragma unroll
-                        for (int p = 0; p < N; p++) W2[q][p] = cw[p] * tCl[q][p];
-#pragma unroll
-                    for (int p = 0; p < N; p++) t2 = t2 + W2[p][p];
-                    mm(inv, W2, Ti);
-                    mm(Ti, tCl, W4);
-                    const cd t4 = trace(W4);
-                    cd ia[N];
-#pragma unroll
-                    for (int p = 0; p < N; p++) {
-                        cd s = mk(0.0, 0.0);
-#pragma unroll
-                        for (int q = 0; q < N; q++) s = cfma(inv[p][q], a[q], s);
-                        ia[p] = s;
-                    }
-                    const cd t3 = dot(a, ia);
-                    const cd t5 = quad(a, W4, ia);
-                    return 36.0 * (t3 * t4) + 24.0 * t5 - 36.0 * (t1 * t4) - 36.0 * (t2 * t3) + 36.0 * (t1 * t2);
-                };
-                {
-                    cd sk[N];
-                    cd t1 = mk(0.0, 0.0);
-#pragma unroll
-                    for (int p = 0; p < N; p++) {
-                        cd u = mk(0.0, 0.0);
-#pragma unroll
-                        for (int q = 0; q < N; q++) u = u + tCk[q][p];
-                        sk[p] = u;
-                        t1 = t1 + u;
-                    }
-                    double cw[N];
-#pragma unroll
-                    for (int p = 0; p < N; p++)
-                        cw[p] = (mass[0] + mass[p + 1]) / (mass[0] * mass[0] * mass[p + 1] * mass[p + 1]);
-                    dmv = dmv + 0.125 * (S * third(sk, t1, cw));
-                }
-#pragma unroll
-                for (int k = 0; k < N - 1; k++) {
-                    cd a[N];
-                    double cw[N];
-#pragma unroll
-                    for (int p = 0; p < N; p++) {
-                        a[p] = tCk[p][k];
-                        cw[p] = p <= k ? 0.0
-                                       : (mass[k + 1] + mass[p + 1]) /
-                                             (mass[k + 1] * mass[k + 1] * mass[p + 1] * mass[p + 1]);
-                    }
-                    dmv = dmv + 0.125 * (S * third(a, tCk[k][k], cw));
-                }
-                acc.add(1, dmv);
-            }
-
-            }
-
-            if constexpr (SEC == 3) {
-            // Drachmanised Darwin, src/matelem.f90:1875-1929
-            // ME_dXd_dYd with X = E_ii, Y = E_jj is rank one on both sides:
-            // tCk E_ii tCk = a a', tCl E_jj tCl = b b' (a = tCk(:,i),
-            // b = tCl(:,j)), so tr3 = a'C^-1 a, tr4 = b'C^-1 b and
-            // tr5 = (a'C^-1 b)^2; with X = ones, tCk X tCk = s s' (s the
-            // column sums of tCk).
-            {
-                cd W1[N][N], M3[N][N];
-                const double im0 = 1.0 / (mass[0] * mass[0]);
-#pragma unroll
-                for (int p = 0; p < N; p++)
-#pragma unroll
-                    for (int q = 0; q < N; q++)
-                        W1[p][q] = mk(p == q ? im0 + 1.0 / (mass[p + 1] * mass[p + 1]) : im0, 0.0);
-                const cd trx = clxcl(W1, tCl, M3);  // M3 = tCl W1 tCl, trx = tr(tCl W1)
-                const cd trm = trmm(inv, M3);
-                // first and second terms: E ME_dXd(W1)/4 and the sum of ME_dXd_over_rij(W1)
-                cd dd = 0.25 * (ea.energy * (6.0 * ((trm - trx) * S)));
-                int P = 0;
-#pragma unroll
-                for (int a = 0; a < N; a++)
-#pragma unroll
-                    for (int b = a; b < N; b++, P++) {
-                        const double wq = (a == b) ? sp.q0 * sp.q[a] : sp.q[a] * sp.q[b];
-                        const cd rxr = rm[P] * (0.5 * (3.0 * trm - cdiv(quad(pv.d[P], M3, pv.d[P]), pv.tr[P])));
-                        dd = dd - (0.25 * wq) * (4.0 * rxr - 6.0 * (trx * rm[P]));
-                    }
-                // C^-1 tCk and C^-1 tCl
-                cd Vk[N][N], Vl[N][N];
-                mm(inv, tCk, Vk);
-                mm(inv, tCl, Vl);
-                // third term: X = ones, Y = diag((m0 + m_j) / (m0^2 m_j^2))
-                {
-                    cd s[N], is[N];
-                    cd t1 = mk(0.0, 0.0), t2 = mk(0.0, 0.0);
-#pragma unroll
-                    for (int p = 0; p < N; p++) {
-                        cd u = mk(0.0, 0.0), w = mk(0.0, 0.0);
-#pragma unroll
-                        for (int q = 0; q < N; q++) {
-                            u = u + tCk[q][p];
-                            w = w + Vk[p][q];  // (C^-1 tCk 1)_p = (C^-1 s)_p
-                        }
-                        s[p] = u;
-                        is[p] = w;
-                        t1 = t1 + u;
-                    }
-                    cd MM[N][N];  // C^-1 tCl D tCl = Vl D tCl
-                    double w[N];
-#pragma unroll
-                    for (int p = 0; p < N; p++) {
-                        w[p] = (mass[0] + mass[p + 1]) / (mass[0] * mass[0] * mass[p + 1] * mass[p + 1]);
-                        t2 = rfma(w[p], tCl[p][p], t2);
-                    }
-#pragma unroll
-                    for (int p = 0; p < N; p++)
-#pragma unroll
-                        for (int q = 0; q < N; q++) {
-                            cd a = mk(0.0, 0.0);
-#pragma unroll
-                            for (int k = 0; k < N; k++) a = cfma(w[k] * Vl[p][k], tCl[k][q], a);
-                            MM[p][q] = a;
-                        }
-                    const cd t3 = dot(s, is);
-                    const cd t4 = trace(MM);
-                    const cd t5 = quad(s, MM, is);
-                    dd = dd + 0.125 * ((36.0 * (t3 * t4) + 24.0 * t5 - 36.0 * (t1 * t4) - 36.0 * (t2 * t3) +
-                                        36.0 * (t1 * t2)) * S);
-                }
-                // fourth term: pairs i < j with X = E_ii, Y = E_jj
-#pragma unroll
-                for (int i = 0; i < N; i++) {
-                    cd a[N];
-#pragma unroll
-                    for (int p = 0; p < N; p++) a[p] = tCk[p][i];
-                    cd t3 = mk(0.0, 0.0);
-#pragma unroll
-                    for (int p = 0; p < N; p++) t3 = cfma(a[p], Vk[p][i], t3);  // a' C^-1 a
-#pragma unroll
-                    for (int j = i + 1; j < N; j++) {
-                        cd t4 = mk(0.0, 0.0), x = mk(0.0, 0.0);
-#pragma unroll
-                        for (int p = 0; p < N; p++) {
-                            t4 = cfma(tCl[p][j], Vl[p][j], t4);  // b' C^-1 b
-                            x = cfma(a[p], Vl[p][j], x);         // a' C^-1 b
-                        }
-                        const cd t1 = tCk[i][i], t2 = tCl[j][j];
-                        const cd t5 = x * x;
-                        const double cw = (mass[i + 1] + mass[j + 1]) /
-                                          (mass[i + 1] * mass[i + 1] * mass[j + 1] * mass[j + 1]);
-                        dd = dd + (0.125 * cw) * ((36.0 * (t3 * t4) + 24.0 * t5 - 36.0 * (t1 * t4) -
-                                                   36.0 * (t2 * t3) + 36.0 * (t1 * t2)) * S);
-                    }
-                }
-                acc.add(0, dd);
-            }
-            }
+            acc.add(6 * NP + 4, mv);
+            acc.add(6 * NP + 5, dd);
+            acc.add(6 * NP + 6, (-0.5 * PI_D) * dw);
+            acc.add(6 * NP + 7, dd);
+            acc.add(6 * NP + 8, 4.0 * oo);
         }
     }
+    if ((lane & 3) == 0)
+#pragma unroll
+        for (int g = 0; g < Acc<NV>::G; g++) red[tid >> 5][g * 8 + (lane >> 2)] = acc.sum[g];
     __syncthreads();
-    // block sums in a fixed order; the section's slice of partial holds zero
-    // for the values of the other sections
-    double* out = partial + ((size_t)SEC * gridDim.x + blockIdx.x) * 2 * nv;
-    for (int a = tid; a < 2 * nv; a += EXPC_BLK) out[a] = 0.0;
-    __syncthreads();
-    for (int l = tid; l < 2 * nvs; l += EXPC_BLK) {
+    for (int l = tid; l < 2 * NV; l += EXPC_BLK) {
         double s = 0.0;
-        for (int t = 0; t < EXPC_BLK; t++) s += sacc[l * EXPC_BLK + t];
-        const int li = l < nvs ? l : l - nvs;
-        out[sec_global<N, SEC>(li) + (l < nvs ? 0 : nv)] = s;
+        for (int wp = 0; wp < EXPC_BLK / 32; wp++) s += red[wp][l];
+        partial[(size_t)blockIdx.x * 2 * NV + (l & 1) * NV + (l >> 1)] = s;
     }
 }
 
@@ -930,7 +549,7 @@ __global__ void __launch_bounds__(EXPC_BLK) k_expc(const double* __restrict__ pa
 // per grid point), src/matelem.f90:1931-1960; blockIdx.y selects a chunk
 // of `gchunk` grid entries (grid points times values).
 template <int N>
-__global__ void __launch_bounds__(EXPC_BLK) k_expc_grid(const double* __restrict__ params, int npt,
+__global__ void __launch_bounds__(GRID_BLK) k_expc_grid(const double* __restrict__ params, int npt,
                                                         const cd* __restrict__ cvec, const double* __restrict__ diagS,
                                                         const double* __restrict__ terms, ExpcArgs ea,
                                                         const double* __restrict__ cf_grid, int ncf,
@@ -942,10 +561,10 @@ __global__ void __launch_bounds__(EXPC_BLK) k_expc_grid(const double* __restrict
     const int tid = threadIdx.x;
     const int g0 = blockIdx.y * gchunk;
     const int g1 = min(ngrid, g0 + gchunk);
-    for (int g = g0; g < g1; g++) sacc[(g - g0) * EXPC_BLK + tid] = 0.0;
+    for (int g = g0; g < g1; g++) sacc[(g - g0) * GRID_BLK + tid] = 0.0;
     const SysParams& sp = ea.sp;
-    for (long long pidx = (long long)blockIdx.x * EXPC_BLK + tid; pidx < ea.npairs;
-         pidx += (long long)gridDim.x * EXPC_BLK) {
+    for (long long pidx = (long long)blockIdx.x * GRID_BLK + tid; pidx < ea.npairs;
+         pidx += (long long)gridDim.x * GRID_BLK) {
         int pi, pj;
         pair_of(pidx, pi, pj);
         double Ak[N][N], Bk[N][N], Al[N][N], Bl[N][N], dk, dl;
@@ -990,8 +609,8 @@ __global__ void __launch_bounds__(EXPC_BLK) k_expc_grid(const double* __restrict
             cd xr[NP + N + 1], px[NP + N + 1];  // 1/x and pre/(sqrt(x) x)
 #pragma unroll
             for (int v = 0; v < NP + N + 1; v++) {
-                xr[v] = crcp(x[v]);
-                px[v] = cdiv(pre, csqrt(x[v]) * x[v]);
+                const cd rs = crsqrt(x[v], xr[v]);
+                px[v] = pre * (rs * xr[v]);
             }
             for (int g = g0; g < g1; g++) {
                 int v, k;
@@ -1010,39 +629,34 @@ __global__ void __launch_bounds__(EXPC_BLK) k_expc_grid(const double* __restrict
 #pragma unroll
                 for (int u = 0; u < NP + N + 1; u++)
                     if (u == v) O = px[u] * cexp_((-r * r) * xr[u]);
-                sacc[(g - g0) * EXPC_BLK + tid] += w * (p1 * O.x + p2 * O.y);
+                sacc[(g - g0) * GRID_BLK + tid] += w * (p1 * O.x + p2 * O.y);
             }
         }
     }
     __syncthreads();
-    for (int g = g0 + tid; g < g1; g += EXPC_BLK) {
+    for (int g = g0 + tid; g < g1; g += GRID_BLK) {
         double s = 0.0;
-        for (int t = 0; t < EXPC_BLK; t++) s += sacc[(g - g0) * EXPC_BLK + t];
+        for (int t = 0; t < GRID_BLK; t++) s += sacc[(g - g0) * GRID_BLK + t];
         partial[(size_t)blockIdx.x * ngrid + g] = s;
     }
 }
 
-// out[a] = sum over blocks of partial[b][a]; the second half (the error
-// bounds) times epsilon when `eps_from` < count.
-__global__ void k_expc_sum(const double* __restrict__ partial, int nblocks, int count, int eps_from,
-                           double* __restrict__ out)
+// out[a] = sum over blocks of partial[b][a], one CTA a value, in a fixed
+// order; the second half (the error bounds) times epsilon when `eps_from` <
+// count.
+__global__ void __launch_bounds__(128) k_expc_sum(const double* __restrict__ partial, int nblocks, int count,
+                                                  int eps_from, double* __restrict__ out)
 {
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= count) return;
+    __shared__ double sh[128];
+    const int a = blockIdx.x;
     double s = 0.0;
-    for (int b = 0; b < nblocks; b++) s += partial[(size_t)b * count + a];
-    out[a] = a >= eps_from ? s * DBL_EPSILON : s;
-}
-
-template <int N, int SEC>
-int launch_sec(Ctx& c, const ExpcArgs& ea, const double* terms, const cd* cvec, double* partial, int nblocks)
-{
-    const size_t smem = (size_t)2 * sec_nv<N, SEC>() * EXPC_BLK * sizeof(double);
-    if (cudaFuncSetAttribute(k_expc<N, SEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return -2;
-    k_expc<N, SEC><<<nblocks, EXPC_BLK, smem, c.stream>>>(c.params, c.npt, cvec, c.diagS, terms, ea, partial);
-    c.launches += 1;
-    return 0;
+    for (int b = threadIdx.x; b < nblocks; b += 128) s += partial[(size_t)b * count + a];
+    sh[threadIdx.x] = s;
+    for (int h = 64; h >= 1; h >>= 1) {
+        __syncthreads();
+        if (threadIdx.x < h) sh[threadIdx.x] += sh[threadIdx.x + h];
+    }
+    if (threadIdx.x == 0) out[a] = (a >= eps_from) ? sh[0] * DBL_EPSILON : sh[0];
 }
 
 template <int N>
@@ -1050,21 +664,18 @@ int launch_n(Ctx& c, const ExpcArgs& ea, const double* terms, const cd* cvec, co
              const double* dg, int ndens, double* partial, int nblocks, double* out, double* gpartial, int gblocks,
              int gchunk, int ngrid, double* gout)
 {
-    if (launch_sec<N, 0>(c, ea, terms, cvec, partial, nblocks) || launch_sec<N, 1>(c, ea, terms, cvec, partial, nblocks) ||
-        launch_sec<N, 2>(c, ea, terms, cvec, partial, nblocks) || launch_sec<N, 3>(c, ea, terms, cvec, partial, nblocks))
-        return -2;
-    k_expc_sum<<<(2 * ea.nv + 127) / 128, 128, 0, c.stream>>>(partial, EXPC_SECTIONS * nblocks, 2 * ea.nv, ea.nv,
-                                                               out);
-    c.launches += 1;
+    k_expc<N><<<nblocks, EXPC_BLK, 0, c.stream>>>(c.params, c.npt, cvec, c.diagS, terms, ea, partial);
+    k_expc_sum<<<2 * ea.nv, 128, 0, c.stream>>>(partial, nblocks, 2 * ea.nv, ea.nv, out);
+    c.launches += 2;
     if (ngrid > 0) {
-        const size_t gsm = (size_t)gchunk * EXPC_BLK * sizeof(double);
+        const size_t gsm = (size_t)gchunk * GRID_BLK * sizeof(double);
         if (cudaFuncSetAttribute(k_expc_grid<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsm) !=
             cudaSuccess)
             return -2;
         dim3 grid(gblocks, (ngrid + gchunk - 1) / gchunk);
-        k_expc_grid<N><<<grid, EXPC_BLK, gsm, c.stream>>>(c.params, c.npt, cvec, c.diagS, terms, ea, cfg, ncf, dg,
+        k_expc_grid<N><<<grid, GRID_BLK, gsm, c.stream>>>(c.params, c.npt, cvec, c.diagS, terms, ea, cfg, ncf, dg,
                                                           ndens, gchunk, gpartial, ngrid);
-        k_expc_sum<<<(ngrid + 127) / 128, 128, 0, c.stream>>>(gpartial, gblocks, ngrid, ngrid, gout);
+        k_expc_sum<<<ngrid, 128, 0, c.stream>>>(gpartial, gblocks, ngrid, ngrid, gout);
         c.launches += 2;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -1083,9 +694,24 @@ int expectation_values(Ctx& c, int nbasis, const double* masses, int nterms, con
     ea.sp = c.sp;
     double mtot = 0.0;
     for (int i = 0; i <= n; i++) {
-        ea.mass[i] = masses[i];
-        mtot += masses[i];
+        const double m = masses[i];
+        mtot += m;
+        ea.im2[i] = 1.0 / (m * m);
+        ea.im3[i] = 1.0 / (m * m * m);
     }
+    for (int a = 0; a < n; a++)
+        for (int b = a; b < n; b++) {
+            // a = b: the pair of particle a with particle 0
+            const double ma = a == b ? masses[0] : masses[a + 1], mb = masses[b + 1];
+            const double(&M)[NMAX * NMAX] = c.sp.M;
+            ea.wq[a][b] = a == b ? c.sp.q0 * c.sp.q[a] : c.sp.q[a] * c.sp.q[b];
+            ea.cw[a][b] = (ma + mb) / (ma * ma * mb * mb);
+            ea.wdw[a][b] = (1.0 / (ma * ma) + 1.0 / (mb * mb)) * ea.wq[a][b];
+            ea.woo[a][b] = (a == b ? 1.0 : -1.0) * ea.wq[a][b] / (ma * mb);
+            ea.icm[a][b] = 1.0 / (2.0 * PI_D *
+                                  (a == b ? M[a * NMAX + a]
+                                          : M[a * NMAX + a] + M[b * NMAX + b] - M[a * NMAX + b] - M[a * NMAX + b]));
+        }
     // Glob_bvc, src/workproc.f90:612-621
     for (int i = 0; i <= n; i++)
         for (int p = 0; p < n; p++) ea.bvc[p][i] = -masses[p + 1] / mtot;
@@ -1112,10 +738,10 @@ int expectation_values(Ctx& c, int nbasis, const double* masses, int nterms, con
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.dev);
     const long long blocks_needed = (ea.npairs + EXPC_BLK - 1) / EXPC_BLK;
-    const int nblocks = (int)std::min<long long>(blocks_needed, (long long)sms * 8);
+    const int nblocks = (int)std::min<long long>(blocks_needed, (long long)sms * EXPC_MINB * 2);
     const int ngrid = ncf * np + ndens * (n + 1);
     const int gchunk = 48;  // 48 x 64 doubles of shared memory per block
-    const int gblocks = (int)std::min<long long>(blocks_needed, (long long)sms * 2);
+    const int gblocks = (int)std::min<long long>((ea.npairs + GRID_BLK - 1) / GRID_BLK, (long long)sms * 2);
 
     double *d_terms = nullptr, *d_part = nullptr, *d_out = nullptr, *d_gpart = nullptr, *d_gout = nullptr,
            *d_cfg = nullptr, *d_dg = nullptr;
@@ -1132,7 +758,7 @@ int expectation_values(Ctx& c, int nbasis, const double* masses, int nterms, con
     };
     const size_t nv = ea.nv;
     if (alloc((void**)&d_terms, th.size() * sizeof(double)) &&
-        alloc((void**)&d_part, (size_t)EXPC_SECTIONS * nblocks * 2 * nv * sizeof(double)) &&
+        alloc((void**)&d_part, (size_t)nblocks * 2 * nv * sizeof(double)) &&
         alloc((void**)&d_out, 2 * nv * sizeof(double)) &&
         alloc((void**)&d_gpart, (size_t)gblocks * ngrid * sizeof(double)) &&
         alloc((void**)&d_gout, (size_t)ngrid * sizeof(double)) &&
