@@ -171,12 +171,14 @@ int ghepiis_core(Ctx& c, int k, int n, double apprlambda, double tol, int max_it
         return ECG_ESINGULAR;
     }
     bool notconverged = true;
-    double nd = 0.0, prev = DBL_MAX;
+    double nd = 0.0, prev = DBL_MAX, last = 0.0;
     int it = 0;
     while (notconverged && it < max_iter) {
         CKR(invit_step(c, n, it == 0));
         CKR(read_red(c));
         nd = c.red_h[RD_NORMDIFF];
+        c.last_gain = it > 0 ? nd / last : 0.0;
+        last = nd;
         if (trace_on()) fprintf(stderr, "ecg: GHEPIIS(%d,%d) iteration %d NormOfDiff %.3e\n", k, n, it + 1, nd);
         if (tol > 0.0) {
             if (nd <= tol) notconverged = false;
@@ -222,7 +224,15 @@ int ghepiis(Ctx& c, int k, int n, double apprlambda, double tol, int max_iter, i
 // eigenvalue lies outside the bracket and so farther from its centre.
 // ---------------------------------------------------------------------------
 constexpr int G_MAX_FACT = 400;   // bound on the factorisations of one call
-constexpr int G_EXTRA_BISECT = 10;  // halvings after isolation: faster inverse iteration
+// Halvings after isolation.  One costs a factorisation (155 us at K = 240, 0.6
+// ms at K = 1000), an inverse iteration 55 to 100 us, and a bracket of width w
+// in a gap g makes the iteration gain a factor of 2 g / w a step: few halvings,
+// and none of a bracket that is narrow already.  G_EXTRA_MOST of them where
+// the iteration did not get there.  K = 240 from a nearby basis's eigenvalue
+// (a bracket of 2e-6): 0.9 ms against 2.4 with ten halvings in every case.
+constexpr int G_EXTRA_BISECT = 4;
+constexpr int G_EXTRA_MOST = 10;
+constexpr double G_NARROW = 1e-5;
 
 // nu(sigma) into *nu; *zero = 1 when a pivot was exactly zero
 int g_count(Ctx& c, int n, double sigma, int* nu, int* zero)
@@ -310,28 +320,7 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
         if ((r = count(hi, &nhi))) return r;
         if (c.g_last_factorizations > G_MAX_FACT) return ECG_ENOCONV;
     }
-    // bisect until the bracket holds the which-th eigenvalue alone, then a
-    // few halvings more
-    int extra = 0;
-    for (;;) {
-        const bool isolated = (nlo == which - 1) && (nhi == which);
-        if (isolated && extra >= G_EXTRA_BISECT) break;
-        if (hi - lo <= 4.0 * DBL_EPSILON * std::max(fabs(lo), fabs(hi))) break;
-        if (c.g_last_factorizations > G_MAX_FACT) return ECG_ENOCONV;
-        double mid = 0.5 * (lo + hi);
-        if ((r = count(mid, &nu))) return r;
-        if (nu >= which) {
-            hi = mid;
-            nhi = nu;
-        } else {
-            lo = mid;
-            nlo = nu;
-        }
-        if (isolated) extra++;
-    }
-    // inverse iteration at the centre of the isolating bracket
-    double sigma = 0.5 * (lo + hi);
-    CKR(g_shift(c, c.H, c.S, c.diagH, nullptr, n, sigma));
+    // the start of the iteration: the last call's vector, or ones
     if (c.g_last_which > 0) {
         CK(cudaMemcpyAsync(c.c, c.x, (size_t)n * sizeof(cd), cudaMemcpyDeviceToDevice, c.stream));
     } else {
@@ -339,18 +328,55 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
         CK(cudaMemcpyAsync(c.c, ones.data(), (size_t)n * sizeof(cd), cudaMemcpyHostToDevice, c.stream));
         CK(cudaStreamSynchronize(c.stream));
     }
-    double lam = 0.0, ra = 0.0;
-    int it = 0;
-    const int e = ghepiis_core(c, 1, n, sigma, 1e-12, 20, want_vector ? 0 : -1, &lam, &ra, &it);
-    c.g_last_factorizations++;
-    if (e < 0) return e;
-    if (e == ECG_ESINGULAR) return ECG_ENOCONV;
-    // the converged eigenvalue is the bracket's; otherwise the bisection's own
-    // estimate.  A bisection point that met the eigenvalue to rounding (the
-    // first one does when the same basis is solved again) became an end of the
-    // bracket on either side of it, so the ends count with a margin.
-    const double margin = 1e-3 * (hi - lo) + 64.0 * DBL_EPSILON * fabs(sigma);
-    *energy = (lam >= lo - margin && lam <= hi + margin) ? lam : sigma;
+    int extra = 0, it = 0;
+    for (bool again = false;; again = true) {
+        // bisect until the bracket holds the which-th eigenvalue alone, then a
+        // few halvings more
+        for (;;) {
+            const double size = std::max(fabs(lo), fabs(hi));
+            const bool isolated = (nlo == which - 1) && (nhi == which);
+            if (isolated && extra >= (again ? G_EXTRA_MOST : G_EXTRA_BISECT)) break;
+            if (isolated && !again && hi - lo <= G_NARROW * std::max(1.0, size)) break;
+            if (hi - lo <= 4.0 * DBL_EPSILON * size) break;
+            if (c.g_last_factorizations > G_MAX_FACT) return ECG_ENOCONV;
+            double mid = 0.5 * (lo + hi);
+            if ((r = count(mid, &nu))) return r;
+            if (nu >= which) {
+                hi = mid;
+                nhi = nu;
+            } else {
+                lo = mid;
+                nlo = nu;
+            }
+            if (isolated) extra++;
+        }
+        // inverse iteration at the centre of the isolating bracket
+        const double sigma = 0.5 * (lo + hi);
+        CKR(g_shift(c, c.H, c.S, c.diagH, nullptr, n, sigma));
+        double lam = 0.0, ra = 0.0;
+        const int e = ghepiis_core(c, 1, n, sigma, 1e-12, 20, want_vector ? 0 : -1, &lam, &ra, &it);
+        c.g_last_factorizations++;
+        if (e < 0) return e;
+        // the converged eigenvalue is the bracket's; otherwise the bisection's
+        // own estimate.  A bisection point that met the eigenvalue to rounding
+        // (the first one does when the same basis is solved again) became an
+        // end of the bracket on either side of it, so the ends count with a
+        // margin.
+        const double margin = 1e-3 * (hi - lo) + 64.0 * DBL_EPSILON * fabs(sigma);
+        const bool inside = e != ECG_ESINGULAR && lam >= lo - margin && lam <= hi + margin;
+        // once more in a narrower bracket if the shift met the eigenvalue, the
+        // iteration found another one, or it was still gaining when it ended
+        // (standing still, it is on its floor, which no shift lowers)
+        const bool gaining = e == ECG_ENOCONV && (ra > 1e-6 || c.last_gain < 0.9);
+        if (!again && extra < G_EXTRA_MOST && (!inside || gaining)) {
+            if (e == ECG_ESINGULAR) continue;
+            CK(cudaMemcpyAsync(c.c, c.x, (size_t)n * sizeof(cd), cudaMemcpyDeviceToDevice, c.stream));
+            continue;
+        }
+        if (e == ECG_ESINGULAR) return ECG_ENOCONV;
+        *energy = inside ? lam : sigma;
+        break;
+    }
     c.last_numiter = it;
     if (want_vector) CK(cudaMemcpyAsync(c.c, c.x, (size_t)n * sizeof(cd), cudaMemcpyDeviceToDevice, c.stream));
     CK(cudaStreamSynchronize(c.stream));

@@ -195,6 +195,7 @@ struct Ctx {
     cudaEvent_t ev[16];
     double stage_ms[8] = {0};
     int last_numiter = 0;
+    double last_gain = 0.0;  // NormOfDiff of GHEPIIS's last iteration over the one before
 
     CandWork cand;           // batched candidate evaluation
 
