@@ -103,17 +103,6 @@ double elapsed(Ctx& c, int a, int b)
     return ms;
 }
 
-int read_red(Ctx& c)
-{
-    CK(cudaMemcpyAsync(c.red_h, c.red, RD_COUNT * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    CK(cudaMemcpyAsync(c.status_h, c.status, ST_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.bytes_d2h += RD_COUNT * sizeof(double) + ST_COUNT * sizeof(int);
-    CK(cudaStreamSynchronize(c.stream));
-    // a cooperative solve that gave up waiting leaves an unusable step
-    if (c.status_h[ST_SOLVE_TIMEOUT]) return ECG_ECUDA;
-    return 0;
-}
-
 int compute_hs(Ctx& c, int nmin, int nmax, double approx_e)
 {
     if (nmin < 1 || nmax < nmin || nmax > c.ld) return ECG_EARG;
@@ -146,61 +135,66 @@ int ghepiis_core(Ctx& c, int k, int n, double apprlambda, double tol, int max_it
     *rel_acc = DBL_MAX;
     *num_iter = 0;
     CK(cudaMemsetAsync(c.status, 0, ST_COUNT * sizeof(int), c.stream));
+    CK(cudaMemsetAsync(c.red, 0, RD_COUNT * sizeof(double), c.stream));
     CKR(ldlh_factor(c, k - 1, n));
-    CK(cudaMemcpyAsync(c.status_h, c.status, ST_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    c.bytes_d2h += ST_COUNT * sizeof(int);
-    CK(cudaStreamSynchronize(c.stream));
+    // the factorisation's own status, for the host to see below
+    int* const fact_status = c.status_h + ST_COUNT;
+    CK(cudaMemcpyAsync(fact_status, c.status, ST_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+    CK(cudaMemsetAsync(c.counters + 2, 0, sizeof(int), c.stream));  // the solves' abort word
     mark(c, 2);
-    if (c.status_h[ST_SOLVE_TIMEOUT]) {
-        // a bounded wait of the factorisation ran out: no factor, or none of
-        // the one new row
-        const bool row = k > 1 && n == k;
-        c.fact_n = row ? k - 1 : 0;
-        if (!row)
-            c.blk_start.clear();
-        else if (!c.blk_start.empty() && c.blk_start.back() == k - 1)
-            c.blk_start.pop_back();
-        return ECG_ECUDA;
-    }
-    if (c.status_h[ST_ZERO_PIVOT] != 0) {
-        // LDLHF returned ErrorCode = 1 (src/linalg.f90:377-380); the factor
-        // is incomplete, so no row of it may be reused.
-        c.fact_n = 0;
-        c.blk_start.clear();
-        mark(c, 3);
-        return ECG_ESINGULAR;
-    }
+    // Iterations are enqueued several at a time, the Rayleigh quotient behind
+    // them, and the host looks once: after convergence, and where the
+    // factorisation failed, the rest of the launches return at once.  As many
+    // as the last call took, then two at a time: a look costs the stream 15 to
+    // 20 us (an iteration at n = 500 takes 50), an empty iteration 8.
+    int batch = std::min(8, c.last_numiter > 0 ? c.last_numiter : 3);
+    if (trace_on()) batch = 1;
     bool notconverged = true;
-    double nd = 0.0, prev = DBL_MAX, last = 0.0;
+    double nd = 0.0;
     int it = 0;
-    while (notconverged && it < max_iter) {
-        CKR(invit_step(c, n, it == 0));
-        CKR(read_red(c));
-        nd = c.red_h[RD_NORMDIFF];
-        c.last_gain = it > 0 ? nd / last : 0.0;
-        last = nd;
-        if (trace_on()) fprintf(stderr, "ecg: GHEPIIS(%d,%d) iteration %d NormOfDiff %.3e\n", k, n, it + 1, nd);
-        if (tol > 0.0) {
-            if (nd <= tol) notconverged = false;
-        } else {
-            if (nd > prev && nd <= fabs(tol)) notconverged = false;
-            prev = nd;
+    for (bool first = true;; first = false) {
+        const int m = std::min(batch, max_iter - it);
+        for (int i = 0; i < m; i++) CKR(invit_step(c, n, tol));
+        const bool last = it + m >= max_iter;
+        CKR(invit_rayleigh(c, n, last, specif_norm));
+        CK(cudaMemcpyAsync(c.red_h, c.red, RD_COUNT * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+        CK(cudaMemcpyAsync(c.status_h, c.status, ST_COUNT * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+        c.bytes_d2h += RD_COUNT * sizeof(double) + (first ? 2 : 1) * ST_COUNT * sizeof(int);
+        CK(cudaStreamSynchronize(c.stream));
+        if (first && fact_status[ST_SOLVE_TIMEOUT]) {
+            // a bounded wait of the factorisation ran out: no factor, or none of
+            // the one new row
+            const bool row = k > 1 && n == k;
+            c.fact_n = row ? k - 1 : 0;
+            if (!row)
+                c.blk_start.clear();
+            else if (!c.blk_start.empty() && c.blk_start.back() == k - 1)
+                c.blk_start.pop_back();
+            return ECG_ECUDA;
         }
-        it++;
+        if (first && fact_status[ST_ZERO_PIVOT] != 0) {
+            // LDLHF returned ErrorCode = 1 (src/linalg.f90:377-380); the factor
+            // is incomplete, so no row of it may be reused.
+            c.fact_n = 0;
+            c.blk_start.clear();
+            mark(c, 3);
+            return ECG_ESINGULAR;
+        }
+        // a cooperative solve that gave up waiting leaves an unusable step
+        if (c.status_h[ST_SOLVE_TIMEOUT]) return ECG_ECUDA;
+        it = (int)c.red_h[RD_ITERS];
+        nd = c.red_h[RD_NORMDIFF];
+        notconverged = c.red_h[RD_DONE] == 0.0;
+        if (trace_on()) fprintf(stderr, "ecg: GHEPIIS(%d,%d) iteration %d NormOfDiff %.3e\n", k, n, it, nd);
+        if (!notconverged || last) break;
+        batch = trace_on() ? 1 : 2;
     }
     mark(c, 3);
     *rel_acc = nd;
     *num_iter = it;
     c.last_numiter = it;
-    CKR(invit_rayleigh(c, n));
-    CKR(read_red(c));
-    const double t1 = c.red_h[RD_T1], t2 = c.red_h[RD_T2];
-    *lambda = t2 / t1 + apprlambda;
-    if (specif_norm == 0) {
-        CKR(vec_scale(c, c.x, n, 1.0 / sqrt(t1)));
-    } else if (specif_norm == 1) {
-        CKR(vec_scale(c, c.x, n, 1.0 / sqrt(c.red_h[RD_XX])));
-    }
+    c.last_gain = c.red_h[RD_GAIN];
+    *lambda = c.red_h[RD_T2] / c.red_h[RD_T1] + apprlambda;
     return notconverged ? ECG_ENOCONV : ECG_OK;
 }
 
@@ -565,7 +559,7 @@ int ecg_ctx_create(int n, const double* mass_matrix_host, const double* charges_
     r |= dalloc(&c.dblk, L + 2);
     r |= dalloc(&c.xw, L);
     if (!r) {
-        if (cudaMallocHost((void**)&c.status_h, ST_COUNT * sizeof(int)) != cudaSuccess ||
+        if (cudaMallocHost((void**)&c.status_h, 2 * ST_COUNT * sizeof(int)) != cudaSuccess ||
             cudaMallocHost((void**)&c.bounds_h, (L + 2) * sizeof(int)) != cudaSuccess ||
             cudaMallocHost((void**)&c.red_h, RD_COUNT * sizeof(double)) != cudaSuccess ||
             cudaMallocHost((void**)&c.gcnt_h, 4 * sizeof(int)) != cudaSuccess) {

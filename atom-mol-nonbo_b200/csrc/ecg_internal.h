@@ -220,6 +220,9 @@ enum RedSlot {
     RD_T1 = 1,       // x^H B x
     RD_T2 = 2,       // x^H M x
     RD_XX = 3,       // x^H x
+    RD_DONE = 4,     // the iteration has converged
+    RD_ITERS = 5,    // iterations done
+    RD_GAIN = 6,     // NormOfDiff over the iteration before's
     RD_COUNT = 8
 };
 
@@ -284,10 +287,9 @@ int ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long
 int ldlh_factor_traced(Ctx& c, int n, unsigned long long* out, long long cap, long long* count);
 
 // ---- launchers (invit.cu) ----
-int invit_step(Ctx& c, int n, bool first);
-int invit_rayleigh(Ctx& c, int n);
+int invit_step(Ctx& c, int n, double tol);
+int invit_rayleigh(Ctx& c, int n, bool always, int specif_norm);
 int border_row(Ctx& c, int m0, int nexist);
-int vec_scale(Ctx& c, cd* v, int n, double s);
 
 inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? 0 : -2; }
 

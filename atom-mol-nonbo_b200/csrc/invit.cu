@@ -12,6 +12,7 @@
 // partials in a fixed order and applies the panel's precomputed inverse
 // block, so results are deterministic run to run.
 #include <algorithm>
+#include <float.h>
 #include "ecg_internal.h"
 #include "wait_value.cuh"
 #include "warp_sums.cuh"
@@ -40,11 +41,25 @@ __device__ __forceinline__ cd warp_sum(cd s)
     return s;
 }
 
+// Whether a launch of the iteration has nothing to do: the host enqueues
+// several iterations and the Rayleigh quotient without looking in between.
+__device__ __forceinline__ bool idle(const double* red, const int* status)
+{
+    return red[RD_DONE] != 0.0 || status[ST_ZERO_PIVOT] != 0 || status[ST_SOLVE_TIMEOUT] != 0;
+}
+// The same for the Rayleigh quotient behind them.
+__device__ __forceinline__ bool idle_rayleigh(const double* red, const int* status, int always)
+{
+    return (!always && red[RD_DONE] == 0.0) || status[ST_ZERO_PIVOT] != 0 || status[ST_SOLVE_TIMEOUT] != 0;
+}
+
 // w(i) = sum_j conj(B(j,i)) v(j); one warp per column, four accumulators.
 // The solves' vectors y and x are marked as not computed on the way.
 __global__ void __launch_bounds__(256) k_hemv(const cd* __restrict__ B, int ld, int n, const cd* __restrict__ v,
-                                              cd* __restrict__ w, cd* __restrict__ y, cd* __restrict__ x)
+                                              cd* __restrict__ w, cd* __restrict__ y, cd* __restrict__ x,
+                                              const double* __restrict__ red, const int* __restrict__ status)
 {
+    if (idle(red, status)) return;
     const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (col >= n) return;
@@ -250,8 +265,9 @@ __global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_fwd_coop(const cd* __res
                                                   int nb, const cd* __restrict__ w, cd* __restrict__ y,
                                                   cd* __restrict__ z, const cd* __restrict__ invD,
                                                   const cd* __restrict__ linv, const cd* __restrict__ lmf,
-                                                  int* __restrict__ status, int* abort_word)
+                                                  int* status, int* abort_word, const double* __restrict__ idle_red)
 {
+    if (idle_red && idle(idle_red, status)) return;
     extern __shared__ double2 sm[];
     double2* Ls = sm;                          // Linv_j, [r][q]
     double2* Ms = sm + LDL_NB * LS_LD;         // NEIGH: M_j, [r][q]
@@ -346,8 +362,9 @@ template <bool NEIGH>
 __global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_bwd_coop(const cd* __restrict__ A, int ld, const int* __restrict__ bstart,
                                                   int nb, const cd* __restrict__ z, cd* __restrict__ x,
                                                   const cd* __restrict__ linv, const cd* __restrict__ lnb,
-                                                  int* __restrict__ status, int* abort_word)
+                                                  int* status, int* abort_word, const double* __restrict__ idle_red)
 {
+    if (idle(idle_red, status)) return;
     extern __shared__ double2 sm[];
     double2* Ls = sm;
     double2* red = sm + LDL_NB * LS_LD;  // [8][64] warp partials
@@ -446,12 +463,13 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh)
     }
 }
 
-// Normalisation and convergence measure of one step from the solution xw;
-// ends with v <- x.
+// Normalisation, convergence measure and convergence of one step from the
+// solution xw (src/linalg.f90:1894-1908); ends with v <- x.
 __global__ void __launch_bounds__(1024) k_iter_norm(int n, const cd* __restrict__ xw, cd* __restrict__ x,
-                                                    cd* __restrict__ v, double sqrtn,
-                                                    double* __restrict__ red)
+                                                    cd* __restrict__ v, double sqrtn, double tol,
+                                                    double* __restrict__ red, const int* __restrict__ status)
 {
+    if (idle(red, status)) return;
     __shared__ double sh[32 * 3];
     __shared__ double smax[32];
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
@@ -487,7 +505,14 @@ __global__ void __launch_bounds__(1024) k_iter_norm(int n, const cd* __restrict_
     }
     __syncthreads();
     block_sum<1>(d, sh);
-    if (tid == 0) red[RD_NORMDIFF] = sqrtn * sqrt(d[0]);
+    if (tid == 0) {
+        const double nd = sqrtn * sqrt(d[0]), it = red[RD_ITERS];
+        const double prev = it > 0.0 ? red[RD_NORMDIFF] : DBL_MAX;
+        red[RD_NORMDIFF] = nd;
+        red[RD_ITERS] = it + 1.0;
+        red[RD_GAIN] = nd / prev;
+        red[RD_DONE] = (tol > 0.0 ? nd <= tol : (nd > prev && nd <= fabs(tol))) ? 1.0 : 0.0;
+    }
     __syncthreads();
     for (int j = tid; j < n; j += 1024) v[j] = x[j];
 }
@@ -495,8 +520,10 @@ __global__ void __launch_bounds__(1024) k_iter_norm(int n, const cd* __restrict_
 // Per-column terms of x^H A x over the lower triangle (VMMHMV,
 // src/linalg.f90:1195-1206) for A = B (blockIdx.y = 0) and A = M (1).
 __global__ void __launch_bounds__(256) k_vmm_cols(const cd* __restrict__ B, const cd* __restrict__ M, int ld, int n,
-                                                  const cd* __restrict__ x, double* __restrict__ colval)
+                                                  const cd* __restrict__ x, double* __restrict__ colval,
+                                                  const double* __restrict__ red, const int* __restrict__ status, int always)
 {
+    if (idle_rayleigh(red, status, always)) return;
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (k >= n) return;
@@ -520,10 +547,14 @@ __global__ void __launch_bounds__(256) k_vmm_cols(const cd* __restrict__ B, cons
     }
 }
 
-__global__ void __launch_bounds__(1024) k_vmm_reduce(int n, const double* __restrict__ colval,
-                                                     const cd* __restrict__ x, double* __restrict__ red)
+// The three quadratic forms; x is then scaled to x^H B x = 1 (specif_norm 0)
+// or x^H x = 1 (1).
+__global__ void __launch_bounds__(1024) k_vmm_reduce(int n, const double* __restrict__ colval, cd* __restrict__ x,
+                                                     double* __restrict__ red, const int* __restrict__ status, int always,
+                                                     int specif_norm)
 {
     __shared__ double sh[32 * 3];
+    if (idle_rayleigh(red, status, always)) return;
     double acc[3] = {0.0, 0.0, 0.0};
     for (int j = threadIdx.x; j < n; j += 1024) {
         acc[0] += colval[j];
@@ -537,14 +568,11 @@ __global__ void __launch_bounds__(1024) k_vmm_reduce(int n, const double* __rest
         red[RD_T2] = acc[1];
         red[RD_XX] = acc[2];
     }
-}
-
-__global__ void k_vec_scale(cd* __restrict__ v, int n, double s)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) {
-        const cd a = v[j];
-        v[j] = cd{s * a.x, s * a.y};
+    if (specif_norm != 0 && specif_norm != 1) return;
+    const double f = 1.0 / sqrt(specif_norm == 0 ? acc[0] : acc[2]);
+    for (int j = threadIdx.x; j < n; j += 1024) {
+        const cd a = x[j];
+        x[j] = cd{a.x * f, a.y * f};
     }
 }
 
@@ -678,16 +706,16 @@ __global__ void __launch_bounds__(1024) k_border_finish(cd* __restrict__ A, int 
     }
 }
 
-static int launch_fwd(Ctx& c, int nb, bool neigh)
+// red: the iteration's state, or null outside it.
+static int launch_fwd(Ctx& c, int nb, bool neigh, const double* red)
 {
     const size_t sm = coop_smem(neigh);
     int* abort_word = c.counters + 2;
-    if (cudaMemsetAsync(abort_word, 0, sizeof(int), c.stream) != cudaSuccess) return -2;
     const int* bs = c.dblk;
     const cd *H = c.F, *w = c.w, *invD = c.invD, *linv = c.linv, *lmf = c.lmf;
     int ld = c.ld;
     void* args[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&w, &c.yv, &c.zv, (void*)&invD, (void*)&linv, (void*)&lmf,
-                    &c.status, &abort_word};
+                    &c.status, &abort_word, (void*)&red};
     const void* k = neigh ? (const void*)k_fwd_coop<true> : (const void*)k_fwd_coop<false>;
     if (cudaLaunchCooperativeKernel(k, nb, 256, args, sm, c.stream) != cudaSuccess) return -2;
     c.launches++;
@@ -697,14 +725,15 @@ static int launch_fwd(Ctx& c, int nb, bool neigh)
 static int solve_cooperative(Ctx& c, bool neigh)
 {
     int nb = (int)c.blk_start.size();
-    const int r = launch_fwd(c, nb, neigh);
+    const double* red = c.red;
+    const int r = launch_fwd(c, nb, neigh, red);
     if (r) return r;
     int* abort_word = c.counters + 2;
     const int* bs = c.dblk;
     const cd *H = c.F, *linv = c.linv, *lnb = c.lnb, *zv = c.zv;
     int ld = c.ld;
     void* args[] = {(void*)&H, &ld, (void*)&bs, &nb, (void*)&zv, &c.xw, (void*)&linv, (void*)&lnb,
-                    &c.status, &abort_word};
+                    &c.status, &abort_word, (void*)&red};
     const void* k = neigh ? (const void*)k_bwd_coop<true> : (const void*)k_bwd_coop<false>;
     if (cudaLaunchCooperativeKernel(k, nb, 256, args, coop_smem(neigh), c.stream) != cudaSuccess) return -2;
     c.launches++;
@@ -718,7 +747,8 @@ int border_row(Ctx& c, int m0, int nexist)
     const bool neigh = nexist <= coop_capacity(c, true);
     if (nexist < 1 || (!neigh && nexist > coop_capacity(c, false))) return 1;
     k_border_rhs<<<(m0 + 255) / 256, 256, 0, c.stream>>>(c.F, c.ld, m0, c.w, c.yv);
-    const int r = launch_fwd(c, nexist, neigh);
+    if (cudaMemsetAsync(c.counters + 2, 0, sizeof(int), c.stream) != cudaSuccess) return -2;  // the abort word
+    const int r = launch_fwd(c, nexist, neigh, nullptr);
     if (r) return r;
     int p0 = 0;  // first row of the last existing panel
     for (int s : c.blk_start)
@@ -729,9 +759,9 @@ int border_row(Ctx& c, int m0, int nexist)
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int invit_step(Ctx& c, int n, bool /*first*/)
+int invit_step(Ctx& c, int n, double tol)
 {
-    k_hemv<<<(n * 32 + 255) / 256, 256, 0, c.stream>>>(c.S, c.ld, n, c.c, c.w, c.yv, c.xw);
+    k_hemv<<<(n * 32 + 255) / 256, 256, 0, c.stream>>>(c.S, c.ld, n, c.c, c.w, c.yv, c.xw, c.red, c.status);
     c.launches++;
     const int nb = (int)c.blk_start.size();
     // the neighbour products take a second 64 x 64 block of shared memory
@@ -744,24 +774,18 @@ int invit_step(Ctx& c, int n, bool /*first*/)
     else
         r = solve_multi_launch(c, n);
     if (r) return r;
-    k_iter_norm<<<1, 1024, 0, c.stream>>>(n, c.xw, c.x, c.c, sqrt(2.0 * n), c.red);
+    k_iter_norm<<<1, 1024, 0, c.stream>>>(n, c.xw, c.x, c.c, sqrt(2.0 * n), tol, c.red, c.status);
     c.launches++;
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int invit_rayleigh(Ctx& c, int n)
+// Once the iteration has converged, or `always`.
+int invit_rayleigh(Ctx& c, int n, bool always, int specif_norm)
 {
     dim3 g((n * 32 + 255) / 256, 2);
-    k_vmm_cols<<<g, 256, 0, c.stream>>>(c.S, c.F, c.ld, n, c.x, c.colval);
-    k_vmm_reduce<<<1, 1024, 0, c.stream>>>(n, c.colval, c.x, c.red);
+    k_vmm_cols<<<g, 256, 0, c.stream>>>(c.S, c.F, c.ld, n, c.x, c.colval, c.red, c.status, always);
+    k_vmm_reduce<<<1, 1024, 0, c.stream>>>(n, c.colval, c.x, c.red, c.status, always, specif_norm);
     c.launches += 2;
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-}
-
-int vec_scale(Ctx& c, cd* v, int n, double s)
-{
-    k_vec_scale<<<(n + 255) / 256, 256, 0, c.stream>>>(v, n, s);
-    c.launches++;
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
