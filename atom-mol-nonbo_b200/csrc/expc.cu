@@ -19,7 +19,7 @@
 // tCl - X (all symmetric).  Put in, the long sums the reference takes term
 // by term leave
 //   kinetic            6 S tr[M X]
-//   mass-velocity      -(36/8) (5/3) S (X_k l summed squared / m0^3 + sum_i X_ii^2 / m_i^3)
+//   mass-velocity      -(36/8) (5/3) S ((sum of all X_kl)^2 / m0^3 + sum_i X_ii^2 / m_i^3)
 //   ME_dXd_dYd         36 X_ii X_jj + 24 X_ij^2 (X = E_ii, Y = E_jj)
 //   orbit-orbit        -8 X_ij <1/r_P> of each (i, j)
 // so the Drachmanised mass-velocity and Darwin sums are one value (the

@@ -6,11 +6,14 @@
 //   tc = x^H v / v^H v, NormOfDiff = sqrt(2n) ||x - tc v||
 //   t1 = x^H B x, t2 = x^H M x VMMHMV on the lower triangles
 //
-// The triangular solves walk the panels of the LDL^H factor.  Each panel
-// step is one launch whose CTAs share the dot products against the already
-// solved part; the last CTA to finish (atomic ticket, no waiting) sums the
-// partials in a fixed order and applies the panel's precomputed inverse
-// block, so results are deterministic run to run.
+// The triangular solves walk the panels of the LDL^H factor, one cooperative
+// launch each with a CTA per panel (below); beyond the co-resident CTAs each
+// panel step is one launch whose CTAs share the dot products against the
+// already solved part, and the last CTA to finish (atomic ticket, no waiting)
+// sums the partials in a fixed order and applies the panel's precomputed
+// inverse block.  Results are deterministic run to run.  The host enqueues
+// several steps and the Rayleigh quotient at a time (ghepiis_core); launches
+// after convergence return at once.
 #include <algorithm>
 #include <float.h>
 #include "ecg_internal.h"

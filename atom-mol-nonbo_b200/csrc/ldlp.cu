@@ -22,7 +22,8 @@
 // CTA 0, alone on its SM, runs the chain D(s) -> T(s, s+1) -> B(s, s+1,
 // s+1) -> D(s+1) with the diagonal tile kept in registers.  The other
 // CTAs (all co-resident: cooperative launch) take every other task from a
-// list in a fixed order through one atomic counter; an update whose next
+// list in a fixed order through one atomic counter; updates far from their
+// panels are one task for four of them, and a nearer one whose group's next
 // panels are already final applies them too (rank up to 256).  The list is
 // a topological order of the dependency graph, made on the host by list
 // scheduling on as many simulated workers as the grid has CTAs, always
@@ -40,7 +41,7 @@
 // with D; 47 us with an elimination through shared memory and substitution
 // in T), and the list's updates run at 95 % of the tensor cores, so whole
 // factorisations take 0.31 ms at K = 500 (0.46 before both), 0.88 at 1500
-// (1.24), 3.79 at 4000 (4.94), 47.2 at 10000 (57.2 per panel step).  Two CTAs an SM take 217 KB of
+// (1.24), 3.63 at 4000 (4.94), 45.5 at 10000 (57.2 per panel step).  Two CTAs an SM take 217 KB of
 // shared memory and leave about 28 KB of L1, so a spilled register comes back
 // from L2: the chain with 200 bytes of stack ran D(s) in 32 us, with 32 bytes
 // in 18.  Every array of the chain is sized to stay within 128 registers.
