@@ -19,6 +19,7 @@
 #include "ecg_internal.h"
 #include "wait_value.cuh"
 #include "warp_sums.cuh"
+#include "zmma.cuh"
 
 namespace ecg {
 
@@ -207,19 +208,21 @@ __device__ __forceinline__ bool wait_panel(const cd* p, int n, double2* sv, int*
 }
 
 // Rows [j0, j0 + b) of a per-panel 64-column block (linv, lmf, lnb) into
-// Ls[r][q] for q < bq, zeros elsewhere.
+// Ls[r][q] for q < bq, zeros elsewhere: asynchronous copies, all in flight at
+// once (through registers the two blocks of a CTA took 4 us, a third of the
+// whole solve at n = 201).
 __device__ __forceinline__ void load_linv(const cd* __restrict__ linv, int j0, int b, double2* Ls, int bq = -1)
 {
     if (bq < 0) bq = b;
-    for (int e = threadIdx.x; e < LDL_NB * LDL_NB; e += blockDim.x) {
-        const int r = e / LDL_NB, q = e % LDL_NB;
-        double2 v = make_double2(0.0, 0.0);
-        if (r < b && q < bq) {
-            const cd a = ld2(linv + (size_t)(j0 + r) * LDL_NB + q);
-            v = make_double2(a.x, a.y);
-        }
-        Ls[r * LS_LD + q] = v;
+    const int q = threadIdx.x & 63, r0 = threadIdx.x >> 6;
+    const cd* src = linv + (size_t)(j0 + r0) * LDL_NB + q;
+#pragma unroll 4
+    for (int i = 0; i < 16; i++) {
+        const int r = r0 + 4 * i;
+        const bool in = r < b && q < bq;
+        cp_async16(Ls + r * LS_LD + q, in ? src + (size_t)(4 * i) * LDL_NB : linv, in ? 16 : 0);
     }
+    cp_async_commit();
 }
 
 // Row r = tid / 4 of the product of a 64 x 64 block in shared memory with
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_fwd_coop(const cd* __res
                                                   const cd* __restrict__ linv, const cd* __restrict__ lmf,
                                                   int* status, int* abort_word, const double* __restrict__ idle_red)
 {
-    if (idle_red && idle(idle_red, status)) return;
+    const bool off = idle_red && idle(idle_red, status);
     extern __shared__ double2 sm[];
     double2* Ls = sm;                          // Linv_j, [r][q]
     double2* Ms = sm + LDL_NB * LS_LD;         // NEIGH: M_j, [r][q]
@@ -280,6 +283,10 @@ __global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_fwd_coop(const cd* __res
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     load_linv(linv, j0, b, Ls);
     if (NEIGH && j > 0) load_linv(lmf, j0, b, Ms, j0 - bstart[j - 1]);
+    if (off) {  // looked at while the blocks are on their way
+        cp_async_wait<0>();
+        return;
+    }
     // this panel's right-hand side and pivots, read before the waits
     const int r = threadIdx.x >> 2;
     const cd wj = (threadIdx.x < b) ? ld2(w + j0 + threadIdx.x) : mk(0.0, 0.0);
@@ -345,6 +352,7 @@ __global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_fwd_coop(const cd* __res
         const double sum = warp_transpose_sum<16>(v);
         if ((lane & 1) == 0) reinterpret_cast<double*>(t)[16 * wp + (lane >> 1)] = sum;
     }
+    cp_async_wait<0>();
     __syncthreads();
     if (threadIdx.x < LDL_NB) t[threadIdx.x] = make_double2(wj.x - t[threadIdx.x].x, wj.y - t[threadIdx.x].y);
     __syncthreads();
@@ -367,7 +375,7 @@ __global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_bwd_coop(const cd* __res
                                                   const cd* __restrict__ linv, const cd* __restrict__ lnb,
                                                   int* status, int* abort_word, const double* __restrict__ idle_red)
 {
-    if (idle(idle_red, status)) return;
+    const bool off = idle(idle_red, status);
     extern __shared__ double2 sm[];
     double2* Ls = sm;
     double2* red = sm + LDL_NB * LS_LD;  // [8][64] warp partials
@@ -378,6 +386,10 @@ __global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_bwd_coop(const cd* __res
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     load_linv(linv, j0, b, Ls);
     if (NEIGH && j + 1 < nb) load_linv(lnb, j0, b, Ns, bstart[j + 2] - j1);
+    if (off) {
+        cp_async_wait<0>();
+        return;
+    }
     const int r = threadIdx.x >> 2;
     const cd zj = (threadIdx.x < b) ? ld2(z + j0 + threadIdx.x) : mk(0.0, 0.0);  // read before the waits
     cd a0 = mk(0.0, 0.0), a1 = mk(0.0, 0.0);  // rows lane, lane + 32
@@ -426,6 +438,7 @@ __global__ void __launch_bounds__(256, NEIGH ? 1 : 2) k_bwd_coop(const cd* __res
     }
     red[wp * LDL_NB + lane] = make_double2(a0.x, a0.y);
     red[wp * LDL_NB + lane + 32] = make_double2(a1.x, a1.y);
+    cp_async_wait<0>();
     __syncthreads();
     if (threadIdx.x < LDL_NB) {
         cd s = mk(0.0, 0.0);
