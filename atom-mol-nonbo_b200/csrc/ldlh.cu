@@ -326,11 +326,12 @@ __global__ void __launch_bounds__(256) k_ldl_linv(const cd* __restrict__ A, int 
 // stored like linv, row r of panel j at [(p0 + r) * 64 + q].  With them a
 // solve's panel j applies the neighbouring panel's solution as one 64 x 64
 // product once that panel is published, everything else being done before.
-// One 64 x 64 x 64 complex product per CTA on the FP64 tensor cores, in two
-// chunks of the inner dimension: 8 us for all panels at K = 4000 (a product
-// of FMA loops over one chunk of 133 KB, one CTA an SM: 37 us).
-constexpr int MN_K = 32, MN_LDA = LDL_NB + 2, MN_LDB = MN_K + 4;  // pitches as zmma.cuh wants them
-constexpr size_t MN_SMEM = (size_t)(MN_K * MN_LDA + LDL_NB * MN_LDB) * sizeof(double2);
+// A CTA takes 16 columns (blockIdx.z) of a 64 x 64 x 64 complex product on
+// the FP64 tensor cores, its operands loaded at once: 9.3 us at
+// K = 500, 19.5 at K = 4000 (whole products, 8.4 us of one SM each, in two
+// chunks of the inner dimension: 20.4 and 22.4 us).
+constexpr int MN_N = 16, MN_LDA = LDL_NB + 2, MN_LDB = LDL_NB + 4;  // pitches as zmma.cuh wants them
+constexpr size_t MN_SMEM = (size_t)(LDL_NB * MN_LDA + MN_N * MN_LDB) * sizeof(double2);
 
 __global__ void __launch_bounds__(256) k_ldl_mn(const cd* __restrict__ A, int ld, const int* __restrict__ bstart,
                                                  int nb, int first, const cd* __restrict__ linv, cd* __restrict__ lmf,
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(256) k_ldl_mn(const cd* __restrict__ A, int ld
 {
     extern __shared__ double2 sm[];
     double2* As = sm;                    // [k][m]: Linv_j (forward) or its transpose (backward, conjugated in the product)
-    double2* Bs = sm + MN_K * MN_LDA;    // [n][k]: conj(U(o0 + n, p0 + k)) or U(p0 + k, o0 + n)
+    double2* Bs = sm + LDL_NB * MN_LDA;  // [n][k]: conj(U(o0 + n, p0 + k)) or U(p0 + k, o0 + n)
     const int j = first + blockIdx.x;
     const bool fwd = blockIdx.y == 0;
     if (fwd ? j < 1 : j + 1 >= nb) return;
@@ -346,50 +347,49 @@ __global__ void __launch_bounds__(256) k_ldl_mn(const cd* __restrict__ A, int ld
     const int o0 = fwd ? bstart[j - 1] : bstart[j + 1];
     const int bo = fwd ? p0 - o0 : bstart[j + 2] - o0;
     const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
-    const int wm = (wp >> 2) * 32, wn = (wp & 3) * 16;
-    ZAcc<4, 2> acc;
+    const int n0 = blockIdx.z * MN_N;
+    // linv's rows are contiguous, U's columns are
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int e = tid + 256 * u;
+        const int nn = n0 + (fwd ? (e & 15) : (e >> 6)), k = fwd ? (e >> 4) : (e & 63);
+        double2 y = make_double2(0.0, 0.0);
+        if (nn < bo && k < b) {
+            const cd v = ldg2(A + (fwd ? (size_t)(o0 + nn) + (size_t)(p0 + k) * ld
+                                       : (size_t)(p0 + k) + (size_t)(o0 + nn) * ld));
+            y = make_double2(v.x, fwd ? -v.y : v.y);
+        }
+        Bs[(nn - n0) * MN_LDB + k] = y;
+    }
+#pragma unroll
+    for (int u = 0; u < 16; u++) {
+        const int e = tid + 256 * u;
+        const int m = fwd ? (e >> 6) : (e & 63), k = fwd ? (e & 63) : (e >> 6);
+        const bool in = m < b && k < b;
+        cp_async16(As + k * MN_LDA + m, in ? linv + (fwd ? (size_t)(p0 + m) * LDL_NB + k : (size_t)(p0 + k) * LDL_NB + m) : linv,
+                   in ? 16 : 0);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    ZAcc<1, 2> acc;
     acc.zero();
-    for (int k0 = 0; k0 < LDL_NB; k0 += MN_K) {
+    if (fwd) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const int e = tid + 256 * u;
-            // linv's rows are contiguous, U's columns are
-            const int ma = fwd ? (e >> 5) : (e & 63), ka = k0 + (fwd ? (e & 31) : (e >> 6));
-            const int nn = fwd ? (e & 63) : (e >> 5), kb = k0 + (fwd ? (e >> 6) : (e & 31));
-            double2 x = make_double2(0.0, 0.0), y = x;
-            if (ma < b && ka < b) {
-                const cd v = ldg2(linv + (fwd ? (size_t)(p0 + ma) * LDL_NB + ka : (size_t)(p0 + ka) * LDL_NB + ma));
-                x = make_double2(v.x, v.y);
-            }
-            if (nn < bo && kb < b) {
-                const cd v = ldg2(A + (fwd ? (size_t)(o0 + nn) + (size_t)(p0 + kb) * ld
-                                           : (size_t)(p0 + kb) + (size_t)(o0 + nn) * ld));
-                y = make_double2(v.x, fwd ? -v.y : v.y);
-            }
-            As[(ka - k0) * MN_LDA + ma] = x;
-            Bs[nn * MN_LDB + kb - k0] = y;
-        }
-        __syncthreads();
-        if (fwd) {
+        for (int kk = 0; kk < LDL_NB; kk += 4) zmma_k4<1, 2, MN_LDA, MN_LDB, false>(acc, As, Bs, 8 * wp, 0, kk, lane);
+    } else {
 #pragma unroll
-            for (int kk = 0; kk < MN_K; kk += 4) zmma_k4<4, 2, MN_LDA, MN_LDB, false>(acc, As, Bs, wm, wn, kk, lane);
-        } else {
-#pragma unroll
-            for (int kk = 0; kk < MN_K; kk += 4) zmma_k4<4, 2, MN_LDA, MN_LDB, true>(acc, As, Bs, wm, wn, kk, lane);
-        }
-        __syncthreads();
+        for (int kk = 0; kk < LDL_NB; kk += 4) zmma_k4<1, 2, MN_LDA, MN_LDB, true>(acc, As, Bs, 8 * wp, 0, kk, lane);
     }
     const int g = lane >> 2, t = lane & 3;
     cd* out = fwd ? lmf : lnb;
 #pragma unroll
-    for (int mt = 0; mt < 4; mt++)
+    for (int nt = 0; nt < 2; nt++)
 #pragma unroll
-        for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                const int m = wm + mt * 8 + g, n = wn + nt * 8 + 2 * t + e;
-                if (m < b) out[(size_t)(p0 + m) * LDL_NB + n] = cd{acc.r[mt][nt][e], acc.i[mt][nt][e]};
-            }
+        for (int e = 0; e < 2; e++) {
+            const int m = 8 * wp + g, n = n0 + nt * 8 + 2 * t + e;
+            if (m < b) out[(size_t)(p0 + m) * LDL_NB + n] = cd{acc.r[0][nt][e], acc.i[0][nt][e]};
+        }
 }
 
 // Panel rows beyond the diagonal block, by substitution:
@@ -699,7 +699,7 @@ static void enqueue_factor(Ctx& c, int m0, int n, const std::vector<int>& starts
         k_ldl_linv<<<nblk - nexist, 256, 2 * sm1, c.stream>>>(c.F, c.ld, c.dblk, nexist, c.linv);
         // the last existing panel's N changes with the first new panel
         const int f = std::max(nexist - 1, 0);
-        k_ldl_mn<<<dim3(nblk - f, 2), 256, MN_SMEM, c.stream>>>(c.F, c.ld, c.dblk, nblk, f, c.linv, c.lmf, c.lnb);
+        k_ldl_mn<<<dim3(nblk - f, 2, LDL_NB / MN_N), 256, MN_SMEM, c.stream>>>(c.F, c.ld, c.dblk, nblk, f, c.linv, c.lmf, c.lnb);
         c.launches += 2;
     }
 }
@@ -716,7 +716,7 @@ static int enqueue_persist(Ctx& c, int n, const unsigned* tasks, int ntasks, boo
     const int r = ldlp_enqueue(c, n, tasks, ntasks, trace);
     if (r || !solves) return r;
     const int nblk = (n + LDL_NB - 1) / LDL_NB;
-    k_ldl_mn<<<dim3(nblk, 2), 256, MN_SMEM, c.stream>>>(c.F, c.ld, c.dblk, nblk, 0, c.linv, c.lmf, c.lnb);
+    k_ldl_mn<<<dim3(nblk, 2, LDL_NB / MN_N), 256, MN_SMEM, c.stream>>>(c.F, c.ld, c.dblk, nblk, 0, c.linv, c.lmf, c.lnb);
     c.launches++;
     return 0;
 }
