@@ -182,8 +182,7 @@ struct Ctx {
     int factor_mode = 0;        // 0: persistent kernel for m0 = 0, 1: one launch per panel step
     int lp_grid = 0;            // co-resident CTAs of the persistent kernel (0: not yet known)
     int lp_sms = 1;             // SMs of the device
-    unsigned* lp_cnt = nullptr; // tile counters, then the next-task counter and the abort word
-    size_t lp_cap = 0;          // capacity of lp_cnt (unsigned)
+    unsigned* lp_cnt = nullptr; // tile counters and control words, in every cached graph: allocated once
     unsigned* lp_direct = nullptr;  // task list of the uncaptured fallback, for lp_direct_n rows
     int lp_direct_n = 0, lp_direct_count = 0;
 
@@ -280,7 +279,7 @@ int ldlh_factor(Ctx& c, int m0, int n, bool solves = true);
 int ldlp_grid(Ctx& c);
 int ldlp_tasks(Ctx& c, int n, unsigned** tasks, int* count);
 long long ldlp_task_total(int n);
-int ldlp_reserve(Ctx& c, int np);
+int ldlp_reserve(Ctx& c);
 int ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long long* trace = nullptr);
 // One persistent factorisation of rows 0..n-1 of the current matrix with a
 // per-task timing record (4 values per task, see ecg_factor_trace).

@@ -781,7 +781,7 @@ int ldlh_factor(Ctx& c, int m0, int n, bool solves)
         unsigned* tasks = nullptr;
         int ntasks = 0;
         if (persist) {
-            const int r = ldlp_reserve(c, nb);
+            const int r = ldlp_reserve(c);
             if (r) return r;
             const int t = ldlp_tasks(c, n, &tasks, &ntasks);
             if (t) return t;
@@ -860,7 +860,7 @@ int ldlh_factor_traced(Ctx& c, int n, unsigned long long* out, long long cap, lo
     if (cudaMemcpyAsync(c.dblk, c.bounds_h, (nb + 1) * sizeof(int), cudaMemcpyHostToDevice, c.stream) !=
         cudaSuccess)
         return -2;
-    if (ldlp_reserve(c, nb)) return -3;
+    if (ldlp_reserve(c)) return -3;
     unsigned* tasks = nullptr;
     int ntasks = 0;
     if (ldlp_tasks(c, n, &tasks, &ntasks)) return -2;

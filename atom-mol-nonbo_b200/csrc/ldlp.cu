@@ -1209,19 +1209,18 @@ long long ldlp_task_total(int n)
 }
 
 // Tile counters and the control words (next task, abort word, trace
-// records, the chain CTA's SM) for np panels.
-int ldlp_reserve(Ctx& c, int np)
+// records, the chain CTA's SM), once for the largest factorisation this
+// context can take here (60 KB at 5000 rows, 0.24 MB at 12800).  The cached
+// graphs of every size hold this address, so it never moves.
+int ldlp_reserve(Ctx& c)
 {
-    const size_t need = (size_t)np * (np + 1) / 2 * 3 + 4;
-    if (c.lp_cap >= need) return 0;
-    if (c.lp_cnt) cudaFree(c.lp_cnt);
-    c.lp_cnt = nullptr;
-    c.lp_cap = 0;
-    if (cudaMalloc(&c.lp_cnt, need * sizeof(unsigned)) != cudaSuccess) {
+    if (c.lp_cnt) return 0;
+    const size_t np = (std::min(c.ld, LDL_PERSIST_MAX) + LDL_NB - 1) / LDL_NB;
+    if (cudaMalloc(&c.lp_cnt, (np * (np + 1) / 2 * 3 + 4) * sizeof(unsigned)) != cudaSuccess) {
         cudaGetLastError();
+        c.lp_cnt = nullptr;
         return -3;
     }
-    c.lp_cap = need;
     return 0;
 }
 
