@@ -1270,19 +1270,30 @@ int ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long
 
 }  // namespace ecg
 
-// Host-only diagnostic: every task of the persistent factorisation of n
-// rows for a grid of `workers` CTAs in the scheduler's start order (the
-// chain CTA's tasks included; the kernel's list is this order without
-// them).  No GPU needed.
-extern "C" int ecg_ldl_schedule(int n, int workers, unsigned* out, long long cap, long long* count)
+// Host-only diagnostics: the tasks of the persistent factorisation of n rows
+// for a grid of `workers` CTAs in the scheduler's start order, the chain
+// CTA's included.  No GPU needed.
+static int task_order(int n, int workers, bool group, unsigned* out, long long cap, long long* count)
 {
     using namespace ecg;
     if (n < 1 || workers < 1 || !count) return -1;
     const int np = (n + LDL_NB - 1) / LDL_NB;
     if (np > 200) return -1;
     std::vector<unsigned> full, list;
-    lp_schedule(np, workers, LpCost(), false, list, &full);
+    lp_schedule(np, workers, LpCost(), group, list, &full);
     *count = (long long)full.size();
     if (out && cap >= (long long)full.size()) std::copy(full.begin(), full.end(), out);
     return 0;
+}
+
+// Every update a task of its own, which the kernel does not run.
+extern "C" int ecg_ldl_schedule(int n, int workers, unsigned* out, long long cap, long long* count)
+{
+    return task_order(n, workers, false, out, cap, count);
+}
+
+// What the kernel runs: its list is this order without the chain's tasks.
+extern "C" int ecg_ldl_task_list(int n, int workers, unsigned* out, long long cap, long long* count)
+{
+    return task_order(n, workers, true, out, cap, count);
 }

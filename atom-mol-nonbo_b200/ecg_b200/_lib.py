@@ -64,6 +64,7 @@ PROTOTYPES = {
     "ecg_set_factor_mode": (C.c_int, [_vp, C.c_int]),
     "ecg_factor_trace": (C.c_int, [_vp, C.c_int, C.c_void_p, C.c_longlong, C.POINTER(C.c_longlong)]),
     "ecg_ldl_schedule": (C.c_int, [C.c_int, C.c_int, C.c_void_p, C.c_longlong, C.POINTER(C.c_longlong)]),
+    "ecg_ldl_task_list": (C.c_int, [C.c_int, C.c_int, C.c_void_p, C.c_longlong, C.POINTER(C.c_longlong)]),
     "ecg_io_bytes": (C.c_int, [_vp, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]),
     "ecg_probe_fp64_peak": (C.c_int, [C.c_int, _dp]),
     "ecg_probe_fp64_tensor_peak": (C.c_int, [C.c_int, _dp]),

@@ -331,7 +331,7 @@ int ecg_set_factor_mode(ecg_ctx* ctx, int mode);
 /* Factorise rows 1..n of the context's current matrix (the lower triangle
  * that ecg_compute_mat_elem / ecg_ghepiis leave: H - lambda~ S) once with
  * the persistent kernel, outside any graph, recording per task: the task
- * code (as ecg_ldl_schedule) | CTA << 32 | panels applied << 48 (0: found
+ * code (as ecg_ldl_task_list) | CTA << 32 | panels applied << 48 (0: found
  * already applied), and the GPU's globaltimer (ns) when the CTA began
  * waiting for the task's tiles, when they were ready and when the task was
  * published.  *count receives the number of records; records (capacity cap
@@ -347,15 +347,23 @@ int ecg_factor_trace(ecg_ctx* ctx, int n, unsigned long long* records, long long
  * No counterpart in the reference: a diagnostic that lets a test make a
  * wait run out without a fault. */
 int ecg_set_wait_limit(ecg_ctx* ctx, int polls);
-/* The task order of the persistent factorisation of n rows (n <= 12800)
+/* A task order of the factorisation of n rows (n <= 12800) by 64 x 64 tiles
  * for a grid of `workers` CTAs, on the host (no GPU needed): codes
  * type << 30 | h << 29 | s << 20 | R << 10 | C, type 0 = D(s) (diagonal
  * tile s), 1 = T(s, C) (panel rows of tile (s, C)), 2 = B(s, R, C) (update
  * of tile (R, C) by panel s; for R <= s + 2, other than (s+1, s+1), two
- * tasks on the column halves h = 0, 1), 64-row tiles.  *count receives the
- * length; out (capacity cap) is filled when it is large enough.  No
- * counterpart in the reference: exposes the task order to tests. */
+ * tasks on the column halves h = 0, 1), 64-row tiles.  Every update is a
+ * task of its own here; the persistent kernel runs ecg_ldl_task_list's.
+ * *count receives the length; out (capacity cap) is filled when it is large
+ * enough.  No counterpart in the reference: exposes the task order to
+ * tests. */
 int ecg_ldl_schedule(int n, int workers, unsigned* out, long long cap, long long* count);
+/* The task order the persistent factorisation of n rows runs on a grid of
+ * `workers` CTAs besides the chain's: as ecg_ldl_schedule, with the updates
+ * of a tile (R, C) by the four panels s..s+3 (s a multiple of 4), R >= s + 8,
+ * as one task of code B(s, R, C) with h = 1.  The kernel's CTAs take these
+ * tasks in this order, the chain CTA D(s), T(s, s+1) and B(s, s+1, s+1). */
+int ecg_ldl_task_list(int n, int workers, unsigned* out, long long cap, long long* count);
 /* Bytes this context has copied host->device and device->host so far. */
 int ecg_io_bytes(ecg_ctx* ctx, long long* h2d, long long* d2h);
 /* The fused adjoint gradient of ecg_energy_ib_adjoint, for callers that
