@@ -92,6 +92,7 @@ struct CgArgs {
     const cd *E1, *e2;
     cd* P;             // two partial tiles a CTA
     int* status;
+    const int* limitp;  // poll limit of the call's waits: at 0 the first one here runs out too
 };
 
 // first chunk of tile row it, and the chunks before tile t (column by column)
@@ -161,6 +162,15 @@ __global__ void __launch_bounds__(256, 2) k_cgemm(const __grid_constant__ CgArgs
         fence_async_global();
         for (int i = 0; i < TMA_ST && u0 + i < u1; i++) issue(i);
     }
+    // a wait ran out at the piece's chunk ch
+    auto give_up = [&](int ch) {
+        if (lane == 0) atomicExch(a.status + ST_SOLVE_TIMEOUT, 1);
+        if (tid == 0) ring.drain(rst, rph, (int)(u1 - u0) - ring_refilled(ch, (int)(u1 - u0)));
+    };
+    if (__ldg(a.limitp) == 0) {
+        give_up(0);
+        return;
+    }
     constexpr int MT = 4, NT = 2;
     double accr[MT][NT][2], acci[MT][NT][2];
     auto zero = [&] {
@@ -178,7 +188,7 @@ __global__ void __launch_bounds__(256, 2) k_cgemm(const __grid_constant__ CgArgs
     for (long long u = u0; u < u1; u++) {
         const bool ok = bar_wait(ring.full + 8u * ring.st, ring.ph);
         if (!__all_sync(0xffffffffu, ok)) {
-            if (lane == 0) atomicExch(a.status + ST_SOLVE_TIMEOUT, 1);
+            give_up((int)(u - u0));
             return;
         }
         const int it = t % a.mt;
@@ -993,6 +1003,7 @@ int launch_gemm(Ctx& c, cd* A, int nbase, int ncols, cd* B, cd* C, const cd* E1,
     a.e2 = e2;
     a.P = cw.Pk;
     a.status = c.status;
+    a.limitp = cw.abort_word + 1;
     const int pieces = (int)std::min<long long>(cw.gemm_grid, a.total);
     k_cgemm<TRI><<<pieces, 256, CG_SMEM, c.stream>>>(a);
     k_cgemm_sum<TRI><<<dim3(a.ntile, CG_TILE / 256), 256, 0, c.stream>>>(a, pieces);

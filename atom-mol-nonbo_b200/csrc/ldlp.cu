@@ -465,7 +465,8 @@ __device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half,
     __syncthreads();  // dp
     bool ok = true;
     const int f0 = pg * TMA_KC + (t4 ^ pg);  // fragment slots of k = t4 and, with ^ 4, of k = 4 + t4
-    for (int ch = 0; ch < nch; ch++) {
+    int ch = 0;
+    for (; ch < nch; ch++) {
         ok = bar_wait(ring.full + 8u * ring.st, ring.ph);
         if (!__all_sync(0xffffffffu, ok)) break;
         if (wact) {
@@ -511,7 +512,10 @@ __device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half,
             ring.step(rst, rph);
         }
     }
-    if (__syncthreads_or(ok ? 0 : 1)) return false;
+    if (__syncthreads_or(ok ? 0 : 1)) {
+        if (tid == 0) ring.drain(rst, rph, nch - ring_refilled(ch, nch));
+        return false;
+    }
 #pragma unroll
     for (int mt = 0; mt < MT; mt++)
 #pragma unroll
@@ -1116,8 +1120,7 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
         const int half = (task >> 29) & 1;
         if (go == 1) {
             if (!lp_exec<CPLX>(a, type, s, m, R, C, half, lsm, ring)) {
-                // a copy did not arrive: wait for the others in flight, report, stop
-                for (int i = 0; i < TMA_ST; i++) bar_wait(ring.full + 8u * i, ring.ph);
+                // a copy did not arrive, and none is in flight: report, stop
                 if (tid == 0) {
                     atomicExch(a.status + ST_SOLVE_TIMEOUT, 1);
                     atomicExch(a.ctl + 1, 1u);

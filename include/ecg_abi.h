@@ -343,7 +343,8 @@ int ecg_factor_trace(ecg_ctx* ctx, int n, unsigned long long* records, long long
  * solves of GHEPIIS and of the batched candidates, and the tile waits of
  * the persistent factorisation): every wait on another CTA's work gives up
  * after `polls` polls, records the timeout and the call returns ECG_ECUDA
- * with the context still usable.  polls < 0 restores the default (2^22).
+ * with the context still usable; with polls = 0 the candidates' GEMM gives
+ * up on its bulk copies too.  polls < 0 restores the default (2^22).
  * No counterpart in the reference: a diagnostic that lets a test make a
  * wait run out without a fault. */
 int ecg_set_wait_limit(ecg_ctx* ctx, int polls);
