@@ -323,12 +323,20 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
         CK(cudaStreamSynchronize(c.stream));
     }
     int extra = 0, it = 0;
+    // the first bracket that held the eigenvalue alone: no other is inside it
+    bool alone = false;
+    double alone_lo = 0.0, alone_hi = 0.0;
     for (bool again = false;; again = true) {
         // bisect until the bracket holds the which-th eigenvalue alone, then a
         // few halvings more
         for (;;) {
             const double size = std::max(fabs(lo), fabs(hi));
             const bool isolated = (nlo == which - 1) && (nhi == which);
+            if (isolated && !alone) {
+                alone = true;
+                alone_lo = lo;
+                alone_hi = hi;
+            }
             if (isolated && extra >= (again ? G_EXTRA_MOST : G_EXTRA_BISECT)) break;
             if (isolated && !again && hi - lo <= G_NARROW * std::max(1.0, size)) break;
             if (hi - lo <= 4.0 * DBL_EPSILON * size) break;
@@ -358,13 +366,25 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
         // margin.
         const double margin = 1e-3 * (hi - lo) + 64.0 * DBL_EPSILON * fabs(sigma);
         const bool inside = e != ECG_ESINGULAR && lam >= lo - margin && lam <= hi + margin;
-        // once more in a narrower bracket if the shift met the eigenvalue, the
-        // iteration found another one, or it was still gaining when it ended
-        // (standing still, it is on its floor, which no shift lowers)
-        const bool gaining = e == ECG_ENOCONV && (ra > 1e-6 || c.last_gain < 0.9);
-        if (!again && extra < G_EXTRA_MOST && (!inside || gaining)) {
+        // An iteration leaves at most this share of the other eigenvectors.
+        // Only where it is well below one does a residual that stands still
+        // mean that the iteration is on its floor, which no shift lowers, and
+        // a small one that the vector is as close.
+        const double rate = alone ? fabs(lam - sigma) / std::min(sigma - alone_lo, alone_hi - sigma) : 0.0;
+        const bool found = e == ECG_OK ? rate <= 0.9 : (ra <= 1e-6 && c.last_gain >= 0.9 && rate <= 0.5);
+        // otherwise once more in a narrower bracket, as also where the shift
+        // met the eigenvalue or the iteration found another one, whose vector
+        // is then no start
+        const bool narrower = extra < G_EXTRA_MOST && hi - lo > 4.0 * DBL_EPSILON * std::max(fabs(lo), fabs(hi));
+        if (!again && narrower && !(inside && found)) {
             if (e == ECG_ESINGULAR) continue;
-            CK(cudaMemcpyAsync(c.c, c.x, (size_t)n * sizeof(cd), cudaMemcpyDeviceToDevice, c.stream));
+            if (inside) {
+                CK(cudaMemcpyAsync(c.c, c.x, (size_t)n * sizeof(cd), cudaMemcpyDeviceToDevice, c.stream));
+            } else {
+                std::vector<cd> ones(n, cd{1.0, 0.0});
+                CK(cudaMemcpyAsync(c.c, ones.data(), (size_t)n * sizeof(cd), cudaMemcpyHostToDevice, c.stream));
+                CK(cudaStreamSynchronize(c.stream));
+            }
             continue;
         }
         if (e == ECG_ESINGULAR) return ECG_ENOCONV;
