@@ -146,9 +146,10 @@ int ghepiis_core(Ctx& c, int k, int n, double apprlambda, double tol, int max_it
     // them, and the host looks once: after convergence, and where the
     // factorisation failed, the rest of the launches return at once.  As many
     // as the last call took, then two at a time: a look costs the stream 15 to
-    // 20 us (an iteration at n = 500 takes 50), an empty iteration 8.
-    int batch = std::min(8, c.last_numiter > 0 ? c.last_numiter : 3);
-    if (trace_on()) batch = 1;
+    // 20 us (an iteration at n = 500 takes 50), an empty iteration 8.  One at
+    // a time where a step is a launch per panel: 600 of them at 300 panels.
+    const bool single = trace_on() || invit_by_panels(c);
+    int batch = single ? 1 : std::min(8, c.last_numiter > 0 ? c.last_numiter : 3);
     bool notconverged = true;
     double nd = 0.0;
     int it = 0;
@@ -187,7 +188,7 @@ int ghepiis_core(Ctx& c, int k, int n, double apprlambda, double tol, int max_it
         notconverged = c.red_h[RD_DONE] == 0.0;
         if (trace_on()) fprintf(stderr, "ecg: GHEPIIS(%d,%d) iteration %d NormOfDiff %.3e\n", k, n, it, nd);
         if (!notconverged || last) break;
-        batch = trace_on() ? 1 : 2;
+        batch = single ? 1 : 2;
     }
     mark(c, 3);
     *rel_acc = nd;

@@ -286,6 +286,7 @@ int ldlp_enqueue(Ctx& c, int n, const unsigned* tasks, int ntasks, unsigned long
 int ldlh_factor_traced(Ctx& c, int n, unsigned long long* out, long long cap, long long* count);
 
 // ---- launchers (invit.cu) ----
+bool invit_by_panels(Ctx& c);
 int invit_step(Ctx& c, int n, double tol);
 int invit_rayleigh(Ctx& c, int n, bool always, int specif_norm);
 int border_row(Ctx& c, int m0, int nexist);

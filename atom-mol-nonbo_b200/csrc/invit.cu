@@ -12,8 +12,9 @@
 // already solved part, and the last CTA to finish (atomic ticket, no waiting)
 // sums the partials in a fixed order and applies the panel's precomputed
 // inverse block.  Results are deterministic run to run.  The host enqueues
-// several steps and the Rayleigh quotient at a time (ghepiis_core); launches
-// after convergence return at once.
+// several steps (one where a step is a launch per panel) and the Rayleigh
+// quotient at a time (ghepiis_core); launches after convergence return at
+// once.
 #include <algorithm>
 #include <float.h>
 #include "ecg_internal.h"
@@ -91,8 +92,10 @@ __global__ void __launch_bounds__(256) k_hemv(const cd* __restrict__ B, int ld, 
 __global__ void __launch_bounds__(256) k_fwd(const cd* __restrict__ A, int ld, int j0, int j1, int chunk,
                                              const cd* __restrict__ w, cd* __restrict__ y, cd* __restrict__ z,
                                              const cd* __restrict__ invD, const cd* __restrict__ linv,
-                                             cd* __restrict__ part, int* __restrict__ counter)
+                                             cd* __restrict__ part, int* __restrict__ counter,
+                                             const double* __restrict__ red, const int* __restrict__ status)
 {
+    if (idle(red, status)) return;
     __shared__ cd t[LDL_NB];
     __shared__ int last;
     const int b = j1 - j0;
@@ -134,8 +137,10 @@ __global__ void __launch_bounds__(256) k_fwd(const cd* __restrict__ A, int ld, i
 __global__ void __launch_bounds__(256) k_bwd(const cd* __restrict__ A, int ld, int j0, int j1, int n, int chunk,
                                              const cd* __restrict__ z, cd* __restrict__ x,
                                              const cd* __restrict__ linv, cd* __restrict__ part,
-                                             int* __restrict__ counter)
+                                             int* __restrict__ counter, const double* __restrict__ red,
+                                             const int* __restrict__ status)
 {
+    if (idle(red, status)) return;
     __shared__ cd sred[4][LDL_NB];
     __shared__ cd t[LDL_NB];
     __shared__ int last;
@@ -635,7 +640,7 @@ static int solve_multi_launch(Ctx& c, int n)
         G = G < 1 ? 1 : (G > SOLVE_G_MAX ? SOLVE_G_MAX : G);
         const int chunk = (j0 + G - 1) / G;
         k_fwd<<<G, 256, 0, c.stream>>>(c.F, c.ld, j0, j1, chunk > 0 ? chunk : 1, c.w, c.yv, c.zv, c.invD, c.linv,
-                                      c.spart, c.counters);
+                                      c.spart, c.counters, c.red, c.status);
         c.launches++;
     }
     for (int i = nb - 1; i >= 0; i--) {
@@ -645,7 +650,7 @@ static int solve_multi_launch(Ctx& c, int n)
         G = G < 1 ? 1 : (G > SOLVE_G_MAX ? SOLVE_G_MAX : G);
         const int chunk = (rest + G - 1) / G;
         k_bwd<<<G, 256, 0, c.stream>>>(c.F, c.ld, j0, j1, n, chunk > 0 ? chunk : 1, c.zv, c.xw, c.linv, c.spart,
-                                      c.counters + 1);
+                                      c.counters + 1, c.red, c.status);
         c.launches++;
     }
     return 0;
@@ -775,6 +780,9 @@ int border_row(Ctx& c, int m0, int nexist)
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+// Whether a step is a launch per panel: more panels than co-resident CTAs.
+bool invit_by_panels(Ctx& c) { return (int)c.blk_start.size() > coop_capacity(c, false); }
+
 int invit_step(Ctx& c, int n, double tol)
 {
     k_hemv<<<(n * 32 + 255) / 256, 256, 0, c.stream>>>(c.S, c.ld, n, c.c, c.w, c.yv, c.xw, c.red, c.status);
@@ -785,7 +793,7 @@ int invit_step(Ctx& c, int n, double tol)
     int r;
     if (nb <= coop_capacity(c, true))
         r = solve_cooperative(c, true);
-    else if (nb <= coop_capacity(c, false))
+    else if (!invit_by_panels(c))
         r = solve_cooperative(c, false);
     else
         r = solve_multi_launch(c, n);
