@@ -186,6 +186,10 @@ struct Ctx {
     unsigned* lp_direct = nullptr;  // task list of the uncaptured fallback, for lp_direct_n rows
     int lp_direct_n = 0, lp_direct_count = 0;
 
+    // shared-memory limits of the kernels that need more than 48 KB, which
+    // belong to the device: set by each context
+    bool attr_ldl = false, attr_lp = false, attr_grad = false, attr_adj = false;
+
     // bookkeeping
     long long launches = 0;
     long long bytes_h2d = 0, bytes_d2h = 0;

@@ -574,8 +574,6 @@ __global__ void __launch_bounds__(256, TC == 64 ? 3 : 4) k_ldl_bulk(cd* __restri
             }
 }
 
-static bool g_ldl_attr = false;
-
 // Trailing update by panel [p0, p1) of rows [r0, rend), columns
 // [max(r, c0), n).
 // k rows [p0, p1) of U and of vb (vb(q, c) at vb[c * vld + q - p0]).
@@ -721,9 +719,9 @@ static int enqueue_persist(Ctx& c, int n, const unsigned* tasks, int ntasks, boo
     return 0;
 }
 
-static void ldl_attrs()
+static void ldl_attrs(Ctx& c)
 {
-    if (g_ldl_attr) return;
+    if (c.attr_ldl) return;
     const size_t sm1 = LDL_NB * DG_LD * sizeof(double2);
     cudaFuncSetAttribute(k_ldl_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1);
     cudaFuncSetAttribute(k_ldl_diag<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DG_SMEM);
@@ -732,7 +730,7 @@ static void ldl_attrs()
     cudaFuncSetAttribute(k_ldl_mn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MN_SMEM);
     cudaFuncSetAttribute(k_ldl_bulk<32, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)blk_smem<32>());
     cudaFuncSetAttribute(k_ldl_bulk<16, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)blk_smem<16>());
-    g_ldl_attr = true;
+    c.attr_ldl = true;
 }
 
 // Factorise rows m0..n-1 of M = H - lambda~ S given the factor of rows
@@ -747,7 +745,7 @@ int ldlh_factor(Ctx& c, int m0, int n, bool solves)
 {
     if (m0 < 0 || m0 > n || n > c.ld) return -1;
     if (m0 > c.fact_n) return -1;
-    ldl_attrs();
+    ldl_attrs(c);
     // block list: existing blocks truncated at m0, then new 64-row blocks
     std::vector<int> starts;
     for (int s : c.blk_start)
@@ -852,7 +850,7 @@ int ldlh_factor_traced(Ctx& c, int n, unsigned long long* out, long long cap, lo
     if (n < 1 || n > c.ld) return -1;
     if (ldlp_grid(c) <= 0) return -1;
     const int nb = (n + LDL_NB - 1) / LDL_NB;
-    ldl_attrs();
+    ldl_attrs(c);
     std::vector<int> starts;
     for (int s = 0; s < n; s += LDL_NB) starts.push_back(s);
     for (int i = 0; i < nb; i++) c.bounds_h[i] = starts[i];

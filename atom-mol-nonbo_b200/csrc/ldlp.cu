@@ -1145,12 +1145,10 @@ __global__ void __launch_bounds__(256, 2) k_ldl_persist(const __grid_constant__ 
     }
 }
 
-static bool g_lp_attr = false;
-
 // Grid of the persistent kernel (co-resident CTAs), 0 if unavailable.
 int ldlp_grid(Ctx& c)
 {
-    if (!g_lp_attr) {
+    if (!c.attr_lp) {
         if (cudaFuncSetAttribute(k_ldl_persist<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LP_SMEM) !=
                 cudaSuccess ||
             cudaFuncSetAttribute(k_ldl_persist<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LP_SMEM) !=
@@ -1158,7 +1156,7 @@ int ldlp_grid(Ctx& c)
             cudaGetLastError();
             return 0;
         }
-        g_lp_attr = true;
+        c.attr_lp = true;
     }
     if (c.lp_grid > 0) return c.lp_grid;
     int per_sm = 0, sms = 0;

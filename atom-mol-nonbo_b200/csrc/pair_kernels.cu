@@ -1466,10 +1466,9 @@ static int grad_n(Ctx& c, int r0, int r1, int nfru, double approx_e)
     constexpr int NT = (N <= 4) ? 128 : 64;
     constexpr int NP = Sym<N>::NP;
     const size_t smem = sizeof(double2) * ((size_t)4 * NP * NT + BraShared<N>::ENTRIES * TILE);
-    static bool attr = false;
-    if (!attr) {
+    if (!c.attr_grad) {
         cudaFuncSetAttribute(k_pair_grad<N, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
+        c.attr_grad = true;
     }
     const int Rlo = r0 / TILE, Rhi = (r1 + TILE - 1) / TILE;
     const long long nt = tile_count(Rlo, Rhi);
@@ -1500,11 +1499,10 @@ static int adjoint_n(Ctx& c, int nfru, int nfa, double E)
         c.part_bytes = need;
     }
     constexpr size_t smem = adjoint_smem<N>();
-    static bool attr = false;
-    if (!attr) {
+    if (!c.attr_adj) {
         cudaFuncSetAttribute(k_adjoint<N, 8, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(k_adjoint<N, 4, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
+        c.attr_adj = true;
     }
     auto run = [&](int v) {
         if (v == 0)
