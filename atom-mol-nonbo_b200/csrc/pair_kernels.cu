@@ -763,9 +763,11 @@ __global__ void __launch_bounds__(TILE) k_adjoint_row(SysParams sp, const double
     v[NV - 1] = ra;
     const double sum = warp_transpose_sum<M>(v);
     const int x = lane / (32 / M);
-    if (lane % (32 / M) == 0 && x < NV) {
-        part[((tile * 2 + 0) * TILE + k % TILE) * NV + x] = sum;
-        part[((tile * 2 + 1) * TILE + k % TILE) * NV + x] = 0.0;
+    if (lane % (32 / M) == 0 && x < NV) part[((tile * 2 + 0) * TILE + k % TILE) * NV + x] = sum;
+    // the tile's other rows, and its columns from k on, have no share
+    for (int y = 0; y < NV; y++) {
+        if (lane != k % TILE) part[((tile * 2 + 0) * TILE + lane) * NV + y] = 0.0;
+        if (l >= k) part[((tile * 2 + 1) * TILE + lane) * NV + y] = 0.0;
     }
 }
 
