@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from ecg_b200 import Context, EcgError
+from gpu_util import problem
 from test_gpu_candidates import base_problem
 
 pytestmark = pytest.mark.gpu
@@ -35,3 +36,26 @@ def test_candidates_gemm_copies(K0):
         ctx.set_wait_limit(-1)
         E1, err1, it1, _ = batch(ctx)
     assert np.array_equal(E0, E1, equal_nan=True) and np.array_equal(err0, err1) and np.array_equal(it0, it1)
+
+
+@pytest.mark.parametrize("K", [130, 400])
+def test_iteration_solves(K):
+    """A factorisation by one launch per panel step has no waits, so those of
+    GHEPIIS's triangular solves run out first."""
+    sysm, params, lam, _ = problem(1, K)
+
+    def solve(ctx):
+        ctx.set_vectors(K, last_eigvec=np.ones(K, dtype=np.complex128))
+        return ctx.energy_ia(1, K, lam, 1e-10) + (ctx.vectors(K)[1],)
+
+    with Context(sysm, K) as ctx:
+        ctx.set_factor_mode(1)
+        ctx.set_params(params)
+        before = solve(ctx)
+        ctx.set_wait_limit(0)
+        with pytest.raises(EcgError) as ei:
+            solve(ctx)
+        assert ei.value.status == ECG_ECUDA
+        ctx.set_wait_limit(-1)
+        after = solve(ctx)
+    assert after[:3] == before[:3] and np.array_equal(after[3], before[3])
