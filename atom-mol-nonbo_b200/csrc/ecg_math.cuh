@@ -79,9 +79,10 @@ __host__ __device__ constexpr int vech_index(int N, int i, int j)
 }
 
 // 1/sqrt(x) for positive normal x without a branch: the hardware's seed y
-// (rsqrt.approx.ftz.f64, about 20 bits), then one step of Householder's
-// method of third order, the Taylor series of (1 - e)^(-1/2) to e^2 with
-// e = 1 - x y^2, whose remainder (5/16) e^3 is below 2^-60.  Zero,
+// (rsqrt.approx.ftz.f64), then one step of Householder's method of third
+// order, the Taylor series of (1 - e)^(-1/2) to e^2 with e = 1 - x y^2.
+// |e| is at most 2^-19.0 over all upper words of the mantissa (measured), so
+// the remainder (5/16) e^3 is below 2^-58.  Zero,
 // subnormal, infinite or NaN x gives NaN.  rsqrt() and the divide are
 // accurate for every x and so end in a branch; the pair term takes up to
 // sixteen of them (n = 3), and without the branches their chains overlap.

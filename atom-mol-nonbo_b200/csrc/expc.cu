@@ -30,7 +30,7 @@
 // TrCJCJ(i,j,p,q) of src/matelem.f90:1270-1300 is never assigned for
 // i = j < p < q (n >= 3) but is read by the 1/(r_ij r_pq) loop; the
 // reference's ifort build keeps local arrays in zero-initialised static
-// storage, so those entries are zero there.  pair_pair() reproduces that.
+// storage, so those entries are zero there.  k_expc takes zero for them too.
 #include <float.h>
 #include <algorithm>
 #include "ecg_internal.h"

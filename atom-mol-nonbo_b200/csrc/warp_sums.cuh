@@ -5,8 +5,8 @@
 namespace ecg {
 
 // Sum v[0..M) (M a power of two, at most 32) over the warp's lanes: every
-// step exchanges half of the values a lane still holds, so 2 M - 1 values
-// travel instead of the 5 M of a butterfly per value.  Lane i returns the
+// step exchanges half of the values a lane still holds, so M - 1 +
+// log2(32 / M) values travel instead of the 5 M of a butterfly per value.  Lane i returns the
 // sum of value i / (32 / M).
 template <int M>
 __device__ __forceinline__ double warp_transpose_sum(double (&v)[M])

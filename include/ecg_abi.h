@@ -300,9 +300,10 @@ int ecg_adjoint_finish(ecg_ctx* ctx, int nfru, int nfa, const void* part_dev, do
 /* Shapes the context's autotuner chose (-1: not tuned yet).  The pair
  * kernels' shape is chosen once per context by timing every candidate
  * shape on the first large launch (the outputs do not depend on it):
- *   pair_shape     k_pair_energy, 0..3: warps per 32 x 32 pair tile (8, 8,
+ *   pair_shape     k_pair_energy, 0..3: warps per 32 x 32 pair tile (8, 4,
  *                  4, 4) x register budget (2, 3, 2, 4 CTAs per SM);
- *   adjoint_shape  k_adjoint, 0..1: 1 or 2 CTAs per SM;
+ *   adjoint_shape  k_adjoint, 0..1: 8 warps per tile at 1 CTA per SM, or 4
+ *                  at 3;
  *   cand_row_shape k_cand_row, 0..4: warps x candidates per warp.
  * times_ms (may be NULL) receives the 4 + 2 timings of the first two.  No
  * counterpart in the reference, whose linalg_setparam table
