@@ -290,12 +290,19 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
     int nu = 0, zero = 0;
     double lo = center - delta, hi = center + delta;
     int nlo, nhi;
+    // the widest bracket the counts know to hold the eigenvalue alone: the
+    // lowest point with which - 1 below it, the highest with which
+    double alone_lo = which == 1 ? -DBL_MAX : DBL_MAX, alone_hi = which == n ? DBL_MAX : -DBL_MAX;
     auto count = [&](double& s, int* v) -> int {
         // an exactly zero pivot leaves the count undefined: move sigma by a few ulps
         for (int tries = 0; tries < 8; tries++) {
             const int r = g_count(c, n, s, v, &zero);
             if (r) return r;
-            if (!zero) return 0;
+            if (!zero) {
+                if (*v == which - 1) alone_lo = std::min(alone_lo, s);
+                if (*v == which) alone_hi = std::max(alone_hi, s);
+                return 0;
+            }
             s = s + (fabs(s) + 1e-300) * 1e-14 * (tries + 1);
         }
         return ECG_ENOCONV;
@@ -324,20 +331,12 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
         CK(cudaStreamSynchronize(c.stream));
     }
     int extra = 0, it = 0;
-    // the first bracket that held the eigenvalue alone: no other is inside it
-    bool alone = false;
-    double alone_lo = 0.0, alone_hi = 0.0;
     for (bool again = false;; again = true) {
         // bisect until the bracket holds the which-th eigenvalue alone, then a
         // few halvings more
         for (;;) {
             const double size = std::max(fabs(lo), fabs(hi));
             const bool isolated = (nlo == which - 1) && (nhi == which);
-            if (isolated && !alone) {
-                alone = true;
-                alone_lo = lo;
-                alone_hi = hi;
-            }
             if (isolated && extra >= (again ? G_EXTRA_MOST : G_EXTRA_BISECT)) break;
             if (isolated && !again && hi - lo <= G_NARROW * std::max(1.0, size)) break;
             if (hi - lo <= 4.0 * DBL_EPSILON * size) break;
@@ -371,7 +370,7 @@ int energy_ga(Ctx& c, int nmin, int nmax, int needed, int which, int want_vector
         // Only where it is well below one does a residual that stands still
         // mean that the iteration is on its floor, which no shift lowers, and
         // a small one that the vector is as close.
-        const double rate = alone ? fabs(lam - sigma) / std::min(sigma - alone_lo, alone_hi - sigma) : 0.0;
+        const double rate = alone_lo < alone_hi ? fabs(lam - sigma) / std::min(sigma - alone_lo, alone_hi - sigma) : 0.0;
         const bool found = e == ECG_OK ? rate <= 0.9 : (ra <= 1e-6 && c.last_gain >= 0.9 && rate <= 0.5);
         // otherwise once more in a narrower bracket, as also where the shift
         // met the eigenvalue or the iteration found another one, whose vector
