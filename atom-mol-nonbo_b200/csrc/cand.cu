@@ -92,7 +92,7 @@ struct CgArgs {
     const cd *E1, *e2;
     cd* P;             // two partial tiles a CTA
     int* status;
-    const int* limitp;  // poll limit of the call's waits: at 0 the first one here runs out too
+    int give_up;       // the call's poll limit is 0: the first wait here runs out too
 };
 
 // first chunk of tile row it, and the chunks before tile t (column by column)
@@ -165,9 +165,12 @@ __global__ void __launch_bounds__(256, 2) k_cgemm(const __grid_constant__ CgArgs
     // a wait ran out at the piece's chunk ch
     auto give_up = [&](int ch) {
         if (lane == 0) atomicExch(a.status + ST_SOLVE_TIMEOUT, 1);
-        if (tid == 0) ring.drain(rst, rph, (int)(u1 - u0) - ring_refilled(ch, (int)(u1 - u0)));
+        if (tid == 0) {
+            const int n = (int)(u1 - u0), r = ring_refilled(ch, n);
+            ring_drain(ring.full, r % TMA_ST, (unsigned)(r / TMA_ST) & 1u, n - r);
+        }
     };
-    if (__ldg(a.limitp) == 0) {
+    if (a.give_up) {
         give_up(0);
         return;
     }
@@ -185,12 +188,10 @@ __global__ void __launch_bounds__(256, 2) k_cgemm(const __grid_constant__ CgArgs
     int k0 = k;  // where the tile's segment begins
     bool first = true;
     const int f0 = pg * TMA_KC + (t4 ^ pg);  // fragment slots of k = t4 and, with ^ 4, of k = 4 + t4
-    for (long long u = u0; u < u1; u++) {
+    long long u = u0;
+    for (; u < u1; u++) {
         const bool ok = bar_wait(ring.full + 8u * ring.st, ring.ph);
-        if (!__all_sync(0xffffffffu, ok)) {
-            give_up((int)(u - u0));
-            return;
-        }
+        if (!__all_sync(0xffffffffu, ok)) break;
         const int it = t % a.mt;
         const double2* Us = stages + ring.st * 2 * CG_OP + (wr * MT) * 64;
         const double2* Vs = stages + ring.st * 2 * CG_OP + CG_OP + (wc * NT) * 64;
@@ -258,6 +259,7 @@ __global__ void __launch_bounds__(256, 2) k_cgemm(const __grid_constant__ CgArgs
             first = false;
         }
     }
+    if (u < u1) give_up((int)(u - u0));
 }
 
 // Tiles that fell into several pieces: their partial sums, in order.  One
@@ -1003,7 +1005,7 @@ int launch_gemm(Ctx& c, cd* A, int nbase, int ncols, cd* B, cd* C, const cd* E1,
     a.e2 = e2;
     a.P = cw.Pk;
     a.status = c.status;
-    a.limitp = cw.abort_word + 1;
+    a.give_up = c.wait_limit == 0;
     const int pieces = (int)std::min<long long>(cw.gemm_grid, a.total);
     k_cgemm<TRI><<<pieces, 256, CG_SMEM, c.stream>>>(a);
     k_cgemm_sum<TRI><<<dim3(a.ntile, CG_TILE / 256), 256, 0, c.stream>>>(a, pieces);
@@ -1038,7 +1040,7 @@ int run_iteration(Ctx& c, int nbase, int count, int ncols, int nb, double tol)
     CandWork& cw = c.cand;
     long long tl;
     memcpy(&tl, &tol, sizeof(tl));
-    std::vector<int> key = {nbase, count, ncols, nb, (int)(tl & 0xffffffff), (int)(tl >> 32)};
+    std::vector<int> key = {nbase, count, ncols, nb, (int)(tl & 0xffffffff), (int)(tl >> 32), c.wait_limit == 0};
     CandWork::IterGraph* g = nullptr;
     for (auto& e : cw.graphs)
         if (e.key == key) g = &e;

@@ -513,7 +513,7 @@ __device__ bool lp_update(const LpArgs& a, int s, int m, int R, int C, int half,
         }
     }
     if (__syncthreads_or(ok ? 0 : 1)) {
-        if (tid == 0) ring.drain(rst, rph, nch - ring_refilled(ch, nch));
+        if (tid == 0) ring_drain(ring.full, rst, rph, nch - ring_refilled(ch, nch));
         return false;
     }
 #pragma unroll

@@ -86,21 +86,25 @@ struct TmaRing {
             p ^= 1u;
         }
     }
-    // Thread 0, after a wait that ran out: a CTA does not leave while a copy
-    // may still write its shared memory.  `uses` are to come from the one of
-    // stage i and parity p on, the oldest not known to have arrived; of them
-    // those of the next TMA_ST stages, on either side of the ring's end, may
-    // be in flight (one that was not asked for runs into the limit).
-    __device__ __forceinline__ void drain(int i, unsigned p, int uses) const
-    {
-        for (int u = 0; u < min(uses, TMA_ST); u++) {
-            bar_wait(full + 8u * i, p);
-            step(i, p);
-        }
-    }
 };
 // Stages refilled before chunk ch of n, one a chunk from the third on.
 __device__ __forceinline__ int ring_refilled(int ch, int n) { return max(0, min(ch, n - TMA_ST + 2) - 2); }
+// Thread 0, after a wait that ran out: a CTA does not leave while a copy may
+// still write its shared memory.  `uses` are to come from the one of stage i
+// and parity p on, the oldest not known to have arrived; of them those of the
+// next TMA_ST stages, on either side of the ring's end, may be in flight (one
+// that was not asked for runs into the limit).  A call, because its code
+// inside the candidates' GEMM costs that 1 %.
+static __device__ __noinline__ void ring_drain(unsigned full, int i, unsigned p, int uses)
+{
+    for (int u = 0; u < min(uses, TMA_ST); u++) {
+        bar_wait(full + 8u * i, p);
+        if (++i == TMA_ST) {
+            i = 0;
+            p ^= 1u;
+        }
+    }
+}
 
 // Tensor map of the rows x cols matrix at A (column-major complex) as doubles
 // by columns, boxes of TMA_KC complex rows x `box_cols` columns, 128-byte
